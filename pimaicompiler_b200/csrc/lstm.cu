@@ -38,7 +38,7 @@ int launch_gemm_wx_simt(const __half* W, const __half* X, const __half* bias, vo
 int launch_gemm_wx(const __half* W, const __half* X, const __half* bias, void* Y, int N, int K, int J, int ldx,
                    int ldy, int act, int y_is_f32, cudaStream_t st);
 int launch_gemm_wx_time_major(const __half* W, const __half* X, void* Y, int N, int K, int J, int ldx, int ldy, int batch,
-                              cudaStream_t st);
+                              long seq_rows, cudaStream_t st);
 }  // namespace pimb200
 
 using namespace pimb200;
@@ -2293,6 +2293,7 @@ struct SeqLayout {
     int T, B;                       // B = batch_sizes[0] for packed input
     const int64_t* batch_sizes;     // NULL for padded input
     std::vector<long> row0;         // packed: first row of timestep t
+    long x_seq_rows = 0;            // batch-first input: rows from one sequence to the next (0 = T)
 };
 
 static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool reverse, const float* G, long g_tstride,
@@ -2694,6 +2695,8 @@ static int lstm_forward_impl(pimb200_lstm* h, const __half* x, const SeqLayout& 
     long rows = 0;  // rows of the flattened [rows, features] activations
     if (packed) rows = sq.row0[T - 1] + (long)sq.batch_sizes[T - 1];
     else rows = (long)T * B;
+    const long x_seq = sq.x_seq_rows > 0 ? sq.x_seq_rows : T;
+    const long in_rows = batch_first ? (B - 1) * x_seq + T : rows;   // rows of x up to the last used one
     int rc;
     // packed input of several steps: as a padded lock-step batch on the persistent recurrences (needs the 128-bit GEMM
     // path for the padded rows; the streamed kernels below take every other case)
@@ -2701,10 +2704,10 @@ static int lstm_forward_impl(pimb200_lstm* h, const __half* x, const SeqLayout& 
         return lstm_forward_packed_lockstep(h, x, sq, h0, c0, y, hn, cn, st);
     // decode form: seq_len 1, every extent a multiple of 8 and 16-byte aligned -> one fused cell launch per layer
     bool cell = !packed && T == 1 && h->variant != PIMB200_LSTM_PERSISTENT && h->variant != PIMB200_LSTM_PERSISTENT_TAGGED &&
-                H % 8 == 0 && h->I % 8 == 0 && aligned16(x) && aligned16(y) && (!h0 || aligned16(h0));
+                H % 8 == 0 && h->I % 8 == 0 && aligned16(x) && aligned16(y) && (!h0 || aligned16(h0)) && (!batch_first || x_seq == T);
     const bool cell_gemm = cell && B >= kCellGemmMinB;   // lock-step decode of many sequences: products as GEMMs
     if (cell_gemm && (rc = grow(&h->G, &h->G_cap, (size_t)2 * B * 4 * H)) != PIMB200_OK) return rc;
-    if (!cell && (rc = grow(&h->G, &h->G_cap, (size_t)rows * 4 * H)) != PIMB200_OK) return rc;
+    if (!cell && (rc = grow(&h->G, &h->G_cap, (size_t)in_rows * 4 * H)) != PIMB200_OK) return rc;
     if (L > 1 && (rc = grow(&h->ybuf[0], &h->y_cap[0], (size_t)rows * D * H)) != PIMB200_OK) return rc;
     if (L > 2 && (rc = grow(&h->ybuf[1], &h->y_cap[1], (size_t)rows * D * H)) != PIMB200_OK) return rc;
     if (cell) {
@@ -2753,7 +2756,7 @@ static int lstm_forward_impl(pimb200_lstm* h, const __half* x, const SeqLayout& 
         long in_t, in_b, out_t, out_b;
         if (packed) { in_t = 1; in_b = 1; out_t = 1; out_b = 1; }  // row = row0[t] + b
         else {
-            in_t = (first && batch_first) ? 1 : B;  in_b = (first && batch_first) ? T : 1;
+            in_t = (first && batch_first) ? 1 : B;  in_b = (first && batch_first) ? x_seq : 1;
             out_t = (last && batch_first) ? 1 : B;  out_b = (last && batch_first) ? T : 1;
         }
         for (int d = 0; d < D; ++d) {
@@ -2764,12 +2767,12 @@ static int lstm_forward_impl(pimb200_lstm* h, const __half* x, const SeqLayout& 
             long g_t = in_t, g_b = in_b;
             rc = PIMB200_ERR_UNSUPPORTED;
             if (first && batch_first && !packed && B > 1 && T > 1) {
-                rc = launch_gemm_wx_time_major(h->w_ih[ld], X, h->G, 4 * H, Il, (int)rows, Il, 4 * H, B, st);
+                rc = launch_gemm_wx_time_major(h->w_ih[ld], X, h->G, 4 * H, Il, (int)rows, Il, 4 * H, B, x_seq, st);
                 if (rc == PIMB200_OK) { g_t = B; g_b = 1; }
             }
             if (rc == PIMB200_ERR_UNSUPPORTED)
-                rc = launch_gemm_wx(h->w_ih[ld], X, nullptr, h->G, 4 * H, Il, (int)rows, Il, 4 * H, PIMB200_ACT_NONE, 1,
-                                    st);
+                rc = launch_gemm_wx(h->w_ih[ld], X, nullptr, h->G, 4 * H, Il, (int)(first ? in_rows : rows), Il, 4 * H,
+                                    PIMB200_ACT_NONE, 1, st);
             if (rc != PIMB200_OK) return rc;
             if (wave_fits(h, l, T, B, packed)) {
                 // layers l and l + 1 in one launch, one step apart; the pair's output is layer l + 1's
@@ -2801,6 +2804,13 @@ extern "C" int pimb200_lstm_forward(pimb200_lstm* h, const void* x, int T, int B
     return lstm_forward_impl(h, static_cast<const __half*>(x), sq, static_cast<const __half*>(h0),
                              static_cast<const __half*>(c0), static_cast<__half*>(y), static_cast<__half*>(hn),
                              static_cast<__half*>(cn), batch_first ? 1 : 0, static_cast<cudaStream_t>(stream));
+}
+
+// Batch-first forward whose input sequences lie x_seq_rows >= T rows apart (only the first T of each are read).
+int lstm_forward_batch_first(pimb200_lstm* h, const __half* x, long x_seq_rows, int T, int B, __half* y, cudaStream_t st) {
+    SeqLayout sq;
+    sq.T = T; sq.B = B; sq.batch_sizes = nullptr; sq.x_seq_rows = x_seq_rows;
+    return lstm_forward_impl(h, x, sq, nullptr, nullptr, y, nullptr, nullptr, 1, st);
 }
 
 // Decode step of a one-layer, one-direction handle for B >= 8 sequences with strided rows: x rows x_ld halves apart, the

@@ -118,6 +118,18 @@ def test_rnnt_batch_of_utterances_matches_single():
     assert toks3 == toks and torch.equal(logits3, logits)
 
 
+@pytest.mark.parametrize("n_utts,T", [(3, 41), (37, 27), (65, 9), (129, 7)])
+def test_rnnt_odd_length_batches(n_utts, T):
+    # a frame behind the last whole stack, batch sizes that do not divide the projection GEMM's 128-row tile
+    cfg = to.RnntConfig(feat_dim=24, enc_hidden=64, pred_hidden=32, joint_hidden=48, vocab=11, blank=10)
+    w = to.make_rnnt_weights(cfg, seed=9, gain=2.0, logit_gain=6.0)
+    dec = _decoder(cfg, w)
+    feats = [to.make_features(T, cfg, 500 + i) for i in range(n_utts)]
+    toks, logits = dec.decode(torch.stack(feats).to(torch.float16).cuda(), want_logits=True)
+    for i in sorted({0, 1, n_utts // 2, n_utts - 1}):
+        _check_utterance(cfg, w, feats[i], toks[i], logits[i].cpu().numpy(), co.rnnt_greedy)
+
+
 @pytest.mark.parametrize("n_utts", [12, 19])
 def test_rnnt_tensor_core_greedy_small_model(n_utts):
     # a model whose shapes the tensor-core greedy kernel accepts (PH, JH multiples of 64, 16 CTAs per cluster); more
