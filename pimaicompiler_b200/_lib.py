@@ -139,6 +139,26 @@ def lib() -> C.CDLL:
     return _lib
 
 
+_native = None
+
+
+def native():
+    """The native call path of the short ops (`_pimb200_ops`), loaded once.  Raises if it is not built."""
+    global _native
+    if _native is None:
+        import importlib.util
+        lib()
+        path = os.path.join(PKG_DIR, "_pimb200_ops.so")
+        if not os.path.exists(path):
+            raise RuntimeError(f"{path} is missing: build it with `python -m pimaicompiler_b200.host.build`")
+        spec = importlib.util.spec_from_file_location("_pimb200_ops", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.set_check(check)
+        _native = module
+    return _native
+
+
 class Pimb200Error(RuntimeError):
     def __init__(self, status: int, where: str):
         self.status = status

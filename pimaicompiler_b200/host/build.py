@@ -1,5 +1,5 @@
-"""In-tree build of the C++ host-side mirror (`_pimb200_host`), against this interpreter's libtorch and
-libpimb200.so.  Usage: ``python -m pimaicompiler_b200.host.build``."""
+"""In-tree build of the C++ host-side mirror (`_pimb200_host`) and of the native call path of `ops.py`
+(`_pimb200_ops`), against this interpreter's libtorch and libpimb200.so.  Usage: ``python -m pimaicompiler_b200.host.build``."""
 from __future__ import annotations
 
 import os
@@ -13,12 +13,14 @@ PKG = os.path.dirname(HERE)
 ROOT = os.path.dirname(PKG)
 OUT = os.path.join(PKG, "_pimb200_host.so")
 SOURCES = ["tensor_ops.cpp", "stream_executor.cpp", "op_executors.cpp", "bindings.cpp"]
+OPS_OUT = os.path.join(PKG, "_pimb200_ops.so")
+OPS_SOURCE = "fast_ops.cpp"
 
 
 def needs_build() -> bool:
-    if not os.path.exists(OUT):
+    if not os.path.exists(OUT) or not os.path.exists(OPS_OUT):
         return True
-    t = os.path.getmtime(OUT)
+    t = min(os.path.getmtime(OUT), os.path.getmtime(OPS_OUT))
     deps = [os.path.join(HERE, f) for f in os.listdir(HERE) if f.endswith((".cpp", ".h"))]
     deps.append(os.path.join(ROOT, "include", "pimb200.h"))
     return any(os.path.getmtime(d) > t for d in deps)
@@ -48,12 +50,13 @@ def build(force: bool = False) -> str:
         return obj
 
     with ThreadPoolExecutor(max_workers=4) as ex:
-        objs = list(ex.map(cc, SOURCES))
-    link = ["g++", "-shared", "-o", OUT, *objs, f"-L{tlib}", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
-            "-ltorch_python", f"-L{PKG}", "-lpimb200", f"-Wl,-rpath,{tlib}", "-Wl,-rpath,$ORIGIN"]
-    res = subprocess.run(link, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError("link failed:\n" + res.stdout + res.stderr)
+        *objs, ops_obj = list(ex.map(cc, [*SOURCES, OPS_SOURCE]))
+    for out, parts in ((OUT, objs), (OPS_OUT, [ops_obj])):
+        link = ["g++", "-shared", "-o", out, *parts, f"-L{tlib}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10",
+                "-lc10_cuda", "-ltorch_python", f"-L{PKG}", "-lpimb200", f"-Wl,-rpath,{tlib}", "-Wl,-rpath,$ORIGIN"]
+        res = subprocess.run(link, capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError("link failed:\n" + res.stdout + res.stderr)
     return OUT
 
 

@@ -66,24 +66,15 @@ def shutdown(device: Optional[int] = None) -> None:
 def gemv_mv(W: torch.Tensor, x: torch.Tensor, bias: Optional[torch.Tensor] = None, act: int = ACT_NONE,
             out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """y[N] = act(W[N,K] @ x[K] + bias)."""
-    _req_half_cuda(W, x, bias)
-    N, K = W.shape
-    assert x.numel() == K
-    y = out if out is not None else torch.empty(N, dtype=torch.float16, device=W.device)
-    check(_lib.lib().pimb200_gemv_mv(_ptr(W), _ptr(x), _ptr(bias), _ptr(y), N, K, act, _stream()), "gemv_mv")
-    return y
+    return (_lib._native or _lib.native()).gemv_mv(W, x, bias, act, out)
 
 
 def gemv_vm(x: torch.Tensor, A: torch.Tensor, bias: Optional[torch.Tensor] = None, act: int = ACT_NONE,
             out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """y[N] = act(x[K] @ A[K,N] + bias)."""
-    _req_half_cuda(A, x, bias)
-    init(A.device.index)
-    K, N = A.shape
-    assert x.numel() == K
-    y = out if out is not None else torch.empty(N, dtype=torch.float16, device=A.device)
-    check(_lib.lib().pimb200_gemv_vm(_ptr(x), _ptr(A), _ptr(bias), _ptr(y), K, N, act, _stream()), "gemv_vm")
-    return y
+    if A.is_cuda:
+        init(A.device.index)
+    return (_lib._native or _lib.native()).gemv_vm(x, A, bias, act, out)
 
 
 def dot_vv(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
@@ -107,16 +98,7 @@ def bmm_row(x: torch.Tensor, A: torch.Tensor, out: Optional[torch.Tensor] = None
 def gemm_wx(W: torch.Tensor, X: torch.Tensor, bias: Optional[torch.Tensor] = None, act: int = ACT_NONE,
             out_f32: bool = False, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Y[J,N] = act(X[J,K] @ W[N,K]^T + bias).  Rows of X and of `out` may be strided (column slices of wider buffers)."""
-    _req_half_cuda(W, bias)
-    _req_half_cuda_rows(X)
-    N, K = W.shape
-    J = X.shape[0]
-    assert X.shape[1] == K and X.stride(1) == 1
-    if out is None:
-        out = torch.empty(J, N, dtype=torch.float32 if out_f32 else torch.float16, device=W.device)
-    check(_lib.lib().pimb200_gemm_wx(_ptr(W), _ptr(X), _ptr(bias), _ptr(out), N, K, J, X.stride(0), out.stride(0), act,
-                                     1 if out.dtype == torch.float32 else 0, _stream()), "gemm_wx")
-    return out
+    return (_lib._native or _lib.native()).gemm_wx(W, X, bias, act, out_f32, out)
 
 
 def gemm_wx_grouped(problems: Sequence[tuple], act: int = ACT_NONE) -> list:
@@ -378,11 +360,13 @@ class Lstm:
         check(_lib.lib().pimb200_lstm_create(arr, len(params), num_layers, 1 if bidirectional else 0, input_size,
                                              hidden_size, 1 if has_biases else 0, C.byref(handle)), "lstm_create")
         self._h = handle
+        self._handle = handle.value   # the same address as a plain number, for the native call path
 
     def close(self) -> None:
         if getattr(self, "_h", None):
             _lib.lib().pimb200_lstm_destroy(self._h)
             self._h = None
+            self._handle = 0
 
     def __del__(self):
         try:
@@ -404,21 +388,8 @@ class Lstm:
 
     def forward(self, x: torch.Tensor, h0: Optional[torch.Tensor] = None, c0: Optional[torch.Tensor] = None,
                 batch_first: bool = False, out=None):
-        _req_half_cuda(x, h0, c0)
-        if batch_first:
-            B, T, _ = x.shape
-        else:
-            T, B, _ = x.shape
-        DH = self.D * self.H
-        if out is None:
-            y = torch.empty((B, T, DH) if batch_first else (T, B, DH), dtype=torch.float16, device=x.device)
-            hn = torch.empty(self.L * self.D, B, self.H, dtype=torch.float16, device=x.device)
-            cn = torch.empty_like(hn)
-        else:
-            y, hn, cn = out
-        check(_lib.lib().pimb200_lstm_forward(self._h, _ptr(x), T, B, _ptr(h0), _ptr(c0), _ptr(y), _ptr(hn),
-                                              _ptr(cn), 1 if batch_first else 0, _stream()), "lstm_forward")
-        return y, hn, cn
+        return (_lib._native or _lib.native()).lstm_forward(self._handle, self.L * self.D, self.D, self.H, x, h0, c0,
+                                                            batch_first, out)
 
     def forward_step(self, x: torch.Tensor, h0: Optional[torch.Tensor], c0: Optional[torch.Tensor], y: torch.Tensor,
                      hn: torch.Tensor, cn: torch.Tensor, residual: Optional[torch.Tensor] = None) -> bool:
@@ -437,14 +408,5 @@ class Lstm:
 
     def forward_packed(self, data: torch.Tensor, batch_sizes: torch.Tensor, h0: Optional[torch.Tensor] = None,
                        c0: Optional[torch.Tensor] = None):
-        _req_half_cuda(data, h0, c0)
-        bs = [int(v) for v in batch_sizes.tolist()]
-        T = len(bs)
-        B = bs[0]
-        arr = (C.c_int64 * T)(*bs)
-        y = torch.empty(data.shape[0], self.D * self.H, dtype=torch.float16, device=data.device)
-        hn = torch.empty(self.L * self.D, B, self.H, dtype=torch.float16, device=data.device)
-        cn = torch.empty_like(hn)
-        check(_lib.lib().pimb200_lstm_forward_packed(self._h, _ptr(data), arr, T, _ptr(h0), _ptr(c0), _ptr(y),
-                                                     _ptr(hn), _ptr(cn), _stream()), "lstm_forward_packed")
-        return y, hn, cn
+        return (_lib._native or _lib.native()).lstm_forward_packed(self._handle, self.L * self.D, self.D, self.H, data,
+                                                                   batch_sizes, h0, c0)
