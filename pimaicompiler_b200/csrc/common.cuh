@@ -49,7 +49,32 @@ constexpr size_t kSplitKMaxFloats = size_t(1) << 22;  // 16 MiB of fp32 partial 
 constexpr int kSplitKMaxTiles = 4096;
 DeviceCtx* current_ctx();  // nullptr when pimb200_init was not called for the current device
 
+// A launch that may start while the kernel before it on the stream is still running (programmatic dependent launch): its
+// CTAs are scheduled and set up as soon as that kernel's CTAs have all called pdl_launch_dependents(), and block in
+// pdl_wait() until it has completed and its writes are visible.  Every kernel launched this way calls pdl_wait() before
+// it touches global memory.  It saves the gap between two short kernels, about a microsecond.
+// CLUSTER: CTAs per thread-block cluster.
+template <int CLUSTER = 1, typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = grid;
+    lc.blockDim = block;
+    lc.dynamicSmemBytes = smem;
+    lc.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = CLUSTER; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    lc.attrs = at;
+    lc.numAttrs = CLUSTER > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&lc, kernel, P(args)...);
+}
+
 // ---- device side -----------------------------------------------------------
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ uint4 ldg_stream_v4(const void* p) {
     // weights are read once per launch: keep them out of L1
     uint4 r;

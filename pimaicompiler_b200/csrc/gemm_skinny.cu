@@ -23,8 +23,10 @@ constexpr int kSkinnyThreads = kSkinnyWarps * 32;
 constexpr int kSkinnyRows = 16;
 constexpr int kSkinnyMaxJ = 32;
 constexpr int kSkinnyMaxBlockedJ = 256;                     // column-blocked form: at most 8 blocks of 32 rows ...
-constexpr int kSkinnyMaxBlockedN = 2048;                    // ... of a matrix of at most 16 tcgen05 row tiles ...
+constexpr int kSkinnyMaxBlockedN = 2048;                    // ... of a matrix of at most 2048 rows ...
 constexpr size_t kSkinnyMaxBlockedNK = (size_t)8 << 20;     // ... and 16 MB
+constexpr int kSkinnyMaxBlockedCtas = kNumSmB200;           // ... in one wave of CTAs: 3.5 us at 512 x 512, 128 rows (tcgen05
+                                                            // 4.1), but 7.9 at 2048 x 512, 160 rows (4.2)
 
 // not volatile: the compiler may move these loads and products freely (volatile asm statements keep their order, which
 // would put every block's loads behind the previous block's products and serialise the HBM round trips)
@@ -364,7 +366,8 @@ int launch_gemm_wx_skinny(const __half* W, const __half* X, const __half* bias, 
     // More than 32 activation rows run as column blocks of 32 (grid.y) when the weight matrix is small: W then comes
     // from L2 for all but the first block, and a matrix of a few 128-row tiles would leave most SMs of the tcgen05
     // kernel's grid without work (a Transformer layer's 512 x 512 projections for 128 sequences: 4 tiles).
-    if (J > kSkinnyMaxJ && (J > kSkinnyMaxBlockedJ || N > kSkinnyMaxBlockedN || (size_t)N * K > kSkinnyMaxBlockedNK))
+    if (J > kSkinnyMaxJ && (J > kSkinnyMaxBlockedJ || N > kSkinnyMaxBlockedN || (size_t)N * K > kSkinnyMaxBlockedNK ||
+                            ceil_div(N, kSkinnyRows) * ceil_div(J, kSkinnyMaxJ) > kSkinnyMaxBlockedCtas))
         return PIMB200_ERR_UNSUPPORTED;
     SkinnyArgs a{W, X, bias, Y, N, K, J, ldx, ldy, act, y_is_f32};
     const int nt = J > kSkinnyMaxJ ? 4 : ceil_div(J, 8);

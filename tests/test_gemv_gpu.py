@@ -168,6 +168,23 @@ def test_few_row_gemm_ragged_shapes(N, K, J):
     assert _lib.lib().pimb200_gemm_last_status() == 0
 
 
+@pytest.mark.parametrize("N,K,J", [(2304, 8, 33), (2056, 64, 127), (2500, 72, 128), (4097, 136, 129), (65, 200, 257), (63, 1032, 300),
+                                   (4104, 192, 2500), (260, 2048, 1025), (512, 512, 9000)])
+@pytest.mark.parametrize("f32", [False, True])
+def test_gemm_row_tiles(N, K, J, f32):
+    # edges of the row-major tcgen05 kernel: one and two CTAs per tile, partial row and column tiles, odd numbers of K
+    # blocks, more tiles than SMs, output rows that no tensor map takes (odd N) and rows inside a wider buffer
+    ops = _ops()
+    W, b, X = _c2_inputs(N, K, J, seed=N + K + J)
+    ref = torch.relu(X.cuda() @ W.cuda().T + b.cuda())
+    out = torch.full((J, N + 24), 7.0, dtype=torch.float32 if f32 else torch.float16, device="cuda")
+    got = ops.gemm_wx(to_dev(W), to_dev(X), to_dev(b), ops.ACT_RELU, out=out[:, :N])
+    assert_close(got, ref, GEMV_ATOL, GEMV_RTOL, f"gemm {N}x{K}x{J}")
+    assert bool((out[:, N:] == 7.0).all())
+    from pimaicompiler_b200 import _lib
+    assert _lib.lib().pimb200_gemm_last_status() == 0
+
+
 @pytest.mark.parametrize("N,K,J", [(4096, 240, 200), (512, 1024, 500), (4096, 2048, 130), (130, 72, 17), (128, 64, 16),
                                    (256, 8, 3), (1280, 320, 29)])
 def test_dense_gemm_tensor_core_and_simt_agree_with_oracle(N, K, J):
