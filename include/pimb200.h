@@ -238,6 +238,18 @@ int pimb200_additive_attention(const void* q, const void* keys_proj, const void*
                                const void* v, const void* bias, void* ctx, float* scores, int n_seq, long max_len, int H,
                                long row_stride, long seq_stride, long ctx_stride, void* stream);
 
+/* The end of a greedy decode step for J streams in lock step: idx[j] = arg max over n of fp16(W[n,:] . X[j,:] + bias[n])
+ * (lowest index among equal maxima; int64 in DEVICE memory), and, when emb is given, the next step's input
+ * x_next[j, :] = emb[idx[j], :] + pos (rows of d elements, d a multiple of 8; pos one row or NULL).  The same as
+ * pimb200_gemm_wx, pimb200_argmax_rows, pimb200_gather_rows and pimb200_add_f16 one after the other, without the logits in
+ * memory.  `workspace`: pimb200_greedy_token_workspace(N, J) bytes of device memory, 16-byte aligned.  Shapes or
+ * alignments without a kernel (K a multiple of 8, of 64 up to 32 streams) return PIMB200_ERR_UNSUPPORTED.  Stands for the
+ * addmm / argmax / embedding nodes of a decode step (executeAtenAddmm, executeAtenArgmax
+ * aten_ops_executor.cpp:520-547, executeAtenEmbedding 1233-1300). */
+size_t pimb200_greedy_token_workspace(int N, int J);
+int pimb200_greedy_token(const void* W, const void* X, const void* bias, int N, int K, int J, int ldx, void* workspace,
+                         long long* idx, const void* emb, const void* pos, void* x_next, int d, void* stream);
+
 typedef struct pimb200_lstm pimb200_lstm;
 
 /* One-time weight layout step.  params = the flat list at::lstm takes:

@@ -47,6 +47,8 @@ struct SkinnyArgs {
     const __half* bias;   // [N] or NULL
     void* Y;              // [J, ldy] fp16 or fp32
     int N, K, J, ldx, ldy, act, y_is_f32;
+    float* best_v;        // arg max form: [CTAs][J] largest output of the CTA's rows and its index
+    int* best_i;
 };
 
 // NT: n-tiles of 8 activation rows; MTW: 16-row weight tiles per warp (1 or 2; they share the warp's X fragments).
@@ -58,6 +60,8 @@ __global__ void __launch_bounds__(kSkinnyThreads) gemm_skinny_kernel(SkinnyArgs 
     constexpr int ROWS = MTW * kSkinnyRows;
     constexpr int UB = 4 / MTW;
     __shared__ float part[KS][ROWS][NT * 8 + 1];
+    pdl_launch_dependents();
+    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int n0 = blockIdx.x * ROWS;
@@ -166,6 +170,8 @@ __global__ void __launch_bounds__(kSkinnyThreads) gemm_skinny_grouped_kernel(con
     constexpr int KS = kSkinnyWarps;
     constexpr int UB = 4;
     __shared__ float part[KS][kSkinnyRows][NT * 8 + 1];
+    pdl_launch_dependents();
+    pdl_wait();
     const SkinnyArgs& a = ga.p[blockIdx.z];
     const int n0 = blockIdx.x * kSkinnyRows;
     const int j_base = blockIdx.y * kSkinnyMaxJ;
@@ -242,10 +248,14 @@ __device__ __forceinline__ uint4 lds_v4(uint32_t addr) {
     return r;
 }
 
-template <int NT, bool FULL>   // FULL: K a multiple of 128 (no partial group of K blocks)
+// FULL: K a multiple of 128 (no partial group of K blocks).  ARGMAX: nothing is stored but, per CTA and activation row, the
+// largest output (rounded to fp16, as it would be stored) and the lowest index that has it.
+template <int NT, bool FULL, bool ARGMAX>
 __global__ void __launch_bounds__(kSkinnyThreads, 2) gemm_skinny_rows_kernel(SkinnyArgs a, int tiles) {
     constexpr int UB = 4;                                            // 32-wide K blocks per register buffer
     extern __shared__ __align__(16) unsigned char sk_smem[];
+    pdl_launch_dependents();
+    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int K = a.K;                                               // K % 64 == 0 (checked by the launcher)
@@ -285,6 +295,13 @@ __global__ void __launch_bounds__(kSkinnyThreads, 2) gemm_skinny_rows_kernel(Ski
     for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
     const uint32_t xaddr = (uint32_t)__cvta_generic_to_shared(sk_smem) + (uint32_t)(g * xs + t * 16);
     const int s1 = g & 1;                                            // odd rows: 64-byte halves of a 128-byte pair swapped
+    float top[NT][2];
+    int at[NT][2];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+        top[j][0] = top[j][1] = -INFINITY;
+        at[j][0] = at[j][1] = 0x7fffffff;
+    }
     auto step = [&](const uint4 (&w)[UB][2], int tile, int grp) {
 #pragma unroll
         for (int u = 0; u < UB; ++u)
@@ -312,6 +329,11 @@ __global__ void __launch_bounds__(kSkinnyThreads, 2) gemm_skinny_rows_kernel(Ski
                     float v = acc[j][2 * h + e] + bv;
                     acc[j][2 * h + e] = 0.f;
                     if (n >= a.N || col >= a.J) continue;
+                    if (ARGMAX) {   // a lane's rows come in ascending order
+                        v = __half2float(__float2half_rn(v));
+                        if (v > top[j][e] || (at[j][e] == 0x7fffffff && v == v)) { top[j][e] = v; at[j][e] = n; }
+                        continue;
+                    }
                     if (a.act == PIMB200_ACT_RELU) v = fmaxf(v, 0.f);
                     if (a.y_is_f32) static_cast<float*>(a.Y)[(size_t)col * a.ldy + n] = v;
                     else static_cast<__half*>(a.Y)[(size_t)col * a.ldy + n] = __float2half_rn(v);
@@ -333,9 +355,45 @@ __global__ void __launch_bounds__(kSkinnyThreads, 2) gemm_skinny_rows_kernel(Ski
         load_group(w0, lt, lg); advance(lt, lg);
         step(w1, ct, cg); advance(ct, cg);
     }
+    if (ARGMAX) {
+        // over the eight lanes that hold other rows of the same columns, then over the warps
+        __shared__ float red_v[kSkinnyWarps][NT * 8];
+        __shared__ int red_i[kSkinnyWarps][NT * 8];
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) {
+                    const float ov = __shfl_xor_sync(0xffffffffu, top[j][e], o);
+                    const int oi = __shfl_xor_sync(0xffffffffu, at[j][e], o);
+                    if (ov > top[j][e] || (ov == top[j][e] && oi < at[j][e])) { top[j][e] = ov; at[j][e] = oi; }
+                }
+                if (g == 0) {
+                    red_v[warp][j * 8 + 2 * t + e] = top[j][e];
+                    red_i[warp][j * 8 + 2 * t + e] = at[j][e];
+                }
+            }
+        __syncthreads();
+        const int col = threadIdx.x;
+        if (col < NT * 8 && col < a.J) {
+            float v = red_v[0][col];
+            int i = red_i[0][col];
+#pragma unroll
+            for (int w = 1; w < kSkinnyWarps; ++w)
+                if (red_v[w][col] > v || (red_v[w][col] == v && red_i[w][col] < i)) { v = red_v[w][col]; i = red_i[w][col]; }
+            a.best_v[(size_t)blockIdx.x * a.J + col] = v;
+            a.best_i[(size_t)blockIdx.x * a.J + col] = i;
+        }
+    }
 }
 
-template <int NT>
+int skinny_rows_grid(int N, size_t smem) {
+    const int per_sm = smem <= 110 * 1024 ? 2 : 1;
+    return min(ceil_div(ceil_div(N, kSkinnyRows), kSkinnyWarps), kNumSmB200 * per_sm);
+}
+
+template <int NT, bool ARGMAX>
 int launch_skinny_rows(const SkinnyArgs& a, cudaStream_t st) {
     const size_t smem = (size_t)NT * 8 * a.K * 2;
     if (a.K % 64 != 0 || smem > 200 * 1024) return PIMB200_ERR_UNSUPPORTED;
@@ -344,18 +402,15 @@ int launch_skinny_rows(const SkinnyArgs& a, cudaStream_t st) {
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return PIMB200_ERR_UNSUPPORTED;
     if (!attr_set[dev]) {
-        if (cudaFuncSetAttribute(gemm_skinny_rows_kernel<NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
-            cudaFuncSetAttribute(gemm_skinny_rows_kernel<NT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
+        if (cudaFuncSetAttribute(gemm_skinny_rows_kernel<NT, true, ARGMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
+            cudaFuncSetAttribute(gemm_skinny_rows_kernel<NT, false, ARGMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
             return PIMB200_ERR_LAUNCH;
         attr_set[dev] = true;
     }
     const int tiles = ceil_div(a.N, kSkinnyRows);
-    const int per_sm = smem <= 110 * 1024 ? 2 : 1;
-    DeviceCtx* ctx = current_ctx();
-    const int grid = min(ceil_div(tiles, kSkinnyWarps), (ctx ? ctx->sm_count : kNumSmB200) * per_sm);
-    if (a.K % 128 == 0) gemm_skinny_rows_kernel<NT, true><<<grid, kSkinnyThreads, smem, st>>>(a, tiles);
-    else gemm_skinny_rows_kernel<NT, false><<<grid, kSkinnyThreads, smem, st>>>(a, tiles);
-    return launch_status();
+    const dim3 grid(skinny_rows_grid(a.N, smem)), block(kSkinnyThreads);
+    if (a.K % 128 == 0) return cuda_status(launch_pdl(gemm_skinny_rows_kernel<NT, true, ARGMAX>, grid, block, smem, st, a, tiles));
+    return cuda_status(launch_pdl(gemm_skinny_rows_kernel<NT, false, ARGMAX>, grid, block, smem, st, a, tiles));
 }
 }  // namespace
 
@@ -369,32 +424,49 @@ int launch_gemm_wx_skinny(const __half* W, const __half* X, const __half* bias, 
     if (J > kSkinnyMaxJ && (J > kSkinnyMaxBlockedJ || N > kSkinnyMaxBlockedN || (size_t)N * K > kSkinnyMaxBlockedNK ||
                             ceil_div(N, kSkinnyRows) * ceil_div(J, kSkinnyMaxJ) > kSkinnyMaxBlockedCtas))
         return PIMB200_ERR_UNSUPPORTED;
-    SkinnyArgs a{W, X, bias, Y, N, K, J, ldx, ldy, act, y_is_f32};
+    SkinnyArgs a{W, X, bias, Y, N, K, J, ldx, ldy, act, y_is_f32, nullptr, nullptr};
     const int nt = J > kSkinnyMaxJ ? 4 : ceil_div(J, 8);
     const int jblocks = ceil_div(J, kSkinnyMaxJ);
     if (nt >= 2 && N >= 16384 && jblocks == 1) {
         // a warp per row tile with X in shared memory, when the CTA's copy of X fits
-        const int rc = nt == 2 ? launch_skinny_rows<2>(a, st) : nt == 3 ? launch_skinny_rows<3>(a, st) : launch_skinny_rows<4>(a, st);
+        const int rc = nt == 2 ? launch_skinny_rows<2, false>(a, st) : nt == 3 ? launch_skinny_rows<3, false>(a, st)
+                                                                    : launch_skinny_rows<4, false>(a, st);
         if (rc != PIMB200_ERR_UNSUPPORTED) return rc;
     }
+    cudaError_t rc = cudaSuccess;
     if (N >= 2048) {
         const dim3 grid(ceil_div(N, 2 * kSkinnyRows), jblocks);
         switch (nt) {
-            case 1: gemm_skinny_kernel<1, 2><<<grid, kSkinnyThreads, 0, st>>>(a); break;
-            case 2: gemm_skinny_kernel<2, 2><<<grid, kSkinnyThreads, 0, st>>>(a); break;
-            case 3: gemm_skinny_kernel<3, 2><<<grid, kSkinnyThreads, 0, st>>>(a); break;
-            default: gemm_skinny_kernel<4, 2><<<grid, kSkinnyThreads, 0, st>>>(a); break;
+            case 1: rc = launch_pdl(gemm_skinny_kernel<1, 2>, grid, dim3(kSkinnyThreads), 0, st, a); break;
+            case 2: rc = launch_pdl(gemm_skinny_kernel<2, 2>, grid, dim3(kSkinnyThreads), 0, st, a); break;
+            case 3: rc = launch_pdl(gemm_skinny_kernel<3, 2>, grid, dim3(kSkinnyThreads), 0, st, a); break;
+            default: rc = launch_pdl(gemm_skinny_kernel<4, 2>, grid, dim3(kSkinnyThreads), 0, st, a); break;
         }
     } else {
         const dim3 grid(ceil_div(N, kSkinnyRows), jblocks);
         switch (nt) {
-            case 1: gemm_skinny_kernel<1, 1><<<grid, kSkinnyThreads, 0, st>>>(a); break;
-            case 2: gemm_skinny_kernel<2, 1><<<grid, kSkinnyThreads, 0, st>>>(a); break;
-            case 3: gemm_skinny_kernel<3, 1><<<grid, kSkinnyThreads, 0, st>>>(a); break;
-            default: gemm_skinny_kernel<4, 1><<<grid, kSkinnyThreads, 0, st>>>(a); break;
+            case 1: rc = launch_pdl(gemm_skinny_kernel<1, 1>, grid, dim3(kSkinnyThreads), 0, st, a); break;
+            case 2: rc = launch_pdl(gemm_skinny_kernel<2, 1>, grid, dim3(kSkinnyThreads), 0, st, a); break;
+            case 3: rc = launch_pdl(gemm_skinny_kernel<3, 1>, grid, dim3(kSkinnyThreads), 0, st, a); break;
+            default: rc = launch_pdl(gemm_skinny_kernel<4, 1>, grid, dim3(kSkinnyThreads), 0, st, a); break;
         }
     }
-    return launch_status();
+    return cuda_status(rc);
+}
+
+// The arg max form for up to 32 activation rows: best_v / best_i [*parts][J]
+int launch_skinny_argmax(const __half* W, const __half* X, const __half* bias, float* best_v, int* best_i, int* parts, int N, int K,
+                         int J, int ldx, cudaStream_t st) {
+    if (J < 1 || J > kSkinnyMaxJ || K % 64 != 0 || ldx % 8 != 0 || !aligned16(W) || !aligned16(X)) return PIMB200_ERR_UNSUPPORTED;
+    const SkinnyArgs a{W, X, bias, nullptr, N, K, J, ldx, 0, PIMB200_ACT_NONE, 0, best_v, best_i};
+    const int nt = ceil_div(J, 8);
+    *parts = skinny_rows_grid(N, (size_t)nt * 8 * K * 2);
+    switch (nt) {
+        case 1: return launch_skinny_rows<1, true>(a, st);
+        case 2: return launch_skinny_rows<2, true>(a, st);
+        case 3: return launch_skinny_rows<3, true>(a, st);
+        default: return launch_skinny_rows<4, true>(a, st);
+    }
 }
 
 // Up to 8 problems in one launch; PIMB200_ERR_UNSUPPORTED when one of them is not a shape of the few-row kernels (the
@@ -408,20 +480,21 @@ int launch_gemm_wx_grouped(const GemmProblem* pr, int n, cudaStream_t st) {
         if (q.J < 1 || q.J > kSkinnyMaxBlockedJ || q.K % 8 != 0 || q.ldx % 8 != 0 || !aligned16(q.W) || !aligned16(q.X))
             return PIMB200_ERR_UNSUPPORTED;
         if (q.J > kSkinnyMaxJ && (q.N > kSkinnyMaxBlockedN || (size_t)q.N * q.K > kSkinnyMaxBlockedNK)) return PIMB200_ERR_UNSUPPORTED;
-        ga.p[i] = SkinnyArgs{q.W, q.X, q.bias, q.Y, q.N, q.K, q.J, q.ldx, q.ldy, q.act, q.y_is_f32};
+        ga.p[i] = SkinnyArgs{q.W, q.X, q.bias, q.Y, q.N, q.K, q.J, q.ldx, q.ldy, q.act, q.y_is_f32, nullptr, nullptr};
         max_tiles = max(max_tiles, ceil_div(q.N, kSkinnyRows));
         max_jb = max(max_jb, ceil_div(q.J, kSkinnyMaxJ));
         max_j = max(max_j, min(q.J, kSkinnyMaxJ));
     }
-    for (int i = n; i < kGroupedMax; ++i) ga.p[i] = SkinnyArgs{nullptr, nullptr, nullptr, nullptr, 0, 0, 0, 0, 0, 0, 0};
+    for (int i = n; i < kGroupedMax; ++i) ga.p[i] = SkinnyArgs{};
     const dim3 grid(max_tiles, max_jb, n);
+    cudaError_t rc = cudaSuccess;
     switch (ceil_div(max_j, 8)) {
-        case 1: gemm_skinny_grouped_kernel<1><<<grid, kSkinnyThreads, 0, st>>>(ga); break;
-        case 2: gemm_skinny_grouped_kernel<2><<<grid, kSkinnyThreads, 0, st>>>(ga); break;
-        case 3: gemm_skinny_grouped_kernel<3><<<grid, kSkinnyThreads, 0, st>>>(ga); break;
-        default: gemm_skinny_grouped_kernel<4><<<grid, kSkinnyThreads, 0, st>>>(ga); break;
+        case 1: rc = launch_pdl(gemm_skinny_grouped_kernel<1>, grid, dim3(kSkinnyThreads), 0, st, ga); break;
+        case 2: rc = launch_pdl(gemm_skinny_grouped_kernel<2>, grid, dim3(kSkinnyThreads), 0, st, ga); break;
+        case 3: rc = launch_pdl(gemm_skinny_grouped_kernel<3>, grid, dim3(kSkinnyThreads), 0, st, ga); break;
+        default: rc = launch_pdl(gemm_skinny_grouped_kernel<4>, grid, dim3(kSkinnyThreads), 0, st, ga); break;
     }
-    return launch_status();
+    return cuda_status(rc);
 }
 
 }  // namespace pimb200

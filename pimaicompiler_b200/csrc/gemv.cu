@@ -321,6 +321,8 @@ __global__ void __launch_bounds__(256) dot_vv_kernel(const __half* __restrict__ 
 // =============================================================================================
 __global__ void __launch_bounds__(256) add_f16_vec_kernel(const uint4* A, const uint4* __restrict__ B,
                                                           uint4* C, size_t total8, int n8, int bcast) {
+    pdl_launch_dependents();
+    pdl_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total8; i += (size_t)gridDim.x * blockDim.x) {
         uint4 a = A[i];
         uint4 b = B[bcast ? (i % n8) : i];
@@ -346,6 +348,8 @@ template <typename V>
 __global__ void __launch_bounds__(256) copy_2d_kernel(unsigned char* __restrict__ dst, size_t dpitch,
                                                       const unsigned char* __restrict__ src, size_t spitch,
                                                       size_t row_elems, size_t rows) {
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t total = row_elems * rows;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         size_t r = i / row_elems, c = i - r * row_elems;
@@ -370,7 +374,8 @@ static int launch_copy_2d(void* dst, size_t dpitch, const void* src, size_t spit
         return (unsigned)(g > 148 * 16 ? 148 * 16 : (g ? g : 1));
     };
     if ((bits & 15) == 0)
-        copy_2d_kernel<uint4><<<grid_for(total_bytes / 16), 256, 0, st>>>(d, dpitch, s, spitch, row_bytes / 16, rows);
+        return cuda_status(launch_pdl(copy_2d_kernel<uint4>, dim3(grid_for(total_bytes / 16)), dim3(256), 0, st, d, dpitch, s, spitch,
+                                      row_bytes / 16, rows));
     else if ((bits & 3) == 0)
         copy_2d_kernel<uint32_t><<<grid_for(total_bytes / 4), 256, 0, st>>>(d, dpitch, s, spitch, row_bytes / 4, rows);
     else if ((bits & 1) == 0)
@@ -500,8 +505,8 @@ extern "C" int pimb200_add_f16(const void* A, const void* B, void* C, int m, int
         size_t total8 = total / 8;
         size_t g = (total8 + 255) / 256;
         unsigned grid = (unsigned)(g > 148 * 8 ? 148 * 8 : g);
-        add_f16_vec_kernel<<<grid, 256, 0, st>>>(static_cast<const uint4*>(A), static_cast<const uint4*>(B),
-                                                 static_cast<uint4*>(C), total8, n / 8, broadcast_b ? 1 : 0);
+        return cuda_status(launch_pdl(add_f16_vec_kernel, dim3(grid), dim3(256), 0, st, static_cast<const uint4*>(A),
+                                      static_cast<const uint4*>(B), static_cast<uint4*>(C), total8, n / 8, broadcast_b ? 1 : 0));
     } else {
         size_t g = (total + 255) / 256;
         unsigned grid = (unsigned)(g > 148 * 8 ? 148 * 8 : g);

@@ -10,6 +10,7 @@
 // shuffles and one shared-memory hop.
 #include <math_constants.h>
 
+#include "attention.cuh"
 #include "common.cuh"
 
 using namespace pimb200;
@@ -105,6 +106,8 @@ __global__ void __launch_bounds__(T) argmax_rows_kernel(const __half* __restrict
                                                                   long cols) {
     __shared__ float red_v[T / 32];
     __shared__ long long red_i[T / 32];
+    pdl_launch_dependents();
+    pdl_wait();
     const __half* row = x + (size_t)blockIdx.x * cols;
     float bv = -CUDART_INF_F;
     long long bi = cols;   // lowest index among equal maxima wins, as in at::argmax on a contiguous row
@@ -209,6 +212,8 @@ __global__ void masked_fill_f16_kernel(const __half* __restrict__ x, const unsig
 // out[i, :] = table[idx[i], :], rows of row_bytes bytes; an index outside [0, n_table) yields a zero row
 __global__ void gather_rows_kernel(const unsigned char* __restrict__ table, const long long* __restrict__ idx,
                                    unsigned char* __restrict__ out, size_t row_bytes, long n_table, int vec16) {
+    pdl_launch_dependents();
+    pdl_wait();
     const long long r = idx[blockIdx.x];
     const bool ok = r >= 0 && r < n_table;
     const unsigned char* src = table + (size_t)(ok ? r : 0) * row_bytes;
@@ -226,6 +231,8 @@ __global__ void gather_rows_kernel(const unsigned char* __restrict__ table, cons
 // device); an index outside [0, n_table) is skipped
 __global__ void scatter_rows_kernel(unsigned char* __restrict__ table, const long long* __restrict__ idx,
                                     const unsigned char* __restrict__ src, size_t row_bytes, long n_table, int vec16) {
+    pdl_launch_dependents();
+    pdl_wait();
     const long long r = idx[blockIdx.x];
     if (r < 0 || r >= n_table) return;
     unsigned char* dst = table + (size_t)r * row_bytes;
@@ -343,102 +350,6 @@ __global__ void __launch_bounds__(kAttnThreads) attention_rows_kernel(const __ha
     }
 }
 
-// The same batched single-query attention with a WARP per (head, sequence), for head widths of 64 or 128 and up to 128
-// cache rows: lanes along the cache rows for the scores (each lane reads whole 128- or 256-byte key rows, the query comes
-// from shared memory as a broadcast), warp shuffles for the softmax, lanes along the head dimension for the weighted sum
-// (one coalesced row of V per cache row, eight rows of loads in flight).  No block-wide barrier, nothing serial per row.
-constexpr int kWarpAttnWarps = 8;
-constexpr int kWarpAttnMaxLen = 128;
-
-template <int EPL>   // elements of the head dimension per lane: 2 (head_dim 64) or 4 (head_dim 128)
-__global__ void __launch_bounds__(kWarpAttnWarps * 32) attention_rows_warp_kernel(
-    const __half* __restrict__ q, const __half* __restrict__ K, const __half* __restrict__ V, const long long* len_dev,
-    long len_inc, long len_add, long max_len, __half* __restrict__ out, int heads, int n_seq, long kv_stride, long seq_stride,
-    long q_stride, long out_stride, float scale) {
-    constexpr int HD = EPL * 32;
-    constexpr int KPL = kWarpAttnMaxLen / 32;     // cache rows per lane
-    __shared__ __align__(16) float qs[kWarpAttnWarps][HD];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long task = (long)blockIdx.x * kWarpAttnWarps + warp;   // head fastest: the heads of a sequence share cache lines
-    if (task >= (long)heads * n_seq) return;
-    const int h = (int)(task % heads), seq = (int)(task / heads);
-    long L = (len_dev ? (long)len_dev[(size_t)seq * len_inc] : 0) + len_add;
-    L = L < 0 ? 0 : (L > max_len ? max_len : L);
-    const __half* qh = q + (size_t)seq * q_stride + (size_t)h * HD;
-    const __half* Ks = K + (size_t)seq * seq_stride + (size_t)h * HD;
-    const __half* Vs = V + (size_t)seq * seq_stride + (size_t)h * HD;
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) qs[warp][lane * EPL + e] = __half2float(qh[lane * EPL + e]) * scale;
-    __syncwarp();
-    float sc[KPL];
-    float m = -CUDART_INF_F;
-#pragma unroll
-    for (int i = 0; i < KPL; ++i) {
-        const long t = lane + 32 * i;
-        sc[i] = -CUDART_INF_F;
-        if (t < L) {
-            const uint4* kr = reinterpret_cast<const uint4*>(Ks + (size_t)t * kv_stride);
-            float a = 0.f;
-#pragma unroll
-            for (int c = 0; c < HD / 8; ++c) {
-                float kf[8];
-                widen8(__ldg(kr + c), kf);
-                const float4 q0 = *reinterpret_cast<const float4*>(&qs[warp][c * 8]);
-                const float4 q1 = *reinterpret_cast<const float4*>(&qs[warp][c * 8 + 4]);
-                a = fmaf(q0.x, kf[0], a); a = fmaf(q0.y, kf[1], a); a = fmaf(q0.z, kf[2], a); a = fmaf(q0.w, kf[3], a);
-                a = fmaf(q1.x, kf[4], a); a = fmaf(q1.y, kf[5], a); a = fmaf(q1.z, kf[6], a); a = fmaf(q1.w, kf[7], a);
-            }
-            sc[i] = a;
-            m = fmaxf(m, a);
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    float sum = 0.f;
-#pragma unroll
-    for (int i = 0; i < KPL; ++i) {
-        sc[i] = (lane + 32 * i < L) ? expf(sc[i] - m) : 0.f;
-        sum += sc[i];
-    }
-    sum = warp_sum(sum);
-    float acc[EPL];
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) acc[e] = 0.f;
-    const __half* vcol = Vs + lane * EPL;
-#pragma unroll
-    for (int i = 0; i < KPL; ++i) {
-        if ((long)32 * i >= L) break;
-        const int rows = (int)min((long)32, L - 32 * i);
-        for (int t0 = 0; t0 < rows; t0 += 8) {
-            float vf[8][EPL];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const long t = 32 * i + min(t0 + u, rows - 1);       // the tail repeats the last row with weight 0
-                if (EPL == 2) {
-                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(vcol + (size_t)t * kv_stride));
-                    vf[u][0] = f.x; vf[u][1] = f.y;
-                } else {
-                    const uint2 raw = *reinterpret_cast<const uint2*>(vcol + (size_t)t * kv_stride);
-                    const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
-                    const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
-                    vf[u][0] = f0.x; vf[u][1] = f0.y; vf[u][EPL - 2] = f1.x; vf[u][EPL - 1] = f1.y;
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                float p = __shfl_sync(0xffffffffu, sc[i], (t0 + u) & 31);
-                if (t0 + u >= rows) p = 0.f;
-#pragma unroll
-                for (int e = 0; e < EPL; ++e) acc[e] = fmaf(p, vf[u][e], acc[e]);
-            }
-        }
-    }
-    const float inv = L > 0 ? 1.0f / sum : 0.f;
-    __half* o = out + (size_t)seq * out_stride + (size_t)h * HD + lane * EPL;
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) o[e] = __float2half_rn(acc[e] * inv);
-}
-
 // Additive (normalised Bahdanau) attention of a decode step:
 //     e[s]   = sum_h v[h] * tanh(keys_proj[s, h] + q[h] + bias[h]),  s < length
 //     ctx[h] = sum_s softmax(e)[s] * values[s, h]
@@ -454,6 +365,8 @@ __global__ void __launch_bounds__(kAddAttnThreads) additive_scores_kernel(
     const __half* __restrict__ q, const __half* __restrict__ keys_proj, const long long* __restrict__ lengths,
     const __half* __restrict__ v, const __half* __restrict__ bias, float* __restrict__ scores, int n_seq, long max_len,
     int H, long row_stride, long seq_stride) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long row = (long)blockIdx.x * (kAddAttnThreads / 32) + warp;     // (sentence, position), position fastest
     if (row >= (long)n_seq * max_len) return;
@@ -490,6 +403,8 @@ __global__ void __launch_bounds__(kAddAttnThreads) additive_scores_kernel(
 __global__ void __launch_bounds__(kAddAttnSlice / 2) additive_context_kernel(
     const float* __restrict__ scores, const __half* __restrict__ values, const long long* __restrict__ lengths,
     __half* __restrict__ ctx, long max_len, int H, long row_stride, long seq_stride, long ctx_stride) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ float sc[];            // [max_len] softmax weights of this sentence
     __shared__ float red[kAddAttnSlice / 64];
     constexpr int T = kAddAttnSlice / 2;
@@ -567,6 +482,64 @@ __global__ void __launch_bounds__(T) add_layer_norm_rows_kernel(const __half* __
         if (gamma) v *= __half2float(gamma[c]);
         if (beta) v += __half2float(beta[c]);
         out[c] = __float2half_rn(v);
+    }
+}
+
+// The same for rows of up to 2048 elements, a multiple of 8, 16-byte aligned: a warp per row, the row in registers (NV
+// 16-byte pieces per lane), no shared memory and no block-wide barrier.  Many rows: bound by HBM (131072 rows of 512: 155 us
+// with a CTA per row, 4 passes of 2-byte accesses); few rows: by latency, so one warp per CTA.
+template <int NV>
+__global__ void __launch_bounds__(256) add_layer_norm_warp_kernel(const __half* __restrict__ x, const __half* __restrict__ r,
+                                                                  const __half* __restrict__ gamma, const __half* __restrict__ beta,
+                                                                  __half* __restrict__ y, long rows, int cols, float eps) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const long row = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    const uint4* xr = reinterpret_cast<const uint4*>(x + row * cols);
+    const uint4* rr = reinterpret_cast<const uint4*>(r + row * cols);
+    const int n8 = cols >> 3;
+    float v[NV][8], s = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int c = lane + 32 * i;
+        if (c < n8) {
+            float b[8];
+            widen8(xr[c], v[i]);
+            widen8(rr[c], b);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                v[i][e] += b[e];
+                s += v[i][e];
+            }
+        }
+    }
+    const float mean = warp_sum(s) / (float)cols;
+    float q = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+        if (lane + 32 * i < n8)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                v[i][e] -= mean;
+                q = fmaf(v[i][e], v[i][e], q);
+            }
+    const float rstd = rsqrtf(warp_sum(q) / (float)cols + eps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int c = lane + 32 * i;
+        if (c >= n8) continue;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            v[i][e] *= rstd;
+            if (gamma) v[i][e] *= __half2float(gamma[c * 8 + e]);
+            if (beta) v[i][e] += __half2float(beta[c * 8 + e]);
+        }
+        __half2 h[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) h[e] = __floats2half2_rn(v[i][2 * e], v[i][2 * e + 1]);
+        reinterpret_cast<uint4*>(y + row * cols)[c] = *reinterpret_cast<uint4*>(h);
     }
 }
 
@@ -675,14 +648,9 @@ extern "C" int pimb200_argmax_rows(const void* x, long long* idx, long rows, lon
     const __half* xp = static_cast<const __half*>(x);
     const bool vec = cols % 8 == 0 && aligned16(x);
     const unsigned grid = (unsigned)rows;
-    if (cols >= kWideRow) {
-        if (vec) argmax_rows_kernel<1024, true><<<grid, 1024, 0, st>>>(xp, idx, cols);
-        else argmax_rows_kernel<1024, false><<<grid, 1024, 0, st>>>(xp, idx, cols);
-    } else {
-        if (vec) argmax_rows_kernel<128, true><<<grid, 128, 0, st>>>(xp, idx, cols);
-        else argmax_rows_kernel<128, false><<<grid, 128, 0, st>>>(xp, idx, cols);
-    }
-    return launch_status();
+    auto run = [&](auto kernel, int threads) { return cuda_status(launch_pdl(kernel, dim3(grid), dim3(threads), 0, st, xp, idx, cols)); };
+    if (cols >= kWideRow) return vec ? run(argmax_rows_kernel<1024, true>, 1024) : run(argmax_rows_kernel<1024, false>, 1024);
+    return vec ? run(argmax_rows_kernel<128, true>, 128) : run(argmax_rows_kernel<128, false>, 128);
 }
 
 extern "C" int pimb200_layer_norm_rows(const void* x, const void* gamma, const void* beta, void* y, long rows, long cols,
@@ -729,9 +697,9 @@ extern "C" int pimb200_gather_rows(const void* table, const long long* idx, void
     if (n_idx == 0 || row_bytes == 0) return PIMB200_OK;
     if (!table || !idx || !out || n_idx < 0 || n_idx > 0x7fffffffL || n_table <= 0) return PIMB200_ERR_BAD_ARG;
     const int vec16 = (row_bytes % 16 == 0 && aligned16(table) && aligned16(out)) ? 1 : 0;
-    gather_rows_kernel<<<(unsigned)n_idx, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const unsigned char*>(table), idx, static_cast<unsigned char*>(out), row_bytes, n_table, vec16);
-    return launch_status();
+    return cuda_status(launch_pdl(gather_rows_kernel, dim3((unsigned)n_idx), dim3(128), 0, static_cast<cudaStream_t>(stream),
+                                  static_cast<const unsigned char*>(table), idx, static_cast<unsigned char*>(out), row_bytes,
+                                  n_table, vec16));
 }
 
 extern "C" int pimb200_scatter_rows(void* table, const long long* idx, const void* src, long n_idx, size_t row_bytes,
@@ -739,9 +707,9 @@ extern "C" int pimb200_scatter_rows(void* table, const long long* idx, const voi
     if (n_idx == 0 || row_bytes == 0) return PIMB200_OK;
     if (!table || !idx || !src || n_idx < 0 || n_idx > 0x7fffffffL || n_table <= 0) return PIMB200_ERR_BAD_ARG;
     const int vec16 = (row_bytes % 16 == 0 && aligned16(table) && aligned16(src)) ? 1 : 0;
-    scatter_rows_kernel<<<(unsigned)n_idx, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<unsigned char*>(table), idx, static_cast<const unsigned char*>(src), row_bytes, n_table, vec16);
-    return launch_status();
+    return cuda_status(launch_pdl(scatter_rows_kernel, dim3((unsigned)n_idx), dim3(128), 0, static_cast<cudaStream_t>(stream),
+                                  static_cast<unsigned char*>(table), idx, static_cast<const unsigned char*>(src), row_bytes,
+                                  n_table, vec16));
 }
 
 extern "C" int pimb200_attention_row(const void* q, const void* K, const void* V, const long long* len_dev, long len_add,
@@ -770,22 +738,10 @@ extern "C" int pimb200_attention_rows(const void* q, const void* K, const void* 
         out_stride < (long)heads * head_dim)
         return PIMB200_ERR_BAD_ARG;
     if (max_len > kAttnMaxLen || head_dim > 1024) return PIMB200_ERR_UNSUPPORTED;
-    // a warp per (head, sequence) when the head width and the cache length allow it and every row is 16-byte aligned
-    const bool rows16 = aligned16(q) && aligned16(K) && aligned16(V) && kv_stride % 8 == 0 && seq_stride % 8 == 0 && q_stride % 8 == 0;
-    if ((head_dim == 64 || head_dim == 128) && max_len <= kWarpAttnMaxLen && rows16) {
-        const long tasks = (long)heads * n_seq;
-        const unsigned grid = (unsigned)((tasks + kWarpAttnWarps - 1) / kWarpAttnWarps);
-        cudaStream_t st = static_cast<cudaStream_t>(stream);
-        if (head_dim == 64)
-            attention_rows_warp_kernel<2><<<grid, kWarpAttnWarps * 32, 0, st>>>(
-                static_cast<const __half*>(q), static_cast<const __half*>(K), static_cast<const __half*>(V), len_dev, len_inc,
-                len_add, max_len, static_cast<__half*>(out), heads, n_seq, kv_stride, seq_stride, q_stride, out_stride, scale);
-        else
-            attention_rows_warp_kernel<4><<<grid, kWarpAttnWarps * 32, 0, st>>>(
-                static_cast<const __half*>(q), static_cast<const __half*>(K), static_cast<const __half*>(V), len_dev, len_inc,
-                len_add, max_len, static_cast<__half*>(out), heads, n_seq, kv_stride, seq_stride, q_stride, out_stride, scale);
-        return launch_status();
-    }
+    const int rc = launch_attention_decode(static_cast<const __half*>(q), static_cast<const __half*>(K), static_cast<const __half*>(V),
+                                           len_dev, len_inc, len_add, max_len, static_cast<__half*>(out), n_seq, heads, head_dim,
+                                           kv_stride, seq_stride, q_stride, out_stride, scale, static_cast<cudaStream_t>(stream));
+    if (rc != PIMB200_ERR_UNSUPPORTED) return rc;
     const size_t smem = ((size_t)max_len + (size_t)(kAttnThreads / 32) * head_dim) * sizeof(float);
     if (smem + 16 > 48 * 1024) return PIMB200_ERR_UNSUPPORTED;
     attention_rows_kernel<<<dim3((unsigned)heads, (unsigned)n_seq), kAttnThreads, smem, static_cast<cudaStream_t>(stream)>>>(
@@ -805,20 +761,32 @@ extern "C" int pimb200_additive_attention(const void* q, const void* keys_proj, 
     if ((size_t)max_len * sizeof(float) + 64 > 48 * 1024) return PIMB200_ERR_UNSUPPORTED;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const long rows = (long)n_seq * max_len;
-    additive_scores_kernel<<<(unsigned)((rows + kAddAttnThreads / 32 - 1) / (kAddAttnThreads / 32)), kAddAttnThreads, 0, st>>>(
+    const int rc = cuda_status(launch_pdl(
+        additive_scores_kernel, dim3((unsigned)((rows + kAddAttnThreads / 32 - 1) / (kAddAttnThreads / 32))), dim3(kAddAttnThreads), 0, st,
         static_cast<const __half*>(q), static_cast<const __half*>(keys_proj), lengths, static_cast<const __half*>(v),
-        static_cast<const __half*>(bias), scores, n_seq, max_len, H, row_stride, seq_stride);
-    additive_context_kernel<<<dim3((unsigned)((H + kAddAttnSlice - 1) / kAddAttnSlice), (unsigned)n_seq), kAddAttnSlice / 2,
-                              (size_t)max_len * sizeof(float), st>>>(
-        scores, static_cast<const __half*>(values), lengths, static_cast<__half*>(ctx), max_len, H, row_stride, seq_stride,
-        ctx_stride);
-    return launch_status();
+        static_cast<const __half*>(bias), scores, n_seq, max_len, H, row_stride, seq_stride));
+    if (rc != PIMB200_OK) return rc;
+    return cuda_status(launch_pdl(
+        additive_context_kernel, dim3((unsigned)((H + kAddAttnSlice - 1) / kAddAttnSlice), (unsigned)n_seq), dim3(kAddAttnSlice / 2),
+        (size_t)max_len * sizeof(float), st, scores, static_cast<const __half*>(values), lengths, static_cast<__half*>(ctx), max_len, H,
+        row_stride, seq_stride, ctx_stride));
 }
 
 extern "C" int pimb200_add_layer_norm_rows(const void* x, const void* r, const void* gamma, const void* beta, void* y,
                                            long rows, long cols, float eps, void* stream) {
     if (rows == 0 || cols == 0) return PIMB200_OK;
     if (!x || !r || !y || !rows_ok(rows, cols)) return PIMB200_ERR_BAD_ARG;
+    if (cols % 8 == 0 && cols <= 2048 && aligned16(x) && aligned16(r) && aligned16(y)) {
+        const int warps = rows <= 4 * kNumSmB200 ? 1 : 8;
+        const dim3 grid((unsigned)((rows + warps - 1) / warps)), block(warps * 32);
+        auto run = [&](auto kernel) {
+            return cuda_status(launch_pdl(kernel, grid, block, 0, static_cast<cudaStream_t>(stream), static_cast<const __half*>(x),
+                                          static_cast<const __half*>(r), static_cast<const __half*>(gamma),
+                                          static_cast<const __half*>(beta), static_cast<__half*>(y), rows, (int)cols, eps));
+        };
+        return cols <= 256 ? run(add_layer_norm_warp_kernel<1>) : cols <= 512 ? run(add_layer_norm_warp_kernel<2>)
+             : cols <= 1024 ? run(add_layer_norm_warp_kernel<4>) : run(add_layer_norm_warp_kernel<8>);
+    }
     if ((size_t)cols * sizeof(float) + 64 > 48 * 1024) return PIMB200_ERR_UNSUPPORTED;
     add_layer_norm_rows_kernel<128><<<(unsigned)rows, 128, (size_t)cols * sizeof(float), static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __half*>(x), static_cast<const __half*>(r), static_cast<const __half*>(gamma),
@@ -833,6 +801,10 @@ extern "C" int pimb200_attention_block(const void* q, const void* k, const void*
     if (!q || !k || !v || !out || n_seq < 0 || n_seq > 65535 || heads <= 0 || head_dim <= 0 || max_len <= 0 ||
         row_stride < (long)heads * head_dim || out_row_stride < (long)heads * head_dim || seq_stride < 0 || out_seq_stride < 0)
         return PIMB200_ERR_BAD_ARG;
+    const int rc = launch_attention_block(static_cast<const __half*>(q), static_cast<const __half*>(k), static_cast<const __half*>(v),
+                                          lengths, static_cast<__half*>(out), n_seq, max_len, heads, head_dim, row_stride,
+                                          seq_stride, out_row_stride, out_seq_stride, scale, static_cast<cudaStream_t>(stream));
+    if (rc != PIMB200_ERR_UNSUPPORTED) return rc;
     const size_t smem = (size_t)max_len * (head_dim + 2) * 2 + (size_t)max_len * head_dim * 2 +
                         (size_t)(kBlockAttnThreads / 32) * (head_dim + max_len) * sizeof(float);
     if (smem > 48 * 1024 || head_dim % 2 != 0) return PIMB200_ERR_UNSUPPORTED;

@@ -325,6 +325,33 @@ def additive_attention(q: torch.Tensor, keys_proj: torch.Tensor, values: torch.T
     return out
 
 
+def greedy_token_workspace(N: int, J: int, device) -> torch.Tensor:
+    """Device scratch of greedy_token for J streams and a vocabulary of N."""
+    return torch.empty(_lib.lib().pimb200_greedy_token_workspace(N, J), dtype=torch.uint8, device=device)
+
+
+def greedy_token(W: torch.Tensor, X: torch.Tensor, bias: Optional[torch.Tensor], workspace: torch.Tensor, idx: torch.Tensor,
+                 emb: Optional[torch.Tensor] = None, pos: Optional[torch.Tensor] = None,
+                 x_next: Optional[torch.Tensor] = None) -> bool:
+    """idx[j] = arg max of the row W @ X[j] + bias, and x_next[j] = emb[idx[j]] (+ pos): the end of a greedy decode step and
+    the input of the next one, without the logits in memory.  Returns False when the shape has no kernel (use gemm_wx,
+    argmax, gather_rows)."""
+    _req_half_cuda(W, bias, emb, pos, x_next)
+    _req_half_cuda_rows(X)
+    N, K = W.shape
+    J = X.shape[0]
+    if idx.dtype != torch.int64 or not idx.is_cuda or not idx.is_contiguous() or idx.numel() != J:
+        raise TypeError("expected a contiguous CUDA int64 index tensor with one element per row of X")
+    if workspace.numel() * workspace.element_size() < _lib.lib().pimb200_greedy_token_workspace(N, J):
+        raise ValueError("workspace too small")
+    rc = _lib.lib().pimb200_greedy_token(_ptr(W), _ptr(X), _ptr(bias), N, K, J, X.stride(0), _ptr(workspace), _ptr(idx), _ptr(emb),
+                                         _ptr(pos), _ptr(x_next), emb.shape[1] if emb is not None else 0, _stream())
+    if rc == _lib.ERR_UNSUPPORTED:
+        return False
+    check(rc, "greedy_token")
+    return True
+
+
 def tanh(x: torch.Tensor) -> torch.Tensor:
     _req_half_cuda(x)
     y = torch.empty_like(x)

@@ -11,9 +11,9 @@ are independent, so a GPU runs `group` of them in lock step:
     feed-forward pair (ReLU fused into the first GEMM) and two fused residual-add + layer-norm launches;
   * the cross-attention keys and values of all decoder layers come from one GEMM over the encoder output;
   * decoder: all `steps` steps of the group are captured into ONE CUDA graph.  Step t's projection GEMM writes q, k, v
-    straight into row t of a [steps, group, 3d] cache (no append, no device-side position), single-query attention reads
-    rows 0..t of it, the vocabulary projection is a GEMM over the group's rows and the arg max writes row t of the token
-    table, which the next step's embedding gather reads.
+    straight into row t of every sequence's part of a [group, steps, 3d] cache (no append, no device-side position),
+    single-query attention reads rows 0..t of it, and the vocabulary projection, the arg max (which writes row t of the
+    token table) and the next step's embedding are two launches that leave no logits in memory.
 
 `TransformerTranslator.translate` is the user call; `bench.py --workload c5` times it.
 """
@@ -61,10 +61,12 @@ class TransformerTranslator:
         nl = cfg.layers
         self.lengths = torch.ones(G, **i64)
         self.cross = torch.zeros(G, S, nl * 2 * d, **f16)            # encoder side, at its maximum size
-        self.cache = [torch.zeros(T, G, 3 * d, **f16) for _ in range(nl)]
+        self.cache = [torch.zeros(G, T, 3 * d, **f16) for _ in range(nl)]
         self.toks = torch.zeros(T + 1, G, **i64)                     # row 0: start tokens, row t+1: choice of step t
         self.forced = torch.zeros(T + 1, G, **i64)
-        self.logits = torch.zeros(G, cfg.vocab, **f16)
+        self.x0 = torch.zeros(G, d, **f16)                           # the step's input: embedding of the last token + position
+        self.token_ws = ops.greedy_token_workspace(cfg.vocab, G, self.dev)
+        self.logits = None                                           # [G, vocab], where the arg max needs them in memory
         self.logits_all = None
         self._graphs = {}
         self.launches_per_step = 0
@@ -93,14 +95,16 @@ class TransformerTranslator:
     def _step(self, t: int, forced: bool, want_logits: bool) -> int:
         cfg, d, G = self.cfg, self.d, self.G
         n = 0
-        tok = (self.forced if forced else self.toks)[t]
-        x = ops.gather_rows(self.emb_tgt, tok); n += 1
-        x = ops.add_f16(x, self.pe[t]); n += 1
+        if t == 0 or forced or want_logits or self.logits is not None:
+            x = ops.gather_rows(self.emb_tgt, (self.forced if forced else self.toks)[t]); n += 1
+            x = ops.add_f16(x, self.pe[t]); n += 1
+        else:
+            x = self.x0                                                          # left there by the previous step
         for i, L in enumerate(self.dec):
-            row = self.cache[i][t]                                               # [G, 3d]: q, k, v of step t
+            row = self.cache[i][:, t]                                            # [G, 3d]: q, k, v of step t
             ops.gemm_wx(L["qkv"], x, L["qkv_b"], out=row); n += 1
             a = ops.attention_rows(row[:, :d], self.cache[i][:, :, d:2 * d], self.cache[i][:, :, 2 * d:], cfg.heads,
-                                   len_add=t + 1, time_major=True); n += 1
+                                   len_add=t + 1); n += 1
             x = ops.add_layer_norm(x, ops.gemm_wx(L["so"], a, L["so_b"])); n += 2
             cq = ops.gemm_wx(L["cq"], x, L["cq_b"]); n += 1
             ck = self.cross[:, :, (2 * i) * d:(2 * i + 1) * d]
@@ -109,6 +113,12 @@ class TransformerTranslator:
             x = ops.add_layer_norm(x, ops.gemm_wx(L["co"], ca, L["co_b"])); n += 2
             f = ops.gemm_wx(L["f2"], ops.gemm_wx(L["f1"], x, L["f1_b"], ops.ACT_RELU), L["f2_b"]); n += 2
             x = ops.add_layer_norm(x, f); n += 1
+        if not want_logits and self.logits is None:
+            nxt = None if forced or t + 1 >= cfg.max_steps else self.pe[t + 1]
+            if ops.greedy_token(self.Wo, x, None, self.token_ws, self.toks[t + 1], None if nxt is None else self.emb_tgt, nxt,
+                                None if nxt is None else self.x0):
+                return n + 2
+            self.logits = torch.zeros(G, cfg.vocab, dtype=torch.float16, device=self.dev)
         lg = self.logits_all[t] if want_logits else self.logits
         ops.gemm_wx(self.Wo, x, out=lg); n += 1
         ops.argmax(lg, out=self.toks[t + 1]); n += 1

@@ -205,3 +205,28 @@ def test_topk_rows_match_oracle(rows, cols, k):
         assert np.array_equal(i.cpu().numpy(), ri)
         tv, _ = torch.topk(x.float(), k, largest=largest)
         assert np.array_equal(rv, tv.numpy())       # the oracle itself against libtorch
+
+
+@pytest.mark.parametrize("J,V,K,bias", [(1, 500, 64, True), (20, 32320, 1024, True), (32, 777, 128, False), (33, 500, 72, True), (130, 32000, 512, False),
+                                        (600, 1000, 64, True)])
+def test_greedy_token_matches_separate_ops(J, V, K, bias):
+    # vocabulary projection + arg max + next embedding in two launches: few-row and tcgen05 forms, ragged vocabularies, ties
+    from pimaicompiler_b200 import ops
+    g = torch.Generator().manual_seed(J + V)
+    W, X, emb, pos = (torch.randn(*s, generator=g).half().cuda() for s in ((V, K), (J, K), (V, 72), (72,)))
+    b = torch.randn(V, generator=g).half().cuda() if bias else None
+    W[V - 1], W[V // 2] = W[3], W[3]                     # equal logits: the lowest index wins
+    if bias:
+        b[V - 1] = b[V // 2] = b[3] = 30.0
+    ws = ops.greedy_token_workspace(V, J, "cuda")
+    idx, x = torch.full((J,), -1, dtype=torch.int64, device="cuda"), torch.empty(J, 72, dtype=torch.float16, device="cuda")
+    assert ops.greedy_token(W, X, b, ws, idx, emb, pos, x)
+    logits = ops.gemm_wx(W, X, b)
+    ref = X.double() @ W.double().T + (b.double() if bias else 0)
+    best = ref.gather(1, idx[:, None])[:, 0]
+    assert bool((best >= ref.max(1).values - 2e-3 * ref.abs().max(1).values).all())
+    same = ops.argmax(logits) == idx                     # the two forms may sum in another order: ties of rounded logits only
+    assert bool((same | ((logits.gather(1, idx[:, None])[:, 0] - logits.max(1).values).abs() < 0.07)).all())
+    if bias:
+        assert idx.tolist() == [3] * J or not bool((ref[:, 3] > ref.max(1).values - 1e-9).all())
+    assert torch.equal(x, ops.add_f16(ops.gather_rows(emb, idx), pos))
