@@ -62,7 +62,8 @@ struct Maps {
 struct Args {
     const __half* bias;       // [N] or NULL (outputs and arg max)
     int N, J, act;
-    int jrows;                // activation rows per CTA: 128, or the whole timesteps that fit in 128 rows
+    int jrows;                // activation rows per CTA: 128, or J if it is less, or the whole timesteps that fit in 128 rows
+    int bn;                   // weight rows per tile: a multiple of 32 (64 for the cell), at most the template's BN
     int kb1, kb2;             // K blocks of 64 of the first and the second pair
     int j_tiles, n_tiles;     // tiles along the activation rows (of one CTA or a pair) and along the weight rows
     void* Y;
@@ -252,12 +253,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
         // ---------------- TMA producers: warp 0 the activation rows, warp 1 the weight rows, each one stream of K blocks
         //                  over all tiles of this CTA ----------------
         const uint32_t el = elect_one();
-        const uint32_t bytes = (uint32_t)CG * ((uint32_t)a.jrows * BK * 2 + (uint32_t)B_BYTES);   // a K block of both CTAs
+        const uint32_t bytes = (uint32_t)CG * (uint32_t)a.jrows * BK * 2 + (uint32_t)a.bn * BK * 2;   // a K block of both CTAs
         const uint32_t smem0 = smem_u32(smem) + (warp == 0 ? 0 : A_BYTES), lead0 = CG == 1 ? full0 : mapa(full0, 0);
         const bool counts = warp == 0 && rank == 0;            // tells the stage's barrier how many bytes will come
         uint32_t s = 0, par = 1, issued = 0;                   // stage, parity of its "empty" phase, stages issued
         for (int tile = first; tile < tiles && !failed; tile += stride) {
-            const int n0 = (tile % a.n_tiles) * BN + rank * (BN / CG), j0 = ((tile / a.n_tiles) * CG + rank) * a.jrows;
+            const int n0 = (tile % a.n_tiles) * a.bn + rank * (a.bn / CG), j0 = ((tile / a.n_tiles) * CG + rank) * a.jrows;
             const int t0 = a.x_batch > 0 ? j0 / a.x_batch : 0;
             for (int k0 = 0; k0 < kblocks; k0 += KS) {
                 if (!mbar_wait(empty0 + 8 * s, par, abort_flag, a.gen)) { failed = true; break; }
@@ -289,8 +290,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
         // ---------------- MMA issuer (the pair's leader) ----------------
         if (rank == 0) {
             const uint32_t el = elect_one();
-            // D = f32, A = B = f16, both K-major, N = BN, M = 128 or 256
-            const uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(CG * BM >> 4) << 24);
+            // D = f32, A = B = f16, both K-major, N = bn, M = 128 or 256
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(a.bn >> 3) << 17) | ((uint32_t)(CG * BM >> 4) << 24);
             const uint64_t desc0 = make_smem_desc(smem_u32(smem));
             uint32_t s = 0, par = 0;
             int local = 0;
@@ -336,7 +337,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
         for (int tile = first; tile < tiles; tile += stride, ++local) {
             const int as = local & 1;
             const int nt = tile % a.n_tiles;
-            const int n0 = nt * BN, j0 = ((tile / a.n_tiles) * CG + rank) * a.jrows, j = j0 + r;
+            const int n0 = nt * a.bn, n_end = min(a.N, n0 + a.bn), j0 = ((tile / a.n_tiles) * CG + rank) * a.jrows, j = j0 + r;
             if (!mbar_wait(accf0 + 8 * as, (uint32_t)(local >> 1) & 1, abort_flag, a.gen)) {
                 status_raise(a.status, a.gen, PIMB200_ERR_TIMEOUT);
                 break;
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
                 constexpr int CH = EPI == kRowsHalf ? 64 : 32;         // columns per 128-byte chunk
 #pragma unroll 1
                 for (int c = half * CH; c < BN; c += 2 * CH) {
-                    if (n0 + c >= a.N) break;                          // uniform
+                    if (n0 + c >= n_end) break;                        // uniform
                     uint4 bb[CH / 8];                                  // under way while the accumulator is read
                     if (bias_vec) {
 #pragma unroll
@@ -373,13 +374,13 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
                         }
                     } else if (a.bias) {
 #pragma unroll
-                        for (int i = 0; i < CH; ++i) f[i] += (n0 + c + i < a.N) ? __half2float(__ldg(a.bias + n0 + c + i)) : 0.f;
+                        for (int i = 0; i < CH; ++i) f[i] += (n0 + c + i < n_end) ? __half2float(__ldg(a.bias + n0 + c + i)) : 0.f;
                     }
                     if (a.direct) {                                    // rows of Y that no tensor map takes
                         if (row_ok) {
 #pragma unroll
                             for (int i = 0; i < CH; ++i) {
-                                if (n0 + c + i >= a.N) break;
+                                if (n0 + c + i >= n_end) break;
                                 const size_t at = (size_t)j * a.ldy + n0 + c + i;
                                 if (EPI == kRowsHalf) static_cast<__half*>(a.Y)[at] = __float2half_rn(fmaxf(f[i], lo));
                                 else static_cast<float*>(a.Y)[at] = fmaxf(f[i], lo);
@@ -399,6 +400,16 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
                             o[i] = make_uint4(__float_as_uint(fmaxf(f[4 * i], lo)), __float_as_uint(fmaxf(f[4 * i + 1], lo)),
                                               __float_as_uint(fmaxf(f[4 * i + 2], lo)), __float_as_uint(fmaxf(f[4 * i + 3], lo)));
                         }
+                    }
+                    if (n0 + c + CH > n_end && n_end < a.N) {          // half a chunk left of this tile: the map's boxes are whole ones
+                        if (row_ok) {
+                            unsigned char* yp = static_cast<unsigned char*>(a.Y) + ((size_t)j * a.ldy + n0 + c) * (EPI == kRowsHalf ? 2 : 4);
+#pragma unroll
+                            for (int i = 0; i < 8; ++i)
+                                if (n0 + c + (i + 1) * CH / 8 <= n_end) reinterpret_cast<uint4*>(yp)[i] = o[i];
+                        }
+                        __syncwarp();
+                        continue;
                     }
                     // the chunk before the previous one must have been read out of this buffer
                     if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
@@ -424,7 +435,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
 #pragma unroll 1
                 for (int c = half * 32; c < BN; c += 64) {
                     const int nb = n0 + c;
-                    if (nb >= a.N) break;
+                    if (nb >= n_end) break;
                     uint4 bb[4];
                     if (bias_vec) {
 #pragma unroll
@@ -432,7 +443,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
                     }
                     uint32_t v[32];
                     tmem_ld32(acc + (uint32_t)c, v);
-                    const int lim = a.N - nb;
+                    const int lim = n_end - nb;
                     float b[32];
                     if (bias_vec) {
 #pragma unroll
@@ -456,7 +467,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
                 // LSTM cell: 64 columns = the four gates (i, f, g, o side by side) of 16 hidden units
 #pragma unroll 1
                 for (int c = half * 64; c < BN; c += 128) {
-                    if (n0 + c >= a.N) break;
+                    if (n0 + c >= n_end) break;
                     uint32_t v[64];
                     tmem_ld32_nowait(acc + (uint32_t)c, v);
                     tmem_ld32_nowait(acc + (uint32_t)c + 32, v + 32);
@@ -537,44 +548,57 @@ int launch_one(const Maps& m, const Args& a, int dev, cudaStream_t st) {
     return cuda_status(launch_pdl<CG>(gemm_rows_kernel<BN, EPI, CG>, dim3(grid), dim3(THREADS), smem, st, m, a));
 }
 
-struct Plan { int bn, cg; };
+struct Plan { int bn, cg; };       // weight rows per tile, CTAs per tile
 
-// Tile shape: waves of tiles over the SMs (or pairs of them), each as long as the slower of its K blocks and its epilogue,
-// plus the last epilogue, which nothing hides.  Cycles per K block of 64 as measured (single CTAs 64 / 128 / 256 columns:
-// 300 / 400 / 700, pairs 320 / 400 / 520: MMAs where they bound, operand traffic or barrier waits where those do).
-// One wave of short products is quickest with single CTAs, many waves with pairs of 256 columns (also where the epilogue is
-// all that counts: 128000 rows of 4096 x 240 take 470 us with single CTAs, 429 with pairs).
-Plan pick(int N, int J, int jrows, int kblocks, int sms) {
+// Tile shape.  For one, two, ... waves of tiles over the SMs (or pairs of them) the tiles are made as narrow as those waves
+// allow, so that no wave is left half empty (32320 weight rows: 145 tiles of 224 on 148 SMs, not 127 of 256).  A wave takes
+// as long as the slower of its K blocks and its epilogue; the last epilogue comes on top, nothing hides it.  Cycles per K
+// block of 64 as measured (single CTAs of 64 / 128 / 256 columns: 300 / 400 / 700, pairs 320 / 400 / 520: MMAs where they
+// bound, operand traffic or barrier waits where those do).  One wave of short products is quickest with single CTAs, many
+// waves with pairs of 256 columns (also where the epilogue is all that counts: 128000 rows of 4096 x 240 take 470 us with
+// single CTAs, 429 with pairs).
+Plan pick(int N, int J, int jrows, int kblocks, int grain, int sms) {
     static const int per_block[2][3] = {{300, 400, 700}, {320, 400, 520}};
     Plan best{0, 0};
     double cost = 0;
-    for (int cg = J > jrows ? 2 : 1; cg >= 1; --cg)
-        for (int i = 0, bn = 64; i < 3; ++i, bn *= 2) {
-            const long tiles = (long)ceil_div(J, jrows * cg) * ceil_div(N, bn), slots = sms / cg, waves = (tiles + slots - 1) / slots;
-            const double mma = (double)kblocks * per_block[cg - 1][i], epi = 600 + 14 * bn;
+    for (int cg = J > jrows ? 2 : 1; cg >= 1; --cg) {
+        const int slots = sms / cg, j_tiles = ceil_div(J, jrows * cg);
+        int last = 0;
+        for (long w = (long)ceil_div(N, 256) * j_tiles / slots; ; ++w) {
+            const long n_max = w * slots / j_tiles;                    // column tiles that w waves hold
+            if (n_max < 1) continue;
+            int bn = (int)((N + n_max - 1) / n_max);
+            bn = ceil_div(bn, grain) * grain;
+            if (bn > 256) continue;
+            if (bn < 64) bn = 64;
+            if (bn == last) break;
+            last = bn;
+            const long tiles = (long)j_tiles * ceil_div(N, bn), waves = (tiles + slots - 1) / slots;
+            const int* p = per_block[cg - 1];
+            const double per = bn <= 128 ? p[0] + (p[1] - p[0]) * (bn - 64) / 64.0 : p[1] + (p[2] - p[1]) * (bn - 128) / 128.0;
+            const double mma = kblocks * per, epi = 600 + 14 * bn;
             const double c = waves * (300 + (mma > epi ? mma : epi)) + epi;
             if (!best.bn || c < cost) { best = Plan{bn, cg}; cost = c; }
+            if (bn == 64) break;
         }
+    }
     return best;
 }
 
 template <int EPI>
 int launch_plan(Plan p, const Maps& m, Args& a, int dev, cudaStream_t st) {
+    a.bn = p.bn;
     a.n_tiles = ceil_div(a.N, p.bn);
     a.j_tiles = ceil_div(a.J, a.jrows * p.cg);
     if (p.cg == 2) {
-        switch (p.bn) {
-            case 256: return launch_one<256, EPI, 2>(m, a, dev, st);
-            case 128: return launch_one<128, EPI, 2>(m, a, dev, st);
-            default: return launch_one<64, EPI, 2>(m, a, dev, st);
-        }
+        if (p.bn > 128) return launch_one<256, EPI, 2>(m, a, dev, st);
+        return p.bn > 64 ? launch_one<128, EPI, 2>(m, a, dev, st) : launch_one<64, EPI, 2>(m, a, dev, st);
     }
-    switch (p.bn) {
-        case 256: return launch_one<256, EPI, 1>(m, a, dev, st);
-        case 128: return launch_one<128, EPI, 1>(m, a, dev, st);
-        default: return launch_one<64, EPI, 1>(m, a, dev, st);
-    }
+    if (p.bn > 128) return launch_one<256, EPI, 1>(m, a, dev, st);
+    return p.bn > 64 ? launch_one<128, EPI, 1>(m, a, dev, st) : launch_one<64, EPI, 1>(m, a, dev, st);
 }
+
+int tile_rows(int J) { return J < BM ? J : BM; }
 
 bool operands_ok(const void* W, const void* X, int K, long ldx) {
     return K % 8 == 0 && ldx % 8 == 0 && aligned16(W) && aligned16(X);
@@ -592,44 +616,47 @@ int launch_gemm_rows(const __half* W, const __half* X, const __half* bias, void*
     int dev = 0, rc;
     if ((rc = tc_prepare(&dev, &a.status, &a.gen)) != PIMB200_OK) return rc;
     a.bias = bias; a.N = N; a.J = J; a.act = act;
-    a.jrows = x_batch > 0 ? BM / x_batch * x_batch : BM;   // whole timesteps; the tile's other rows are never stored
+    // whole timesteps, or no more rows than there are: a tile's other rows are never stored, and a load of rows past the end
+    // of X costs more than one of rows that exist (32320 x 1024, 32 rows: 19.2 us with boxes of 128)
+    a.jrows = x_batch > 0 ? BM / x_batch * x_batch : tile_rows(J);
     a.x_batch = x_batch;
     a.kb1 = ceil_div(K, BK);
-    const Plan p = pick(N, J, a.jrows, a.kb1, tc_sm_count(dev));
+    const Plan p = pick(N, J, a.jrows, a.kb1, 32, tc_sm_count(dev));
     Maps m = {};
     if (!encode_2d(&m.w, W, N, K, (uint64_t)K * 2, p.bn / p.cg, 2)) return PIMB200_ERR_UNSUPPORTED;
     if (x_batch > 0) {
         if (!encode_x_time_major(&m.x, X, x_batch, J / x_batch, x_seq_rows, K, (uint64_t)ldx * 2, a.jrows / x_batch))
             return PIMB200_ERR_UNSUPPORTED;
-    } else if (!encode_2d(&m.x, X, J, K, (uint64_t)ldx * 2, BM, 2)) {
+    } else if (!encode_2d(&m.x, X, J, K, (uint64_t)ldx * 2, a.jrows, 2)) {
         return PIMB200_ERR_UNSUPPORTED;
     }
-    const int es = y_is_f32 ? 4 : 2, tail = a.jrows % 32;
+    const int es = y_is_f32 ? 4 : 2, tail = a.jrows % 32, whole = a.jrows < 32 ? a.jrows : 32;
     a.Y = Y; a.ldy = ldy;
     a.direct = !aligned16(Y) || (long)ldy * es % 16 != 0;
     if (a.direct) m.y = m.x;   // (prefetched only)
-    else if (!encode_2d(&m.y, Y, J, N, (uint64_t)ldy * es, 32, es) ||
+    else if (!encode_2d(&m.y, Y, J, N, (uint64_t)ldy * es, whole, es) ||
         (tail && !encode_2d(&m.y_tail, Y, J, N, (uint64_t)ldy * es, tail, es)))
         return PIMB200_ERR_UNSUPPORTED;
     return y_is_f32 ? launch_plan<kRowsFloat>(p, m, a, dev, st) : launch_plan<kRowsHalf>(p, m, a, dev, st);
 }
 
-int gemm_rows_parts(int N) { return 2 * ceil_div(N, 256); }
+int gemm_rows_max_parts(int N) { return 2 * ceil_div(N, 64); }
 
-int launch_gemm_rows_argmax(const __half* W, const __half* X, const __half* bias, float* best_v, int* best_i, int N, int K,
-                            int J, int ldx, cudaStream_t st) {
+int launch_gemm_rows_argmax(const __half* W, const __half* X, const __half* bias, float* best_v, int* best_i, int* parts, int N,
+                            int K, int J, int ldx, cudaStream_t st) {
     using namespace tc;
     if (!operands_ok(W, X, K, ldx)) return PIMB200_ERR_UNSUPPORTED;
     Args a = {};
     int dev = 0, rc;
     if ((rc = tc_prepare(&dev, &a.status, &a.gen)) != PIMB200_OK) return rc;
     a.bias = bias; a.N = N; a.J = J; a.act = PIMB200_ACT_NONE;
-    a.jrows = BM;
+    a.jrows = tile_rows(J);
     a.kb1 = ceil_div(K, BK);
-    const Plan p{256, J > BM ? 2 : 1};
+    const Plan p = pick(N, J, a.jrows, a.kb1, 32, tc_sm_count(dev));
+    *parts = 2 * ceil_div(N, p.bn);
     a.best_v = best_v; a.best_i = best_i;
     Maps m = {};   // (y is only prefetched)
-    if (!encode_2d(&m.w, W, N, K, (uint64_t)K * 2, p.bn / p.cg, 2) || !encode_2d(&m.x, X, J, K, (uint64_t)ldx * 2, BM, 2))
+    if (!encode_2d(&m.w, W, N, K, (uint64_t)K * 2, p.bn / p.cg, 2) || !encode_2d(&m.x, X, J, K, (uint64_t)ldx * 2, a.jrows, 2))
         return PIMB200_ERR_UNSUPPORTED;
     m.y = m.x;
     return launch_plan<kRowsArgmax>(p, m, a, dev, st);
@@ -644,18 +671,18 @@ int launch_gemm_rows_cell(const RowsCell& c, cudaStream_t st) {
     Args a = {};
     int dev = 0, rc;
     if ((rc = tc_prepare(&dev, &a.status, &a.gen)) != PIMB200_OK) return rc;
-    a.N = 4 * c.H; a.J = c.J; a.jrows = BM;
+    a.N = 4 * c.H; a.J = c.J; a.jrows = tile_rows(c.J);
     a.kb1 = ceil_div(c.I, BK);
     a.kb2 = c.h0 ? ceil_div(c.H, BK) : 0;
     a.cell_bias = c.bias; a.c0 = c.c0; a.y = c.y; a.y_ld = c.y_ld; a.hn = c.hn; a.cn = c.cn; a.res = c.res; a.res_ld = c.res_ld;
     a.H = c.H;
-    const Plan p = pick(a.N, a.J, BM, a.kb1 + a.kb2, tc_sm_count(dev));
+    const Plan p = pick(a.N, a.J, a.jrows, a.kb1 + a.kb2, 64, tc_sm_count(dev));
     Maps m = {};
     if (!encode_2d(&m.w, c.Wx, a.N, c.I, (uint64_t)c.I * 2, p.bn / p.cg, 2) ||
-        !encode_2d(&m.x, c.x, c.J, c.I, (uint64_t)c.x_ld * 2, BM, 2))
+        !encode_2d(&m.x, c.x, c.J, c.I, (uint64_t)c.x_ld * 2, a.jrows, 2))
         return PIMB200_ERR_UNSUPPORTED;
     if (c.h0 && (!encode_2d(&m.w2, c.Wh, a.N, c.H, (uint64_t)c.H * 2, p.bn / p.cg, 2) ||
-                 !encode_2d(&m.x2, c.h0, c.J, c.H, (uint64_t)c.H * 2, BM, 2)))
+                 !encode_2d(&m.x2, c.h0, c.J, c.H, (uint64_t)c.H * 2, a.jrows, 2)))
         return PIMB200_ERR_UNSUPPORTED;
     m.y = m.x;
     return launch_plan<kRowsCell>(p, m, a, dev, st);

@@ -26,10 +26,10 @@ int tc_sm_count(int dev);
 int launch_gemm_rows(const __half* W, const __half* X, const __half* bias, void* Y, int N, int K, int J, int ldx, int ldy,
                      int act, int y_is_f32, int x_batch, long x_seq_rows, cudaStream_t st);
 
-// The largest of fp16(act(X W^T + bias)) of every row in pieces: best_v / best_i [parts][J], parts = gemm_rows_parts(N).
-int gemm_rows_parts(int N);
-int launch_gemm_rows_argmax(const __half* W, const __half* X, const __half* bias, float* best_v, int* best_i, int N, int K,
-                            int J, int ldx, cudaStream_t st);
+// The largest of fp16(X W^T + bias) of every row in pieces: best_v / best_i [*parts][J], *parts <= gemm_rows_max_parts(N).
+int gemm_rows_max_parts(int N);
+int launch_gemm_rows_argmax(const __half* W, const __half* X, const __half* bias, float* best_v, int* best_i, int* parts, int N,
+                            int K, int J, int ldx, cudaStream_t st);
 
 // One LSTM step of J sequences: gates = X Wx^T + H0 Wh^T + bias (H0 may be NULL), cell update, y = h (+ residual)
 struct RowsCell {
@@ -46,5 +46,6 @@ struct RowsCell {
     int I, H, J;
 };
 int launch_gemm_rows_cell(const RowsCell& c, cudaStream_t st);
+int launch_lstm_cell_skinny(const RowsCell& c, cudaStream_t st);   // up to 32 sequences (gemm_skinny.cu)
 
 }  // namespace pimb200

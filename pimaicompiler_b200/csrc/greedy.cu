@@ -80,7 +80,7 @@ using namespace pimb200;
 
 extern "C" size_t pimb200_greedy_token_workspace(int N, int J) {
     if (N <= 0 || J <= 0) return 0;
-    const size_t parts = J <= 32 ? kMaxParts : gemm_rows_parts(N);
+    const size_t parts = J <= 32 ? kMaxParts : gemm_rows_max_parts(N);
     return parts * J * (sizeof(float) + sizeof(int));
 }
 
@@ -91,10 +91,10 @@ extern "C" int pimb200_greedy_token(const void* W, const void* X, const void* bi
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const __half *w = static_cast<const __half*>(W), *x = static_cast<const __half*>(X), *b = static_cast<const __half*>(bias);
     float* best_v = static_cast<float*>(workspace);
-    int parts = J <= 32 ? kMaxParts : gemm_rows_parts(N);
+    int parts = J <= 32 ? kMaxParts : gemm_rows_max_parts(N);
     int* best_i = reinterpret_cast<int*>(best_v + (size_t)parts * J);
     const int rc = J <= 32 ? launch_skinny_argmax(w, x, b, best_v, best_i, &parts, N, K, J, ldx, st)
-                           : launch_gemm_rows_argmax(w, x, b, best_v, best_i, N, K, J, ldx, st);
+                           : launch_gemm_rows_argmax(w, x, b, best_v, best_i, &parts, N, K, J, ldx, st);
     if (rc != PIMB200_OK) return rc;
     auto run = [&](auto kernel, int slices) {
         return cuda_status(launch_pdl(kernel, dim3(ceil_div(J, kRows)), dim3(kRows * slices), 0, st, best_v, best_i, parts, J, N, idx,
