@@ -13,7 +13,7 @@
 //     slots of two products, and the B fragment (X, read through L1: it is small and shared by all CTAs) is taken
 //     from the same k positions.  No shared-memory staging, no shuffles;
 //   * the K-partials meet in shared memory; the CTA's rows x J outputs get bias, activation and the fp16 (or fp32) store.
-#include "common.cuh"
+#include "gemm_rows.cuh"
 
 namespace pimb200 {
 
@@ -148,6 +148,101 @@ __global__ void __launch_bounds__(kSkinnyThreads) gemm_skinny_kernel(SkinnyArgs 
         if (a.act == PIMB200_ACT_RELU) v = fmaxf(v, 0.f);
         if (a.y_is_f32) static_cast<float*>(a.Y)[(size_t)(j_base + j) * a.ldy + n] = v;
         else static_cast<__half*>(a.Y)[(size_t)(j_base + j) * a.ldy + n] = __float2half_rn(v);
+    }
+}
+
+// One LSTM step of up to 32 sequences in one launch: the products with W_ih and W_hh as one walk over the K blocks of both
+// (their eight warps' partial sums meet once), gate math in the epilogue.  A CTA owns 32 packed gate rows = 8 hidden units.
+// As two products and a gate kernel a step of 9 sequences (2048 inputs, H = 1024) took 12.8 us, the first 1.1 of each
+// kernel in launch and ramp; one launch takes 8.9.  The weights are constants of the handle, so the first group of them is
+// loaded before the kernel's predecessor has finished.
+template <int NT>
+__global__ void __launch_bounds__(kSkinnyThreads) lstm_cell_skinny_kernel(const __grid_constant__ RowsCell a) {
+    constexpr int KS = kSkinnyWarps, ROWS = 2 * kSkinnyRows, UB = 2;
+    __shared__ float part[KS][ROWS][NT * 8 + 1];
+    pdl_launch_dependents();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane >> 2, t = lane & 3;
+    const int n0 = blockIdx.x * ROWS;                              // 4H is a multiple of 32
+    const int bx = a.I >> 5, blocks = bx + (a.h0 ? a.H >> 5 : 0);  // 32-wide K blocks of both products
+    const int per = (blocks + KS - 1) / KS;
+    const int b_lo = min(blocks, warp * per), b_hi = min(blocks, b_lo + per);
+    const __half* wi = a.Wx + (size_t)(n0 + g) * a.I + 8 * t;
+    const __half* wh = a.Wh + (size_t)(n0 + g) * a.H + 8 * t;
+    float acc[2][NT][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[m][j][i] = 0.f;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    uint4 wc[UB][2][2], xc[UB][NT], wn[UB][2][2], xn[UB][NT];
+    auto load_w = [&](uint4 (&w)[UB][2][2], int b0) {
+#pragma unroll
+        for (int u = 0; u < UB; ++u) {
+            const int b = b0 + u;
+            const bool in = b < b_hi, first = b < bx;
+            const __half* p = first ? wi + (size_t)b * 32 : wh + (size_t)(b - bx) * 32;
+            const size_t row8 = (size_t)8 * (first ? a.I : a.H);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) w[u][q >> 1][q & 1] = in ? ldg_w(p + q * row8) : zero;   // rows g, g+8, g+16, g+24
+        }
+    };
+    auto load_x = [&](uint4 (&x)[UB][NT], int b0) {
+#pragma unroll
+        for (int u = 0; u < UB; ++u) {
+            const int b = b0 + u;
+            const bool in = b < b_hi, first = b < bx;
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+                const int row = min(j * 8 + g, a.J - 1);           // rows past J repeat the last one
+                const __half* p = first ? a.x + (size_t)row * a.x_ld + b * 32 : a.h0 + (size_t)row * a.H + (b - bx) * 32;
+                x[u][j] = in ? __ldg(reinterpret_cast<const uint4*>(p + 8 * t)) : zero;
+            }
+        }
+    };
+    auto multiply = [&](const uint4 (&w)[UB][2][2], const uint4 (&x)[UB][NT]) {
+#pragma unroll
+        for (int u = 0; u < UB; ++u)
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    mma16816(acc[m][j], w[u][m][0].x, w[u][m][1].x, w[u][m][0].y, w[u][m][1].y, x[u][j].x, x[u][j].y);
+                    mma16816(acc[m][j], w[u][m][0].z, w[u][m][1].z, w[u][m][0].w, w[u][m][1].w, x[u][j].z, x[u][j].w);
+                }
+    };
+    load_w(wc, b_lo);
+    pdl_wait();
+    load_x(xc, b_lo);
+    for (int b0 = b_lo; b0 < b_hi; b0 += 2 * UB) {
+        load_w(wn, b0 + UB); load_x(xn, b0 + UB);
+        multiply(wc, xc);
+        load_w(wc, b0 + 2 * UB); load_x(xc, b0 + 2 * UB);
+        multiply(wn, xn);
+    }
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) part[warp][m * 16 + g + (e >> 1) * 8][j * 8 + 2 * t + (e & 1)] = acc[m][j][e];
+    __syncthreads();
+    const int ul = threadIdx.x & 7, u = (n0 >> 2) + ul;            // a thread per (sequence, unit)
+    for (int j = threadIdx.x >> 3; j < a.J; j += kSkinnyThreads / 8) {
+        const float4 b4 = *reinterpret_cast<const float4*>(a.bias + (size_t)u * 4);
+        float z[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int w = 0; w < KS; ++w)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) z[q] += part[w][ul * 4 + q][j];
+        const float cprev = a.c0 ? __half2float(a.c0[(size_t)j * a.H + u]) : 0.f;
+        const float cnew = sigmoidf_(z[1] + b4.y) * cprev + sigmoidf_(z[0] + b4.x) * tanhf_(z[2] + b4.z);
+        const __half hh = __float2half_rn(sigmoidf_(z[3] + b4.w) * tanhf_(cnew));
+        a.y[(size_t)j * a.y_ld + u] = a.res ? __float2half_rn(__half2float(hh) + __half2float(a.res[(size_t)j * a.res_ld + u])) : hh;
+        if (a.hn) a.hn[(size_t)j * a.H + u] = hh;
+        if (a.cn) a.cn[(size_t)j * a.H + u] = __float2half_rn(cnew);
     }
 }
 
@@ -452,6 +547,18 @@ int launch_gemm_wx_skinny(const __half* W, const __half* X, const __half* bias, 
         }
     }
     return cuda_status(rc);
+}
+
+int launch_lstm_cell_skinny(const RowsCell& c, cudaStream_t st) {
+    if (c.J < 1 || c.J > kSkinnyMaxJ || c.I % 32 != 0 || c.H % 32 != 0 || c.x_ld % 8 != 0 || !aligned16(c.x) || (c.h0 && !aligned16(c.h0)))
+        return PIMB200_ERR_UNSUPPORTED;
+    const dim3 grid(4 * c.H / (2 * kSkinnyRows)), block(kSkinnyThreads);
+    switch (ceil_div(c.J, 8)) {
+        case 1: return cuda_status(launch_pdl(lstm_cell_skinny_kernel<1>, grid, block, 0, st, c));
+        case 2: return cuda_status(launch_pdl(lstm_cell_skinny_kernel<2>, grid, block, 0, st, c));
+        case 3: return cuda_status(launch_pdl(lstm_cell_skinny_kernel<3>, grid, block, 0, st, c));
+        default: return cuda_status(launch_pdl(lstm_cell_skinny_kernel<4>, grid, block, 0, st, c));
+    }
 }
 
 // The arg max form for up to 32 activation rows: best_v / best_i [*parts][J]

@@ -270,10 +270,14 @@ __global__ void __launch_bounds__(256) lstm_cell_kernel(CellArgs a) {
 // cell kernel above would stream both matrices once per four sequences, so the two products run as GEMMs over the B
 // rows (one pass over each matrix whatever B is) into fp32 gate terms, and this kernel applies bias and gate math:
 // a thread per (sequence, hidden unit), the unit's four gate terms one 16-byte load from each product.
-// From kCellRowsMinB sequences on, both products and the gate math are one tcgen05 kernel (gemm_rows.cu): the gate terms
-// never leave the chip (512 sequences, 2048 inputs, H = 1024: 27.6 us as two products and this kernel, 15.4 us as one).
+// Where the shape allows, both products and the gate math are one kernel instead, on mma.sync up to 32 sequences
+// (gemm_skinny.cu) and on tcgen05 above (gemm_rows.cu): the gate terms never leave the chip (512 sequences, 2048 inputs,
+// H = 1024: 27.6 us as two products and this kernel, 15.4 us as one).
 constexpr int kCellGemmMinB = 8;
 constexpr int kCellRowsMinB = 33;
+static int launch_cell(const RowsCell& c, cudaStream_t st) {
+    return c.J < kCellRowsMinB ? launch_lstm_cell_skinny(c, st) : launch_gemm_rows_cell(c, st);
+}
 struct CellPointArgs {
     const float* Gx;     // [B, 4H]  W_ih x, packed gate order (unit-major)
     const float* Gh;     // [B, 4H]  W_hh h0, or NULL when h0 is zero
@@ -2731,10 +2735,10 @@ static int lstm_forward_impl(pimb200_lstm* h, const __half* x, const SeqLayout& 
                 a.hn = hn ? hn + (size_t)ld * B * H : nullptr;
                 a.cn = cn ? cn + (size_t)ld * B * H : nullptr;
                 a.I = in_size(h, l); a.H = H; a.B = B;
-                if (cell_gemm && B >= kCellRowsMinB) {
+                if (cell_gemm) {
                     const RowsCell rc_args{a.Wih, a.Whh, a.bias, a.x, a.x_bstride, a.h0, a.c0, a.y, a.y_bstride, a.hn, a.cn,
                                            nullptr, 0, a.I, H, B};
-                    rc = launch_gemm_rows_cell(rc_args, st);
+                    rc = launch_cell(rc_args, st);
                     if (rc == PIMB200_OK) continue;
                     if (rc != PIMB200_ERR_UNSUPPORTED) return rc;
                 }
@@ -2840,11 +2844,11 @@ extern "C" int pimb200_lstm_forward_step(pimb200_lstm* h, const void* x, long x_
     std::lock_guard<std::mutex> lk(h->mu);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int rc;
-    if (B >= kCellRowsMinB) {
+    {
         const RowsCell cell{h->w_ih[0], h->w_hh[0], h->bias[0], static_cast<const __half*>(x), x_ld, static_cast<const __half*>(h0),
                             static_cast<const __half*>(c0), static_cast<__half*>(y), y_ld, static_cast<__half*>(hn),
                             static_cast<__half*>(cn), static_cast<const __half*>(residual), residual_ld, I, H, B};
-        rc = launch_gemm_rows_cell(cell, st);
+        rc = launch_cell(cell, st);
         if (rc != PIMB200_ERR_UNSUPPORTED) return rc;
     }
     if ((rc = grow(&h->G, &h->G_cap, (size_t)2 * B * 4 * H)) != PIMB200_OK) return rc;
