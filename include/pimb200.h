@@ -218,6 +218,17 @@ int pimb200_attention_block(const void* q, const void* k, const void* v, const l
                             long max_len, int heads, int head_dim, long row_stride, long seq_stride, long out_row_stride,
                             long out_seq_stride, float scale, void* stream);
 
+/* The two forms above over packed rows: sequence j's rows are rows row0[j] .. row0[j] + L_j - 1 (int64 in DEVICE memory) of
+ * K and V (in the block form of q and out too), all sequences' rows one after the other without padding; the sequence
+ * strides are not used. */
+int pimb200_attention_rows_packed(const void* q, const void* K, const void* V, const long long* row0, const long long* len_dev,
+                                  long len_inc, long len_add, long max_len, void* out, int n_seq, int heads, int head_dim,
+                                  long kv_stride, long seq_stride, long q_stride, long out_stride, float scale, void* stream);
+int pimb200_attention_block_packed(const void* q, const void* k, const void* v, const long long* lengths,
+                                   const long long* row0, void* out, int n_seq, long max_len, int heads, int head_dim,
+                                   long row_stride, long seq_stride, long out_row_stride, long out_seq_stride, float scale,
+                                   void* stream);
+
 /* y = layer_norm(x + r) over the last dimension (gamma / beta optional): the residual add and the normalisation that
  * follow every Transformer sub-layer, two interpreter nodes in the reference (executeAtenAdd aten_ops_executor.cpp:110-166,
  * executeAtenLayerNorm).  cols * 4 bytes of shared memory per row. */
@@ -237,6 +248,13 @@ int pimb200_add_layer_norm_rows(const void* x, const void* r, const void* gamma,
 int pimb200_additive_attention(const void* q, const void* keys_proj, const void* values, const long long* lengths,
                                const void* v, const void* bias, void* ctx, float* scores, int n_seq, long max_len, int H,
                                long row_stride, long seq_stride, long ctx_stride, void* stream);
+
+/* The same with the context written `copies` times, copy_stride elements apart: straight into the concatenated input of
+ * every decoder cell that takes it.  Rows without 16-byte alignment return PIMB200_ERR_UNSUPPORTED for copies > 1. */
+int pimb200_additive_attention_copies(const void* q, const void* keys_proj, const void* values, const long long* lengths,
+                                      const void* v, const void* bias, void* ctx, float* scores, int n_seq, long max_len, int H,
+                                      long row_stride, long seq_stride, long ctx_stride, int copies, long copy_stride,
+                                      void* stream);
 
 /* The end of a greedy decode step for J streams in lock step: idx[j] = arg max over n of fp16(W[n,:] . X[j,:] + bias[n])
  * (lowest index among equal maxima; int64 in DEVICE memory), and, when emb is given, the next step's input

@@ -52,9 +52,15 @@ SIGNATURES = {
                                     C.c_long, C.c_long, C.c_float, _vp]),
     "pimb200_attention_block": (_i, [_vp, _vp, _vp, _vp, _vp, _i, C.c_long, _i, _i, C.c_long, C.c_long, C.c_long, C.c_long,
                                      C.c_float, _vp]),
+    "pimb200_attention_rows_packed": (_i, [_vp, _vp, _vp, _vp, _vp, C.c_long, C.c_long, C.c_long, _vp, _i, _i, _i, C.c_long,
+                                           C.c_long, C.c_long, C.c_long, C.c_float, _vp]),
+    "pimb200_attention_block_packed": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, C.c_long, _i, _i, C.c_long, C.c_long, C.c_long,
+                                            C.c_long, C.c_float, _vp]),
     "pimb200_add_layer_norm_rows": (_i, [_vp, _vp, _vp, _vp, _vp, C.c_long, C.c_long, C.c_float, _vp]),
     "pimb200_additive_attention": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, C.c_long, _i, C.c_long, C.c_long,
                                         C.c_long, _vp]),
+    "pimb200_additive_attention_copies": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, C.c_long, _i, C.c_long, C.c_long,
+                                               C.c_long, _i, C.c_long, _vp]),
     "pimb200_gather_rows": (_i, [_vp, _vp, _vp, C.c_long, _sz, C.c_long, _vp]),
     "pimb200_scatter_rows": (_i, [_vp, _vp, _vp, C.c_long, _sz, C.c_long, _vp]),
     "pimb200_greedy_token_workspace": (_sz, [_i, _i]),

@@ -71,7 +71,7 @@ __device__ __forceinline__ void decode_chunk(DecodeState& st, const float* qf, c
 
 template <int HD, int CL>
 __global__ void __launch_bounds__(128) attention_decode_kernel(const __half* __restrict__ q, const __half* __restrict__ K,
-                                                               const __half* __restrict__ V, const long long* len_dev,
+                                                               const __half* __restrict__ V, const long long* row0, const long long* len_dev,
                                                                long len_inc, long len_add, long max_len, __half* __restrict__ out,
                                                                int heads, int n_seq, long kv_stride, long seq_stride, long q_stride,
                                                                long out_stride, float scale) {
@@ -85,8 +85,8 @@ __global__ void __launch_bounds__(128) attention_decode_kernel(const __half* __r
     const int h = (int)(task % heads), seq = (int)(task / heads);
     long L = (len_dev ? (long)len_dev[(size_t)seq * len_inc] : 0) + len_add;
     L = L < 0 ? 0 : (L > max_len ? max_len : L);
-    const __half* Ks = K + (size_t)seq * seq_stride + (size_t)h * HD + sub * 8;
-    const __half* Vs = V + (size_t)seq * seq_stride + (size_t)h * HD + sub * 8;
+    const size_t at0 = (row0 ? (size_t)row0[seq] * kv_stride : (size_t)seq * seq_stride) + (size_t)h * HD + sub * 8;
+    const __half *Ks = K + at0, *Vs = V + at0;
     float qf[8];
     DecodeState ds;
     ds.m = -CUDART_INF_F;
@@ -157,7 +157,8 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
 template <int HD, int KT>   // KT: tiles of 16 positions
 __global__ void __launch_bounds__(kBlockWarps * 32) attention_block_mma_kernel(
     const __half* __restrict__ Q, const __half* __restrict__ K, const __half* __restrict__ V, const long long* __restrict__ lengths,
-    __half* __restrict__ out, long max_len, long row_stride, long seq_stride, long out_row_stride, long out_seq_stride, float scale) {
+    const long long* __restrict__ row0, __half* __restrict__ out, long max_len, long row_stride, long seq_stride, long out_row_stride,
+    long out_seq_stride, float scale) {
     constexpr int PITCH = HD * 2 + 16;                  // bytes per shared row
     constexpr int CPR = HD / 8;                         // 16-byte chunks per row
     extern __shared__ __align__(16) unsigned char smem[];
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(kBlockWarps * 32) attention_block_mma_kernel(
     long Ll = lengths ? (long)lengths[seq] : max_len;
     const int L = (int)(Ll < 0 ? 0 : (Ll > max_len ? max_len : Ll));
     const int tiles = (L + 15) >> 4, rows = tiles * 16;
-    const size_t base = (size_t)seq * seq_stride + (size_t)h * HD;
+    const size_t base = (row0 ? (size_t)row0[seq] * row_stride : (size_t)seq * seq_stride) + (size_t)h * HD;
     unsigned char *sQ = smem, *sK = smem + (size_t)KT * 16 * PITCH, *sV = sK + (size_t)KT * 16 * PITCH;
     for (int i = threadIdx.x; i < rows * CPR; i += kBlockWarps * 32) {
         const int r = i / CPR, c = i % CPR;
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(kBlockWarps * 32) attention_block_mma_kernel(
         *reinterpret_cast<uint4*>(sV + r * PITCH + c * 16) = d;
     }
     __syncthreads();
-    __half* o = out + (size_t)seq * out_seq_stride + (size_t)h * HD;
+    __half* o = out + (row0 ? (size_t)row0[seq] * out_row_stride : (size_t)seq * out_seq_stride) + (size_t)h * HD;
     const uint32_t q0 = (uint32_t)__cvta_generic_to_shared(sQ), k0 = (uint32_t)__cvta_generic_to_shared(sK), v0 = (uint32_t)__cvta_generic_to_shared(sV);
     // ldmatrix rows of a lane: A and V take rows lane % 16 at column half lane / 16; K takes eight keys per matrix
     const uint32_t arow = (uint32_t)((lane & 15) * PITCH + (lane >> 4) * 16);
@@ -276,12 +277,13 @@ __global__ void __launch_bounds__(kBlockWarps * 32) attention_block_mma_kernel(
                 *reinterpret_cast<uint4*>(o + (size_t)(qt * 16 + r) * out_row_stride + c * 8) = *reinterpret_cast<const uint4*>(so + r * PITCH + c * 16);
         }
     }
+    if (row0) return;                                                                         // packed rows: there are none past the length
     for (long i = (long)L * CPR + threadIdx.x; i < max_len * CPR; i += kBlockWarps * 32)      // rows past the length
         *reinterpret_cast<uint4*>(o + (size_t)(i / CPR) * out_row_stride + (i % CPR) * 8) = make_uint4(0u, 0u, 0u, 0u);
 }
 
 template <int HD, int KT>
-int launch_block(const __half* q, const __half* k, const __half* v, const long long* lengths, __half* out, int n_seq, long max_len,
+int launch_block(const __half* q, const __half* k, const __half* v, const long long* lengths, const long long* row0, __half* out, int n_seq, long max_len,
                  int heads, long row_stride, long seq_stride, long out_row_stride, long out_seq_stride, float scale, cudaStream_t st) {
     constexpr size_t smem = (size_t)3 * KT * 16 * (HD * 2 + 16);
     static bool attr_set[64];                           // cudaFuncSetAttribute is per device
@@ -295,25 +297,25 @@ int launch_block(const __half* q, const __half* k, const __half* v, const long l
         }
     }
     return cuda_status(launch_pdl(attention_block_mma_kernel<HD, KT>, dim3(heads, n_seq), dim3(kBlockWarps * 32), smem, st, q, k, v,
-                                  lengths, out, max_len, row_stride, seq_stride, out_row_stride, out_seq_stride, scale));
+                                  lengths, row0, out, max_len, row_stride, seq_stride, out_row_stride, out_seq_stride, scale));
 }
 
 }  // namespace
 
-int launch_attention_block(const __half* q, const __half* k, const __half* v, const long long* lengths, __half* out, int n_seq,
+int launch_attention_block(const __half* q, const __half* k, const __half* v, const long long* lengths, const long long* row0, __half* out, int n_seq,
                            long max_len, int heads, int head_dim, long row_stride, long seq_stride, long out_row_stride,
                            long out_seq_stride, float scale, cudaStream_t st) {
     if ((head_dim != 64 && head_dim != 128) || max_len > 128 || row_stride % 8 || seq_stride % 8 || out_row_stride % 8 ||
         out_seq_stride % 8 || !aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(out))
         return PIMB200_ERR_UNSUPPORTED;
     auto run = [&](auto f) {
-        return f(q, k, v, lengths, out, n_seq, max_len, heads, row_stride, seq_stride, out_row_stride, out_seq_stride, scale, st);
+        return f(q, k, v, lengths, row0, out, n_seq, max_len, heads, row_stride, seq_stride, out_row_stride, out_seq_stride, scale, st);
     };
     if (head_dim == 64) return max_len <= 64 ? run(launch_block<64, 4>) : run(launch_block<64, 8>);
     return max_len <= 64 ? run(launch_block<128, 4>) : run(launch_block<128, 8>);
 }
 
-int launch_attention_decode(const __half* q, const __half* K, const __half* V, const long long* len_dev, long len_inc,
+int launch_attention_decode(const __half* q, const __half* K, const __half* V, const long long* row0, const long long* len_dev, long len_inc,
                             long len_add, long max_len, __half* out, int n_seq, int heads, int head_dim, long kv_stride,
                             long seq_stride, long q_stride, long out_stride, float scale, cudaStream_t st) {
     if ((head_dim != 64 && head_dim != 128) || kv_stride % 8 || seq_stride % 8 || q_stride % 8 || out_stride % 8 || !aligned16(q) ||
@@ -324,7 +326,7 @@ int launch_attention_decode(const __half* q, const __half* K, const __half* V, c
     const int warps = tasks <= 4 * kNumSmB200 ? 1 : 4;
     const dim3 grid((unsigned)((tasks + warps - 1) / warps)), block(warps * 32);
     auto run = [&](auto kernel) {
-        return cuda_status(launch_pdl(kernel, grid, block, 0, st, q, K, V, len_dev, len_inc, len_add, max_len, out, heads, n_seq, kv_stride,
+        return cuda_status(launch_pdl(kernel, grid, block, 0, st, q, K, V, row0, len_dev, len_inc, len_add, max_len, out, heads, n_seq, kv_stride,
                                       seq_stride, q_stride, out_stride, scale));
     };
     // the longest attended length that the host knows of decides how many rows a warp has in flight (and its registers)

@@ -301,7 +301,8 @@ __global__ void __launch_bounds__(kAttnThreads) attention_row_kernel(const __hal
 // Batched form of attention_row_kernel: blockIdx.y is the sequence; every sequence has its own cache (seq_stride
 // elements after the previous one) and its own length (len_dev[seq * len_inc]).
 __global__ void __launch_bounds__(kAttnThreads) attention_rows_kernel(const __half* __restrict__ q, const __half* __restrict__ K,
-                                                                      const __half* __restrict__ V, const long long* len_dev,
+                                                                      const __half* __restrict__ V, const long long* row0,
+                                                                      const long long* len_dev,
                                                                       long len_inc, long len_add, long max_len,
                                                                       __half* __restrict__ out, int hd, long kv_stride,
                                                                       long seq_stride, long q_stride, long out_stride,
@@ -314,8 +315,8 @@ __global__ void __launch_bounds__(kAttnThreads) attention_rows_kernel(const __ha
     L = L < 0 ? 0 : (L > max_len ? max_len : L);
     (void)heads;
     const __half* qh = q + (size_t)seq * q_stride + (size_t)h * hd;
-    const __half* Ks = K + (size_t)seq * seq_stride + (size_t)h * hd;
-    const __half* Vs = V + (size_t)seq * seq_stride + (size_t)h * hd;
+    const size_t at0 = (row0 ? (size_t)row0[seq] * kv_stride : (size_t)seq * seq_stride) + (size_t)h * hd;
+    const __half *Ks = K + at0, *Vs = V + at0;
     for (long t = warp; t < L; t += kAttnThreads / 32) {
         const __half* kr = Ks + (size_t)t * kv_stride;
         float a = 0.f;
@@ -456,6 +457,140 @@ __global__ void __launch_bounds__(kAddAttnSlice / 2) additive_context_kernel(
     }
 }
 
+// Both halves in one launch for rows of 16-byte pieces: a cluster of C CTAs per sentence.  The CTAs share the source
+// positions for the scores (a warp per position), exchange the scores through distributed shared memory, and share the
+// columns of H for the context.  Keys and values are read once each; MUFU bounds the scores, so four tanh share one
+// reciprocal: tanh(x) = 1 - 2 / (1 + e^2x), and with d = 1 + e^2x the four quotients v / d come from 1 / (d0 d1 d2 d3)
+// (2x is capped at 20, where tanh is 1 in fp32, so the product stays finite): 1.25 MUFU per element instead of 2.
+// The first rows of values are loaded before the scores are known.  512 sentences (one CTA each): 22 + 13 us as two
+// launches; few sentences take up to eight CTAs each.
+constexpr int kBahdanauThreads = 256;
+constexpr int kBahdanauAhead = 8;        // value rows in flight per thread
+
+__device__ __forceinline__ float ex2_(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+template <int C>
+__global__ void __launch_bounds__(kBahdanauThreads) bahdanau_kernel(
+    const __half* __restrict__ q, const __half* __restrict__ keys_proj, const __half* __restrict__ values,
+    const long long* __restrict__ lengths, const __half* __restrict__ v, const __half* __restrict__ bias, __half* __restrict__ ctx,
+    float* __restrict__ scores, long max_len, int H, long row_stride, long seq_stride, long ctx_stride, int copies, long copy_stride) {
+    constexpr int WARPS = kBahdanauThreads / 32;
+    constexpr float kScale = 2.885390082f;                  // 2 / ln 2: e^2x = 2^(kScale x)
+    extern __shared__ float bsm[];
+    float* qb = bsm;                                        // [H] kScale * (q + bias)
+    float* vs = qb + H;                                     // [H]
+    float* red = vs + H;                                    // [8 * threads] partial contexts
+    float* sc = red + 8 * kBahdanauThreads;                 // [max_len] scores of the sentence, then weights
+    __shared__ float vsum[WARPS];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int rank = blockIdx.x, seq = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    long Ll = lengths ? (long)lengths[seq] : max_len;
+    const int L = (int)(Ll < 0 ? 0 : (Ll > max_len ? max_len : Ll));
+    const int n8 = H >> 3, nch = n8 / C, groups = kBahdanauThreads / nch;   // 16-byte pieces per row, of this CTA, rows side by side
+    const int ch = tid % nch, grp = tid / nch;
+    const __half* vals = values + (size_t)seq * seq_stride + (size_t)(rank * nch + ch) * 8;
+    uint4 va[kBahdanauAhead];
+#pragma unroll
+    for (int i = 0; i < kBahdanauAhead; ++i) {
+        const int s = grp + i * groups;
+        va[i] = s < L ? __ldg(reinterpret_cast<const uint4*>(vals + (size_t)s * row_stride)) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    float my_v = 0.f;
+    for (int h = tid; h < H; h += kBahdanauThreads) {
+        qb[h] = kScale * (__half2float(q[(size_t)seq * H + h]) + (bias ? __half2float(bias[h]) : 0.f));
+        const float f = __half2float(v[h]);
+        vs[h] = f;
+        my_v += f;
+    }
+    my_v = warp_sum(my_v);
+    if (lane == 0) vsum[warp] = my_v;
+    __syncthreads();
+    float vtot = 0.f;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) vtot += vsum[w];
+    // ---- scores: warp w of CTA r takes positions r + C * (w + 8 i) ----
+    for (int s = rank + C * warp; s < L; s += C * WARPS) {
+        const uint4* kr = reinterpret_cast<const uint4*>(keys_proj + (size_t)seq * seq_stride + (size_t)s * row_stride);
+        float a = 0.f;
+#pragma unroll 4
+        for (int c = lane; c < n8; c += 32) {
+            float k[8];
+            widen8(__ldg(kr + c), k);
+#pragma unroll
+            for (int o = 0; o < 8; o += 4) {
+                const float4 b = *reinterpret_cast<const float4*>(qb + c * 8 + o), w = *reinterpret_cast<const float4*>(vs + c * 8 + o);
+                const float d0 = 1.f + ex2_(fminf(fmaf(k[o], kScale, b.x), 28.85390082f)), d1 = 1.f + ex2_(fminf(fmaf(k[o + 1], kScale, b.y), 28.85390082f)),
+                            d2 = 1.f + ex2_(fminf(fmaf(k[o + 2], kScale, b.z), 28.85390082f)), d3 = 1.f + ex2_(fminf(fmaf(k[o + 3], kScale, b.w), 28.85390082f));
+                const float p01 = d0 * d1, p23 = d2 * d3;
+                const float n01 = fmaf(w.x, d1, w.y * d0), n23 = fmaf(w.z, d3, w.w * d2);
+                a = fmaf(fmaf(n01, p23, n23 * p01), rcp_approx(p01 * p23), a);
+            }
+        }
+        a = vtot - 2.f * warp_sum(a);
+        if (lane == 0) scores[(size_t)seq * max_len + s] = a;
+        if (C == 1) {
+            if (lane == 0) sc[s] = a;
+        } else if (lane < C) {
+            uint32_t dst;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"((uint32_t)__cvta_generic_to_shared(sc + s)), "r"(lane));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(a) : "memory");
+        }
+    }
+    if (C == 1) __syncthreads();
+    else {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+    // ---- softmax: every warp on its own, then the weights once ----
+    float m = -CUDART_INF_F;
+    for (int s = lane; s < L; s += 32) m = fmaxf(m, sc[s]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    float sum = 0.f;
+    for (int s = lane; s < L; s += 32) sum += expf(sc[s] - m);
+    sum = warp_sum(sum);
+    const float inv = L > 0 ? 1.0f / sum : 0.f;
+    // ---- context: this CTA's columns ----
+    float acc[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+    for (int s0 = grp; s0 < L; s0 += groups * kBahdanauAhead) {
+#pragma unroll
+        for (int i = 0; i < kBahdanauAhead; ++i) {
+            const int s = s0 + i * groups;
+            const float p = s < L ? expf(sc[s] - m) : 0.f;
+            float f[8];
+            widen8(va[i], f);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[e] = fmaf(p, f[e], acc[e]);
+        }
+#pragma unroll
+        for (int i = 0; i < kBahdanauAhead; ++i) {
+            const int s = s0 + (i + kBahdanauAhead) * groups;
+            if (s < L) va[i] = __ldg(reinterpret_cast<const uint4*>(vals + (size_t)s * row_stride));
+        }
+    }
+    if (groups > 1) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) red[e * kBahdanauThreads + tid] = acc[e];
+        __syncthreads();
+        if (grp > 0) return;
+        for (int g2 = 1; g2 < groups; ++g2)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[e] += red[e * kBahdanauThreads + g2 * nch + ch];
+    }
+    __half2 o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[e] = __floats2half2_rn(acc[2 * e] * inv, acc[2 * e + 1] * inv);
+    __half* dst = ctx + (size_t)seq * ctx_stride + (size_t)(rank * nch + ch) * 8;
+    for (int i = 0; i < copies; ++i) *reinterpret_cast<uint4*>(dst + i * copy_stride) = *reinterpret_cast<uint4*>(o);
+}
+
 // y = layer_norm(x + r) per row: the residual connection and the normalisation behind every Transformer sub-layer in one
 // pass (the sum lives in shared memory as fp32; each thread re-reads only the entries it wrote).
 template <int T>
@@ -551,8 +686,8 @@ constexpr int kBlockAttnThreads = 128;
 
 __global__ void __launch_bounds__(kBlockAttnThreads) attention_block_kernel(
     const __half* __restrict__ Q, const __half* __restrict__ K, const __half* __restrict__ V,
-    const long long* __restrict__ lengths, __half* __restrict__ out, long max_len, int hd, long row_stride, long seq_stride,
-    long out_row_stride, long out_seq_stride, float scale) {
+    const long long* __restrict__ lengths, const long long* __restrict__ row0, __half* __restrict__ out, long max_len, int hd,
+    long row_stride, long seq_stride, long out_row_stride, long out_seq_stride, float scale) {
     extern __shared__ __align__(16) unsigned char blk_smem[];
     const int h = blockIdx.x, seq = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kp = hd + 2;                                   // padded key row (halves): lanes on different rows, different banks
@@ -562,7 +697,9 @@ __global__ void __launch_bounds__(kBlockAttnThreads) attention_block_kernel(
     float* ps = qs + (kBlockAttnThreads / 32) * hd;           // [warps][max_len]
     long L = lengths ? (long)lengths[seq] : max_len;
     L = L < 0 ? 0 : (L > max_len ? max_len : L);
-    const size_t base = (size_t)seq * seq_stride + (size_t)h * hd;
+    const size_t base = (row0 ? (size_t)row0[seq] * row_stride : (size_t)seq * seq_stride) + (size_t)h * hd;
+    const size_t out0 = (row0 ? (size_t)row0[seq] * out_row_stride : (size_t)seq * out_seq_stride) + (size_t)h * hd;
+    const long n_rows = row0 ? L : max_len;                   // packed rows: there are none past the length
     for (long i = threadIdx.x; i < L * hd; i += kBlockAttnThreads) {
         const long s_ = i / hd;
         const int c = (int)(i % hd);
@@ -572,8 +709,8 @@ __global__ void __launch_bounds__(kBlockAttnThreads) attention_block_kernel(
     __syncthreads();
     float* qw = qs + warp * hd;
     float* pw = ps + (size_t)warp * max_len;
-    for (long qi = warp; qi < max_len; qi += kBlockAttnThreads / 32) {
-        __half* o = out + (size_t)seq * out_seq_stride + (size_t)qi * out_row_stride + (size_t)h * hd;
+    for (long qi = warp; qi < n_rows; qi += kBlockAttnThreads / 32) {
+        __half* o = out + out0 + (size_t)qi * out_row_stride;
         if (qi >= L) {
             for (int c = lane; c < hd; c += 32) o[c] = __float2half_rn(0.f);
             continue;
@@ -732,6 +869,14 @@ extern "C" int pimb200_attention_rows(const void* q, const void* K, const void* 
                                       long len_add, long max_len, void* out, int n_seq, int heads, int head_dim,
                                       long kv_stride, long seq_stride, long q_stride, long out_stride, float scale,
                                       void* stream) {
+    return pimb200_attention_rows_packed(q, K, V, nullptr, len_dev, len_inc, len_add, max_len, out, n_seq, heads, head_dim, kv_stride,
+                                         seq_stride, q_stride, out_stride, scale, stream);
+}
+
+extern "C" int pimb200_attention_rows_packed(const void* q, const void* K, const void* V, const long long* row0, const long long* len_dev,
+                                             long len_inc, long len_add, long max_len, void* out, int n_seq, int heads,
+                                             int head_dim, long kv_stride, long seq_stride, long q_stride, long out_stride,
+                                             float scale, void* stream) {
     if (n_seq == 0) return PIMB200_OK;
     if (!q || !K || !V || !out || n_seq < 0 || n_seq > 65535 || heads <= 0 || head_dim <= 0 || max_len <= 0 ||
         kv_stride < (long)heads * head_dim || seq_stride < 0 || len_inc < 0 || q_stride < (long)heads * head_dim ||
@@ -739,27 +884,62 @@ extern "C" int pimb200_attention_rows(const void* q, const void* K, const void* 
         return PIMB200_ERR_BAD_ARG;
     if (max_len > kAttnMaxLen || head_dim > 1024) return PIMB200_ERR_UNSUPPORTED;
     const int rc = launch_attention_decode(static_cast<const __half*>(q), static_cast<const __half*>(K), static_cast<const __half*>(V),
-                                           len_dev, len_inc, len_add, max_len, static_cast<__half*>(out), n_seq, heads, head_dim,
-                                           kv_stride, seq_stride, q_stride, out_stride, scale, static_cast<cudaStream_t>(stream));
+                                           row0, len_dev, len_inc, len_add, max_len, static_cast<__half*>(out), n_seq, heads,
+                                           head_dim, kv_stride, seq_stride, q_stride, out_stride, scale, static_cast<cudaStream_t>(stream));
     if (rc != PIMB200_ERR_UNSUPPORTED) return rc;
     const size_t smem = ((size_t)max_len + (size_t)(kAttnThreads / 32) * head_dim) * sizeof(float);
     if (smem + 16 > 48 * 1024) return PIMB200_ERR_UNSUPPORTED;
     attention_rows_kernel<<<dim3((unsigned)heads, (unsigned)n_seq), kAttnThreads, smem, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __half*>(q), static_cast<const __half*>(K), static_cast<const __half*>(V), len_dev, len_inc, len_add,
+        static_cast<const __half*>(q), static_cast<const __half*>(K), static_cast<const __half*>(V), row0, len_dev, len_inc, len_add,
         max_len, static_cast<__half*>(out), head_dim, kv_stride, seq_stride, q_stride, out_stride, scale);
     return launch_status();
 }
+
+namespace {
+template <int C>
+int launch_bahdanau(const __half* q, const __half* kp, const __half* values, const long long* lengths, const __half* v, const __half* bias,
+                    __half* ctx, float* scores, int n_seq, long max_len, int H, long row_stride, long seq_stride, long ctx_stride, int copies,
+                    long copy_stride, cudaStream_t st) {
+    const size_t smem = ((size_t)2 * H + 8 * kBahdanauThreads + max_len) * sizeof(float);
+    return cuda_status(launch_pdl<C>(bahdanau_kernel<C>, dim3(C, n_seq), dim3(kBahdanauThreads), smem, st, q, kp, values, lengths, v, bias, ctx,
+                                     scores, max_len, H, row_stride, seq_stride, ctx_stride, copies, copy_stride));
+}
+}  // namespace
 
 extern "C" int pimb200_additive_attention(const void* q, const void* keys_proj, const void* values, const long long* lengths,
                                           const void* v, const void* bias, void* ctx, float* scores, int n_seq,
                                           long max_len, int H, long row_stride, long seq_stride, long ctx_stride,
                                           void* stream) {
+    return pimb200_additive_attention_copies(q, keys_proj, values, lengths, v, bias, ctx, scores, n_seq, max_len, H, row_stride, seq_stride,
+                                             ctx_stride, 1, 0, stream);
+}
+
+extern "C" int pimb200_additive_attention_copies(const void* q, const void* keys_proj, const void* values, const long long* lengths,
+                                                 const void* v, const void* bias, void* ctx, float* scores, int n_seq, long max_len,
+                                                 int H, long row_stride, long seq_stride, long ctx_stride, int copies, long copy_stride,
+                                                 void* stream) {
     if (n_seq == 0) return PIMB200_OK;
+    if (copies < 1 || (copies > 1 && copy_stride < H)) return PIMB200_ERR_BAD_ARG;
     if (!q || !keys_proj || !values || !v || !ctx || !scores || n_seq < 0 || n_seq > 65535 || max_len <= 0 || H <= 0 ||
         row_stride < H || seq_stride < 0 || ctx_stride < H)
         return PIMB200_ERR_BAD_ARG;
     if ((size_t)max_len * sizeof(float) + 64 > 48 * 1024) return PIMB200_ERR_UNSUPPORTED;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (H % 8 == 0 && row_stride % 8 == 0 && seq_stride % 8 == 0 && ctx_stride % 8 == 0 && copy_stride % 8 == 0 && aligned16(keys_proj) &&
+        aligned16(values) && aligned16(ctx) && ((size_t)2 * H + 8 * kBahdanauThreads + max_len) * sizeof(float) + 64 <= 48 * 1024) {
+        // CTAs per sentence: as many as keep the grid within two CTAs per SM, if the pieces of a row split evenly
+        auto run = [&](auto f) {
+            return f(static_cast<const __half*>(q), static_cast<const __half*>(keys_proj), static_cast<const __half*>(values), lengths,
+                     static_cast<const __half*>(v), static_cast<const __half*>(bias), static_cast<__half*>(ctx), scores, n_seq, max_len, H,
+                     row_stride, seq_stride, ctx_stride, copies, copy_stride, st);
+        };
+        auto fits = [&](int c) { return (H / 8) % c == 0 && H / 8 / c <= kBahdanauThreads && kBahdanauThreads % (H / 8 / c) == 0; };
+        for (int c = 8; c >= 1; c /= 2) {
+            if (!fits(c) || (c > 1 && (long)n_seq * c > 2 * kNumSmB200)) continue;
+            return c == 8 ? run(launch_bahdanau<8>) : c == 4 ? run(launch_bahdanau<4>) : c == 2 ? run(launch_bahdanau<2>) : run(launch_bahdanau<1>);
+        }
+    }
+    if (copies > 1) return PIMB200_ERR_UNSUPPORTED;
     const long rows = (long)n_seq * max_len;
     const int rc = cuda_status(launch_pdl(
         additive_scores_kernel, dim3((unsigned)((rows + kAddAttnThreads / 32 - 1) / (kAddAttnThreads / 32))), dim3(kAddAttnThreads), 0, st,
@@ -797,19 +977,26 @@ extern "C" int pimb200_add_layer_norm_rows(const void* x, const void* r, const v
 extern "C" int pimb200_attention_block(const void* q, const void* k, const void* v, const long long* lengths, void* out,
                                        int n_seq, long max_len, int heads, int head_dim, long row_stride, long seq_stride,
                                        long out_row_stride, long out_seq_stride, float scale, void* stream) {
+    return pimb200_attention_block_packed(q, k, v, lengths, nullptr, out, n_seq, max_len, heads, head_dim, row_stride, seq_stride,
+                                          out_row_stride, out_seq_stride, scale, stream);
+}
+
+extern "C" int pimb200_attention_block_packed(const void* q, const void* k, const void* v, const long long* lengths, const long long* row0,
+                                              void* out, int n_seq, long max_len, int heads, int head_dim, long row_stride,
+                                              long seq_stride, long out_row_stride, long out_seq_stride, float scale, void* stream) {
     if (n_seq == 0) return PIMB200_OK;
     if (!q || !k || !v || !out || n_seq < 0 || n_seq > 65535 || heads <= 0 || head_dim <= 0 || max_len <= 0 ||
         row_stride < (long)heads * head_dim || out_row_stride < (long)heads * head_dim || seq_stride < 0 || out_seq_stride < 0)
         return PIMB200_ERR_BAD_ARG;
     const int rc = launch_attention_block(static_cast<const __half*>(q), static_cast<const __half*>(k), static_cast<const __half*>(v),
-                                          lengths, static_cast<__half*>(out), n_seq, max_len, heads, head_dim, row_stride,
+                                          lengths, row0, static_cast<__half*>(out), n_seq, max_len, heads, head_dim, row_stride,
                                           seq_stride, out_row_stride, out_seq_stride, scale, static_cast<cudaStream_t>(stream));
     if (rc != PIMB200_ERR_UNSUPPORTED) return rc;
     const size_t smem = (size_t)max_len * (head_dim + 2) * 2 + (size_t)max_len * head_dim * 2 +
                         (size_t)(kBlockAttnThreads / 32) * (head_dim + max_len) * sizeof(float);
     if (smem > 48 * 1024 || head_dim % 2 != 0) return PIMB200_ERR_UNSUPPORTED;
     attention_block_kernel<<<dim3((unsigned)heads, (unsigned)n_seq), kBlockAttnThreads, smem, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __half*>(q), static_cast<const __half*>(k), static_cast<const __half*>(v), lengths,
+        static_cast<const __half*>(q), static_cast<const __half*>(k), static_cast<const __half*>(v), lengths, row0,
         static_cast<__half*>(out), max_len, head_dim, row_stride, seq_stride, out_row_stride, out_seq_stride, scale);
     return launch_status();
 }

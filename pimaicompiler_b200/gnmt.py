@@ -9,11 +9,11 @@ hundreds of them runs `group` sentences in lock step instead:
   * encoder: the group's sentences, sorted by length, go through each layer as packed batches of up to 128 sentences
     (aten::lstm's packed overload, which the library runs as a padded lock-step batch on the persistent weight-stationary
     recurrence, the backward direction of the first layer on the sentences reversed one by one);
-  * decoder: one step for the whole group is 4 x (two GEMMs over the group's rows + the gate kernel, which writes the
-    cell's output, for the last two cells with the residual added, straight into the next cell's concatenated input), one
-    attention launch (a CTA per sentence, own source length), the vocabulary projection as a GEMM (the 66 MB matrix is
-    read once per step for all sentences) and a row-wise arg max; two steps (state buffers alternate) are captured into
-    one CUDA graph and replayed, the chosen tokens staying on the device until the group is done.
+  * decoder: one step for the whole group is four cells (each one launch: both products and the gate math; the output, for
+    the last two with the residual added, goes straight into the next cell's concatenated input), the query projection, one
+    attention launch (which writes the context into the other halves of those inputs), and the vocabulary projection with
+    its arg max and the next token's embedding (two launches, no logits in memory).  All steps are captured into one CUDA
+    graph; the chosen tokens stay on the device until the group is done.
 
 `GnmtTranslator.translate` is the user call; `bench.py --workload c4` times it.
 """
@@ -21,6 +21,7 @@ from __future__ import annotations
 
 from typing import List, Optional, Sequence
 
+import numpy as np
 import torch
 
 from . import ops
@@ -33,29 +34,33 @@ def stage_groups(sentences: Sequence[torch.Tensor], G: int, enc_batch: int, max_
     timestep) and `dst`, the row t * G + j of the padded [S, G] buffer each packed row belongs to.  A ragged last group
     is filled with one-token dummies.  With `pin` the tensors that travel to the device are in pinned host memory."""
     keep = (lambda t: t.pin_memory()) if pin else (lambda t: t)
-    order = sorted(range(len(sentences)), key=lambda i: -int(sentences[i].shape[0]))
+    n = len(sentences)
+    lens = np.fromiter((s.shape[0] for s in sentences), np.int64, n)
+    if n and (lens.max() > max_len or lens.min() < 1):
+        raise ValueError("sentence length outside 1..max_len")
+    flat = torch.cat(list(sentences)).numpy() if n else np.zeros(0, np.int64)
+    start = np.cumsum(lens) - lens
+    order = np.argsort(-lens, kind="stable")
     groups = []
-    for g0 in range(0, len(order), G):
+    for g0 in range(0, n, G):
         idx = order[g0:g0 + G]
-        lens = [int(sentences[i].shape[0]) for i in idx]
-        if max(lens) > max_len or min(lens) < 1:
-            raise ValueError("sentence length outside 1..max_len")
-        lens_all = lens + [1] * (G - len(idx))
-        toks = [sentences[i] for i in idx] + [torch.full((1,), 4, dtype=torch.int64)] * (G - len(idx))
+        lens_all = np.ones(G, np.int64)
+        lens_all[:len(idx)] = lens[idx]
+        first = np.zeros(G, np.int64)                        # where a sentence's tokens begin in `flat`
+        first[:len(idx)] = start[idx]
         slices = []
         for j0 in range(0, G, enc_batch):
-            j1 = min(j0 + enc_batch, G)
-            sl_lens = lens_all[j0:j1]
-            nb, Ss = j1 - j0, sl_lens[0]
-            pad = torch.full((Ss, nb), 4, dtype=torch.int64)
-            for b in range(nb):
-                pad[:sl_lens[b], b] = toks[j0 + b]
-            steps_col = torch.arange(Ss, dtype=torch.int64).view(Ss, 1)
-            mask = steps_col < torch.tensor(sl_lens, dtype=torch.int64).view(1, nb)      # [t, b]: sentence b has a step t
-            dst = (steps_col * G + j0 + torch.arange(nb, dtype=torch.int64).view(1, nb))[mask]
-            slices.append({"ids": keep(pad[mask]), "dst": keep(dst), "batch_sizes": mask.sum(1)})
-        groups.append({"idx": idx, "S": max(lens_all), "lengths": keep(torch.tensor(lens_all, dtype=torch.int64)),
-                       "slices": slices})
+            sl_lens, nb = lens_all[j0:j0 + enc_batch], min(enc_batch, G - j0)
+            steps_col = np.arange(sl_lens[0])[:, None]
+            mask = steps_col < sl_lens                       # [t, b]: sentence b has a step t
+            at = (first[j0:j0 + enc_batch] + steps_col)[mask]
+            ids = flat[at]
+            if j0 + nb > len(idx):                           # one-token dummies
+                ids[(steps_col * 0 + np.arange(j0, j0 + nb))[mask] >= len(idx)] = 4
+            dst = (steps_col * G + np.arange(j0, j0 + nb))[mask]
+            slices.append({"ids": keep(torch.from_numpy(ids)), "dst": keep(torch.from_numpy(dst)),
+                           "batch_sizes": torch.from_numpy(mask.sum(1))})
+        groups.append({"idx": idx.tolist(), "S": int(lens_all[0]), "lengths": keep(torch.from_numpy(lens_all)), "slices": slices})
     return groups
 
 
@@ -83,20 +88,20 @@ class GnmtTranslator:
         self.enc_out = torch.zeros(S, G, H, **f16)
         self.keys_proj = torch.zeros(S, G, H, **f16)
         self.lengths = torch.ones(G, **i64)
-        # decoder step buffers (addresses fixed: the step is replayed from a CUDA graph)
-        self.tok = torch.zeros(G, **i64)
-        self.step_idx = torch.zeros(1, **i64)
+        # decoder step buffers (addresses fixed: the steps are replayed from a CUDA graph)
         self.x = torch.zeros(G, H, **f16)
         self.q = torch.zeros(G, H, **f16)
         self.scores = torch.zeros(G, S, dtype=torch.float32, device=self.dev)
         self.y = [torch.zeros(1, G, H, **f16) for _ in range(4)]
         self.r2 = torch.zeros(G, H, **f16)
         self.r3 = torch.zeros(G, H, **f16)
-        self.cat = [torch.zeros(G, 2 * H, **f16) for _ in range(3)]
-        self.logits = torch.zeros(G, V, **f16)
+        self.cats = torch.zeros(G, 3, 2 * H, **f16)                     # inputs [previous output | context] of the last three cells
+        self.cat = [self.cats[:, i] for i in range(3)]
         self.state = [[torch.zeros(1, G, H, **f16) for _ in range(8)] for _ in range(2)]   # h0..3, c0..3, two sets
-        self.toks_out = torch.zeros(cfg.max_steps, G, **i64)
-        self.forced = None
+        self.token_ws = ops.greedy_token_workspace(V, G, self.dev)
+        self.toks = torch.zeros(cfg.max_steps + 1, G, **i64)            # row 0: start tokens, row t+1: choice of step t
+        self.forced = torch.zeros(cfg.max_steps + 1, G, **i64)          # row t: token fed to step t
+        self.logits = None                                              # [G, V], where the arg max needs them in memory
         self.logits_out = None
         self._graphs = {}
         self.launches_per_step = 0
@@ -126,109 +131,89 @@ class GnmtTranslator:
         return Sg
 
     # ------------------------------------------------------------------------------------------------ decoder
-    def _step(self, src: List[torch.Tensor], dst: List[torch.Tensor]) -> int:
-        """One decode step of the whole group; state read from `src`, written to `dst`.  Returns its launch count."""
-        H, G, w = self.H, self.G, self.w
-        row = 2 * H * 2          # bytes per row of a concatenation buffer
-        half = H * 2
+    def _step(self, t: int, forced: bool, want_logits: bool) -> int:
+        """One decode step of the whole group.  Returns its launch count."""
+        H, G, w, cfg = self.H, self.G, self.w, self.cfg
+        src, dst = self.state[t & 1], self.state[1 - (t & 1)]
+        row, half = 3 * 2 * H * 2, H * 2        # bytes from row to row of a concatenated input, of half of it
         n = 0
         cat = self.cat
-        ops.gather_rows(w["emb_tgt"], self.tok, out=self.x); n += 1
+        if t == 0 or forced or want_logits or self.logits is not None:
+            ops.gather_rows(w["emb_tgt"], (self.forced if forced else self.toks)[t], out=self.x); n += 1
         # groups of 8 or more sentences: every cell writes its output (the last two with their residual added) straight
         # into the first half of the next cell's concatenated input, as the reference's labelled GNMT graph does
         fused = self.lstm["dec0"].forward_step(self.x, src[0][0], src[4][0], cat[0][:, :H], dst[0][0], dst[4][0])
-        if fused:
-            n += 3
-            y0 = cat[0][:, :H]
-        else:
-            self.lstm["dec0"].forward(self.x.view(1, G, H), src[0], src[4], out=(self.y[0], dst[0], dst[4])); n += 1
-            y0 = self.y[0].view(G, H)
-            ops.copy_2d(cat[0], 0, row, y0, 0, half, half, G); n += 1
+        n += 1
+        y0 = cat[0][:, :H]
+        if not fused:
+            self.lstm["dec0"].forward(self.x.view(1, G, H), src[0], src[4], out=(self.y[0], dst[0], dst[4]))
+            ops.copy_2d(self.cats, 0, row, self.y[0], 0, half, half, G); n += 1
         ops.gemm_wx(w["Wq"], y0, out=self.q); n += 1
         ops.additive_attention(self.q, self.keys_proj, self.enc_out, self.lengths, self.v_norm, w["att_b"],
-                               out=cat[0][:, H:], scores=self.scores); n += 2
-        for i in (1, 2):          # the context is the second half of every layer's input
-            ops.copy_2d(cat[i], half, row, cat[0], half, row, half, G); n += 1
+                               out=cat[0][:, H:], scores=self.scores, copies=3, copy_stride=2 * H); n += 1
         if fused:
-            self.lstm["dec1"].forward_step(cat[0], src[1][0], src[5][0], cat[1][:, :H], dst[1][0], dst[5][0]); n += 3
+            self.lstm["dec1"].forward_step(cat[0], src[1][0], src[5][0], cat[1][:, :H], dst[1][0], dst[5][0])
             self.lstm["dec2"].forward_step(cat[1], src[2][0], src[6][0], cat[2][:, :H], dst[2][0], dst[6][0],
-                                           residual=cat[1][:, :H]); n += 3
+                                           residual=cat[1][:, :H])
             self.lstm["dec3"].forward_step(cat[2], src[3][0], src[7][0], self.r3, dst[3][0], dst[7][0],
                                            residual=cat[2][:, :H]); n += 3
         else:
-            self.lstm["dec1"].forward(cat[0].view(1, G, 2 * H), src[1], src[5], out=(self.y[1], dst[1], dst[5])); n += 1
-            y1 = self.y[1].view(G, H)
-            ops.copy_2d(cat[1], 0, row, y1, 0, half, half, G); n += 1
-            self.lstm["dec2"].forward(cat[1].view(1, G, 2 * H), src[2], src[6], out=(self.y[2], dst[2], dst[6])); n += 1
-            ops.add_f16(self.y[2].view(G, H), y1, out=self.r2); n += 1
-            ops.copy_2d(cat[2], 0, row, self.r2, 0, half, half, G); n += 1
-            self.lstm["dec3"].forward(cat[2].view(1, G, 2 * H), src[3], src[7], out=(self.y[3], dst[3], dst[7])); n += 1
-            ops.add_f16(self.y[3].view(G, H), self.r2, out=self.r3); n += 1
-        ops.gemm_wx(w["Wc"], self.r3, w["bc"], out=self.logits); n += 1
-        ops.argmax(self.logits, out=self.tok); n += 1
-        # record the chosen tokens (and, for the parity tests, the logits) in row step_idx of the output tables
-        ops.scatter_rows(self.toks_out.view(self.cfg.max_steps, G), self.step_idx, self.tok.view(1, G)); n += 1
-        if self.logits_out is not None:
-            ops.scatter_rows(self.logits_out.view(self.logits_out.shape[0], -1), self.step_idx, self.logits.view(1, -1)); n += 1
-        if self.forced is not None:   # teacher forcing: the fed-back token comes from a table instead of the arg max
-            ops.gather_rows(self.forced, self.step_idx, out=self.tok.view(1, G)); n += 1
-        self.step_idx.add_(1)
-        return n
+            def cell(i):                         # of whole rows: the concatenated input is a slice
+                x = cat[i - 1].contiguous().view(1, G, 2 * H)
+                self.lstm[f"dec{i}"].forward(x, src[i], src[4 + i], out=(self.y[i], dst[i], dst[4 + i]))
+                return self.y[i].view(G, H)
+            y1 = cell(1)
+            ops.copy_2d(self.cats, 2 * half, row, y1, 0, half, half, G)
+            ops.add_f16(cell(2), y1, out=self.r2)
+            ops.copy_2d(self.cats, 4 * half, row, self.r2, 0, half, half, G)
+            ops.add_f16(cell(3), self.r2, out=self.r3); n += 10
+        if not want_logits and self.logits is None:
+            last = forced or t + 1 >= cfg.max_steps
+            if ops.greedy_token(w["Wc"], self.r3, w["bc"], self.token_ws, self.toks[t + 1], None if last else w["emb_tgt"], None,
+                                None if last else self.x):
+                return n + 2
+            self.logits = torch.zeros(G, self.V, dtype=torch.float16, device=self.dev)
+        lg = self.logits_out[t] if want_logits else self.logits
+        ops.gemm_wx(w["Wc"], self.r3, w["bc"], out=lg)
+        ops.argmax(lg, out=self.toks[t + 1])
+        return n + 2
 
-    def _graph(self, key):
-        """Two steps (state set 0 -> 1 -> 0) captured once per (forced, logits) mode."""
+    def _graph(self, steps: int, forced: bool, want_logits: bool):
+        """All steps, captured once per (steps, forced, logits) mode."""
+        key = (steps, forced, want_logits)
         if key in self._graphs:
             return self._graphs[key]
         side = torch.cuda.Stream(device=self.dev)
         side.wait_stream(torch.cuda.current_stream(self.dev))
         with torch.cuda.stream(side):          # warm-up outside capture: buffers of the LSTM handles grow here
-            self._step(self.state[0], self.state[1])
-            self._step(self.state[1], self.state[0])
+            self._step(0, forced, want_logits)
         torch.cuda.current_stream(self.dev).wait_stream(side)
         torch.cuda.synchronize(self.dev)
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
-            n = self._step(self.state[0], self.state[1])
-            self._step(self.state[1], self.state[0])
-        self.launches_per_step = n
+            for t in range(steps):
+                self.launches_per_step = self._step(t, forced, want_logits)
         self._graphs[key] = g
         return g
 
     def decode(self, steps: int, forced: Optional[torch.Tensor] = None, want_logits: bool = False):
-        """Greedy decode of the encoded group for `steps` steps (rounded up to an even count internally).  Returns the
-        token table [steps, G] (device, int64) and, when asked, the logits [steps, G, V]."""
+        """Greedy decode of the encoded group for `steps` steps (one graph launch).  Returns the token table [steps, G]
+        (device, int64) and, when asked, the logits [steps, G, V]."""
         cfg, G = self.cfg, self.G
-        steps2 = steps + (steps & 1)
-        if steps2 > cfg.max_steps + (cfg.max_steps & 1) or steps2 > self.toks_out.shape[0] + 1:
+        if steps > cfg.max_steps:
             raise ValueError("more steps than the configuration's maximum")
-        if self.toks_out.shape[0] < steps2:
-            self.toks_out = torch.zeros(steps2, G, dtype=torch.int64, device=self.dev)
-            self._graphs.clear()
+        if want_logits and (self.logits_out is None or self.logits_out.shape[0] < steps):
+            self.logits_out = torch.zeros(steps, G, self.V, dtype=torch.float16, device=self.dev)
+            self._graphs = {k: v for k, v in self._graphs.items() if not k[2]}
         if forced is not None:
-            f = torch.zeros(steps2, G, dtype=torch.int64, device=self.dev)
-            f[:steps] = forced.to(self.dev)
-            if self.forced is None or self.forced.shape != f.shape:
-                self.forced = f
-                self._graphs.clear()
-            else:
-                self.forced.copy_(f)
-        elif self.forced is not None:
-            self.forced = None
-            self._graphs.clear()
-        if want_logits and (self.logits_out is None or self.logits_out.shape[0] < steps2):
-            self.logits_out = torch.zeros(steps2, G, self.V, dtype=torch.float16, device=self.dev)
-            self._graphs.clear()
-        if not want_logits and self.logits_out is not None:
-            self.logits_out = None
-            self._graphs.clear()
-        g = self._graph((forced is not None, want_logits))
+            self.forced[0].fill_(cfg.bos)
+            self.forced[1:steps].copy_(forced[:steps - 1].to(self.dev))          # step t is fed the token forced at t - 1
+        g = self._graph(steps, forced is not None, want_logits)
         for s in self.state[0]:
             s.zero_()
-        self.tok.fill_(cfg.bos)
-        self.step_idx.zero_()
-        for _ in range(steps2 // 2):
-            g.replay()
-        toks = self.toks_out[:steps]
+        self.toks[0].fill_(cfg.bos)
+        g.replay()
+        toks = self.toks[1:steps + 1]
         return (toks, self.logits_out[:steps]) if want_logits else (toks, None)
 
     # ------------------------------------------------------------------------------------------------ user call
@@ -278,14 +263,15 @@ class GnmtTranslator:
                 for j, i in enumerate(idx):
                     f[:, j] = torch.tensor(list(forced[i])[:run_steps], dtype=torch.int64)
             toks, logits = self.run_group(self.to_device(group), run_steps, f, want_logits)
-            host = torch.empty(toks.shape, dtype=torch.int64).pin_memory()
+            host = torch.empty(toks.shape, dtype=torch.int64, pin_memory=True)
             host.copy_(toks, non_blocking=True)
             pending.append((idx, host, logits.float().cpu() if want_logits else None))
             torch.cuda.current_stream(self.dev).synchronize()   # the next group reuses the token table
             self.check_status()
         for idx, host, logits in pending:
+            rows = host.t().tolist()                        # [G][steps] in one call
             for j, i in enumerate(idx):
-                seq = host[:, j].tolist()
+                seq = rows[j]
                 if steps is None and cfg.eos in seq:
                     seq = seq[:seq.index(cfg.eos) + 1]
                 out_toks[i] = seq

@@ -295,6 +295,38 @@ def attention_block(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, heads: in
     return out
 
 
+def attention_rows_packed(q: torch.Tensor, K: torch.Tensor, V: torch.Tensor, heads: int, row0: torch.Tensor, lengths: torch.Tensor,
+                          max_len: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """attention_rows over packed keys and values [rows, heads*hd] (last dimension contiguous): sequence j's rows begin at
+    row0[j], lengths[j] of them (int64 on the device, at most max_len)."""
+    _req_half_cuda_rows(q, K, V)
+    n, d = q.shape
+    hd = d // heads
+    if K.stride() != V.stride():
+        raise ValueError("K and V must share their strides")
+    if out is None:
+        out = torch.empty(n, d, dtype=torch.float16, device=q.device)
+    check(_lib.lib().pimb200_attention_rows_packed(_ptr(q), _ptr(K), _ptr(V), _ptr(row0), _ptr(lengths), 1, 0, max_len, _ptr(out), n,
+                                                   heads, hd, K.stride(0), 0, q.stride(0), out.stride(0), 1.0 / math.sqrt(hd),
+                                                   _stream()), "attention_rows_packed")
+    return out
+
+
+def attention_block_packed(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, heads: int, row0: torch.Tensor, lengths: torch.Tensor,
+                           max_len: int) -> torch.Tensor:
+    """attention_block over packed rows: q, k, v [rows, heads*hd] views with equal strides."""
+    _req_half_cuda_rows(q, k, v)
+    rows, d = q.shape
+    hd = d // heads
+    if not (q.stride() == k.stride() == v.stride()):
+        raise ValueError("q, k, v must share their strides")
+    out = torch.empty(rows, d, dtype=torch.float16, device=q.device)
+    check(_lib.lib().pimb200_attention_block_packed(_ptr(q), _ptr(k), _ptr(v), _ptr(lengths), _ptr(row0), _ptr(out), lengths.numel(),
+                                                    max_len, heads, hd, q.stride(0), 0, out.stride(0), 0, 1.0 / math.sqrt(hd),
+                                                    _stream()), "attention_block_packed")
+    return out
+
+
 def add_layer_norm(x: torch.Tensor, r: torch.Tensor, gamma: Optional[torch.Tensor] = None, beta: Optional[torch.Tensor] = None,
                    eps: float = 1e-5, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """layer_norm(x + r) over the last dimension."""
@@ -309,9 +341,10 @@ def add_layer_norm(x: torch.Tensor, r: torch.Tensor, gamma: Optional[torch.Tenso
 
 def additive_attention(q: torch.Tensor, keys_proj: torch.Tensor, values: torch.Tensor, lengths: Optional[torch.Tensor],
                        v: torch.Tensor, bias: Optional[torch.Tensor], out: Optional[torch.Tensor] = None,
-                       scores: Optional[torch.Tensor] = None) -> torch.Tensor:
+                       scores: Optional[torch.Tensor] = None, copies: int = 1, copy_stride: int = 0) -> torch.Tensor:
     """Normalised Bahdanau attention for n sentences: q [n, H]; keys_proj / values time-major [S, n, H] (contiguous);
-    lengths int64 [n] on the device; v, bias [H].  `out` may be a column slice of a wider [n, *] buffer."""
+    lengths int64 [n] on the device; v, bias [H].  `out` may be a column slice of a wider [n, *] buffer; the context is
+    written `copies` times, copy_stride elements apart."""
     _req_half_cuda(q, v, bias)
     _req_half_cuda_rows(keys_proj, values)
     S, n, H = keys_proj.shape
@@ -319,9 +352,9 @@ def additive_attention(q: torch.Tensor, keys_proj: torch.Tensor, values: torch.T
         out = torch.empty(n, H, dtype=torch.float16, device=q.device)
     if scores is None:
         scores = torch.empty(n, S, dtype=torch.float32, device=q.device)
-    check(_lib.lib().pimb200_additive_attention(_ptr(q), _ptr(keys_proj), _ptr(values), _ptr(lengths), _ptr(v), _ptr(bias),
-                                                _ptr(out), _ptr(scores), n, S, H, keys_proj.stride(0), keys_proj.stride(1),
-                                                out.stride(0), _stream()), "additive_attention")
+    check(_lib.lib().pimb200_additive_attention_copies(
+        _ptr(q), _ptr(keys_proj), _ptr(values), _ptr(lengths), _ptr(v), _ptr(bias), _ptr(out), _ptr(scores), n, S, H,
+        keys_proj.stride(0), keys_proj.stride(1), out.stride(0), copies, copy_stride, _stream()), "additive_attention")
     return out
 
 

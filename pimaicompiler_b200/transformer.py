@@ -6,9 +6,10 @@ batch-1 addmm, each attention as matmul -> softmax -> matmul with per-head resha
 an at::cat (runtime/source/executor/op_executor/aten_ops_executor.cpp:181-216, 2488-2505, 3402-3436, 772-819).  Sequences
 are independent, so a GPU runs `group` of them in lock step:
 
-  * encoder: the group's sequences, sorted by length and padded, form one [group, S, d] batch; each layer is one fused
-    q/k/v projection GEMM, one attention launch (a CTA per head and sequence, own length), the output projection, the
-    feed-forward pair (ReLU fused into the first GEMM) and two fused residual-add + layer-norm launches;
+  * encoder: the tokens of the group's sequences, one sequence behind the other without padding, are the rows of every
+    product; each layer is one fused q/k/v projection GEMM, one attention launch (a CTA per head and sequence, own rows),
+    the output projection, the feed-forward pair (ReLU fused into the first GEMM) and two fused residual-add + layer-norm
+    launches;
   * the cross-attention keys and values of all decoder layers come from one GEMM over the encoder output;
   * decoder: all `steps` steps of the group are captured into ONE CUDA graph.  Step t's projection GEMM writes q, k, v
     straight into row t of every sequence's part of a [group, steps, 3d] cache (no append, no device-side position),
@@ -21,6 +22,7 @@ from __future__ import annotations
 
 from typing import List, Optional, Sequence
 
+import numpy as np
 import torch
 
 from . import ops
@@ -60,7 +62,8 @@ class TransformerTranslator:
         i64 = dict(dtype=torch.int64, device=self.dev)
         nl = cfg.layers
         self.lengths = torch.ones(G, **i64)
-        self.cross = torch.zeros(G, S, nl * 2 * d, **f16)            # encoder side, at its maximum size
+        self.row0 = torch.zeros(G, **i64)                            # first encoder row of every sequence
+        self.cross = torch.zeros(G * S, nl * 2 * d, **f16)           # encoder side, packed rows, at its maximum size
         self.cache = [torch.zeros(G, T, 3 * d, **f16) for _ in range(nl)]
         self.toks = torch.zeros(T + 1, G, **i64)                     # row 0: start tokens, row t+1: choice of step t
         self.forced = torch.zeros(T + 1, G, **i64)
@@ -73,23 +76,20 @@ class TransformerTranslator:
 
     # ------------------------------------------------------------------------------------------------ encoder
     def encode(self, group: dict) -> None:
-        """One staged group (see stage(); tensors on the device): `ids` [G, S_g] int64 (padded with any valid id) and
-        `lengths` [G] int64.  Fills the cross-attention keys / values of every decoder layer."""
-        cfg, d, G = self.cfg, self.d, self.G
-        ids = group["ids"]
-        Sg = ids.shape[1]
-        n = G * Sg
+        """One staged group (see stage(); tensors on the device).  Fills the cross-attention keys / values of every decoder
+        layer."""
+        cfg, d = self.cfg, self.d
+        n = group["ids"].numel()
         self.lengths.copy_(group["lengths"])
-        x = ops.gather_rows(self.emb_src, ids.reshape(-1))                       # [n, d]
-        x = ops.add_f16(x.view(G, Sg * d), self.pe[:Sg].reshape(1, Sg * d)).view(n, d)   # positions: one row per sequence
+        self.row0.copy_(group["row0"])
+        x = ops.add_f16(ops.gather_rows(self.emb_src, group["ids"]), ops.gather_rows(self.pe, group["pos"]))    # [n, d]
         for L in self.enc:
-            qkv = ops.gemm_wx(L["qkv"], x, L["qkv_b"]).view(G, Sg, 3 * d)
-            a = ops.attention_block(qkv[:, :, :d], qkv[:, :, d:2 * d], qkv[:, :, 2 * d:], cfg.heads, self.lengths)
-            x = ops.add_layer_norm(x, ops.gemm_wx(L["so"], a.view(n, d), L["so_b"]))
+            qkv = ops.gemm_wx(L["qkv"], x, L["qkv_b"])
+            a = ops.attention_block_packed(qkv[:, :d], qkv[:, d:2 * d], qkv[:, 2 * d:], cfg.heads, self.row0, self.lengths, group["S"])
+            x = ops.add_layer_norm(x, ops.gemm_wx(L["so"], a, L["so_b"]))
             f = ops.gemm_wx(L["f2"], ops.gemm_wx(L["f1"], x, L["f1_b"], ops.ACT_RELU), L["f2_b"])
             x = ops.add_layer_norm(x, f)
-        kv = ops.gemm_wx(self.ckv, x, self.ckv_b).view(G, Sg, -1)
-        self.cross[:, :Sg].copy_(kv)
+        ops.gemm_wx(self.ckv, x, self.ckv_b, out=self.cross[:n])
 
     # ------------------------------------------------------------------------------------------------ decoder
     def _step(self, t: int, forced: bool, want_logits: bool) -> int:
@@ -107,9 +107,9 @@ class TransformerTranslator:
                                    len_add=t + 1); n += 1
             x = ops.add_layer_norm(x, ops.gemm_wx(L["so"], a, L["so_b"])); n += 2
             cq = ops.gemm_wx(L["cq"], x, L["cq_b"]); n += 1
-            ck = self.cross[:, :, (2 * i) * d:(2 * i + 1) * d]
-            cv = self.cross[:, :, (2 * i + 1) * d:(2 * i + 2) * d]
-            ca = ops.attention_rows(cq, ck, cv, cfg.heads, len_dev=self.lengths, len_inc=1); n += 1
+            ck = self.cross[:, (2 * i) * d:(2 * i + 1) * d]
+            cv = self.cross[:, (2 * i + 1) * d:(2 * i + 2) * d]
+            ca = ops.attention_rows_packed(cq, ck, cv, cfg.heads, self.row0, self.lengths, cfg.max_len); n += 1
             x = ops.add_layer_norm(x, ops.gemm_wx(L["co"], ca, L["co_b"])); n += 2
             f = ops.gemm_wx(L["f2"], ops.gemm_wx(L["f1"], x, L["f1_b"], ops.ACT_RELU), L["f2_b"]); n += 2
             x = ops.add_layer_norm(x, f); n += 1
@@ -160,30 +160,33 @@ class TransformerTranslator:
 
     # ------------------------------------------------------------------------------------------------ user call
     def stage(self, sequences: Sequence[torch.Tensor]):
-        """Sorts by length and packs lock-step groups: dicts of `idx` (sequence indices), `ids` (padded [G, S_g]) and
-        `lengths` [G], the tensors in pinned host memory."""
-        G = self.G
-        order = sorted(range(len(sequences)), key=lambda i: -int(sequences[i].shape[0]))
+        """Packs lock-step groups, longest sequences first: dicts of `idx` (sequence indices), `S` (longest length) and, in
+        pinned host memory, `ids` and `pos` (token and position of every row, one sequence behind the other), `lengths` [G]
+        and `row0` [G] (first row of every sequence).  A ragged last group is filled with one-token dummies."""
+        G, n = self.G, len(sequences)
+        lens = np.fromiter((s.shape[0] for s in sequences), np.int64, n)
+        if n and (lens.max() > self.cfg.max_len or lens.min() < 1):
+            raise ValueError("sequence length outside 1..max_len")
+        order = np.argsort(-lens, kind="stable").tolist()
+        pin = lambda t: t.pin_memory()
+        dummy = torch.full((1,), 4, dtype=torch.int64)
         groups = []
-        for g0 in range(0, len(order), G):
+        for g0 in range(0, n, G):
             idx = order[g0:g0 + G]
-            lens = [int(sequences[i].shape[0]) for i in idx]
-            if max(lens) > self.cfg.max_len or min(lens) < 1:
-                raise ValueError("sequence length outside 1..max_len")
-            ids = torch.full((G, max(lens)), 4, dtype=torch.int64)
-            for j, i in enumerate(idx):
-                ids[j, :lens[j]] = sequences[i]
-            lens_t = torch.ones(G, dtype=torch.int64)
-            lens_t[:len(idx)] = torch.tensor(lens, dtype=torch.int64)
-            groups.append({"idx": idx, "ids": ids.pin_memory(), "lengths": lens_t.pin_memory()})
+            lens_g = np.ones(G, np.int64)
+            lens_g[:len(idx)] = lens[idx]
+            row0 = np.cumsum(lens_g) - lens_g
+            ids = torch.cat([sequences[i] for i in idx] + [dummy] * (G - len(idx)))
+            pos = np.arange(ids.numel()) - np.repeat(row0, lens_g)
+            groups.append({"idx": idx, "S": int(lens_g[0]), "ids": pin(ids), "pos": pin(torch.from_numpy(pos)),
+                           "lengths": pin(torch.from_numpy(lens_g)), "row0": pin(torch.from_numpy(row0))})
         return groups
 
     def to_device(self, group: dict) -> dict:
-        return {"idx": group["idx"], "ids": group["ids"].to(self.dev, non_blocking=True),
-                "lengths": group["lengths"].to(self.dev, non_blocking=True)}
+        return {k: v.to(self.dev, non_blocking=True) if isinstance(v, torch.Tensor) else v for k, v in group.items()}
 
     def h2d_bytes(self, group: dict) -> int:
-        return 8 * (group["ids"].numel() + group["lengths"].numel())
+        return 8 * sum(v.numel() for v in group.values() if isinstance(v, torch.Tensor))
 
     def check_status(self) -> None:
         """Raises if a bounded wait of the tensor-core GEMM gave up since the last check."""
@@ -211,14 +214,15 @@ class TransformerTranslator:
                 for j, i in enumerate(idx):
                     f[:, j] = torch.tensor(list(forced[i])[:run_steps], dtype=torch.int64)
             toks, logits = self.decode(run_steps, f, want_logits)
-            host = torch.empty(toks.shape, dtype=torch.int64).pin_memory()
+            host = torch.empty(toks.shape, dtype=torch.int64, pin_memory=True)
             host.copy_(toks, non_blocking=True)
             pending.append((idx, host, logits.float().cpu() if want_logits else None))
             torch.cuda.current_stream(self.dev).synchronize()   # the next group reuses the token table
             self.check_status()
         for idx, host, logits in pending:
+            rows = host.t().tolist()                        # [G][steps] in one call
             for j, i in enumerate(idx):
-                seq = host[:, j].tolist()
+                seq = rows[j]
                 if steps is None and cfg.eos in seq:
                     seq = seq[:seq.index(cfg.eos) + 1]
                 out_toks[i] = seq

@@ -12,6 +12,7 @@ import pytest
 import torch
 
 from oracle import c_oracle as co
+from tests.util import assert_close
 
 pytestmark = pytest.mark.gpu
 GOLD = os.path.join(os.path.dirname(__file__), "golden")
@@ -230,3 +231,44 @@ def test_greedy_token_matches_separate_ops(J, V, K, bias):
     if bias:
         assert idx.tolist() == [3] * J or not bool((ref[:, 3] > ref.max(1).values - 1e-9).all())
     assert torch.equal(x, ops.add_f16(ops.gather_rows(emb, idx), pos))
+
+
+@pytest.mark.parametrize("heads,hd,lens", [(8, 64, [64, 33, 32, 17, 1]), (2, 128, [128, 65, 9]), (3, 16, [9, 4, 1])])
+def test_packed_attention_matches_padded(heads, hd, lens):
+    # rows of all sequences one behind the other against the padded forms of the same sequences
+    from pimaicompiler_b200 import ops
+    g = torch.Generator().manual_seed(heads + hd)
+    n, S, d = len(lens), max(lens), heads * hd
+    qkv = torch.randn(sum(lens), 3 * d, generator=g).half().cuda()
+    ln = torch.tensor(lens, device="cuda")
+    row0 = torch.cumsum(ln, 0) - ln
+    pad = torch.zeros(n, S, 3 * d, dtype=torch.float16, device="cuda")
+    for j, L in enumerate(lens):
+        pad[j, :L] = qkv[int(row0[j]):int(row0[j]) + L]
+    q, k, v = (qkv[:, i * d:(i + 1) * d] for i in range(3))
+    got = ops.attention_block_packed(q, k, v, heads, row0, ln, S)
+    ref = ops.attention_block(*(pad[:, :, i * d:(i + 1) * d] for i in range(3)), heads, ln)
+    for j, L in enumerate(lens):
+        assert torch.equal(got[int(row0[j]):int(row0[j]) + L], ref[j, :L])
+    one = torch.randn(n, d, generator=g).half().cuda()
+    assert torch.equal(ops.attention_rows_packed(one, k, v, heads, row0, ln, S),
+                       ops.attention_rows(one, pad[:, :, d:2 * d], pad[:, :, 2 * d:], heads, len_dev=ln, len_inc=1))
+
+
+@pytest.mark.parametrize("n", [1, 20, 40, 80, 300])
+def test_additive_attention_copies(n):
+    # one to eight CTAs per sentence, the context written three times
+    from pimaicompiler_b200 import ops
+    g = torch.Generator().manual_seed(n)
+    S, H = 37, 1024
+    q, v, b = (torch.randn(*s, generator=g).half().cuda() for s in ((n, H), (H,), (H,)))
+    kp, val = (torch.randn(S, n, H, generator=g).half().cuda() for _ in range(2))
+    ln = torch.randint(1, S + 1, (n,), generator=g).cuda()
+    out = torch.zeros(n, 3, 2 * H, dtype=torch.float16, device="cuda")
+    ops.additive_attention(q, kp, val, ln, v * 0.05, b, out=out[:, 0, H:], copies=3, copy_stride=2 * H)
+    e = (torch.tanh(kp.float() + (q.float() + b.float())) * (v * 0.05).float()).sum(2)
+    e = e.masked_fill(torch.arange(S, device="cuda")[:, None] >= ln, float("-inf"))
+    ref = (torch.softmax(e, 0)[:, :, None] * val.float()).sum(0)
+    assert_close(out[:, 0, H:], ref, 2e-3, 2e-3, "context")
+    assert torch.equal(out[:, 1, H:], out[:, 0, H:]) and torch.equal(out[:, 2, H:], out[:, 0, H:])
+    assert float(out[:, :, :H].abs().max()) == 0.0
