@@ -33,6 +33,7 @@
 #include "tc_common.cuh"
 
 #include "gemm_rows.cuh"
+#include "lstm_direct.cuh"
 
 namespace pimb200 {
 int launch_gemm_wx_simt(const __half* W, const __half* X, const __half* bias, void* Y, int N, int K, int J, int ldx,
@@ -804,7 +805,7 @@ constexpr int kWideThreads = kPersistThreads;
 constexpr int kWideKq = 4;         // K-split of the tensor-core phase across warps
 constexpr int kWideMaxKtw = 16;    // k-tiles per warp held in registers (H <= 1024)
 
-template <int NT>  // 2, 4 or 8 tiles of 8 sequences
+template <int NT>  // 4 or 8 tiles of 8 sequences
 __global__ void __launch_bounds__(kWideThreads, 1) lstm_persistent_wide_kernel(BulkArgs a) {
     constexpr int BP = NT * 8;
     constexpr int NH = NT / 2;                       // n-tiles per warp
@@ -1047,275 +1048,6 @@ __global__ void __launch_bounds__(kWideThreads, 1) lstm_persistent_wide_kernel(B
         }
         if (__syncthreads_or(timed_out)) return;
         if (tr && tid == 0) tr[7] = clock64();
-    }
-}
-
-// ---------------------------------------------------------------------------------------------
-// two stacked layers as a wavefront (up to 8 sequences, H a multiple of 16 up to 1024): layer A at timestep s and layer
-// B at timestep s - 2 in the same step of ONE launch, so a pair of layers costs T + 2 dependent steps instead of 2T.
-// It is the wide kernel with its two sequence tiles given to the two layers: slots 0..7 of the exchange records and of
-// the hidden-state buffer hold layer A's sequences, slots 8..15 layer B's; the warps of tile half 0 keep layer A's
-// W_hh slice in registers, those of tile half 1 layer B's, and the exchange moves both layers' states in the same
-// records, flags and bulk copies.  Layer B's input is layer A's output, which every CTA holds after the gather:
-// W_ih(B) . h_A is one more product per step, shared by all eight warps (a K quarter of one m-tile each), with the CTA's
-// 32 rows of W_ih(B) kept in shared memory (read as mma A fragments, rows padded by 16 bytes: conflict-free); it is made
-// a step ahead of its use, under the exchange (see the step loop), and summed by layer B's gate threads next to the
-// partials of W_hh(B) . h_B.  Layer A's input projection stays hoisted (G); layer B has none.
-// ---------------------------------------------------------------------------------------------
-struct WaveArgs {
-    const __half* Whh[2];      // packed [4H, H] of layer A, layer B
-    const __half* WihB;        // packed [4H, H]: layer B's input matrix
-    const float* bias[2];
-    const float* G;            // layer A's input-projection terms (fp32)
-    long g_tstride, g_bstride;
-    const __half* h0[2];
-    const __half* c0[2];
-    __half* y;                 // layer B's output
-    long y_tstride, y_bstride;
-    int y_vec;
-    __half* hn[2];
-    __half* cn[2];
-    uint4* data;
-    uint32_t* flags;
-    uint32_t tag_base;
-    int* status;
-    int gen;
-    int H, T, B;
-    int poll_limit;
-};
-
-__global__ void __launch_bounds__(kWideThreads, 1) lstm_persistent_wave_kernel(WaveArgs a) {
-    constexpr int BP = 16;                           // slots: 8 per layer
-    constexpr int ZP = BP + 1;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int H = a.H, T = a.T, B = a.B;
-    const int wp = H + 8;                            // row pitch of the W_ih(B) slice (halves)
-    __half* hs = reinterpret_cast<__half*>(smem_raw);                         // [H/8][BP][8]
-    float* zpart = reinterpret_cast<float*>(hs + (size_t)BP * H);             // [kWideKq][8 units][ZP][4 gates]
-    float* zpart2 = zpart + (size_t)kWideKq * 8 * ZP * 4;                     // same shape: partials of W_ih(B) . h_A
-    unsigned short* hpub = reinterpret_cast<unsigned short*>(zpart2 + (size_t)kWideKq * 8 * ZP * 4);  // [BP][8]
-    __half* wib = reinterpret_cast<__half*>(hpub + (size_t)BP * 8);           // [32 rows][wp]
-    uint64_t* gbar = reinterpret_cast<uint64_t*>(wib + (size_t)32 * wp);
-    const uint32_t gbar_addr = (uint32_t)__cvta_generic_to_shared(gbar);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int n_cta = gridDim.x, cta = blockIdx.x;
-    const int u0 = cta * 8;
-    const int ktiles = H >> 4;
-    const int cpw = (n_cta + kPersistWarps - 1) / kPersistWarps;
-    if (tid == 0) {
-        pimb200::tc::mbar_init(gbar_addr, (uint32_t)((n_cta + cpw - 1) / cpw));
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    const int kq = warp & (kWideKq - 1), nh = (warp >> 2) & 1;   // nh: the layer whose tile this warp multiplies
-    const int b_n = lane >> 2, b_k = (lane & 3) * 2;
-    uint32_t afrag[kWideMaxKtw][2][4];
-    {
-        const __half* wbase = a.Whh[nh] + (size_t)u0 * 4 * H;
-#pragma unroll
-        for (int i = 0; i < kWideMaxKtw; ++i)
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    afrag[i][m][r] = 0u;
-                    if (kWideKq * i + kq < ktiles) {
-                        const int row = m * 16 + b_n + (r & 1) * 8;
-                        const int k = (kWideKq * i + kq) * 16 + b_k + (r >> 1) * 8;
-                        afrag[i][m][r] = __ldg(reinterpret_cast<const uint32_t*>(wbase + (size_t)row * H + k));
-                    }
-                }
-    }
-    {
-        const int H8 = H >> 3;
-        const uint4* src = reinterpret_cast<const uint4*>(a.WihB + (size_t)u0 * 4 * H);
-        for (int i = tid; i < 32 * H8; i += kWideThreads) {
-            const int r = i / H8, c8 = i - r * H8;
-            *reinterpret_cast<uint4*>(wib + (size_t)r * wp + c8 * 8) = __ldg(src + (size_t)r * H8 + c8);
-        }
-    }
-    for (int i = tid; i < BP * H; i += kWideThreads) {
-        const int slot = i / H, k = i - slot * H, n = slot & 7;
-        const __half* h0 = a.h0[slot >> 3];
-        hs[((size_t)(k >> 3) * BP + slot) * 8 + (k & 7)] = (n < B && h0) ? h0[(size_t)n * H + k] : __float2half_rn(0.f);
-    }
-    for (int i = tid; i < BP * 8; i += kWideThreads) hpub[i] = 0;
-
-    // gate pair of this thread: unit tid / 16, slot tid % 16 (threads 128..255 have none)
-    const int gu = tid < 8 * BP ? tid / BP : 0, slot = tid < 8 * BP ? tid % BP : 0;
-    const int layer = slot >> 3, gn = slot & 7;
-    const bool live = tid < 8 * BP && gn < B;
-    float c = 0.f;
-    __half hh = __float2half_rn(0.f);
-    float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f), gx = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (live) {
-        const int u = u0 + gu;
-        c = a.c0[layer] ? __half2float(a.c0[layer][(size_t)gn * H + u]) : 0.f;
-        hh = a.h0[layer] ? a.h0[layer][(size_t)gn * H + u] : __float2half_rn(0.f);
-        bias4 = *reinterpret_cast<const float4*>(a.bias[layer] + (size_t)u * 4);
-        if (layer == 0) gx = __ldcg(reinterpret_cast<const float4*>(a.G + (size_t)gn * a.g_bstride + (size_t)u * 4));
-    }
-    __syncthreads();
-
-    // Layer B runs TWO steps behind layer A: its input product W_ih(B) . h_A(t) is then computed from the states already in
-    // shared memory right after this CTA has released its flag, while the other CTAs' flags are still on their way (a
-    // stretch in which the warps would only spin), and lies ready in zpart2 when layer B's gates need it a step later.
-    // One step behind, that product sat between the gather and the gates, on the step's critical path (3.4 us per step).
-    for (int s = 0; s <= T + 1; ++s) {
-        const int par = s & 1;
-        const bool act = layer == 0 ? (s < T) : (s >= 2);      // this thread's layer has a timestep in this step
-        const int t = layer == 0 ? s : s - 2;
-        // ---- 1. K-partial Z tiles: W_hh . h of the warp's layer
-        {
-            float acc[2][4];
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) acc[m][i] = 0.f;
-            const __half* brow = hs + ((size_t)(nh * 8 + b_n)) * 8 + b_k;
-#pragma unroll
-            for (int i = 0; i < kWideMaxKtw; ++i) {
-                if (kWideKq * i + kq < ktiles) {   // warp-uniform
-                    const int kt = kWideKq * i + kq;
-                    const __half* hp = brow + (size_t)(2 * kt) * BP * 8;
-                    const uint32_t b0 = *reinterpret_cast<const uint32_t*>(hp);
-                    const uint32_t b1 = *reinterpret_cast<const uint32_t*>(hp + (size_t)BP * 8);
-                    mma_16816(acc[0], afrag[i][0], b0, b1);
-                    mma_16816(acc[1], afrag[i][1], b0, b1);
-                }
-            }
-            float* zq = zpart + (size_t)kq * 8 * ZP * 4;
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int r = m * 16 + b_n + (i >> 1) * 8, n = nh * 8 + b_k + (i & 1);
-                    zq[((size_t)(r >> 2) * ZP + n) * 4 + (r & 3)] = acc[m][i];
-                }
-        }
-        __syncthreads();
-        // ---- 2. gates (a layer without a timestep in this step keeps its state)
-        if (live) {
-            if (act) {
-                float zi = gx.x + bias4.x, zf = gx.y + bias4.y, zg = gx.z + bias4.z, zo = gx.w + bias4.w;
-#pragma unroll
-                for (int k = 0; k < kWideKq; ++k) {
-                    const float4 zk = *reinterpret_cast<const float4*>(zpart + ((size_t)(k * 8 + gu) * ZP + slot) * 4);
-                    zi += zk.x; zf += zk.y; zg += zk.z; zo += zk.w;
-                }
-                if (layer == 1) {   // the input product made during the previous step's exchange
-#pragma unroll
-                    for (int k = 0; k < kWideKq; ++k) {
-                        const float4 zk = *reinterpret_cast<const float4*>(zpart2 + ((size_t)(k * 8 + gu) * ZP + slot) * 4);
-                        zi += zk.x; zf += zk.y; zg += zk.z; zo += zk.w;
-                    }
-                }
-                c = sigmoidf_(zf) * c + sigmoidf_(zi) * tanhf_(zg);
-                hh = __float2half_rn(sigmoidf_(zo) * tanhf_(c));
-            }
-            const int u = u0 + gu;
-            hpub[slot * 8 + gu] = __half_as_ushort(hh);
-            if (act) {
-                if (layer == 1 && !a.y_vec) a.y[(size_t)t * a.y_tstride + (size_t)gn * a.y_bstride + u] = hh;
-                if (t == T - 1) {
-                    if (a.hn[layer]) a.hn[layer][(size_t)gn * H + u] = hh;
-                    if (a.cn[layer]) a.cn[layer][(size_t)gn * H + u] = __float2half_rn(c);
-                }
-            }
-        }
-        __syncthreads();
-        // ---- 3. publish both layers' records
-        if (tid < BP && (tid & 7) < B) {
-            const uint4 v = *reinterpret_cast<const uint4*>(hpub + tid * 8);
-            if (s <= T) {
-                a.data[((size_t)par * n_cta + cta) * BP + tid] = v;
-                asm volatile("fence.proxy.async.global;" ::: "memory");
-            }
-            if (tid >= 8 && s >= 2 && a.y_vec)
-                *reinterpret_cast<uint4*>(a.y + (size_t)(s - 2) * a.y_tstride + (size_t)(tid & 7) * a.y_bstride + u0) = v;
-        }
-        if (s == T + 1) break;
-        __syncthreads();
-        const uint32_t tag = a.tag_base + (uint32_t)s + 1u;
-        if (tid < kBulkFlagCopies)
-            asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(a.flags + (((size_t)tid * 2 + par) * n_cta + cta) * 32), "r"(tag) : "memory");
-        // ---- 3b. layer B's input product for the NEXT step, from layer A's states still in shared memory (the output of
-        //      A's timestep s - 1, which B reaches at step s + 1): warp (kq, nh) takes its K quarter of m-tile nh.  The
-        //      barrier behind it keeps every warp's reads of hs ahead of the bulk copies issued below.
-        {
-            float acc2[4] = {0.f, 0.f, 0.f, 0.f};
-            const __half* xrow = hs + (size_t)b_n * 8 + b_k;      // layer A's slots: tile 0
-            const __half* arow = wib + (size_t)(nh * 16 + b_n) * wp + b_k;
-#pragma unroll 4
-            for (int i = 0; i < kWideMaxKtw; ++i) {
-                if (kWideKq * i + kq < ktiles) {
-                    const int kt = kWideKq * i + kq;
-                    const __half* hp = xrow + (size_t)(2 * kt) * BP * 8;
-                    const uint32_t b0 = *reinterpret_cast<const uint32_t*>(hp);
-                    const uint32_t b1 = *reinterpret_cast<const uint32_t*>(hp + (size_t)BP * 8);
-                    const __half* ap = arow + kt * 16;
-                    uint32_t af[4];
-                    af[0] = *reinterpret_cast<const uint32_t*>(ap);
-                    af[1] = *reinterpret_cast<const uint32_t*>(ap + (size_t)8 * wp);
-                    af[2] = *reinterpret_cast<const uint32_t*>(ap + 8);
-                    af[3] = *reinterpret_cast<const uint32_t*>(ap + (size_t)8 * wp + 8);
-                    mma_16816(acc2, af, b0, b1);
-                }
-            }
-            float* zq2 = zpart2 + (size_t)kq * 8 * ZP * 4;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = nh * 16 + b_n + (i >> 1) * 8, n = 8 + b_k + (i & 1);
-                zq2[((size_t)(r >> 2) * ZP + n) * 4 + (r & 3)] = acc2[i];
-            }
-        }
-        __syncthreads();
-        // ---- 4./5. flags and gather, one group of CTAs per warp (as in the wide kernel)
-        int timed_out = 0;
-        {
-            const int c0 = warp * cpw;
-            const int c1 = c0 + cpw < n_cta ? c0 + cpw : n_cta;
-            if (c0 < n_cta) {   // warp-uniform
-                const int j = c0 + lane;
-                if (j < c1) {
-                    const uint32_t* f = a.flags + (((size_t)(cta % kBulkFlagCopies) * 2 + par) * n_cta + j) * 32;
-                    int polls = 0;
-                    while (true) {
-                        uint32_t v;
-                        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
-                        if (v == tag) break;
-                        if (++polls >= a.poll_limit) { timed_out = 1; break; }
-                        if ((polls & 1023) == 0 && status_aborted(a.status, a.gen)) { timed_out = 1; break; }
-                    }
-                    if (timed_out) status_raise(a.status, a.gen, PIMB200_ERR_TIMEOUT);
-                    uint32_t v;
-                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
-                }
-                const int lost = __any_sync(0xffffffffu, timed_out);
-                if (lane == 0 && !lost) {
-                    const uint32_t off = (uint32_t)c0 * BP * 16u, len = (uint32_t)(c1 - c0) * BP * 16u;
-                    pimb200::tc::mbar_expect_tx(gbar_addr, len);
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-                                 "r"((uint32_t)__cvta_generic_to_shared(hs) + off),
-                                 "l"(reinterpret_cast<const unsigned char*>(a.data + (size_t)par * n_cta * BP) + off), "r"(len),
-                                 "r"(gbar_addr)
-                                 : "memory");
-                } else if (lane == 0) {
-                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(gbar_addr) : "memory");
-                }
-            }
-        }
-        // layer A's input-projection term of the next step
-        if (live && layer == 0 && s + 1 < T) {
-            const float* gp = a.G + (size_t)(s + 1) * a.g_tstride + (size_t)gn * a.g_bstride + (size_t)(u0 + gu) * 4;
-            asm volatile("ld.global.cg.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(gx.x), "=f"(gx.y), "=f"(gx.z), "=f"(gx.w) : "l"(gp));
-        }
-        if (!pimb200::tc::mbar_wait(gbar_addr, (uint32_t)(s & 1), reinterpret_cast<const volatile int*>(a.status) + 1, a.gen)) {
-            for (uint32_t i = 0; i < (1u << 20); ++i)
-                if (pimb200::tc::mbar_try_wait(gbar_addr, (uint32_t)(s & 1))) break;
-            status_raise(a.status, a.gen, PIMB200_ERR_TIMEOUT);
-            timed_out = 1;
-        }
-        if (__syncthreads_or(timed_out)) return;
     }
 }
 
@@ -2012,6 +1744,7 @@ struct pimb200_lstm {
     int variant = PIMB200_LSTM_AUTO;
     int sm_count = kNumSmB200;
     int max_smem_optin = 0;
+    unsigned char* arena = nullptr;   // one allocation: weights, biases, exchange buffers and the status block
     std::vector<__half*> w_ih, w_hh;  // per (l*D+d), packed
     std::vector<float*> bias;         // per (l*D+d), packed fp32
     // workspace, grown on demand
@@ -2033,6 +1766,8 @@ struct pimb200_lstm {
     int packed_lockstep = 1;   // 0: packed input runs timestep by timestep on the streamed kernels
     int wavefront = 1;         // 1: stacked layers of up to 8 sequences run in pairs, one step apart, in one launch
     uint4* xchg = nullptr;  // [kXchgCopies][2][kXchgWords]
+    uint4* direct_buf = nullptr;     // few sequences: two sets of four record buffers, used by alternate launches
+    unsigned direct_launches = 0;
     uint4* bulk_data = nullptr;      // batched variant: [2][n_cta][32] records
     uint32_t* bulk_flags = nullptr;  // [2][n_cta]
     uint32_t bulk_tag = 0;
@@ -2075,9 +1810,7 @@ static int in_size(const pimb200_lstm* h, int l) { return l == 0 ? h->I : h->D *
 extern "C" int pimb200_lstm_destroy(pimb200_lstm* h) {
     if (!h) return PIMB200_OK;
     cudaSetDevice(h->device);
-    for (auto p : h->w_ih) cudaFree(p);
-    for (auto p : h->w_hh) cudaFree(p);
-    for (auto p : h->bias) cudaFree(p);
+    cudaFree(h->arena);
     cudaFree(h->G);
     cudaFree(h->pk_lens);
     cudaFree(h->pk_row0);
@@ -2086,10 +1819,6 @@ extern "C" int pimb200_lstm_destroy(pimb200_lstm* h) {
     cudaFree(h->ybuf[0]);
     cudaFree(h->ybuf[1]);
     cudaFree(h->cstate);
-    cudaFree(h->xchg);
-    cudaFree(h->bulk_data);
-    cudaFree(h->bulk_flags);
-    cudaFree(h->d_status);
     for (auto e : h->prof_ev) cudaEventDestroy(e);
     delete h;
     return PIMB200_OK;
@@ -2111,37 +1840,44 @@ extern "C" int pimb200_lstm_create(const void* const* params, int n_params, int 
     cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, h->device);
     cudaDeviceGetAttribute(&h->max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
     const int H = hidden_size;
+    const size_t ncta = (size_t)ceil_div(H, 8);
+    // one allocation and one fill for everything that lives as long as the handle; what has to start as zeros comes first
+    size_t at = 0;
+    auto take = [&](size_t bytes) { const size_t p = at; at += (bytes + 255) & ~size_t(255); return p; };
+    const size_t o_status = take(8), o_xchg = take(kXchgBytes);
+    // the pipelined kernel's layouts of flags and records (up to kPipeMaxB sequences) are the largest
+    const size_t o_flags = take((size_t)kBulkFlagCopies * 2 * kPipeMaxHalves * kPipeMaxGroups * ncta * 128);
+    const size_t zeros = at;
+    const size_t o_direct = take(kDirectBytes), o_data = take(2 * ncta * kPipeMaxB * 16);
+    std::vector<size_t> o_w;
+    for (int l = 0; l < num_layers; ++l)
+        for (int d = 0; d < D; ++d) {
+            o_w.push_back(take((size_t)4 * H * in_size(h, l) * 2));
+            o_w.push_back(take((size_t)4 * H * H * 2));
+            o_w.push_back(take((size_t)4 * H * 4));
+        }
+    if (cudaMalloc(&h->arena, at) != cudaSuccess) return fail(PIMB200_ERR_NO_MEMORY);
+    cudaMemset(h->arena, 0, zeros);
+    cudaMemset(h->arena + o_direct, 0xff, kDirectBytes);
+    h->d_status = reinterpret_cast<int*>(h->arena + o_status);
+    h->xchg = reinterpret_cast<uint4*>(h->arena + o_xchg);
+    h->bulk_flags = reinterpret_cast<uint32_t*>(h->arena + o_flags);
+    h->direct_buf = reinterpret_cast<uint4*>(h->arena + o_direct);
+    h->bulk_data = reinterpret_cast<uint4*>(h->arena + o_data);
     for (int l = 0; l < num_layers; ++l) {
         for (int d = 0; d < D; ++d) {
-            const int Il = in_size(h, l);
-            const void* const* p = params + (size_t)(l * D + d) * per;
-            __half *wi = nullptr, *wh = nullptr;
-            float* bs = nullptr;
-            if (cudaMalloc(&wi, (size_t)4 * H * Il * 2) != cudaSuccess) return fail(PIMB200_ERR_NO_MEMORY);
-            h->w_ih.push_back(wi);
-            if (cudaMalloc(&wh, (size_t)4 * H * H * 2) != cudaSuccess) return fail(PIMB200_ERR_NO_MEMORY);
-            h->w_hh.push_back(wh);
-            if (cudaMalloc(&bs, (size_t)4 * H * 4) != cudaSuccess) return fail(PIMB200_ERR_NO_MEMORY);
-            h->bias.push_back(bs);
-            lstm_pack_matrix_kernel<<<296, 256>>>(static_cast<const __half*>(p[0]), wi, H, Il);
-            lstm_pack_matrix_kernel<<<296, 256>>>(static_cast<const __half*>(p[1]), wh, H, H);
+            const int ld = l * D + d, Il = in_size(h, l);
+            const void* const* p = params + (size_t)ld * per;
+            h->w_ih.push_back(reinterpret_cast<__half*>(h->arena + o_w[3 * ld]));
+            h->w_hh.push_back(reinterpret_cast<__half*>(h->arena + o_w[3 * ld + 1]));
+            h->bias.push_back(reinterpret_cast<float*>(h->arena + o_w[3 * ld + 2]));
+            lstm_pack_matrix_kernel<<<296, 256>>>(static_cast<const __half*>(p[0]), h->w_ih[ld], H, Il);
+            lstm_pack_matrix_kernel<<<296, 256>>>(static_cast<const __half*>(p[1]), h->w_hh[ld], H, H);
             lstm_pack_bias_kernel<<<ceil_div(4 * H, 256), 256>>>(
                 has_biases ? static_cast<const __half*>(p[2]) : nullptr,
-                has_biases ? static_cast<const __half*>(p[3]) : nullptr, bs, H);
+                has_biases ? static_cast<const __half*>(p[3]) : nullptr, h->bias[ld], H);
         }
     }
-    if (cudaMalloc(&h->xchg, kXchgBytes) != cudaSuccess) return fail(PIMB200_ERR_NO_MEMORY);
-    if (cudaMalloc(&h->d_status, 8) != cudaSuccess) return fail(PIMB200_ERR_NO_MEMORY);
-    cudaMemset(h->xchg, 0, kXchgBytes);
-    {
-        const size_t ncta = (size_t)ceil_div(H, 8);
-        // records of both parities: the pipelined kernel's layout (up to kPipeMaxB sequences) is the largest
-        if (cudaMalloc(&h->bulk_data, 2 * ncta * kPipeMaxB * 16) != cudaSuccess) return fail(PIMB200_ERR_NO_MEMORY);
-        const size_t flag_bytes = (size_t)kBulkFlagCopies * 2 * kPipeMaxHalves * kPipeMaxGroups * ncta * 128;   // the pipelined kernel's layout is the largest
-        if (cudaMalloc(&h->bulk_flags, flag_bytes) != cudaSuccess) return fail(PIMB200_ERR_NO_MEMORY);
-        cudaMemset(h->bulk_flags, 0, flag_bytes);
-    }
-    cudaMemset(h->d_status, 0, 8);
     if ((rc = cuda_status(cudaDeviceSynchronize())) != PIMB200_OK) return fail(rc);
     *out = h;
     return PIMB200_OK;
@@ -2305,6 +2041,21 @@ struct SeqLayout {
     long x_seq_rows = 0;            // batch-first input: rows from one sequence to the next (0 = T)
 };
 
+// the launch on a handle's next set of record buffers; `steps` of `layers` recurrences for the profile
+static int run_direct(pimb200_lstm* h, DirectArgs& a, int layers, int steps, cudaStream_t st) {
+    const unsigned n = h->direct_launches++;
+    a.set = h->direct_buf + (n & 1) * kDirectSetWords;
+    a.other_set = h->direct_buf + ((n & 1) ^ 1) * kDirectSetWords;
+    a.status = h->d_status; a.gen = next_gen(h); a.H = h->H; a.poll_limit = h->poll_limit;
+    if (h->prof) prof_mark(h, st);
+    const int rc = launch_lstm_direct(a, layers, st);
+    if (h->prof) {
+        prof_mark(h, st);
+        h->prof_bytes += (double)layers * steps * 4.0 * h->H * h->H * 2.0;
+    }
+    return rc;
+}
+
 static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool reverse, const float* G, long g_tstride,
                           long g_bstride, const __half* h0, const __half* c0, __half* y, long y_tstride,
                           long y_bstride, __half* hn, __half* cn, cudaStream_t st) {
@@ -2319,7 +2070,7 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
     // (the wide kernel keeps its W_hh slice in registers: H at most 1024)
     const bool wide_ok = (H % 16 == 0) && H <= 16 * kWideKq * kWideMaxKtw;
     const bool wide = wide_ok && h->bulk_wide >= 1;
-    const int wnt = nt < 2 ? 2 : nt;   // the wide kernel's smallest instance takes 16 sequences
+    const int wnt = nt < 4 ? 4 : nt;   // the wide kernel's smallest instance takes 32 sequences
     const size_t bsmem = wide ? wide_smem(H, wnt) : bulk_smem(H, nt);
     const bool bulk_fits = (H % 16 == 0) && (H / 8 <= h->sm_count) && (H / 8 <= kPersistThreads) && B >= (wide ? 1 : 2) &&
                            B <= (h->bulk_wide ? kBulkMaxB : 32) && (nt <= 4 || wide) && !packed && (int)bsmem <= h->max_smem_optin;
@@ -2405,6 +2156,17 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
             return PIMB200_OK;
         }
     }
+    // up to 16 sequences: records polled straight into the registers that multiply them (3.0 thousand cycles per step against
+    // 5.0 with flags and bulk copies); beyond that the polling loads themselves cost more than the flags
+    const bool direct_fits = wide_ok && !packed && B <= kDirectMaxSlots && H / 8 <= h->sm_count && H / 8 <= kDirectMaxCtas &&
+                             (h->bulk_wide == 1 || h->bulk_wide == 2) && (int)direct_smem(H, 1) <= h->max_smem_optin;
+    if (direct_fits && (h->variant == PIMB200_LSTM_PERSISTENT || (h->variant == PIMB200_LSTM_AUTO && T >= 8))) {
+        DirectArgs a = {};
+        a.Whh[0] = h->w_hh[ld]; a.bias[0] = h->bias[ld]; a.G = G; a.g_tstride = g_tstride; a.g_bstride = g_bstride;
+        a.h0[0] = h0; a.c0[0] = c0; a.y = y; a.y_tstride = y_tstride; a.y_bstride = y_bstride; a.hn[0] = hn; a.cn[0] = cn;
+        a.T = T; a.B = B; a.reverse = reverse ? 1 : 0;
+        return run_direct(h, a, 1, T, st);
+    }
     if (B > kBulkMaxB && !packed && h->variant != PIMB200_LSTM_STREAMED && h->variant != PIMB200_LSTM_AUTO)
         return PIMB200_ERR_UNSUPPORTED;   // a persistent variant was requested for a batch only the pipelined kernel takes
     bool use_bulk = false;
@@ -2428,9 +2190,7 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
         a.H = H; a.T = T; a.B = B; a.reverse = reverse ? 1 : 0; a.poll_limit = h->poll_limit;
         a.trace = h->trace;
         h->bulk_tag += (uint32_t)T + 1u;
-        const void* fn = wide ? (wnt == 2   ? (const void*)lstm_persistent_wide_kernel<2>
-                                 : wnt == 4 ? (const void*)lstm_persistent_wide_kernel<4>
-                                            : (const void*)lstm_persistent_wide_kernel<8>)
+        const void* fn = wide ? (wnt == 4 ? (const void*)lstm_persistent_wide_kernel<4> : (const void*)lstm_persistent_wide_kernel<8>)
                               : (nt == 1   ? (const void*)lstm_persistent_bulk_kernel<1>
                                  : nt == 2 ? (const void*)lstm_persistent_bulk_kernel<2>
                                            : (const void*)lstm_persistent_bulk_kernel<4>);
@@ -2652,22 +2412,18 @@ static int lstm_forward_packed_lockstep(pimb200_lstm* h, const __half* data, con
     return PIMB200_OK;
 }
 
-static size_t wave_smem(int H) {
-    return (size_t)16 * H * 2 + (size_t)2 * kWideKq * 8 * 17 * 16 + (size_t)16 * 16 + (size_t)32 * (H + 8) * 2 + 16;
-}
 // Layers l and l + 1 (one direction) as a wavefront: true when the shape is the wave kernel's
 static bool wave_fits(const pimb200_lstm* h, int l, int T, int B, bool packed) {
     const int H = h->H;
     return h->wavefront && !packed && h->D == 1 && l + 1 < h->L && T >= 8 && B >= 1 && B <= 8 && H % 16 == 0 &&
-           H <= 16 * kWideKq * kWideMaxKtw && H / 8 <= h->sm_count && H / 8 <= kPersistThreads && h->bulk_wide >= 1 &&
-           (h->variant == PIMB200_LSTM_AUTO || h->variant == PIMB200_LSTM_PERSISTENT) && (int)wave_smem(H) <= h->max_smem_optin;
+           H / 8 <= kDirectMaxCtas && H / 8 <= h->sm_count && h->bulk_wide >= 1 &&
+           (h->variant == PIMB200_LSTM_AUTO || h->variant == PIMB200_LSTM_PERSISTENT) && (int)direct_smem(H, 2) <= h->max_smem_optin;
 }
 static int run_wave(pimb200_lstm* h, int l, int T, int B, const float* G, long g_tstride, long g_bstride, const __half* h0,
                     const __half* c0, __half* y, long y_tstride, long y_bstride, __half* hn, __half* cn, cudaStream_t st) {
-    const int H = h->H;
-    WaveArgs a;
+    DirectArgs a = {};
     for (int k = 0; k < 2; ++k) {
-        const size_t off = (size_t)(l + k) * B * H;
+        const size_t off = (size_t)(l + k) * B * h->H;
         a.Whh[k] = h->w_hh[l + k];
         a.bias[k] = h->bias[l + k];
         a.h0[k] = h0 ? h0 + off : nullptr;
@@ -2678,21 +2434,8 @@ static int run_wave(pimb200_lstm* h, int l, int T, int B, const float* G, long g
     a.WihB = h->w_ih[l + 1];
     a.G = G; a.g_tstride = g_tstride; a.g_bstride = g_bstride;
     a.y = y; a.y_tstride = y_tstride; a.y_bstride = y_bstride;
-    a.y_vec = (aligned16(y) && y_tstride % 8 == 0 && y_bstride % 8 == 0) ? 1 : 0;
-    a.data = h->bulk_data; a.flags = h->bulk_flags; a.tag_base = h->bulk_tag; a.status = h->d_status; a.gen = next_gen(h);
-    a.H = H; a.T = T; a.B = B; a.poll_limit = h->poll_limit;
-    h->bulk_tag += (uint32_t)T + 3u;
-    const size_t smem = wave_smem(H);
-    const void* fn = (const void*)lstm_persistent_wave_kernel;
-    PIMB200_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    void* kargs[] = {&a};
-    if (h->prof) prof_mark(h, st);
-    PIMB200_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(H / 8), dim3(kWideThreads), kargs, smem, st));
-    if (h->prof) {
-        prof_mark(h, st);
-        h->prof_bytes += 2.0 * T * 4.0 * H * H * 2.0;   // two layers' W_hh per timestep
-    }
-    return PIMB200_OK;
+    a.T = T; a.B = B;
+    return run_direct(h, a, 2, T, st);
 }
 
 static int lstm_forward_impl(pimb200_lstm* h, const __half* x, const SeqLayout& sq, const __half* h0,
