@@ -10,7 +10,7 @@
 //     every 32-bit word is checked, so nothing is assumed about a record arriving in one piece.  There is no flag and no
 //     release: one L2 trip from the writer's store to the reader's load;
 //   * four buffers are used in turn.  At step s a warp of its own writes sentinels into the CTA's records of buffer
-//     (s + 2) % 4 and fences; the next CTA barrier orders that before the CTA publishes step s + 1.  A reader looks at that
+//     (s + 2) % 4 and fences; the next step's barrier orders that before the CTA publishes step s + 1.  A reader looks at that
 //     buffer only after it has read the same CTA's record of step s + 1, and its old contents (step s - 2) have been read
 //     by everyone, since every CTA has published step s - 1.  A launch starts on buffers that the previous launch of the
 //     handle has filled with sentinels (two sets, alternating);
@@ -18,22 +18,24 @@
 //     contraction index is only a summation order, so lane (sequence g, t) of a block takes units 8t .. 8t+7 of it as one
 //     16-byte record, and W_hh lies in registers (or shared memory) in the same order.  No staging, no barrier between
 //     exchange and product: a warp starts multiplying when its own records are there;
-//   * one CTA barrier per step, between the warps' partial sums (double-buffered) and the gates.  Eight lanes hold the
-//     units of one record and store it as four 32-bit words.
+//   * one handover per step: the product warps store their partial sums (double-buffered), arrive at one of two named
+//     barriers and go on to the next step's records; four gate warps wait there.  A product warp is never two steps ahead
+//     of the gates: the records it needs for that depend on all of this CTA's records of the step between.  Eight lanes
+//     hold the units of one record and store it as four 32-bit words.
 // Wavefront: layer B runs two steps behind layer A (see DirectArgs).  Its input product W_ih(B) . h_A of the next step is
-// made from the registers that hold h_A, after the barrier, while the records are on their way, and stays in the
+// made from the registers that hold h_A, while the gates work and the records are on their way, and stays in the
 // accumulators that W_hh(B) . h_B then continues.
-// Measured at H = 1024, one sequence: 5.0 -> 3.0 thousand cycles per step for one layer (exchange 1.9).
+// Measured at H = 1024, one sequence: 5.0 -> 2.5 thousand cycles per step for one layer, 5.3 -> 3.4 for a wavefront.
 // Every wait is bounded; a CTA that gives up raises the status word, and the others, polling, see it.
 #include "lstm_direct.cuh"
 
 namespace pimb200 {
 namespace {
 
-constexpr int kWarps = 8;                       // compute warps, two warpgroups
-constexpr int kThreads = (kWarps + 4) * 32;     // a third warpgroup, of which one warp writes the sentinels, gives its
-                                                // registers to them (168 a thread at launch; 8 x 240 + 4 x 24 = 12 x 168)
-constexpr int kBarThreads = (kWarps + 1) * 32;  // threads at the step barrier
+constexpr int kWarps = 8;                       // product warps, two warpgroups
+constexpr int kGateWarps = 4;                   // 128 cells: 8 units x 16 slots.  They give registers to the product warps
+                                                // (168 a thread at launch: 8 x 216 + 4 x 72 = 12 x 168)
+constexpr int kThreads = (kWarps + kGateWarps) * 32;
 constexpr int kMaxBlocks = 4;                   // K blocks of 32 per warp: H <= 1024
 
 __device__ __forceinline__ void mma_16816(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -46,7 +48,6 @@ __device__ __forceinline__ uint4 ld_relaxed(const uint4* p) {
     asm volatile("ld.relaxed.gpu.global.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void step_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kBarThreads) : "memory"); }
 __device__ __forceinline__ bool arrived(const uint4& v) { return max(max(v.x, v.y), max(v.z, v.w)) != 0xffffffffu; }
 
 // eight columns x 32 rows: w[m][0 / 1] = W[row 16m + g / 16m + g + 8][the lane's eight k], x = the lane's record
@@ -73,8 +74,11 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
     const int n_cta = gridDim.x, cta = blockIdx.x, u0 = cta * 8;
     const int blocks = (n_cta + 3) >> 2;                         // K blocks of four octets
     const int slots = LAYERS * B;
-    // records per CTA in a buffer: 64 to 256 bytes (with less, one 128-byte line takes the stores of too many CTAs)
-    const int stride = slots == 1 ? 8 : (slots <= 4 ? 4 : (slots <= 8 ? 8 : 16));
+    // An odd number of records is padded with a copy of the last one: stores of half a 32-byte sector cost L2 more (one
+    // sequence: 1.49 -> 1.41 us per step).  Records of a CTA in a buffer: 64 to 256 bytes (with less, one 128-byte line takes
+    // the stores of too many CTAs).
+    const int padded = (slots + 1) & ~1;
+    const int stride = slots <= 4 ? 4 : (slots <= 8 ? 8 : 16);
     const size_t buf = (size_t)n_cta * stride;
     if (tid == 0) dead_step = 0;
     for (int i = tid; i < 2 * ZBUF; i += kThreads) zpart[i] = 0.f;   // (warps without a block never write theirs)
@@ -86,24 +90,91 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
             const int ln = i & 31, q = (i >> 5) & 3, o = 4 * (i >> 7) + (ln & 3);
             wib[i] = o < n_cta ? __ldg(reinterpret_cast<const uint4*>(a.WihB + (size_t)(u0 * 4 + q * 8 + (ln >> 2)) * H + 8 * o)) : make_uint4(0u, 0u, 0u, 0u);
         }
+    const int last = T - 1 + (LAYERS == 2 ? 2 : 0);
     __syncthreads();
+
     if (warp >= kWarps) {
-        // ---- sentinels for step s + 2; the fence ends before the next barrier, ahead of the CTA's records of step s + 1
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 24;" ::: "memory");
-        if (warp > kWarps) return;
-        const int last = T - 1 + (LAYERS == 2 ? 2 : 0);
-        for (int s = 0; s <= last; ++s) {
-            step_barrier();
-            if (dead_step != 0 && dead_step <= s + 1) return;
-            if (lane < slots) {
-                uint4* p = a.set + (size_t)((s + 2) & 3) * buf + (size_t)cta * stride + lane;
-                asm volatile("st.relaxed.gpu.global.v4.b32 [%0], {%1,%1,%1,%1};" ::"l"(p), "r"(~0u) : "memory");
+        // ================================ gate warps ================================
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 72;" ::: "memory");
+        // cell of this thread: unit gt % 8 of slot gt / 8 (layer-major); the pad repeats the last slot's
+        const int gt = tid - kWarps * 32, gu = gt & 7, slot = gt >> 3, u = u0 + gu;
+        const bool live = slot < padded, own = slot < slots, has_cells = (warp - kWarps) * 4 < padded;
+        const int cell = own ? slot : slots - 1, layer = LAYERS == 2 && cell >= B ? 1 : 0, gn = cell - layer * B;
+        const bool sweeps = warp == kWarps + kGateWarps - 1;     // writes the sentinels
+        float c = 0.f;
+        __half hh = __float2half_rn(0.f);
+        float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f), gx = bias4;
+        const float* gp = a.G;
+        long g_step = 0;
+        if (live) {
+            if (a.c0[layer]) c = __half2float(a.c0[layer][(size_t)gn * H + u]);
+            if (a.h0[layer]) hh = a.h0[layer][(size_t)gn * H + u];
+            bias4 = *reinterpret_cast<const float4*>(a.bias[layer] + (size_t)u * 4);
+            if (layer == 0) {
+                gp = a.G + (size_t)(a.reverse ? T - 1 : 0) * a.g_tstride + (size_t)gn * a.g_bstride + (size_t)u * 4;
+                g_step = a.reverse ? -a.g_tstride : a.g_tstride;
+                gx = __ldcg(reinterpret_cast<const float4*>(gp));
             }
-            __threadfence();
+        }
+        uint32_t* const record0 = reinterpret_cast<uint32_t*>(a.set + (size_t)cta * stride + slot) + (gu >> 1);
+        __half* yp = a.y + (size_t)(a.reverse ? T - 1 : 0) * a.y_tstride + (size_t)gn * a.y_bstride + u;   // output of the layer's next step
+        const long y_step = a.reverse ? -a.y_tstride : a.y_tstride;
+        const bool y_pairs = (reinterpret_cast<uintptr_t>(a.y) & 3) == 0 && a.y_tstride % 2 == 0 && a.y_bstride % 2 == 0;
+        const float* const zp0 = zpart + layer * ZL + (gu * ZP + gn) * 4;
+        for (int s = 0; s <= last; ++s) {
+            uint32_t* const record = record0 + (unsigned)(s & 3) * (unsigned)buf * 4u;
+            const float* zp = zp0 + (s & 1) * ZBUF;
+            const int t_l = layer == 0 ? s : s - 2;              // the layer's step
+            const bool act = live && t_l >= 0 && t_l < T;        // (a layer without a timestep repeats its state)
+            float4 z = make_float4(gx.x + bias4.x, gx.y + bias4.y, gx.z + bias4.z, gx.w + bias4.w);
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + (s & 1)), "n"(kThreads) : "memory");   // the partial sums are there
+            if (dead_step != 0 && dead_step <= s + 1) return;    // written ahead of the barrier: the same for every gate thread
+            if (has_cells) {
+                if (act) {
+                    float4 q[kWarps];
+#pragma unroll
+                    for (int w = 0; w < kWarps; ++w) q[w] = *reinterpret_cast<const float4*>(zp + w * ZW);
+#pragma unroll
+                    for (int d = kWarps / 2; d > 0; d >>= 1)
+#pragma unroll
+                        for (int w = 0; w < d; ++w) { q[w].x += q[w + d].x; q[w].y += q[w + d].y; q[w].z += q[w + d].z; q[w].w += q[w + d].w; }
+                    z.x += q[0].x; z.y += q[0].y; z.z += q[0].z; z.w += q[0].w;
+                    c = sigmoidf_(z.y) * c + sigmoidf_(z.x) * tanhf_(z.z);
+                    hh = __float2half_rn(sigmoidf_(z.w) * tanhf_(c));
+                }
+                const uint32_t v = (uint32_t)__half_as_ushort(hh);
+                const uint32_t pair = v | (__shfl_down_sync(0xffffffffu, v, 1, 8) << 16);
+                if (live && s < last && (gu & 1) == 0) asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(record), "r"(pair) : "memory");
+                if (act) {
+                    if (layer == LAYERS - 1 && own) {
+                        if (!y_pairs) *yp = hh;
+                        else if ((gu & 1) == 0) *reinterpret_cast<uint32_t*>(yp) = pair;
+                        yp += y_step;
+                    }
+                    if (layer == 0 && s + 1 < T) {               // next step's input-projection term
+                        gp += g_step;
+                        asm volatile("ld.global.cg.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(gx.x), "=f"(gx.y), "=f"(gx.z), "=f"(gx.w) : "l"(gp));
+                    }
+                }
+            }
+            if (sweeps) {
+                // sentinels for step s + 2; the fence ends ahead of the next barrier, and so of the records of step s + 1
+                if (lane < padded) {
+                    uint4* p = a.set + (size_t)((s + 2) & 3) * buf + (size_t)cta * stride + lane;
+                    asm volatile("st.relaxed.gpu.global.v4.b32 [%0], {%1,%1,%1,%1};" ::"l"(p), "r"(~0u) : "memory");
+                }
+                __threadfence();
+            }
+        }
+        if (own) {
+            if (a.hn[layer]) a.hn[layer][(size_t)gn * H + u] = hh;
+            if (a.cn[layer]) a.cn[layer][(size_t)gn * H + u] = __float2half_rn(c);
         }
         return;
     }
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 240;" ::: "memory");
+
+    // ================================ product warps ================================
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;" ::: "memory");
     // this warp's blocks warp, warp + 8, ...: the lane's octet of block i is 4 * block + t4
     uint4 wf[LAYERS][kMaxBlocks][2][2], hv[LAYERS][NT][kMaxBlocks];
 #pragma unroll
@@ -117,49 +188,25 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
                 if (o < n_cta) wf[l][i][q >> 1][q & 1] = __ldg(reinterpret_cast<const uint4*>(a.Whh[l] + (size_t)(u0 * 4 + q * 8 + g) * H + 8 * o));
             }
 #pragma unroll
-            for (int j = 0; j < NT; ++j) {                   // the initial hidden states
+            for (int j = 0; j < NT; ++j) {                       // the initial hidden states
                 const int n = j * 8 + g;
                 uint4 x = make_uint4(0u, 0u, 0u, 0u);
                 if (o < n_cta && n < B && a.h0[l]) {
                     const __half* p = a.h0[l] + (size_t)n * H + 8 * o;
                     __half v[8];
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) v[e] = p[e];  // any alignment
+                    for (int e = 0; e < 8; ++e) v[e] = p[e];      // any alignment
                     x = *reinterpret_cast<const uint4*>(v);
                 }
                 hv[l][j][i] = x;
             }
         }
     }
-    // gate cell of this thread: unit tid % 8 of slot tid / 8 (layer-major)
-    const int gu = tid & 7, slot = tid >> 3, u = u0 + gu;
-    const bool live = slot < slots;
-    const int layer = LAYERS == 2 && slot >= B ? 1 : 0, gn = slot - layer * B;
-    float c = 0.f;
-    __half hh = __float2half_rn(0.f);
-    float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f), gx = bias4;
-    const float* gp = a.G;
-    long g_step = 0;
-    if (live) {
-        if (a.c0[layer]) c = __half2float(a.c0[layer][(size_t)gn * H + u]);
-        if (a.h0[layer]) hh = a.h0[layer][(size_t)gn * H + u];
-        bias4 = *reinterpret_cast<const float4*>(a.bias[layer] + (size_t)u * 4);
-        if (layer == 0) {
-            gp = a.G + (size_t)(a.reverse ? T - 1 : 0) * a.g_tstride + (size_t)gn * a.g_bstride + (size_t)u * 4;
-            g_step = a.reverse ? -a.g_tstride : a.g_tstride;
-            gx = __ldcg(reinterpret_cast<const float4*>(gp));
-        }
-    }
-    uint32_t* const record0 = reinterpret_cast<uint32_t*>(a.set + (size_t)cta * stride + slot) + (gu >> 1);
-    __half* yp = a.y + (size_t)(a.reverse ? T - 1 : 0) * a.y_tstride + (size_t)gn * a.y_bstride + u;   // output of the layer's next step
-    const long y_step = a.reverse ? -a.y_tstride : a.y_tstride;
-    const bool y_pairs = (reinterpret_cast<uintptr_t>(a.y) & 3) == 0 && a.y_tstride % 2 == 0 && a.y_bstride % 2 == 0;
     float accB[2][4];                                            // layer B's input product, made a step ahead
 #pragma unroll
     for (int m = 0; m < 2; ++m)
 #pragma unroll
         for (int e = 0; e < 4; ++e) accB[m][e] = 0.f;
-    const int last = T - 1 + (LAYERS == 2 ? 2 : 0);
     // The lane's records of a step, all asked for together and without conditions: lanes of sequences or octets that do not
     // exist read the last one that does (their products meet no output: a column of its own, or weights of zero)
     uint4 hold[kMaxBlocks];
@@ -180,8 +227,8 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
     };
 
     for (int s = 0; s <= last; ++s) {
-        float* zb = zpart + (s & 1) * ZBUF;
-        // ---- 1. this step's hidden states (published in step s - 1): all that are missing are asked for again together
+        float* zb = zpart + (s & 1) * ZBUF + warp * ZW;
+        // ---- this step's hidden states (published in step s - 1)
         if (s > 0) {
             int polls = 0;
             while (true) {
@@ -195,11 +242,14 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
                 all = __all_sync(0xffffffffu, all);
                 // counted at the first look too: records are often there by then, and a limit of one is no wait at all
                 if (++polls >= a.poll_limit || ((polls & 1023) == 0 && status_aborted(a.status, a.gen))) {
+                    // the gate warps leave behind this step's barrier; the other product warps then wait in vain, too
                     if (lane == 0) {
                         status_raise(a.status, a.gen, PIMB200_ERR_TIMEOUT);
                         dead_step = s + 1;
                     }
-                    break;
+                    __syncwarp();
+                    asm volatile("bar.arrive %0, %1;" ::"r"(1 + (s & 1)), "n"(kThreads) : "memory");
+                    return;
                 }
                 if (all) break;
                 ask(s - 1);
@@ -219,7 +269,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
                     for (int e = 0; e < 4; ++e) acc[l][j][m][e] = (LAYERS == 2 && l == 1) ? accB[m][e] : 0.f;
 #pragma unroll
         for (int i = 0; i < kMaxBlocks; ++i)
-            if (warp + kWarps * i < blocks)                  // warp-uniform
+            if (warp + kWarps * i < blocks)                      // warp-uniform
 #pragma unroll
                 for (int l = 0; l < LAYERS; ++l)
 #pragma unroll
@@ -235,51 +285,13 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
                             const int r = m * 16 + g + (e >> 1) * 8, n = j * 8 + 2 * t4 + (e & 1);
-                            zb[warp * ZW + l * ZL + ((r >> 2) * ZP + n) * 4 + (r & 3)] = acc[l][j][m][e];
+                            zb[l * ZL + ((r >> 2) * ZP + n) * 4 + (r & 3)] = acc[l][j][m][e];
                         }
         }
-        uint32_t* const record = record0 + (unsigned)(s & 3) * (unsigned)buf * 4u;
-        const int t_l = layer == 0 ? s : s - 2;                  // the layer's step
-        const bool act = live && t_l >= 0 && t_l < T;
-        const float* zp = zb + layer * ZL + (gu * ZP + gn) * 4;
-        const float4 zin = make_float4(gx.x + bias4.x, gx.y + bias4.y, gx.z + bias4.z, gx.w + bias4.w);
-        step_barrier();
-        if (dead_step != 0 && dead_step <= s + 1) return;        // written before the barrier: the same for every thread
-        // ---- 2. gates and publication (a layer without a timestep in this step repeats its state)
-        if (warp * 4 < slots) {                                  // the warp has gate cells
-            if (act) {
-                float4 z = zin, q[kWarps];
-#pragma unroll
-                for (int w = 0; w < kWarps; ++w) q[w] = *reinterpret_cast<const float4*>(zp + w * ZW);
-#pragma unroll
-                for (int d = kWarps / 2; d > 0; d >>= 1)
-#pragma unroll
-                    for (int w = 0; w < d; ++w) { q[w].x += q[w + d].x; q[w].y += q[w + d].y; q[w].z += q[w + d].z; q[w].w += q[w + d].w; }
-                z.x += q[0].x; z.y += q[0].y; z.z += q[0].z; z.w += q[0].w;
-                c = sigmoidf_(z.y) * c + sigmoidf_(z.x) * tanhf_(z.z);
-                hh = __float2half_rn(sigmoidf_(z.w) * tanhf_(c));
-            }
-            const uint32_t v = (uint32_t)__half_as_ushort(hh);
-            const uint32_t pair = v | (__shfl_down_sync(0xffffffffu, v, 1, 8) << 16);
-            if (live && s < last && (gu & 1) == 0) asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(record), "r"(pair) : "memory");
-            if (act) {
-                if (layer == LAYERS - 1) {
-                    if (!y_pairs) *yp = hh;
-                    else if ((gu & 1) == 0) *reinterpret_cast<uint32_t*>(yp) = pair;
-                    yp += y_step;
-                }
-                if (layer == 0 && s + 1 < T) {                   // next step's input-projection term
-                    gp += g_step;
-                    asm volatile("ld.global.cg.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(gx.x), "=f"(gx.y), "=f"(gx.z), "=f"(gx.w) : "l"(gp));
-                }
-            }
-        }
-        if (s < last) {      // the first look at the next step's records, on its way during what follows
-            ask(s);
-        }
+        asm volatile("bar.arrive %0, %1;" ::"r"(1 + (s & 1)), "n"(kThreads) : "memory");
         if (LAYERS == 2) {
-            // ---- 3. layer B's input product of the next step: B's step s - 1 takes A's output of that step, published in
-            //         step s - 1 and held in `hold`
+            // ---- layer B's input product of the next step: B's step s - 1 takes A's output of that step, published in
+            //      step s - 1 and held in `hold`
 #pragma unroll
             for (int m = 0; m < 2; ++m)
 #pragma unroll
@@ -295,10 +307,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
                 }
             }
         }
-    }
-    if (live) {
-        if (a.hn[layer]) a.hn[layer][(size_t)gn * H + u] = hh;
-        if (a.cn[layer]) a.cn[layer][(size_t)gn * H + u] = __float2half_rn(c);
+        if (s < last) ask(s);                                    // the first look at the next step's records
     }
 }
 
