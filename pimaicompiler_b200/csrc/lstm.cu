@@ -2156,8 +2156,8 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
             return PIMB200_OK;
         }
     }
-    // up to 16 sequences: records polled straight into the registers that multiply them (3.0 thousand cycles per step against
-    // 5.0 with flags and bulk copies); beyond that the polling loads themselves cost more than the flags
+    // up to 16 sequences: records polled straight into the registers that multiply them (1.3 to 2.0 us per step against
+    // 2.8 with flags and bulk copies); beyond that the polling loads themselves cost more than the flags
     const bool direct_fits = wide_ok && !packed && B <= kDirectMaxSlots && H / 8 <= h->sm_count && H / 8 <= kDirectMaxCtas &&
                              (h->bulk_wide == 1 || h->bulk_wide == 2) && (int)direct_smem(H, 1) <= h->max_smem_optin;
     if (direct_fits && (h->variant == PIMB200_LSTM_PERSISTENT || (h->variant == PIMB200_LSTM_AUTO && T >= 8))) {

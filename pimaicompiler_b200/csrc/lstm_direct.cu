@@ -25,7 +25,7 @@
 // Wavefront: layer B runs two steps behind layer A (see DirectArgs).  Its input product W_ih(B) . h_A of the next step is
 // made from the registers that hold h_A, while the gates work and the records are on their way, and stays in the
 // accumulators that W_hh(B) . h_B then continues.
-// Measured at H = 1024, one sequence: 5.0 -> 2.5 thousand cycles per step for one layer, 5.3 -> 3.4 for a wavefront.
+// Measured at H = 1024, one sequence: 2.80 -> 1.30 us per step for one layer, 2.72 -> 1.81 for a wavefront.
 // Every wait is bounded; a CTA that gives up raises the status word, and the others, polling, see it.
 #include "lstm_direct.cuh"
 
@@ -39,7 +39,7 @@ constexpr int kThreads = (kWarps + kGateWarps) * 32;
 constexpr int kMaxBlocks = 4;                   // K blocks of 32 per warp: H <= 1024
 
 __device__ __forceinline__ void mma_16816(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
@@ -128,7 +128,6 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
             const bool act = live && t_l >= 0 && t_l < T;        // (a layer without a timestep repeats its state)
             float4 z = make_float4(gx.x + bias4.x, gx.y + bias4.y, gx.z + bias4.z, gx.w + bias4.w);
             asm volatile("bar.sync %0, %1;" ::"r"(1 + (s & 1)), "n"(kThreads) : "memory");   // the partial sums are there
-            if (dead_step != 0 && dead_step <= s + 1) return;    // written ahead of the barrier: the same for every gate thread
             if (has_cells) {
                 if (act) {
                     float4 q[kWarps];
@@ -157,6 +156,8 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
                     }
                 }
             }
+            // a wait gave up (written ahead of the barrier: the same for every gate thread; what was published is not used)
+            if (dead_step != 0 && dead_step <= s + 1) return;
             if (sweeps) {
                 // sentinels for step s + 2; the fence ends ahead of the next barrier, and so of the records of step s + 1
                 if (lane < padded) {
@@ -226,6 +227,10 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
                 for (int i = 0; i < kMaxBlocks; ++i) hv[l][j][i] = ld_relaxed(src[j] + (at + off[i] + (unsigned)(l * B)));
     };
 
+    // Cycles from a step's handover to the first look at the next one's records.  A look that comes too early costs another
+    // trip of some 900 cycles, and the more records there are the more it delays them.  Measured optima at H = 1024 (us per
+    // step without and with): 1 sequence 1.34 / 1.30, 8 1.52 / 1.39, 16 2.46 / 2.04, wavefront of 1 1.86 / 1.81, of 8 2.37 / 2.17.
+    const unsigned look = slots > 8 ? 1900u : (LAYERS == 2 ? 1300u : (slots > 4 ? 1100u : 1000u));
     for (int s = 0; s <= last; ++s) {
         float* zb = zpart + (s & 1) * ZBUF + warp * ZW;
         // ---- this step's hidden states (published in step s - 1)
@@ -289,6 +294,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
                         }
         }
         asm volatile("bar.arrive %0, %1;" ::"r"(1 + (s & 1)), "n"(kThreads) : "memory");
+        const unsigned handed_over = clock();
         if (LAYERS == 2) {
             // ---- layer B's input product of the next step: B's step s - 1 takes A's output of that step, published in
             //      step s - 1 and held in `hold`
@@ -307,7 +313,11 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
                 }
             }
         }
-        if (s < last) ask(s);                                    // the first look at the next step's records
+        // the first look at the next step's records, timed to meet them in L2
+        if (s < last) {
+            while ((unsigned)clock() - handed_over < look) {}
+            ask(s);
+        }
     }
 }
 
