@@ -230,7 +230,8 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
     // Cycles from a step's handover to the first look at the next one's records.  A look that comes too early costs another
     // trip of some 900 cycles, and the more records there are the more it delays them.  Measured optima at H = 1024 (us per
     // step without and with): 1 sequence 1.34 / 1.30, 8 1.52 / 1.39, 16 2.46 / 2.04, wavefront of 1 1.86 / 1.81, of 8 2.37 / 2.17.
-    const unsigned look = slots > 8 ? 1900u : (LAYERS == 2 ? 1300u : (slots > 4 ? 1100u : 1000u));
+    // With fewer CTAs (H = 320 to 640) only the optimum of more than 8 records lies elsewhere (1.3 to 1.5 thousand cycles).
+    const unsigned look = slots > 8 ? (n_cta > 96 ? 1900u : 1400u) : (LAYERS == 2 ? 1350u : (slots > 4 ? 1100u : 1000u));
     for (int s = 0; s <= last; ++s) {
         float* zb = zpart + (s & 1) * ZBUF + warp * ZW;
         // ---- this step's hidden states (published in step s - 1)
