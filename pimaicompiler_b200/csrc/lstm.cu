@@ -397,7 +397,7 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t* r, const void* smem_ptr) {
                  : "r"(addr));
 }
 __device__ __forceinline__ void mma_16816(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
@@ -1061,21 +1061,29 @@ __global__ void __launch_bounds__(kWideThreads, 1) lstm_persistent_wide_kernel(B
 // as many participants in each half's exchange, twice the sequences per launch.  The halves never interact.
 // Within a CTA the sequences are split into NG groups of BPG = 8*NTG that advance independently, and every stage of a
 // step has warps of its own, handing over through mbarriers, so that the stages of different groups overlap:
-//   * warps 0..7 (tensor) split K eight ways (warp w owns k-tiles w, w+8, ...): wait for the group's gathered hidden
+//   * warps 0..7 (tensor) split the product eight ways (K quarter x half of the rows): wait for the group's gathered hidden
 //     states ("full") and for a free partial-sum buffer ("zfree"), multiply, store the K-partials, arrive on "zready".
 //     They never wait for the gates: the tensor pipe stays busy with the next group.
-//   * warps 8..11 (gates) wait for "zready", sum the eight partials, free the buffer, run the cell update (c stays in
-//     fp32 registers for the whole sequence), assemble each sequence's 16-byte records (eight units each) with shuffles,
-//     store them (and the y row) and arrive on "done".  The input-projection terms of the next step are fetched into
-//     shared memory with cp.async a whole step ahead (they stream from HBM).
-//   * warps 12..15 (exchange), one per group: wait for "done", raise this CTA's step flag (release, cumulative over the
-//     gate warps' record stores), then poll the flags of the half's CTAs, one flag per lane and chunk of 32 CTAs, and
-//     hand each chunk's records to the bulk-copy engine as soon as its flags are up (no cluster multicast); the copies
-//     complete on "full".
-// The exchange of one group (two L2 round trips plus the skew of the slowest CTA, ~4-5 thousand cycles) runs under the
-// arithmetic of the other groups; a step of all groups takes about as long as one group's chain.
+//   * warps 8..11 (gates) wait for "zready", sum the four partials, free the buffer, run the cell update (c stays in
+//     fp32 registers for the whole sequence), store each sequence's 16-byte records (eight units each) and the y row and
+//     arrive on "done".  The input-projection terms of the next step are fetched into shared memory with cp.async a whole
+//     step ahead (they stream from HBM).
+//   * warps 12..15 (exchange), one per group: raise this CTA's step flag behind its records, poll the flags of the half's
+//     CTAs, one flag per lane and chunk of 32 CTAs, and hand each chunk's records to the bulk-copy engine as soon as its
+//     flags are up (no cluster multicast); the copies complete on "full".
+// The flag is a hint that is not ordered behind the records: a release cost a store's whole way to L2 and back (1.2 thousand
+// cycles) in every group's chain.  A record that has not been written holds a sentinel, the fp16 pattern 0xffff, which no
+// hidden value has (see lstm_direct.cu: four buffers in turn, this CTA's records of buffer (s + 2) % 4 made sentinels in step
+// s, two sets of buffers for alternate launches).  It is a NaN, so a copy that was too early shows in the tensor warps' sums,
+// without any instruction in their product; they then wait for the records themselves (seen in 1 of 10^4 phases).
+// Measured at H = 1024, us per step: 48 sequences 3.89 -> 3.19, 64 4.13 -> 3.45, 128 4.82 -> 4.78 (with the gate warps'
+// shorter phase: running addresses, 32-bit record stores, 1660 -> 830 cycles at 128; there the tensor warps, 4 x 2000 cycles,
+// are as long as a group's chain).  Copies without flags, timed like the looks of lstm_direct.cu, drift apart: a CTA that
+// looks too early holds up all others, whose looks move out in turn (5.9 us at 128).
+// The exchange of one group runs under the arithmetic of the other groups; a step of all groups takes as long as one
+// group's chain or as the busiest stage, whichever is longer.
 // The tensor warpgroups take registers from the others at start-up (setmaxnreg).  Per-sequence arithmetic (k-tile order
-// inside a warp's accumulator, order of the eight partial sums) is the same for every UPC / NTG / NG, so a sequence's
+// inside a warp's accumulator, order of the four partial sums) is the same for every UPC / NTG / NG, so a sequence's
 // result does not depend on how many sequences share the launch.  Every wait is bounded and ends early once the
 // launch's generation appears in the status block.
 // ---------------------------------------------------------------------------------------------
@@ -1088,10 +1096,11 @@ constexpr int kPipeKq = 4;           // tensor warp = (K quarter, half of the CT
 constexpr int kPipeMh = kPipeTensorWarps / kPipeKq;
 constexpr int kPipeKtw = 16;         // k-tiles per tensor warp held in registers (H <= 1024)
 constexpr int kPipeMaxGroups = 4;    // one exchange warp per group
-constexpr int kPipeMaxHalves = 2;
 constexpr int kPipeMaxB = 128;       // sequences per launch: 2 halves x 4 groups x 16
-constexpr int kPipeChunk = 32;       // CTAs per gather chunk (one flag per lane)
+constexpr int kPipeChunk = 32;       // CTAs per copied piece of a group's records (one flag per lane)
 constexpr int kPipeMaxChunks = 4;    // H <= 1024: at most 128 CTAs per half
+constexpr size_t kPipeSetWords = (size_t)4 * kPipeMaxB * 128;   // records of four buffers
+constexpr size_t kPipeBytes = 2 * kPipeSetWords * 16;
 
 struct PipeArgs {
     const __half* Whh;
@@ -1102,11 +1111,11 @@ struct PipeArgs {
     const __half* c0;
     __half* y;
     long y_tstride, y_bstride;
-    int y_vec;
     __half* hn;
     __half* cn;
-    uint4* data;            // [2 parities][halves][NG][H/8 octets][BPG] 16-byte records (the image of a group's hs)
-    uint32_t* flags;        // [kBulkFlagCopies][2 parities][kPipeMaxHalves][kPipeMaxGroups][slices] step tags, one per 128-byte line
+    uint4* set;             // [4 buffers][halves][NG][H/8 octets][BPG] 16-byte records (the image of a group's hs), all sentinels
+    uint4* other_set;       // the next launch's: filled with sentinels by this one
+    uint32_t* flags;        // [kBulkFlagCopies][2 parities][2 halves][kPipeMaxGroups][slices] step tags, one per 128-byte line
     uint32_t tag_base;
     int* status;
     int gen;
@@ -1173,6 +1182,9 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    for (size_t i = (size_t)blockIdx.x * kPipeThreads + tid; i < kPipeSetWords; i += (size_t)gridDim.x * kPipeThreads)
+        a.other_set[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    const size_t group_words = (size_t)(H >> 3) * BPG, buf_words = (size_t)a.halves * NG * group_words;
     // initial hidden states, in the layout of the exchange records: hs[g][j][n][8] = units 8j..8j+7 of sequence g*BPG+n
     for (int i = tid; i < NG * BPG * H; i += kPipeThreads) {
         const int n = i / H, k = i - n * H;
@@ -1218,10 +1230,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
                 bool ok = true;
                 if (s > 0) ok = mbar_wait_polls(full0 + 8u * g, (uint32_t)((s - 1) & 1), a.status, a.gen, wait_limit);
                 if (tr && tid == 0 && g == 0) tr[1] = clock64();
-                // the partial-sum buffer must have been read by the gate warps (its use two phases ago)
-                if (ok && phase >= 2)
-                    ok = mbar_wait_polls(zfree0 + 8u * zb, (uint32_t)(((phase >> 1) - 1) & 1), a.status, a.gen, wait_limit);
-                if (!ok) { dead = true; break; }
+                if (!__all_sync(0xffffffffu, ok)) { dead = true; break; }
                 if (tr && tid == 0 && g == 0) tr[2] = clock64();
                 float* zq = zpart + (size_t)zb * ZBUF + (size_t)kq * UPC * ZP * 4;
                 float acc[MTW][NTG][4];
@@ -1232,6 +1241,10 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
 #pragma unroll
                         for (int i = 0; i < 4; ++i) acc[m][j][i] = 0.f;
                 const __half* brow = hs + (size_t)g * BPG * H + (size_t)b_n * 8 + b_k;
+                // the partial-sum buffer must have been read by the gate warps (its use two phases ago): asked here, needed
+                // after the product
+                const uint32_t zfree_parity = (uint32_t)(((phase >> 1) - 1) & 1);
+                const bool zfree = phase < 2 || pimb200::tc::mbar_try_wait(zfree0 + 8u * zb, zfree_parity);
                 auto ktile = [&](int i) {
                     const int kt = kPipeKq * i + kq;
                     const __half* hp = brow + (size_t)(2 * kt) * BPG * 8;
@@ -1256,6 +1269,50 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
                     for (int i = 0; i < kPipeKtw; ++i)
                         if (kPipeKq * i + kq < ktiles) ktile(i);   // warp-uniform
                 }
+                // a sentinel is a NaN: a copy that came too early for a record shows in every sum of its sequence (and so does
+                // a NaN of the caller's inputs).  The warp then takes its k-tiles from the records themselves
+                bool nan = false;
+#pragma unroll
+                for (int j = 0; j < NTG; ++j) nan = nan || isnan(acc[0][j][0]) || isnan(acc[0][j][1]);
+                if (s > 0 && __any_sync(0xffffffffu, nan)) {
+                    const uint32_t* rec = reinterpret_cast<const uint32_t*>(a.set + (size_t)((s - 1) & 3) * buf_words + ((size_t)half * NG + g) * group_words + b_n) + (lane & 3);
+#pragma unroll
+                    for (int m = 0; m < MTW; ++m)
+#pragma unroll
+                        for (int j = 0; j < NTG; ++j)
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) acc[m][j][i] = 0.f;
+                    int polls = 0;
+#pragma unroll
+                    for (int i = 0; i < kPipeKtw; ++i) {
+                        const int kt = kPipeKq * i + kq;
+                        if (kt >= ktiles) continue;
+                        uint32_t b0[NTG], b1[NTG];
+                        for (;;) {
+                            bool here = true;
+#pragma unroll
+                            for (int j = 0; j < NTG; ++j) {
+                                asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(b0[j]) : "l"(rec + ((size_t)(2 * kt) * BPG + j * 8) * 4) : "memory");
+                                asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(b1[j]) : "l"(rec + ((size_t)(2 * kt + 1) * BPG + j * 8) * 4) : "memory");
+                            }
+#pragma unroll
+                            for (int j = 0; j < NTG; ++j) here = here && b0[j] != ~0u && b1[j] != ~0u;
+                            if (__all_sync(0xffffffffu, here)) break;
+                            const bool lost = ++polls >= a.poll_limit || ((polls & 255) == 0 && status_aborted(a.status, a.gen));
+                            if (__any_sync(0xffffffffu, lost)) { dead = true; break; }
+                        }
+                        if (dead) break;
+#pragma unroll
+                        for (int j = 0; j < NTG; ++j)
+#pragma unroll
+                            for (int m = 0; m < MTW; ++m) mma_16816(acc[m][j], afrag[i][m], b0[j], b1[j]);
+                    }
+                    if (dead) break;
+                }
+                if (!__all_sync(0xffffffffu, zfree)) {
+                    ok = zfree || mbar_wait_polls(zfree0 + 8u * zb, zfree_parity, a.status, a.gen, wait_limit);
+                    if (!__all_sync(0xffffffffu, ok)) { dead = true; break; }
+                }
 #pragma unroll
                 for (int m = 0; m < MTW; ++m)
 #pragma unroll
@@ -1271,10 +1328,10 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
         }
         if (dead && lane == 0) status_raise(a.status, a.gen, PIMB200_ERR_TIMEOUT);
     } else {
-    // the other two warpgroups hand registers over (one instruction per warpgroup, before the roles split up)
-    if (UPC == 16) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;" ::: "memory");
-    else asm volatile("setmaxnreg.dec.sync.aligned.u32 120;" ::: "memory");
+    // the other two warpgroups hand registers over (UPC 16: 256 x 184 + 128 x 96 + 128 x 48 = 512 x 128)
     if (warp < kPipeTensorWarps + kPipeGateWarps) {
+        if (UPC == 16) asm volatile("setmaxnreg.dec.sync.aligned.u32 96;" ::: "memory");
+        else asm volatile("setmaxnreg.dec.sync.aligned.u32 120;" ::: "memory");
         // ================================ gate warps ================================
         // Eight consecutive lanes hold the eight units of one octet of one sequence, so a 16-byte record is assembled
         // with four shuffles and stored by its first lane.  Cell q = (sequence block sb, octet o) of thread gt:
@@ -1292,27 +1349,35 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
                 const int o = q % OCT, gn = (gt >> 3) + 16 * (q / OCT), n = g * BPG + gn;
                 c[g][q] = (gn < BPG && n < B && a.c0) ? __half2float(a.c0[(size_t)(seq0 + n) * H + u0 + 8 * o + gl]) : 0.f;
             }
+        // Running addresses of the thread's first cell (sequence gt / 8, unit gl): cell q of group g lies g * BPG + 16 * (q / OCT)
+        // sequences and 8 * (q % OCT) units further on
+        const long gn0 = seq0 + (gt >> 3);
+        const float* g_next = a.G + (size_t)(a.reverse ? T - 1 : 0) * a.g_tstride + gn0 * a.g_bstride + (size_t)(u0 + gl) * 4;   // of the next prefetched step
+        const long g_step = a.reverse ? -a.g_tstride : a.g_tstride, y_step = a.reverse ? -a.y_tstride : a.y_tstride;
+        __half* y_row = a.y + (size_t)(a.reverse ? T - 1 : 0) * a.y_tstride + gn0 * a.y_bstride + u0 + gl;
+        const uint32_t gx_slot = (uint32_t)__cvta_generic_to_shared(gxs + gt);
+        uint32_t* const record0 = reinterpret_cast<uint32_t*>(a.set + (size_t)half * NG * group_words + (size_t)slice * OCT * BPG + (gt >> 3)) + (gl >> 1);
+        const bool y_pairs = (reinterpret_cast<uintptr_t>(a.y) & 3) == 0 && a.y_tstride % 2 == 0 && a.y_bstride % 2 == 0;
         // input-projection terms: fetched with cp.async into this thread's own slots a whole step ahead; one commit
         // group per group phase, so "all but the newest NG - 1 groups" is exactly the phase about to be consumed
-        auto prefetch_gx = [&](int g, int t) {
+        auto prefetch_gx = [&](int g) {
 #pragma unroll
             for (int q = 0; q < CPT; ++q) {
-                const int o = q % OCT, gn = (gt >> 3) + 16 * (q / OCT), n = g * BPG + gn;
+                const int o = q % OCT, sb = q / OCT, gn = (gt >> 3) + 16 * sb, n = g * BPG + gn;
                 if (gn < BPG && n < B) {
-                    const float* gp = a.G + (size_t)t * a.g_tstride + (size_t)(seq0 + n) * a.g_bstride + (size_t)(u0 + 8 * o + gl) * 4;
-                    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(gxs + ((size_t)g * CPT + q) * kPipeGateThreads + gt);
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(gp) : "memory");
+                    const float* gp = g_next + (long)(g * BPG + 16 * sb) * a.g_bstride + 32 * o;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(gx_slot + (uint32_t)((g * CPT + q) * kPipeGateThreads * 16)), "l"(gp) : "memory");
                 }
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
 #pragma unroll
-        for (int g = 0; g < NG; ++g) prefetch_gx(g, a.reverse ? T - 1 : 0);   // (empty commit groups for absent sequences)
+        for (int g = 0; g < NG; ++g) prefetch_gx(g);   // (empty commit groups for absent sequences)
         int phase = 0;
         bool dead = false;
         for (int s = 0; s < T && !dead; ++s) {
-            const int t = a.reverse ? T - 1 - s : s;
-            const int par = s & 1;
+            uint32_t* const record_s = record0 + (size_t)(s & 3) * buf_words * 4;
+            g_next += g_step;                                  // the prefetches below are of step s + 1
             long long* tr = a.trace ? a.trace + ((size_t)blockIdx.x * T + s) * 8 : nullptr;
 #pragma unroll
             for (int g = 0; g < NG; ++g) {
@@ -1328,21 +1393,17 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
                 if (tr && gt == 0 && g == 0) tr[4] = clock64();
                 // the cells of a thread are worked side by side (independent chains): partial sums, gate math, then
                 // the shuffles and stores
-                float z[CPT][4];
-                const float* zbp[CPT];
+                float4 z[CPT];
 #pragma unroll
                 for (int q = 0; q < CPT; ++q) {
                     const int o = q % OCT, gn = (gt >> 3) + 16 * (q / OCT);
-                    zbp[q] = zpart + (size_t)zb * ZBUF + ((size_t)(8 * o + gl) * ZP + (gn < BPG ? gn : 0)) * 4;
-                    z[q][0] = 0.f; z[q][1] = 0.f; z[q][2] = 0.f; z[q][3] = 0.f;
+                    const float* zbp = zpart + (size_t)zb * ZBUF + ((8 * o + gl) * ZP + (gn < BPG ? gn : 0)) * 4;
+                    float4 zk[kPipeKq];
+#pragma unroll
+                    for (int k = 0; k < kPipeKq; ++k) zk[k] = *reinterpret_cast<const float4*>(zbp + k * UPC * ZP * 4);
+                    z[q] = make_float4((zk[0].x + zk[1].x) + (zk[2].x + zk[3].x), (zk[0].y + zk[1].y) + (zk[2].y + zk[3].y),
+                                       (zk[0].z + zk[1].z) + (zk[2].z + zk[3].z), (zk[0].w + zk[1].w) + (zk[2].w + zk[3].w));
                 }
-#pragma unroll
-                for (int k = 0; k < kPipeKq; ++k)
-#pragma unroll
-                    for (int q = 0; q < CPT; ++q) {
-                        const float4 zk = *reinterpret_cast<const float4*>(zbp[q] + (size_t)k * UPC * ZP * 4);
-                        z[q][0] += zk.x; z[q][1] += zk.y; z[q][2] += zk.z; z[q][3] += zk.w;
-                    }
                 mbar_arrive(zfree0 + 8u * zb);   // the buffer may be overwritten: its sums are in registers
                 asm volatile("cp.async.wait_group %0;" ::"n"(NG - 1) : "memory");   // this phase's input terms have landed
                 __half hh[CPT];
@@ -1350,78 +1411,90 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
                 for (int q = 0; q < CPT; ++q) {
                     const int o = q % OCT, gn = (gt >> 3) + 16 * (q / OCT), n = g * BPG + gn;
                     float4 gx = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (gn < BPG && n < B) gx = gxs[((size_t)g * CPT + q) * kPipeGateThreads + gt];
+                    if (gn < BPG && n < B) gx = gxs[(g * CPT + q) * kPipeGateThreads + gt];
                     // order of the additions: input term + bias first, then the sum of the four partials
-                    const float zi = (gx.x + bias4[o].x) + z[q][0], zf = (gx.y + bias4[o].y) + z[q][1],
-                                zg = (gx.z + bias4[o].z) + z[q][2], zo = (gx.w + bias4[o].w) + z[q][3];
+                    const float zi = (gx.x + bias4[o].x) + z[q].x, zf = (gx.y + bias4[o].y) + z[q].y,
+                                zg = (gx.z + bias4[o].z) + z[q].z, zo = (gx.w + bias4[o].w) + z[q].w;
                     c[g][q] = sigmoidf_(zf) * c[g][q] + sigmoidf_(zi) * tanhf_(zg);
                     hh[q] = __float2half_rn(sigmoidf_(zo) * tanhf_(c[g][q]));
                 }
+                uint32_t pair[CPT];
 #pragma unroll
                 for (int q = 0; q < CPT; ++q) {
-                    const int o = q % OCT, gn = (gt >> 3) + 16 * (q / OCT), n = g * BPG + gn, u = u0 + 8 * o + gl;
-                    const bool live = gn < BPG && n < B;
-                    // the octet's record {units 0..7} lands in the lane of unit 0
                     const uint32_t v = (uint32_t)__half_as_ushort(hh[q]);
-                    const uint32_t p1 = v | (__shfl_down_sync(0xffffffffu, v, 1, 8) << 16);
-                    const uint32_t p2 = __shfl_down_sync(0xffffffffu, p1, 2, 8);
-                    const uint32_t q1 = __shfl_down_sync(0xffffffffu, p1, 4, 8);
-                    const uint32_t q2 = __shfl_down_sync(0xffffffffu, p2, 4, 8);
-                    if (live) {
-                        const size_t nn = (size_t)(seq0 + n);
-                        if (gl == 0) {
-                            const uint4 rec = make_uint4(p1, p2, q1, q2);
-                            if (s + 1 < T)
-                                a.data[((((size_t)par * a.halves + half) * NG + g) * (H >> 3) + (size_t)slice * OCT + o) * BPG + gn] = rec;
-                            if (a.y_vec) *reinterpret_cast<uint4*>(a.y + (size_t)t * a.y_tstride + nn * a.y_bstride + u0 + 8 * o) = rec;
-                        }
-                        if (!a.y_vec) a.y[(size_t)t * a.y_tstride + nn * a.y_bstride + u] = hh[q];
+                    pair[q] = v | (__shfl_down_sync(0xffffffffu, v, 1, 8) << 16);
+                }
+                // records (of absent sequences too, or the readers would wait for them): four 32-bit stores of even lanes
+                if (s + 1 < T && (gl & 1) == 0) {
+#pragma unroll
+                    for (int q = 0; q < CPT; ++q) {
+                        const int o = q % OCT, sb = q / OCT;
+                        if ((gt >> 3) + 16 * sb < BPG)
+                            asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(record_s + ((size_t)g * group_words + o * BPG + 16 * sb) * 4), "r"(pair[q]) : "memory");
+                    }
+                }
+                // release (CTA scope): the group's exchange warp starts counting when this phase completes
+                mbar_arrive(done0 + 8u * g);
+#pragma unroll
+                for (int q = 0; q < CPT; ++q) {
+                    const int o = q % OCT, sb = q / OCT, gn = (gt >> 3) + 16 * sb, n = g * BPG + gn;
+                    if (gn < BPG && n < B) {
+                        __half* yp = y_row + (long)(g * BPG + 16 * sb) * a.y_bstride + 8 * o;
+                        if (!y_pairs) *yp = hh[q];
+                        else if ((gl & 1) == 0) *reinterpret_cast<uint32_t*>(yp) = pair[q];
                         if (s == T - 1) {
-                            if (a.hn) a.hn[nn * H + u] = hh[q];
-                            if (a.cn) a.cn[nn * H + u] = __float2half_rn(c[g][q]);
+                            const size_t at = (size_t)(seq0 + n) * H + u0 + 8 * o + gl;
+                            if (a.hn) a.hn[at] = hh[q];
+                            if (a.cn) a.cn[at] = __float2half_rn(c[g][q]);
                         }
                     }
                 }
-                // release (CTA scope): the group's exchange warp raises the step flag after this phase completes; its
-                // cross-proxy fence and gpu-scope release are cumulative over the record stores above
-                mbar_arrive(done0 + 8u * g);
-                if (s + 1 < T) prefetch_gx(g, a.reverse ? t - 1 : t + 1);
+                if (s + 1 < T) prefetch_gx(g);
                 else asm volatile("cp.async.commit_group;" ::: "memory");
                 if (tr && gt == 0 && g == 0) tr[5] = clock64();
                 ++phase;
             }
+            y_row += y_step;
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
         if (dead && lane == 0) status_raise(a.status, a.gen, PIMB200_ERR_TIMEOUT);
     } else {
         // ================================ exchange warps: warp 12 + g serves group g ================================
+        if (UPC == 16) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;" ::: "memory");
+        else asm volatile("setmaxnreg.dec.sync.aligned.u32 120;" ::: "memory");
         const int g = warp - (kPipeTensorWarps + kPipeGateWarps);
         if (g < ng_live) {
             const int rep = blockIdx.x % kBulkFlagCopies;
             const uint32_t dst = (uint32_t)__cvta_generic_to_shared(hs + (size_t)g * BPG * H);
             const uint32_t fbar = full0 + 8u * g;
+            uint4* const group0 = a.set + ((size_t)half * NG + g) * group_words;
+            uint4* const mine = group0 + (size_t)slice * OCT * BPG;
             bool dead = false;
             for (int s = 0; s + 1 < T && !dead; ++s) {
                 const int par = s & 1;
                 const uint32_t tag = a.tag_base + (uint32_t)s + 1u;
                 long long* tr = a.trace ? a.trace + ((size_t)blockIdx.x * T + s) * 8 : nullptr;
+                // ---- sentinels for step s + 2: everyone has read what lies there (step s - 2), since everyone's records of
+                //      step s - 1 have been here; the fence is ahead of "full", and so of this CTA's records of step s + 1
+                for (int i = lane; i < OCT * BPG; i += 32)
+                    asm volatile("st.relaxed.gpu.global.v4.b32 [%0], {%1,%1,%1,%1};" ::"l"(mine + (size_t)((s + 2) & 3) * buf_words + i), "r"(~0u) : "memory");
+                __threadfence();
                 if (!mbar_wait_polls(done0 + 8u * g, (uint32_t)(s & 1), a.status, a.gen, wait_limit)) break;
-                // ---- publish: the gate warps' records are out; raise this CTA's step flag in every replica.  The records
-                //      are read by the other CTAs' bulk copies (async proxy): the cross-proxy fence sits on the writer
-                //      side, here, where its wait for the record stores is the wait the release needs anyway (on the
-                //      reader side, in front of the copy, it was measured to cost several thousand cycles per step)
+                // ---- publish: raise this CTA's step flag in every replica, right behind the records (no release: the tensor
+                //      warps look for sentinels).  The records are read by the other CTAs' bulk copies (async proxy): the
+                //      cross-proxy fence sits on the writer's side (in front of the copy it costs several thousand cycles)
                 if (lane < kBulkFlagCopies) asm volatile("fence.proxy.async.global;" ::: "memory");
                 if (lane < kBulkFlagCopies)
-                    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(
-                                     a.flags + ((((((size_t)lane * 2 + par) * kPipeMaxHalves + half) * kPipeMaxGroups + g) * n_slices + slice) * 32)),
+                    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(
+                                     a.flags + ((((((size_t)lane * 2 + par) * 2 + half) * kPipeMaxGroups + g) * n_slices + slice) * 32)),
                                  "r"(tag)
                                  : "memory");
                 if (tr && lane == 0 && g == 0) tr[6] = clock64();
                 // ---- gather: lane l watches slice 32i + l of every chunk i; a chunk's records go to the bulk-copy
                 //      engine as soon as its 32 flags are up
-                const uint32_t* fbase = a.flags + (((((size_t)rep * 2 + par) * kPipeMaxHalves + half) * kPipeMaxGroups + g) * n_slices) * 32;
+                const uint32_t* fbase = a.flags + (((((size_t)rep * 2 + par) * 2 + half) * kPipeMaxGroups + g) * n_slices) * 32;
                 const unsigned char* src =
-                    reinterpret_cast<const unsigned char*>(a.data + (((size_t)par * a.halves + half) * NG + g) * (H >> 3) * BPG);
+                    reinterpret_cast<const unsigned char*>(group0 + (size_t)(s & 3) * buf_words);
                 uint32_t seen = 0;      // bit i: this lane's flag of chunk i carries the tag (or there is no such CTA)
                 uint32_t issued = 0;    // bit i: chunk i's copy has been handed to the copy engine (warp-uniform)
 #pragma unroll
@@ -1448,16 +1521,6 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
 #pragma unroll
                     for (int i = 0; i < kPipeMaxChunks; ++i) {
                         if ((issued >> i & 1u) || !__all_sync(0xffffffffu, seen >> i & 1u)) continue;
-                        // acquire: one acquire load of the flag just seen (polling with acquire loads was measured far
-                        // slower); the warp-wide sync orders every lane's acquire before lane 0's copy
-                        if (i * kPipeChunk + lane < n_slices) {
-                            uint32_t w;
-                            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];"
-                                         : "=r"(w)
-                                         : "l"(fbase + (size_t)(i * kPipeChunk + lane) * 32)
-                                         : "memory");
-                        }
-                        __syncwarp();
                         if (lane == 0) {
                             const int c0 = i * kPipeChunk, c1 = c0 + kPipeChunk < n_slices ? c0 + kPipeChunk : n_slices;
                             const uint32_t off = (uint32_t)c0 * OCT * BPG * 16u, len = (uint32_t)(c1 - c0) * OCT * BPG * 16u;
@@ -1768,6 +1831,8 @@ struct pimb200_lstm {
     uint4* xchg = nullptr;  // [kXchgCopies][2][kXchgWords]
     uint4* direct_buf = nullptr;     // few sequences: two sets of four record buffers, used by alternate launches
     unsigned direct_launches = 0;
+    uint4* pipe_buf = nullptr;       // the same for the pipelined kernel
+    unsigned pipe_launches = 0;
     uint4* bulk_data = nullptr;      // batched variant: [2][n_cta][32] records
     uint32_t* bulk_flags = nullptr;  // [2][n_cta]
     uint32_t bulk_tag = 0;
@@ -1845,10 +1910,10 @@ extern "C" int pimb200_lstm_create(const void* const* params, int n_params, int 
     size_t at = 0;
     auto take = [&](size_t bytes) { const size_t p = at; at += (bytes + 255) & ~size_t(255); return p; };
     const size_t o_status = take(8), o_xchg = take(kXchgBytes);
-    // the pipelined kernel's layouts of flags and records (up to kPipeMaxB sequences) are the largest
-    const size_t o_flags = take((size_t)kBulkFlagCopies * 2 * kPipeMaxHalves * kPipeMaxGroups * ncta * 128);
+    const size_t o_flags = take((size_t)kBulkFlagCopies * 2 * 2 * kPipeMaxGroups * ncta * 128);
     const size_t zeros = at;
-    const size_t o_direct = take(kDirectBytes), o_data = take(2 * ncta * kPipeMaxB * 16);
+    const size_t o_direct = take(kDirectBytes), o_pipe = take(kPipeBytes), sentinels = at - o_direct;
+    const size_t o_data = take(2 * ncta * kBulkMaxB * 16);
     std::vector<size_t> o_w;
     for (int l = 0; l < num_layers; ++l)
         for (int d = 0; d < D; ++d) {
@@ -1858,11 +1923,12 @@ extern "C" int pimb200_lstm_create(const void* const* params, int n_params, int 
         }
     if (cudaMalloc(&h->arena, at) != cudaSuccess) return fail(PIMB200_ERR_NO_MEMORY);
     cudaMemset(h->arena, 0, zeros);
-    cudaMemset(h->arena + o_direct, 0xff, kDirectBytes);
+    cudaMemset(h->arena + o_direct, 0xff, sentinels);
     h->d_status = reinterpret_cast<int*>(h->arena + o_status);
     h->xchg = reinterpret_cast<uint4*>(h->arena + o_xchg);
     h->bulk_flags = reinterpret_cast<uint32_t*>(h->arena + o_flags);
     h->direct_buf = reinterpret_cast<uint4*>(h->arena + o_direct);
+    h->pipe_buf = reinterpret_cast<uint4*>(h->arena + o_pipe);
     h->bulk_data = reinterpret_cast<uint4*>(h->arena + o_data);
     for (int l = 0; l < num_layers; ++l) {
         for (int d = 0; d < D; ++d) {
@@ -2124,11 +2190,13 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
             PipeArgs a;
             a.Whh = h->w_hh[ld]; a.bias = h->bias[ld]; a.G = G; a.g_tstride = g_tstride; a.g_bstride = g_bstride;
             a.h0 = h0; a.c0 = c0; a.y = y; a.y_tstride = y_tstride; a.y_bstride = y_bstride; a.hn = hn; a.cn = cn;
-            a.y_vec = (aligned16(y) && y_tstride % 8 == 0 && y_bstride % 8 == 0) ? 1 : 0;
-            a.data = h->bulk_data; a.flags = h->bulk_flags; a.tag_base = h->bulk_tag; a.status = h->d_status; a.gen = next_gen(h);
+            const unsigned turn = h->pipe_launches++ & 1;
+            a.flags = h->bulk_flags; a.tag_base = h->bulk_tag;
+            h->bulk_tag += (uint32_t)T + 1u;
+            a.set = h->pipe_buf + turn * kPipeSetWords; a.other_set = h->pipe_buf + (turn ^ 1) * kPipeSetWords;
+            a.status = h->d_status; a.gen = next_gen(h);
             a.H = H; a.T = T; a.B = B; a.halves = halves; a.reverse = reverse ? 1 : 0; a.poll_limit = h->poll_limit;
             a.trace = h->trace;
-            h->bulk_tag += (uint32_t)T + 1u;
             const void* fn = nullptr;
             if (upc == 16) {
                 fn = (const void*)lstm_persistent_pipe_kernel<16, 2, 4>;
