@@ -25,6 +25,7 @@
 //                     tcgen05 variant (measured slower).
 // Weights are stored gate-interleaved (packed row u*4+g = original row g*H+u) so the four gate
 // rows of one hidden unit are contiguous and its four pre-activations are one float4 of G.
+#include <algorithm>
 #include <cstdlib>
 #include <mutex>
 #include <vector>
@@ -1076,9 +1077,10 @@ __global__ void __launch_bounds__(kWideThreads, 1) lstm_persistent_wide_kernel(B
 // hidden value has (see lstm_direct.cu: four buffers in turn, this CTA's records of buffer (s + 2) % 4 made sentinels in step
 // s, two sets of buffers for alternate launches).  It is a NaN, so a copy that was too early shows in the tensor warps' sums,
 // without any instruction in their product; they then wait for the records themselves (seen in 1 of 10^4 phases).
-// Measured at H = 1024, us per step: 48 sequences 3.89 -> 3.19, 64 4.13 -> 3.45, 128 4.82 -> 4.78 (with the gate warps'
-// shorter phase: running addresses, 32-bit record stores, 1660 -> 830 cycles at 128; there the tensor warps, 4 x 2000 cycles,
-// are as long as a group's chain).  Copies without flags, timed like the looks of lstm_direct.cu, drift apart: a CTA that
+// Measured at H = 1024, us per step: 48 sequences 3.89 -> 2.94, 64 4.13 -> 3.14, 128 4.82 -> 3.91, together with the gate
+// warps' shorter phase (running addresses, 32-bit record stores: 1660 -> 900 cycles at 128) and the tensor warps' (operands
+// by ldmatrix, the barriers' state asked for ahead of its use, one arrival per warp: 4 x 1500 cycles at 128, of which the
+// products alone are 4 x 1024).  Copies without flags, timed like the looks of lstm_direct.cu, drift apart: a CTA that
 // looks too early holds up all others, whose looks move out in turn (5.9 us at 128).
 // The exchange of one group runs under the arithmetic of the other groups; a step of all groups takes as long as one
 // group's chain or as the busiest stage, whichever is longer.
@@ -1098,6 +1100,9 @@ constexpr int kPipeKtw = 16;         // k-tiles per tensor warp held in register
 constexpr int kPipeMaxGroups = 4;    // one exchange warp per group
 constexpr int kPipeMaxB = 128;       // sequences per launch: 2 halves x 4 groups x 16
 constexpr int kPipeChunk = 32;       // CTAs per copied piece of a group's records (one flag per lane)
+constexpr unsigned kPipeFirstLook = 800;   // cycles from a CTA's own flag to its first look at the others'
+constexpr int kPipeFlagWords = 32;   // a flag has a 128-byte line: 4.8 us per step with a word each (48 sequences), 3.7 with 32 bytes
+constexpr int kPipeFlagCopies = 2;   // replicas of the flags; 4 and 8 cost 1 and 2 % at 48 sequences, nothing at 128
 constexpr int kPipeMaxChunks = 4;    // H <= 1024: at most 128 CTAs per half
 constexpr size_t kPipeSetWords = (size_t)4 * kPipeMaxB * 128;   // records of four buffers
 constexpr size_t kPipeBytes = 2 * kPipeSetWords * 16;
@@ -1115,7 +1120,7 @@ struct PipeArgs {
     __half* cn;
     uint4* set;             // [4 buffers][halves][NG][H/8 octets][BPG] 16-byte records (the image of a group's hs), all sentinels
     uint4* other_set;       // the next launch's: filled with sentinels by this one
-    uint32_t* flags;        // [kBulkFlagCopies][2 parities][2 halves][kPipeMaxGroups][slices] step tags, one per 128-byte line
+    uint32_t* flags;        // [kPipeFlagCopies][2 parities][2 halves][kPipeMaxGroups][slices] step tags, one per 128-byte line
     uint32_t tag_base;
     int* status;
     int gen;
@@ -1128,6 +1133,18 @@ struct PipeArgs {
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// has the phase of that parity completed?  Does not suspend the thread
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
 }
 // bounded mbarrier wait in polls (not clocks); false = gave up or the launch was aborted
 __device__ __forceinline__ bool mbar_wait_polls(uint32_t bar, uint32_t parity, const int* status, int gen, int limit) {
@@ -1174,11 +1191,11 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
     if (tid == 0) {
         for (int g = 0; g < NG; ++g) {
             pimb200::tc::mbar_init(full0 + 8u * g, (uint32_t)nchunks);          // one arrival (+ bytes) per chunk
-            pimb200::tc::mbar_init(done0 + 8u * g, (uint32_t)kPipeGateThreads);
+            pimb200::tc::mbar_init(done0 + 8u * g, (uint32_t)kPipeGateWarps);
         }
         for (int b = 0; b < 2; ++b) {
-            pimb200::tc::mbar_init(zready0 + 8u * b, (uint32_t)kPipeTensorThreads);
-            pimb200::tc::mbar_init(zfree0 + 8u * b, (uint32_t)kPipeGateThreads);
+            pimb200::tc::mbar_init(zready0 + 8u * b, (uint32_t)kPipeTensorWarps);
+            pimb200::tc::mbar_init(zfree0 + 8u * b, (uint32_t)kPipeGateWarps);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -1221,14 +1238,15 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
                     }
         }
         int phase = 0;      // group phases executed so far: selects the partial-sum buffer
+        bool full = true;   // this lane has seen the next phase's records complete
         bool dead = false;
         for (int s = 0; s < T && !dead; ++s) {
             long long* tr = a.trace ? a.trace + ((size_t)blockIdx.x * T + s) * 8 : nullptr;
             for (int g = 0; g < ng_live; ++g, ++phase) {
                 const int zb = phase & 1;
                 if (tr && tid == 0 && g == 0) tr[0] = clock64();
-                bool ok = true;
-                if (s > 0) ok = mbar_wait_polls(full0 + 8u * g, (uint32_t)((s - 1) & 1), a.status, a.gen, wait_limit);
+                bool ok = full;
+                if (!__all_sync(0xffffffffu, ok)) ok = ok || mbar_wait_polls(full0 + 8u * g, (uint32_t)((s - 1) & 1), a.status, a.gen, wait_limit);
                 if (tr && tid == 0 && g == 0) tr[1] = clock64();
                 if (!__all_sync(0xffffffffu, ok)) { dead = true; break; }
                 if (tr && tid == 0 && g == 0) tr[2] = clock64();
@@ -1240,19 +1258,25 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
                     for (int j = 0; j < NTG; ++j)
 #pragma unroll
                         for (int i = 0; i < 4; ++i) acc[m][j][i] = 0.f;
-                const __half* brow = hs + (size_t)g * BPG * H + (size_t)b_n * 8 + b_k;
+                // ldmatrix: lane l names row l % 8 (a sequence's record) of matrix l / 8 = (8 sequences, half of the k-tile)
+                const uint32_t brow = (uint32_t)__cvta_generic_to_shared(hs + (size_t)g * BPG * H) + (uint32_t)(((lane >> 3 & 1) * BPG + (lane >> 4 & (NTG > 1)) * 8 + (lane & 7)) * 16);
                 // the partial-sum buffer must have been read by the gate warps (its use two phases ago): asked here, needed
                 // after the product
                 const uint32_t zfree_parity = (uint32_t)(((phase >> 1) - 1) & 1);
-                const bool zfree = phase < 2 || pimb200::tc::mbar_try_wait(zfree0 + 8u * zb, zfree_parity);
+                const bool zfree = phase < 2 || mbar_test(zfree0 + 8u * zb, zfree_parity);
                 auto ktile = [&](int i) {
                     const int kt = kPipeKq * i + kq;
-                    const __half* hp = brow + (size_t)(2 * kt) * BPG * 8;
+                    const uint32_t hp = brow + (uint32_t)(2 * kt) * BPG * 16;
                     uint32_t b0[NTG], b1[NTG];
+                    if (NTG == 1) {
+                        asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(b0[0]), "=r"(b1[0]) : "r"(hp) : "memory");
+                    } else {
 #pragma unroll
-                    for (int j = 0; j < NTG; ++j) {
-                        b0[j] = *reinterpret_cast<const uint32_t*>(hp + j * 64);
-                        b1[j] = *reinterpret_cast<const uint32_t*>(hp + j * 64 + (size_t)BPG * 8);
+                        for (int j = 0; j + 1 < NTG; j += 2)
+                            asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                                         : "=r"(b0[j]), "=r"(b1[j]), "=r"(b0[j + 1]), "=r"(b1[j + 1])
+                                         : "r"(hp + j * 128)
+                                         : "memory");
                     }
 #pragma unroll
                     for (int j = 0; j < NTG; ++j)
@@ -1313,6 +1337,11 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
                     ok = zfree || mbar_wait_polls(zfree0 + 8u * zb, zfree_parity, a.status, a.gen, wait_limit);
                     if (!__all_sync(0xffffffffu, ok)) { dead = true; break; }
                 }
+                // the next phase's records: asked for here, needed after this phase's epilogue
+                {
+                    const bool wrap = g + 1 == ng_live;
+                    full = s + (wrap ? 1 : 0) == 0 || mbar_test(full0 + 8u * (wrap ? 0 : g + 1), (uint32_t)((wrap ? s : s - 1) & 1));
+                }
 #pragma unroll
                 for (int m = 0; m < MTW; ++m)
 #pragma unroll
@@ -1322,7 +1351,8 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
                             const int r = (mh * MTW + m) * 16 + b_n + (i >> 1) * 8, n = j * 8 + b_k + (i & 1);
                             zq[((size_t)(r >> 2) * ZP + n) * 4 + (r & 3)] = acc[m][j][i];
                         }
-                mbar_arrive(zready0 + 8u * zb);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(zready0 + 8u * zb);   // (an arrival per thread takes the barrier 32 times as long)
                 if (tr && tid == 0 && g == 0) tr[3] = clock64();
             }
         }
@@ -1404,7 +1434,8 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
                     z[q] = make_float4((zk[0].x + zk[1].x) + (zk[2].x + zk[3].x), (zk[0].y + zk[1].y) + (zk[2].y + zk[3].y),
                                        (zk[0].z + zk[1].z) + (zk[2].z + zk[3].z), (zk[0].w + zk[1].w) + (zk[2].w + zk[3].w));
                 }
-                mbar_arrive(zfree0 + 8u * zb);   // the buffer may be overwritten: its sums are in registers
+                __syncwarp();
+                if (lane == 0) mbar_arrive(zfree0 + 8u * zb);   // the buffer may be overwritten: its sums are in registers
                 asm volatile("cp.async.wait_group %0;" ::"n"(NG - 1) : "memory");   // this phase's input terms have landed
                 __half hh[CPT];
 #pragma unroll
@@ -1434,7 +1465,8 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
                     }
                 }
                 // release (CTA scope): the group's exchange warp starts counting when this phase completes
-                mbar_arrive(done0 + 8u * g);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(done0 + 8u * g);
 #pragma unroll
                 for (int q = 0; q < CPT; ++q) {
                     const int o = q % OCT, sb = q / OCT, gn = (gt >> 3) + 16 * sb, n = g * BPG + gn;
@@ -1464,7 +1496,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
         else asm volatile("setmaxnreg.dec.sync.aligned.u32 120;" ::: "memory");
         const int g = warp - (kPipeTensorWarps + kPipeGateWarps);
         if (g < ng_live) {
-            const int rep = blockIdx.x % kBulkFlagCopies;
+            const int rep = blockIdx.x % kPipeFlagCopies;
             const uint32_t dst = (uint32_t)__cvta_generic_to_shared(hs + (size_t)g * BPG * H);
             const uint32_t fbar = full0 + 8u * g;
             uint4* const group0 = a.set + ((size_t)half * NG + g) * group_words;
@@ -1483,16 +1515,19 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
                 // ---- publish: raise this CTA's step flag in every replica, right behind the records (no release: the tensor
                 //      warps look for sentinels).  The records are read by the other CTAs' bulk copies (async proxy): the
                 //      cross-proxy fence sits on the writer's side (in front of the copy it costs several thousand cycles)
-                if (lane < kBulkFlagCopies) asm volatile("fence.proxy.async.global;" ::: "memory");
-                if (lane < kBulkFlagCopies)
+                if (lane < kPipeFlagCopies) asm volatile("fence.proxy.async.global;" ::: "memory");
+                if (lane < kPipeFlagCopies)
                     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(
-                                     a.flags + ((((((size_t)lane * 2 + par) * 2 + half) * kPipeMaxGroups + g) * n_slices + slice) * 32)),
+                                     a.flags + ((((((size_t)lane * 2 + par) * 2 + half) * kPipeMaxGroups + g) * n_slices + slice) * kPipeFlagWords)),
                                  "r"(tag)
                                  : "memory");
                 if (tr && lane == 0 && g == 0) tr[6] = clock64();
+                // (a look before anyone's flag can be here only keeps the L2 from them)
+                const unsigned t0 = (unsigned)clock();
+                while ((unsigned)clock() - t0 < kPipeFirstLook) {}
                 // ---- gather: lane l watches slice 32i + l of every chunk i; a chunk's records go to the bulk-copy
                 //      engine as soon as its 32 flags are up
-                const uint32_t* fbase = a.flags + (((((size_t)rep * 2 + par) * 2 + half) * kPipeMaxGroups + g) * n_slices) * 32;
+                const uint32_t* fbase = a.flags + (((((size_t)rep * 2 + par) * 2 + half) * kPipeMaxGroups + g) * n_slices) * kPipeFlagWords;
                 const unsigned char* src =
                     reinterpret_cast<const unsigned char*>(group0 + (size_t)(s & 3) * buf_words);
                 uint32_t seen = 0;      // bit i: this lane's flag of chunk i carries the tag (or there is no such CTA)
@@ -1504,6 +1539,20 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
                 constexpr uint32_t all_chunks = (1u << kPipeMaxChunks) - 1u;
                 int polls = 0;
                 while (issued != all_chunks) {
+                    ++polls;
+                    bool lost = polls >= a.poll_limit;   // (ahead of the look: a limit of one is no wait at all)
+                    if ((polls & 255) == 0 && status_aborted(a.status, a.gen)) lost = true;
+                    if (__any_sync(0xffffffffu, lost)) {
+                        // a flag never came: arrive without bytes for the chunks not issued, so that the barrier still
+                        // completes once the copies that were issued have landed; then leave
+                        if (lane == 0) {
+                            status_raise(a.status, a.gen, PIMB200_ERR_TIMEOUT);
+                            for (int i = 0; i < nchunks; ++i)
+                                if (!(issued >> i & 1u)) mbar_arrive(fbar);
+                        }
+                        dead = true;
+                        break;
+                    }
                     // all of this lane's outstanding flags are loaded before any is looked at: up to four loads in flight
                     uint32_t v[kPipeMaxChunks];
 #pragma unroll
@@ -1512,7 +1561,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
                         if (!(seen >> i & 1u))
                             asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];"
                                          : "=r"(v[i])
-                                         : "l"(fbase + (size_t)(i * kPipeChunk + lane) * 32)
+                                         : "l"(fbase + (size_t)(i * kPipeChunk + lane) * kPipeFlagWords)
                                          : "memory");
                     }
 #pragma unroll
@@ -1531,21 +1580,6 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
                                 : "memory");
                         }
                         issued |= 1u << i;
-                    }
-                    if (issued == all_chunks) break;
-                    ++polls;
-                    bool lost = polls >= a.poll_limit;
-                    if ((polls & 255) == 0 && status_aborted(a.status, a.gen)) lost = true;
-                    if (__any_sync(0xffffffffu, lost)) {
-                        // a flag never came: arrive without bytes for the chunks not issued, so that the barrier still
-                        // completes once the copies that were issued have landed; then leave
-                        if (lane == 0) {
-                            status_raise(a.status, a.gen, PIMB200_ERR_TIMEOUT);
-                            for (int i = 0; i < nchunks; ++i)
-                                if (!(issued >> i & 1u)) mbar_arrive(fbar);
-                        }
-                        dead = true;
-                        break;
                     }
                 }
                 if (tr && lane == 0 && g == 0) tr[7] = clock64();
@@ -1910,7 +1944,7 @@ extern "C" int pimb200_lstm_create(const void* const* params, int n_params, int 
     size_t at = 0;
     auto take = [&](size_t bytes) { const size_t p = at; at += (bytes + 255) & ~size_t(255); return p; };
     const size_t o_status = take(8), o_xchg = take(kXchgBytes);
-    const size_t o_flags = take((size_t)kBulkFlagCopies * 2 * 2 * kPipeMaxGroups * ncta * 128);
+    const size_t o_flags = take(std::max((size_t)kBulkFlagCopies * 2, (size_t)kPipeFlagCopies * 2 * 2 * kPipeMaxGroups) * ncta * kPipeFlagWords * 4);
     const size_t zeros = at;
     const size_t o_direct = take(kDirectBytes), o_pipe = take(kPipeBytes), sentinels = at - o_direct;
     const size_t o_data = take(2 * ncta * kBulkMaxB * 16);
