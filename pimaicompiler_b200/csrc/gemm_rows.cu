@@ -112,6 +112,12 @@ __device__ __forceinline__ void store_half16(__half* p, const uint32_t* w) {
     q[1] = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
+// the larger of the two, NaN where either is one (fmaxf would turn a NaN of the inputs into -inf)
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float m;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+    return m;
+}
 // The producer's and the issuer's loops run with all 32 lanes, and only the instructions themselves are predicated on one
 // elected lane (`el`).  Inside an `if (lane == 0)` the compiler keeps addresses and descriptors in per-thread registers and
 // moves each to the uniform ones that these instructions take: the issuer then needed 600 cycles per K block and the
@@ -382,8 +388,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
                             for (int i = 0; i < CH; ++i) {
                                 if (n0 + c + i >= n_end) break;
                                 const size_t at = (size_t)j * a.ldy + n0 + c + i;
-                                if (EPI == kRowsHalf) static_cast<__half*>(a.Y)[at] = __float2half_rn(fmaxf(f[i], lo));
-                                else static_cast<float*>(a.Y)[at] = fmaxf(f[i], lo);
+                                if (EPI == kRowsHalf) static_cast<__half*>(a.Y)[at] = __float2half_rn(max_nan(f[i], lo));
+                                else static_cast<float*>(a.Y)[at] = max_nan(f[i], lo);
                             }
                         }
                         __syncwarp();
@@ -394,11 +400,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
                     for (int i = 0; i < 8; ++i) {
                         if (EPI == kRowsHalf) {
                             const float* g = f + (8 * i) % CH;
-                            o[i] = make_uint4(pack2(fmaxf(g[0], lo), fmaxf(g[1], lo)), pack2(fmaxf(g[2], lo), fmaxf(g[3], lo)),
-                                              pack2(fmaxf(g[4 % CH], lo), fmaxf(g[5 % CH], lo)), pack2(fmaxf(g[6 % CH], lo), fmaxf(g[7 % CH], lo)));
+                            o[i] = make_uint4(pack2(max_nan(g[0], lo), max_nan(g[1], lo)), pack2(max_nan(g[2], lo), max_nan(g[3], lo)),
+                                              pack2(max_nan(g[4 % CH], lo), max_nan(g[5 % CH], lo)), pack2(max_nan(g[6 % CH], lo), max_nan(g[7 % CH], lo)));
                         } else {
-                            o[i] = make_uint4(__float_as_uint(fmaxf(f[4 * i], lo)), __float_as_uint(fmaxf(f[4 * i + 1], lo)),
-                                              __float_as_uint(fmaxf(f[4 * i + 2], lo)), __float_as_uint(fmaxf(f[4 * i + 3], lo)));
+                            o[i] = make_uint4(__float_as_uint(max_nan(f[4 * i], lo)), __float_as_uint(max_nan(f[4 * i + 1], lo)),
+                                              __float_as_uint(max_nan(f[4 * i + 2], lo)), __float_as_uint(max_nan(f[4 * i + 3], lo)));
                         }
                     }
                     if (n0 + c + CH > n_end && n_end < a.N) {          // half a chunk left of this tile: the map's boxes are whole ones
