@@ -338,10 +338,10 @@ int pimb200_lstm_profile_read(pimb200_lstm* h, double* total_ms, long* recurrenc
 int pimb200_lstm_set_use_tc(pimb200_lstm* h, int on);
 
 /* A/B switch between the batched persistent recurrences (lock-step sequences, H <= 1024): 2 (default) = the
- * pipelined kernel for 33..128 sequences (W_hh slice in registers; the sequences advance as independent groups, so
+ * pipelined kernel for 17..128 sequences (W_hh slice in registers; the sequences advance as independent groups, so
  * one group's hidden-state exchange runs under the other groups' arithmetic; 65..128 sequences as two batch halves)
- * and, for 1..32 sequences, the kernel with the exchange on the compute warps (shorter critical path when there is
- * nothing to overlap); 3 = the pipelined kernel for every batch size; 1 = the exchange-on-compute-warps kernel for
+ * and, for 1..16 sequences, the kernel that polls the other CTAs' records straight into registers; 3 = the pipelined
+ * kernel for every batch size; 1 = the kernel with the exchange on the compute warps for
  * 1..64 sequences; 0 = the K-split kernel with W_hh in shared memory (up to 32 sequences; also what H > 1024 falls
  * back to).  Results agree within the LSTM tolerance; within one kernel they do not depend on the batch size.  No
  * counterpart in the reference. */

@@ -13,16 +13,16 @@
 //                     128-bit loads; any B, any H; the form used by seq_len==1 decoder calls
 //        persistent — one cooperative launch for all T steps; every CTA keeps its slice of W_hh on
 //                     chip for the whole sequence and the CTAs exchange the new hidden states through
-//                     L2 once per step (16-byte records + per-CTA step flags + bulk-copy gather).
-//                     Defaults (H <= 1024, slice in registers as mma fragments): 1..32 lock-step
-//                     sequences run lstm_persistent_wide_kernel (exchange on the compute warps: the
-//                     shortest critical path when there is little to overlap), 33..128 run
+//                     L2 once per step.  Defaults (H <= 1024, slice in registers as mma fragments):
+//                     1..16 lock-step sequences, and two layers of up to 8, run lstm_direct.cu (records
+//                     polled straight into the registers that multiply them), 17..128 run
 //                     lstm_persistent_pipe_kernel (warp-specialised; independent sequence groups,
 //                     so one group's exchange runs under the others' arithmetic; 65..128 as two
-//                     batch halves on CTAs of 16 units).  Kept beside them: the K-split kernel with
-//                     the slice in shared memory (2..32 sequences, any H that fits), the tagged-word
-//                     kernel (up to 8 sequences, data and flag in one 16-byte word) and an opt-in
-//                     tcgen05 variant (measured slower).
+//                     batch halves on CTAs of 16 units).  Kept beside them: the wide kernel (exchange
+//                     on the compute warps, 1..64 sequences), the K-split kernel with the slice in
+//                     shared memory (2..32 sequences, any H that fits), the tagged-word kernel (up to
+//                     8 sequences, data and flag in one 16-byte word) and an opt-in tcgen05 variant
+//                     (measured slower).
 // Weights are stored gate-interleaved (packed row u*4+g = original row g*H+u) so the four gate
 // rows of one hidden unit are contiguous and its four pre-activations are one float4 of G.
 #include <algorithm>
@@ -1875,7 +1875,7 @@ struct pimb200_lstm {
     uint32_t tag_counter = 0;
     int poll_limit = kPersistPollLimit;
     int use_tc = 0;        // 1 = tcgen05 recurrence for 17..64 sequences (measured slower than mma.sync here: opt-in)
-    int bulk_wide = 2;     // 2 = pipelined kernel for 33..128 sequences, wide kernel below (default), 3 = pipelined kernel
+    int bulk_wide = 2;     // 2 = pipelined kernel for 17..128 sequences (default), 3 = pipelined kernel
                            // for every batch size, 1 = wide kernel (exchange on the compute warps, up to 64 sequences),
                            // 0 = K-split kernel with W_hh in shared memory (up to 32 sequences)
     int pipe_group_size = 0;   // sequences per group of the pipelined kernel: 0 = choose by batch size, else 8, 16 or 32
@@ -2202,22 +2202,22 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
         }
         return PIMB200_OK;
     }
-    // pipelined register-resident recurrence: the default for 33..128 lock-step sequences (below that a step is mostly
-    // exchange latency with little to overlap it with, and the wide kernel's shorter chain wins); 65..128 sequences run
-    // as two batch halves on CTAs of 16 hidden units each
+    // pipelined register-resident recurrence: the default for 17..128 lock-step sequences (17..32 in groups of 8: 2.75 to
+    // 2.83 us per step against 3.26 for the wide kernel; at 16 the direct kernel below takes 2.0); 65..128 sequences run as
+    // two batch halves on CTAs of 16 hidden units each (for 33..64, halves of 16-unit CTAs cost 0.1 to 0.4 us more)
     const bool pipe_shape = wide_ok && !packed && B <= kPipeMaxB && (H / 8 <= h->sm_count) && (B <= 64 || H % 16 == 0);
-    const bool pipe_wanted = h->bulk_wide >= 2 && (B > 32 || h->bulk_wide >= 3);
+    const bool pipe_wanted = h->bulk_wide >= 2 && (B > kDirectMaxSlots || h->bulk_wide >= 3);
     if (pipe_shape && pipe_wanted && !tc_fits &&
         (h->variant == PIMB200_LSTM_PERSISTENT || (h->variant == PIMB200_LSTM_AUTO && T >= 8))) {
         const int upc = B > 64 ? 16 : 8, halves = B > 64 ? 2 : 1;
-        const int b_half = halves == 2 ? 64 : B;   // sequences the first half holds
+        const int b_half = halves == 2 ? (B <= 96 ? 48 : 64) : B;   // sequences the first half holds
         // sequences per group (8, 16 or 32) and the smallest instantiated group count (at most 4) that holds a half
         int bpg = h->pipe_group_size;
-        if (bpg == 0) bpg = 16;
+        if (bpg == 0) bpg = B <= 32 ? 8 : 16;
         if (bpg * kPipeMaxGroups < b_half) bpg = 16;
         if (upc == 16) bpg = 16;
         const int need = ceil_div(b_half, bpg);
-        const int ng = need <= 1 ? 1 : (need <= 2 ? 2 : 4);
+        const int ng = need <= 1 ? 1 : (need <= 2 ? 2 : (upc == 16 ? need : 4));   // (two halves of three groups: 3.97 -> 3.50 us at 96)
         const int ntg = bpg / 8;
         const size_t smem = pipe_smem(H, upc, ntg, ng);
         if ((int)smem <= h->max_smem_optin) {
@@ -2233,7 +2233,7 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
             a.trace = h->trace;
             const void* fn = nullptr;
             if (upc == 16) {
-                fn = (const void*)lstm_persistent_pipe_kernel<16, 2, 4>;
+                fn = ng == 3 ? (const void*)lstm_persistent_pipe_kernel<16, 2, 3> : (const void*)lstm_persistent_pipe_kernel<16, 2, 4>;
             } else {
                 switch (ntg * 16 + ng) {
                     case 1 * 16 + 1: fn = (const void*)lstm_persistent_pipe_kernel<8, 1, 1>; break;

@@ -230,6 +230,29 @@ def test_persistent_bounded_wait_reports_timeout_and_context_survives(B, L):
     assert m.last_status() == _lib.ERR_TIMEOUT
 
 
+@pytest.mark.parametrize("H", [48, 320, 1024])
+@pytest.mark.parametrize("B,L", [(1, 1), (3, 2), (8, 2), (9, 1), (15, 1), (16, 1), (17, 1), (32, 1), (33, 1), (49, 1), (65, 1), (96, 1), (97, 1)])
+def test_recurrence_kernels_at_the_edges_of_their_ranges(B, L, H):
+    # batch sizes where the choice of kernel, its groups or its halves change; more steps than the exchange has buffers;
+    # a sequence of NaNs (the exchange's marker for "not written yet" is one) must leave the others alone
+    ops = _ops()
+    g = torch.Generator().manual_seed(B * 11 + H)
+    T, I = 11, 24
+    ps = lstm_params(L, 1, I, H, g)
+    x = h16(torch.randn(T, B, I, generator=g))
+    h0, c0 = (h16(torch.randn(L, B, H, generator=g) * 0.5) for _ in range(2))
+    ref = co.lstm(x.numpy(), [p.numpy() for p in ps], L, False, True, h0.numpy(), c0.numpy(), False)
+    got = _run(ops, ps, x, h0, c0, L, False, True, False, ops.LSTM_PERSISTENT)
+    for name, a, b in zip(("y", "hn", "cn"), got, ref):
+        assert_close(a, b, LSTM_ATOL, LSTM_RTOL, f"{name} B {B} H {H}")
+    if B > 1:
+        x[3, 1] = float("nan")
+        y = _run(ops, ps, x, h0, c0, L, False, True, False, ops.LSTM_PERSISTENT)[0].cpu()
+        assert torch.isnan(y[3:, 1]).all()
+        keep = [b for b in range(B) if b != 1]
+        assert_close(y[:, keep], ref[0][:, keep], LSTM_ATOL, LSTM_RTOL, f"beside a NaN sequence, B {B} H {H}")
+
+
 @pytest.mark.parametrize("T,B,I,H", [(6, 64, 64, 1024), (9, 23, 32, 256), (5, 40, 16, 128)])
 def test_tcgen05_recurrence_variant_matches_oracle(T, B, I, H):
     # the opt-in tensor-memory variant of the batched recurrence must give the same results as the default kernels
