@@ -143,6 +143,11 @@ __device__ __forceinline__ float rcp_approx(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
+// asks for `bytes` (a multiple of 16, 16-byte aligned) to be brought into L2
+__device__ __forceinline__ void prefetch_l2(const __half* p, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 __device__ __forceinline__ float sigmoidf_(float x) { return rcp_approx(1.0f + __expf(-x)); }
 __device__ __forceinline__ float tanhf_(float x) {
     // tanh(x) = 2*sigmoid(2x) - 1

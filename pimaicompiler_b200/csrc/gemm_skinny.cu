@@ -213,6 +213,9 @@ __global__ void __launch_bounds__(kSkinnyThreads) lstm_cell_skinny_kernel(const 
                     mma16816(acc[m][j], w[u][m][0].z, w[u][m][1].z, w[u][m][0].w, w[u][m][1].w, x[u][j].z, x[u][j].w);
                 }
     };
+    // the CTA's rows of both matrices, 128 to 256 KB, on their way into L2 while the predecessor finishes
+    if (threadIdx.x < 32) prefetch_l2(a.Wx + (size_t)(n0 + lane) * a.I, (uint32_t)a.I * 2);
+    else if (threadIdx.x < 64 && a.h0) prefetch_l2(a.Wh + (size_t)(n0 + lane) * a.H, (uint32_t)a.H * 2);
     load_w(wc, b_lo);
     pdl_wait();
     load_x(xc, b_lo);
