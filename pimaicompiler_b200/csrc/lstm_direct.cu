@@ -18,15 +18,23 @@
 //     contraction index is only a summation order, so lane (sequence g, t) of a block takes units 8t .. 8t+7 of it as one
 //     16-byte record, and W_hh lies in registers (or shared memory) in the same order.  No staging, no barrier between
 //     exchange and product: a warp starts multiplying when its own records are there;
-//   * one handover per step: the product warps store their partial sums (double-buffered), arrive at one of two named
-//     barriers and go on to the next step's records; four gate warps wait there.  A product warp is never two steps ahead
-//     of the gates: the records it needs for that depend on all of this CTA's records of the step between.  Eight lanes
-//     hold the units of one record and store it as four 32-bit words.
+//   * one handover per step: the product warps store their partial sums (double-buffered), arrive at the step's named
+//     barrier and go on to the next step's records; four gate warps wait there.  Eight lanes hold the units of one record
+//     and store it as four 32-bit words.
+// How far a product warp can be ahead of its gates: past its look at the records of step s + 1, it holds a record of a CTA
+// that published step s + 1, so all product warps of that CTA held this CTA's records of step s, so the gates here have left
+// the barrier of step s.  While they wait at that of step s + 1, a product warp is thus at most polling in step s + 3:
+// partial sums of two steps suffice, and four barriers, used in turn, never mix two steps' arrivals.
 // Wavefront: layer B runs two steps behind layer A (see DirectArgs).  Its input product W_ih(B) . h_A of the next step is
 // made from the registers that hold h_A, while the gates work and the records are on their way, and stays in the
 // accumulators that W_hh(B) . h_B then continues.
 // Measured at H = 1024, one sequence: 2.80 -> 1.30 us per step for one layer, 2.72 -> 1.81 for a wavefront.
-// Every wait is bounded; a CTA that gives up raises the status word, and the others, polling, see it.
+// Every wait is bounded; a CTA that gives up raises the status word, and the others, polling, see it.  Giving up keeps the
+// handover exact, or the gates would wait at a barrier for ever: a product warp that gives up in step s notes the step
+// (dead_step keeps the smallest), arrives at that step's barrier and leaves.  The gates pass the barrier of the smallest
+// such step, where every product warp has arrived once, and leave behind it without publishing: what the others hold is
+// thus always the sum of all product warps, and the bound on who can be where, above, holds while CTAs give up too.
+// A warp that gives up in a later step arrives at a barrier that nobody waits for.
 #include "lstm_direct.cuh"
 
 namespace pimb200 {
@@ -37,6 +45,7 @@ constexpr int kGateWarps = 4;                   // 128 cells: 8 units x 16 slots
                                                 // (168 a thread at launch: 8 x 216 + 4 x 72 = 12 x 168)
 constexpr int kThreads = (kWarps + kGateWarps) * 32;
 constexpr int kMaxBlocks = 4;                   // K blocks of 32 per warp: H <= 1024
+constexpr int kNotDead = 0x7fffffff;
 
 __device__ __forceinline__ void mma_16816(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -68,7 +77,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float* zpart = reinterpret_cast<float*>(smem_raw);           // [2][warp][layer][unit][ZP][gate]
     uint4* wib = reinterpret_cast<uint4*>(zpart + 2 * ZBUF);      // W_ih(B): [block][m][row half][lane]
-    __shared__ int dead_step;                                    // 1 + the step at which a wait gave up (0: none)
+    __shared__ int dead_step;                                    // the first step in which a wait gave up
     const int H = a.H, T = a.T, B = a.B;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     const int n_cta = gridDim.x, cta = blockIdx.x, u0 = cta * 8;
@@ -80,7 +89,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
     const int padded = (slots + 1) & ~1;
     const int stride = slots <= 4 ? 4 : (slots <= 8 ? 8 : 16);
     const size_t buf = (size_t)n_cta * stride;
-    if (tid == 0) dead_step = 0;
+    if (tid == 0) dead_step = kNotDead;
     for (int i = tid; i < 2 * ZBUF; i += kThreads) zpart[i] = 0.f;   // (warps without a block never write theirs)
     for (size_t i = (size_t)cta * kThreads + tid; i < kDirectSetWords; i += (size_t)n_cta * kThreads)
         a.other_set[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
@@ -127,7 +136,8 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
             const int t_l = layer == 0 ? s : s - 2;              // the layer's step
             const bool act = live && t_l >= 0 && t_l < T;        // (a layer without a timestep repeats its state)
             float4 z = make_float4(gx.x + bias4.x, gx.y + bias4.y, gx.z + bias4.z, gx.w + bias4.w);
-            asm volatile("bar.sync %0, %1;" ::"r"(1 + (s & 1)), "n"(kThreads) : "memory");   // the partial sums are there
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + (s & 3)), "n"(kThreads) : "memory");   // the partial sums are there
+            const bool lost = dead_step <= s;                    // or some are not (noted ahead of the barrier: the same for every gate thread)
             if (has_cells) {
                 if (act) {
                     float4 q[kWarps];
@@ -141,6 +151,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
                     c = sigmoidf_(z.y) * c + sigmoidf_(z.x) * tanhf_(z.z);
                     hh = __float2half_rn(sigmoidf_(z.w) * tanhf_(c));
                 }
+                if (lost) return;
                 const uint32_t v = (uint32_t)__half_as_ushort(hh);
                 const uint32_t pair = v | (__shfl_down_sync(0xffffffffu, v, 1, 8) << 16);
                 if (live && s < last && (gu & 1) == 0) asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(record), "r"(pair) : "memory");
@@ -156,8 +167,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
                     }
                 }
             }
-            // a wait gave up (written ahead of the barrier: the same for every gate thread; what was published is not used)
-            if (dead_step != 0 && dead_step <= s + 1) return;
+            if (lost) return;
             if (sweeps) {
                 // sentinels for step s + 2; the fence ends ahead of the next barrier, and so of the records of step s + 1
                 if (lane < padded) {
@@ -251,10 +261,10 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
                     // the gate warps leave behind this step's barrier; the other product warps then wait in vain, too
                     if (lane == 0) {
                         status_raise(a.status, a.gen, PIMB200_ERR_TIMEOUT);
-                        dead_step = s + 1;
+                        atomicMin(&dead_step, s);
                     }
                     __syncwarp();
-                    asm volatile("bar.arrive %0, %1;" ::"r"(1 + (s & 1)), "n"(kThreads) : "memory");
+                    asm volatile("bar.arrive %0, %1;" ::"r"(1 + (s & 3)), "n"(kThreads) : "memory");
                     return;
                 }
                 if (all) break;
@@ -294,7 +304,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
                             zb[l * ZL + ((r >> 2) * ZP + n) * 4 + (r & 3)] = acc[l][j][m][e];
                         }
         }
-        asm volatile("bar.arrive %0, %1;" ::"r"(1 + (s & 1)), "n"(kThreads) : "memory");
+        asm volatile("bar.arrive %0, %1;" ::"r"(1 + (s & 3)), "n"(kThreads) : "memory");
         const unsigned handed_over = clock();
         if (LAYERS == 2) {
             // ---- layer B's input product of the next step: B's step s - 1 takes A's output of that step, published in

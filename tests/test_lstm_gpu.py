@@ -230,6 +230,36 @@ def test_persistent_bounded_wait_reports_timeout_and_context_survives(B, L):
     assert m.last_status() == _lib.ERR_TIMEOUT
 
 
+@pytest.mark.parametrize("B,L,H", [(1, 1, 1024), (8, 1, 320), (16, 1, 1024), (1, 2, 1024), (8, 2, 256)])
+def test_waits_that_run_out_in_different_steps(B, L, H):
+    # limits of a few polls, which some warps of a CTA reach a step or two before others: every launch returns, a launch that
+    # lost a wait says so, one that did not is right, and so is the next one with the normal limit
+    ops = _ops()
+    from pimaicompiler_b200 import _lib
+    g = torch.Generator().manual_seed(B + L)
+    T, I = 64, 32
+    ps = lstm_params(L, 1, I, H, g)
+    x = h16(torch.randn(T, B, I, generator=g))
+    m = ops.Lstm([to_dev(p) for p in ps], L, False, I, H, True)
+    m.set_variant(ops.LSTM_PERSISTENT)
+    want = [t.clone() for t in m.forward(to_dev(x))]
+    lost = 0
+    for limit in (2, 2, 3, 3, 4, 4, 6, 8, 16):
+        assert _lib.lib().pimb200_lstm_set_poll_limit(m._h, limit) == 0
+        got = m.forward(to_dev(x))
+        torch.cuda.synchronize()
+        status = m.last_status()
+        assert status in (0, _lib.ERR_TIMEOUT)
+        lost += status != 0
+        assert status != 0 or all(torch.equal(a, b) for a, b in zip(got, want))
+        assert _lib.lib().pimb200_lstm_set_poll_limit(m._h, 1 << 21) == 0
+        got = m.forward(to_dev(x))
+        torch.cuda.synchronize()
+        assert m.last_status() == 0
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    assert lost > 0                               # (a limit of two is too few for a launch's first step)
+
+
 @pytest.mark.parametrize("H", [48, 320, 1024])
 @pytest.mark.parametrize("B,L", [(1, 1), (3, 2), (8, 2), (9, 1), (15, 1), (16, 1), (17, 1), (32, 1), (33, 1), (49, 1), (65, 1), (96, 1), (97, 1)])
 def test_recurrence_kernels_at_the_edges_of_their_ranges(B, L, H):
