@@ -486,6 +486,7 @@ __global__ void __launch_bounds__(kBahdanauThreads) bahdanau_kernel(
     float* red = vs + H;                                    // [8 * threads] partial contexts
     float* sc = red + 8 * kBahdanauThreads;                 // [max_len] scores of the sentence, then weights
     __shared__ float vsum[WARPS];
+    if (C > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // this CTA has started: waited for below
     pdl_launch_dependents();
     pdl_wait();
     const int rank = blockIdx.x, seq = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -513,6 +514,8 @@ __global__ void __launch_bounds__(kBahdanauThreads) bahdanau_kernel(
     float vtot = 0.f;
 #pragma unroll
     for (int w = 0; w < WARPS; ++w) vtot += vsum[w];
+    // the cluster's other CTAs have started: their shared memory may be written
+    if (C > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     // ---- scores: warp w of CTA r takes positions r + C * (w + 8 i) ----
     for (int s = rank + C * warp; s < L; s += C * WARPS) {
         const uint4* kr = reinterpret_cast<const uint4*>(keys_proj + (size_t)seq * seq_stride + (size_t)s * row_stride);

@@ -255,6 +255,32 @@ def test_packed_attention_matches_padded(heads, hd, lens):
                        ops.attention_rows(one, pad[:, :, d:2 * d], pad[:, :, 2 * d:], heads, len_dev=ln, len_inc=1))
 
 
+@pytest.mark.parametrize("n", [1, 36, 40, 74, 80])
+def test_additive_attention_clusters_beside_other_work(n):
+    # eight, four and two CTAs per sentence: many launches, one behind the other, while another stream's product fills the SMs,
+    # so that the CTAs of a cluster find room at different times; every launch gives the same context
+    from pimaicompiler_b200 import ops
+    g = torch.Generator().manual_seed(n)
+    S, H = 50, 1024
+    q, v, b = (torch.randn(*s, generator=g).half().cuda() for s in ((n, H), (H,), (H,)))
+    kp, val = (torch.randn(S, n, H, generator=g).half().cuda() for _ in range(2))
+    ln = torch.randint(1, S + 1, (n,), generator=g).cuda()
+    big = torch.randn(4096, 4096, generator=g).half().cuda()
+    ref = ops.additive_attention(q, kp, val, ln, v * 0.05, b).clone()
+    outs = torch.empty(200, n, H, dtype=torch.float16, device="cuda")
+    scores = torch.empty(n, S, device="cuda")
+    vv = v * 0.05
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        for _ in range(20):
+            ops.gemm_wx(big, big)
+    for o in outs:
+        ops.additive_attention(q, kp, val, ln, vv, b, out=o, scores=scores)
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, ref) for o in outs)
+
+
 @pytest.mark.parametrize("n", [1, 20, 40, 80, 300])
 def test_additive_attention_copies(n):
     # one to eight CTAs per sentence, the context written three times
