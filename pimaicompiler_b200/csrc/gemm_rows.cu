@@ -112,12 +112,6 @@ __device__ __forceinline__ void store_half16(__half* p, const uint32_t* w) {
     q[1] = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
-// the larger of the two, NaN where either is one (fmaxf would turn a NaN of the inputs into -inf)
-__device__ __forceinline__ float max_nan(float a, float b) {
-    float m;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
-    return m;
-}
 // The producer's and the issuer's loops run with all 32 lanes, and only the instructions themselves are predicated on one
 // elected lane (`el`).  Inside an `if (lane == 0)` the compiler keeps addresses and descriptors in per-thread registers and
 // moves each to the uniform ones that these instructions take: the issuer then needed 600 cycles per K block and the

@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(kAddAttnSlice / 2) additive_context_kernel(
 // positions for the scores (a warp per position), exchange the scores through distributed shared memory, and share the
 // columns of H for the context.  Keys and values are read once each; MUFU bounds the scores, so four tanh share one
 // reciprocal: tanh(x) = 1 - 2 / (1 + e^2x), and with d = 1 + e^2x the four quotients v / d come from 1 / (d0 d1 d2 d3)
-// (2x is capped at 20, where tanh is 1 in fp32, so the product stays finite): 1.25 MUFU per element instead of 2.
+// (2x is capped at 20, where tanh is 1 in fp32, so the product stays finite; a NaN stays one): 1.25 MUFU per element instead of 2.
 // The first rows of values are loaded before the scores are known.  512 sentences (one CTA each): 22 + 13 us as two
 // launches; few sentences take up to eight CTAs each.
 constexpr int kBahdanauThreads = 256;
@@ -527,8 +527,8 @@ __global__ void __launch_bounds__(kBahdanauThreads) bahdanau_kernel(
 #pragma unroll
             for (int o = 0; o < 8; o += 4) {
                 const float4 b = *reinterpret_cast<const float4*>(qb + c * 8 + o), w = *reinterpret_cast<const float4*>(vs + c * 8 + o);
-                const float d0 = 1.f + ex2_(fminf(fmaf(k[o], kScale, b.x), 28.85390082f)), d1 = 1.f + ex2_(fminf(fmaf(k[o + 1], kScale, b.y), 28.85390082f)),
-                            d2 = 1.f + ex2_(fminf(fmaf(k[o + 2], kScale, b.z), 28.85390082f)), d3 = 1.f + ex2_(fminf(fmaf(k[o + 3], kScale, b.w), 28.85390082f));
+                const float d0 = 1.f + ex2_(min_nan(fmaf(k[o], kScale, b.x), 28.85390082f)), d1 = 1.f + ex2_(min_nan(fmaf(k[o + 1], kScale, b.y), 28.85390082f)),
+                            d2 = 1.f + ex2_(min_nan(fmaf(k[o + 2], kScale, b.z), 28.85390082f)), d3 = 1.f + ex2_(min_nan(fmaf(k[o + 3], kScale, b.w), 28.85390082f));
                 const float p01 = d0 * d1, p23 = d2 * d3;
                 const float n01 = fmaf(w.x, d1, w.y * d0), n23 = fmaf(w.z, d3, w.w * d2);
                 a = fmaf(fmaf(n01, p23, n23 * p01), rcp_approx(p01 * p23), a);

@@ -298,3 +298,31 @@ def test_additive_attention_copies(n):
     assert_close(out[:, 0, H:], ref, 2e-3, 2e-3, "context")
     assert torch.equal(out[:, 1, H:], out[:, 0, H:]) and torch.equal(out[:, 2, H:], out[:, 0, H:])
     assert float(out[:, :, :H].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("n,H", [(2, 1024), (80, 256), (300, 64)])
+@pytest.mark.parametrize("where", ["key", "query", "bias", "infinite keys"])
+def test_additive_attention_of_values_that_are_no_numbers(n, H, where):
+    # a NaN of the inputs is the context of its sentence, and of no other one; infinite keys are tanh's limits
+    from pimaicompiler_b200 import ops
+    g = torch.Generator().manual_seed(n)
+    S = 37
+    q, v, b = (torch.randn(*s, generator=g).half().cuda() for s in ((n, H), (H,), (H,)))
+    kp, val = (torch.randn(S, n, H, generator=g).half().cuda() for _ in range(2))
+    ln = torch.randint(1, S + 1, (n,), generator=g).cuda()
+    ln[1] = 20
+    v = v * 0.05
+    if where == "key":
+        kp[3, 1, 5] = float("nan")
+    elif where == "query":
+        q[1, 7] = float("nan")
+    elif where == "bias":
+        b[H - 1] = float("nan")
+    else:
+        kp[2, 1, 9], kp[3, 1, 9] = float("inf"), float("-inf")
+    got = ops.additive_attention(q, kp, val, ln, v, b)
+    e = (torch.tanh(kp.float() + (q.float() + b.float())) * v.float()).sum(2)
+    e = e.masked_fill(torch.arange(S, device="cuda")[:, None] >= ln, float("-inf"))
+    ref = (torch.softmax(e, 0)[:, :, None] * val.float()).sum(0)
+    assert torch.isnan(ref).any() == (where != "infinite keys")
+    torch.testing.assert_close(got.float(), ref, atol=2e-3, rtol=2e-3, equal_nan=True)
