@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(kBahdanauThreads) bahdanau_kernel(
 #pragma unroll
         for (int i = 0; i < kBahdanauAhead; ++i) {
             const int s = s0 + (i + kBahdanauAhead) * groups;
-            if (s < L) va[i] = __ldg(reinterpret_cast<const uint4*>(vals + (size_t)s * row_stride));
+            va[i] = s < L ? __ldg(reinterpret_cast<const uint4*>(vals + (size_t)s * row_stride)) : make_uint4(0u, 0u, 0u, 0u);   // (0 x inf is a NaN)
         }
     }
     if (groups > 1) {

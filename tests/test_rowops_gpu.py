@@ -326,3 +326,19 @@ def test_additive_attention_of_values_that_are_no_numbers(n, H, where):
     ref = (torch.softmax(e, 0)[:, :, None] * val.float()).sum(0)
     assert torch.isnan(ref).any() == (where != "infinite keys")
     torch.testing.assert_close(got.float(), ref, atol=2e-3, rtol=2e-3, equal_nan=True)
+
+
+@pytest.mark.parametrize("n,H", [(2, 1024), (300, 1024), (80, 512)])
+def test_additive_attention_of_infinite_values(n, H):
+    # an infinity in every live row of one column is that column of the context, and nothing else
+    from pimaicompiler_b200 import ops
+    g = torch.Generator().manual_seed(n)
+    S = 50
+    q, v, b = (torch.randn(*s, generator=g).half().cuda() for s in ((n, H), (H,), (H,)))
+    kp, val = (torch.randn(S, n, H, generator=g).half().cuda() for _ in range(2))
+    ln = torch.randint(1, S + 1, (n,), generator=g).cuda()
+    ln[1] = 21
+    want = ops.additive_attention(q, kp, val, ln, v * 0.05, b).clone()
+    val[:21, 1, 3], val[:21, 1, H - 1] = float("inf"), float("-inf")
+    want[1, 3], want[1, H - 1] = float("inf"), float("-inf")
+    assert torch.equal(ops.additive_attention(q, kp, val, ln, v * 0.05, b), want)
