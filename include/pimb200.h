@@ -250,7 +250,7 @@ int pimb200_additive_attention(const void* q, const void* keys_proj, const void*
                                long row_stride, long seq_stride, long ctx_stride, void* stream);
 
 /* The same with the context written `copies` times, copy_stride elements apart: straight into the concatenated input of
- * every decoder cell that takes it.  Rows without 16-byte alignment return PIMB200_ERR_UNSUPPORTED for copies > 1. */
+ * every decoder cell that takes it (copy_stride at least H for copies > 1). */
 int pimb200_additive_attention_copies(const void* q, const void* keys_proj, const void* values, const long long* lengths,
                                       const void* v, const void* bias, void* ctx, float* scores, int n_seq, long max_len, int H,
                                       long row_stride, long seq_stride, long ctx_stride, int copies, long copy_stride,

@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(kAddAttnThreads) additive_scores_kernel(
 
 __global__ void __launch_bounds__(kAddAttnSlice / 2) additive_context_kernel(
     const float* __restrict__ scores, const __half* __restrict__ values, const long long* __restrict__ lengths,
-    __half* __restrict__ ctx, long max_len, int H, long row_stride, long seq_stride, long ctx_stride) {
+    __half* __restrict__ ctx, long max_len, int H, long row_stride, long seq_stride, long ctx_stride, int copies, long copy_stride) {
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ float sc[];            // [max_len] softmax weights of this sentence
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(kAddAttnSlice / 2) additive_context_kernel(
     if (h >= H) return;
     const __half* vals = values + (size_t)seq * seq_stride + h;
     __half* out = ctx + (size_t)seq * ctx_stride + h;
-    if (h + 1 < H && (row_stride % 2 == 0) && (seq_stride % 2 == 0) && (ctx_stride % 2 == 0) &&
+    if (h + 1 < H && (row_stride % 2 == 0) && (seq_stride % 2 == 0) && (ctx_stride % 2 == 0) && (copy_stride % 2 == 0) &&
         ((reinterpret_cast<uintptr_t>(values) & 3u) == 0) && ((reinterpret_cast<uintptr_t>(ctx) & 3u) == 0)) {
         float a0 = 0.f, a1 = 0.f;
         long s = 0;
@@ -447,12 +447,12 @@ __global__ void __launch_bounds__(kAddAttnSlice / 2) additive_context_kernel(
             a0 = fmaf(sc[s], f.x, a0);
             a1 = fmaf(sc[s], f.y, a1);
         }
-        *reinterpret_cast<__half2*>(out) = __floats2half2_rn(a0 * inv, a1 * inv);
+        for (int i = 0; i < copies; ++i) *reinterpret_cast<__half2*>(out + i * copy_stride) = __floats2half2_rn(a0 * inv, a1 * inv);
     } else {
         for (int e = 0; e < 2 && h + e < H; ++e) {
             float a = 0.f;
             for (long s = 0; s < L; ++s) a = fmaf(sc[s], __half2float(vals[(size_t)s * row_stride + e]), a);
-            out[e] = __float2half_rn(a * inv);
+            for (int i = 0; i < copies; ++i) out[i * copy_stride + e] = __float2half_rn(a * inv);
         }
     }
 }
@@ -942,7 +942,6 @@ extern "C" int pimb200_additive_attention_copies(const void* q, const void* keys
             return c == 8 ? run(launch_bahdanau<8>) : c == 4 ? run(launch_bahdanau<4>) : c == 2 ? run(launch_bahdanau<2>) : run(launch_bahdanau<1>);
         }
     }
-    if (copies > 1) return PIMB200_ERR_UNSUPPORTED;
     const long rows = (long)n_seq * max_len;
     const int rc = cuda_status(launch_pdl(
         additive_scores_kernel, dim3((unsigned)((rows + kAddAttnThreads / 32 - 1) / (kAddAttnThreads / 32))), dim3(kAddAttnThreads), 0, st,
@@ -952,7 +951,7 @@ extern "C" int pimb200_additive_attention_copies(const void* q, const void* keys
     return cuda_status(launch_pdl(
         additive_context_kernel, dim3((unsigned)((H + kAddAttnSlice - 1) / kAddAttnSlice), (unsigned)n_seq), dim3(kAddAttnSlice / 2),
         (size_t)max_len * sizeof(float), st, scores, static_cast<const __half*>(values), lengths, static_cast<__half*>(ctx), max_len, H,
-        row_stride, seq_stride, ctx_stride));
+        row_stride, seq_stride, ctx_stride, copies, copy_stride));
 }
 
 extern "C" int pimb200_add_layer_norm_rows(const void* x, const void* r, const void* gamma, const void* beta, void* y,

@@ -47,6 +47,14 @@ def test_gnmt_small_model_ragged_groups(group):
     assert decided > total // 2
 
 
+@pytest.mark.parametrize("group,hidden", [(8, 96), (4, 40)])
+def test_gnmt_hidden_sizes_without_the_one_launch_attention(group, hidden):
+    cfg = to.GnmtConfig(vocab=300, hidden=hidden, max_steps=12, min_len=3, max_len=17)
+    w = to.make_gnmt_weights(cfg, seed=3, gain=2.0, logit_gain=4.0)
+    decided, total = _follow(cfg, w, to.make_sentences(11, cfg, seed=5), group, 12, 1e-2, 1e-2, 0.05)
+    assert decided > total // 2
+
+
 def test_gnmt_small_model_free_running_matches_oracle():
     # sharper logits: the free-running transcripts themselves must agree while every step's margin is clear
     cfg = to.GnmtConfig(vocab=300, hidden=64, max_steps=16, min_len=3, max_len=17)

@@ -342,3 +342,19 @@ def test_additive_attention_of_infinite_values(n, H):
     val[:21, 1, 3], val[:21, 1, H - 1] = float("inf"), float("-inf")
     want[1, 3], want[1, H - 1] = float("inf"), float("-inf")
     assert torch.equal(ops.additive_attention(q, kp, val, ln, v * 0.05, b), want)
+
+
+@pytest.mark.parametrize("n,H", [(3, 96), (9, 320), (5, 1536), (4, 37)])
+def test_additive_attention_copies_of_any_width(n, H):
+    # widths that the one-launch kernel does not take
+    from pimaicompiler_b200 import ops
+    g = torch.Generator().manual_seed(n)
+    S = 37
+    q, v, b = (torch.randn(*s, generator=g).half().cuda() for s in ((n, H), (H,), (H,)))
+    kp, val = (torch.randn(S, n, H, generator=g).half().cuda() for _ in range(2))
+    ln = torch.randint(1, S + 1, (n,), generator=g).cuda()
+    want = ops.additive_attention(q, kp, val, ln, v * 0.05, b)
+    out = torch.zeros(n, 3, 2 * H, dtype=torch.float16, device="cuda")
+    ops.additive_attention(q, kp, val, ln, v * 0.05, b, out=out[:, 0, H:], copies=3, copy_stride=2 * H)
+    assert all(torch.equal(out[:, i, H:], want) for i in range(3))
+    assert float(out[:, :, :H].abs().max()) == 0.0
