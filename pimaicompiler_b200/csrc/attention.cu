@@ -30,7 +30,7 @@ struct DecodeState {
     float m, sum, acc[8];
 };
 
-// rows c0 .. c0 + CL * 32 / (HD / 8) - 1 of one head; rows past L repeat the last one with weight 0
+// rows c0 .. c0 + CL * 32 / (HD / 8) - 1 of one head; rows past L repeat the last one's key and are without weight
 template <int HD, int CL>
 __device__ __forceinline__ void decode_chunk(DecodeState& st, const float* qf, const __half* Ks, const __half* Vs, long c0, long L,
                                              long kv_stride, int grp) {
@@ -53,15 +53,18 @@ __device__ __forceinline__ void decode_chunk(DecodeState& st, const float* qf, c
     }
 #pragma unroll
     for (int o = LPR; o < 32; o <<= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, o));
-    const float mn = fmaxf(st.m, cm), keep = expf(st.m - mn);     // exp(-inf) = 0 in the first chunk
+    // exp(-inf) = 0 in the first chunk.  While every score so far is -inf there is nothing to rescale, and -inf - -inf would be
+    // a NaN that later scores cannot replace; the reference is 0 then, so that the weights are 0 as well
+    const float mn = fmaxf(st.m, cm), ref = mn == -CUDART_INF_F ? 0.f : mn, keep = expf(st.m - ref);
     st.m = mn;
     st.sum *= keep;
 #pragma unroll
     for (int e = 0; e < 8; ++e) st.acc[e] *= keep;
 #pragma unroll
     for (int i = 0; i < CL; ++i) {
-        const float p = expf(s[i] - mn);
+        const float p = expf(s[i] - ref);
         st.sum += p;
+        if (c0 + i * RPL + grp >= L) vr[i] = make_uint4(0u, 0u, 0u, 0u);   // (0 x inf is a NaN)
         float vf[8];
         widen8(vr[i], vf);
 #pragma unroll

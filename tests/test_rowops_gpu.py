@@ -358,3 +358,40 @@ def test_additive_attention_copies_of_any_width(n, H):
     ops.additive_attention(q, kp, val, ln, v * 0.05, b, out=out[:, 0, H:], copies=3, copy_stride=2 * H)
     assert all(torch.equal(out[:, i, H:], want) for i in range(3))
     assert float(out[:, :, :H].abs().max()) == 0.0
+
+
+def _attention_ref(q, K, V, scale):
+    """In 64 bits; a weight of exactly zero meets no value (0 x inf)."""
+    p = torch.softmax(q.double() @ K.double().T * scale, -1)
+    out = torch.zeros(q.shape[0], V.shape[1], dtype=torch.double, device=q.device)
+    for t in range(K.shape[0]):
+        out += torch.where(p[:, t:t + 1] == 0, 0.0, p[:, t:t + 1] * V[t].double())
+    return out
+
+
+@pytest.mark.parametrize("hd,L", [(64, 5), (64, 33), (128, 61), (64, 200)])
+@pytest.mark.parametrize("what", ["numbers", "infinite last value", "infinite first value", "only the last key finite", "every key infinite", "a key NaN"])
+def test_decode_attention_of_infinities(hd, L, what):
+    # one sequence of three and one element of the rows is special; scores of -inf take no part, whatever chunk they are in
+    from pimaicompiler_b200 import ops
+    g = torch.Generator().manual_seed(L)
+    heads, n = 2, 3
+    d = heads * hd
+    q = (torch.rand(n, d, generator=g) + 0.1).half().cuda()
+    K, V = (torch.randn(n, L, d, generator=g).half().cuda() for _ in range(2))
+    if what == "infinite last value":
+        V[1, L - 1, 3] = float("inf")
+    elif what == "infinite first value":
+        V[1, 0, 3] = float("-inf")
+    elif what == "only the last key finite":
+        K[1, :L - 1, 4] = float("-inf")
+    elif what == "every key infinite":
+        K[1, :, 4] = float("-inf")
+    elif what == "a key NaN":
+        K[1, 2, 4] = float("nan")
+    got = ops.attention_rows(q, K, V, heads, len_dev=torch.full((n,), L, device="cuda"), len_inc=1)
+    for j in range(n):
+        for h in range(heads):
+            c = slice(h * hd, (h + 1) * hd)
+            ref = _attention_ref(q[j:j + 1, c], K[j, :, c], V[j, :, c], hd ** -0.5)
+            torch.testing.assert_close(got[j:j + 1, c].double(), ref, atol=2e-3, rtol=2e-3, equal_nan=True)
