@@ -132,7 +132,7 @@ namespace {
 // Up to 128 positions: queries, keys and values of the head sit in shared memory (rows padded by 16 bytes: conflict-free
 // ldmatrix), and a warp takes 16 query rows at a time through two tensor-core products, S = Q K^T and O = P V, with the
 // whole row of scores in registers between them.  A weight is kept as the sum of two fp16 numbers, so O has the precision
-// of fp32 weights.  The work is 4 * L * L * HD flops per 8 * L * HD bytes, so HBM bounds it; with scalar products from
+// of fp32 weights.  (An infinite value meets the first of them alone: the second may be zero or below.)  The work is 4 * L * L * HD flops per 8 * L * HD bytes, so HBM bounds it; with scalar products from
 // shared memory the 2048 x 8 heads of 64 positions took 1116 us per layer (550 MB).
 // ---------------------------------------------------------------------------------------------
 constexpr int kBlockWarps = 4;
@@ -157,6 +157,23 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
     lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
+// The same for a product with infinite values: no weight above zero has a hi of zero (0 x inf is a NaN)
+__device__ __forceinline__ void split2_nonzero(float a, float b, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    if (a > 0.f && (hi & 0xffffu) == 0u) hi |= 1u;
+    if (b > 0.f && (hi >> 16) == 0u) hi |= 0x10000u;
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+__device__ __forceinline__ bool has_infinity(uint32_t w) { return (w & 0x7c00u) == 0x7c00u || (w & 0x7c000000u) == 0x7c000000u; }   // or a NaN
+__device__ __forceinline__ uint32_t finite_or_zero(uint32_t w) {
+    if ((w & 0x7c00u) == 0x7c00u) w &= 0xffff0000u;
+    if ((w & 0x7c000000u) == 0x7c000000u) w &= 0xffffu;
+    return w;
+}
+
 template <int HD, int KT>   // KT: tiles of 16 positions
 __global__ void __launch_bounds__(kBlockWarps * 32) attention_block_mma_kernel(
     const __half* __restrict__ Q, const __half* __restrict__ K, const __half* __restrict__ V, const long long* __restrict__ lengths,
@@ -173,6 +190,7 @@ __global__ void __launch_bounds__(kBlockWarps * 32) attention_block_mma_kernel(
     const int tiles = (L + 15) >> 4, rows = tiles * 16;
     const size_t base = (row0 ? (size_t)row0[seq] * row_stride : (size_t)seq * seq_stride) + (size_t)h * HD;
     unsigned char *sQ = smem, *sK = smem + (size_t)KT * 16 * PITCH, *sV = sK + (size_t)KT * 16 * PITCH;
+    bool infinite = false;      // a value is an infinity or a NaN: it meets the hi terms alone
     for (int i = threadIdx.x; i < rows * CPR; i += kBlockWarps * 32) {
         const int r = i / CPR, c = i % CPR;
         const size_t at = base + (size_t)r * row_stride + c * 8;
@@ -181,12 +199,13 @@ __global__ void __launch_bounds__(kBlockWarps * 32) attention_block_mma_kernel(
             a = ldg_once(Q + at);
             b = ldg_once(K + at);
             d = ldg_once(V + at);
+            infinite = infinite || has_infinity(d.x) || has_infinity(d.y) || has_infinity(d.z) || has_infinity(d.w);
         }
         *reinterpret_cast<uint4*>(sQ + r * PITCH + c * 16) = a;
         *reinterpret_cast<uint4*>(sK + r * PITCH + c * 16) = b;
         *reinterpret_cast<uint4*>(sV + r * PITCH + c * 16) = d;
     }
-    __syncthreads();
+    infinite = __syncthreads_or(infinite);
     __half* o = out + (row0 ? (size_t)row0[seq] * out_row_stride : (size_t)seq * out_seq_stride) + (size_t)h * HD;
     const uint32_t q0 = (uint32_t)__cvta_generic_to_shared(sQ), k0 = (uint32_t)__cvta_generic_to_shared(sK), v0 = (uint32_t)__cvta_generic_to_shared(sV);
     // ldmatrix rows of a lane: A and V take rows lane % 16 at column half lane / 16; K takes eight keys per matrix
@@ -244,17 +263,22 @@ __global__ void __launch_bounds__(kBlockWarps * 32) attention_block_mma_kernel(
                     sum1 += s[t][n][2] + s[t][n][3];
                 }
                 uint32_t hi[4], lo[4];
-                split2(s[t][0][0], s[t][0][1], hi[0], lo[0]);
-                split2(s[t][0][2], s[t][0][3], hi[1], lo[1]);
-                split2(s[t][1][0], s[t][1][1], hi[2], lo[2]);
-                split2(s[t][1][2], s[t][1][3], hi[3], lo[3]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float a = s[t][i >> 1][2 * (i & 1)], b = s[t][i >> 1][2 * (i & 1) + 1];
+                    if (infinite) split2_nonzero(a, b, hi[i], lo[i]);
+                    else split2(a, b, hi[i], lo[i]);
+                }
 #pragma unroll
                 for (int n = 0; n < HD / 16; ++n) {
                     uint32_t vb[4];
                     ldsm4_trans(vb, v0 + t * 16 * PITCH + arow + n * 32);
                     mma_16816(acc[2 * n], hi, vb[0], vb[1]);
-                    mma_16816(acc[2 * n], lo, vb[0], vb[1]);
                     mma_16816(acc[2 * n + 1], hi, vb[2], vb[3]);
+                    if (infinite)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) vb[i] = finite_or_zero(vb[i]);
+                    mma_16816(acc[2 * n], lo, vb[0], vb[1]);
                     mma_16816(acc[2 * n + 1], lo, vb[2], vb[3]);
                 }
             }

@@ -395,3 +395,31 @@ def test_decode_attention_of_infinities(hd, L, what):
             c = slice(h * hd, (h + 1) * hd)
             ref = _attention_ref(q[j:j + 1, c], K[j, :, c], V[j, :, c], hd ** -0.5)
             torch.testing.assert_close(got[j:j + 1, c].double(), ref, atol=2e-3, rtol=2e-3, equal_nan=True)
+
+
+@pytest.mark.parametrize("hd,L", [(64, 5), (64, 33), (128, 61), (64, 128)])
+@pytest.mark.parametrize("what", ["numbers", "inf", "-inf", "nan", "small weight", "a query NaN", "only the last key finite"])
+def test_block_attention_of_infinities(hd, L, what):
+    # a value that is no finite number is its column of the output wherever its weight is above zero, and no other column
+    from pimaicompiler_b200 import ops
+    g = torch.Generator().manual_seed(L)
+    heads, n = 2, 2
+    d = heads * hd
+    q = (torch.rand(n, L, d, generator=g) + 0.1).half().cuda()
+    K, V = (torch.randn(n, L, d, generator=g).half().cuda() for _ in range(2))
+    if what in ("inf", "-inf", "nan"):
+        V[1, L // 2, 3] = float(what)
+    elif what == "small weight":                       # below the smallest fp16 number, above the smallest fp32 one
+        q[1, :, :hd], K[1, :, :hd] = 1.0, 0.0
+        K[1, L // 2, :hd] = -40.0 / hd ** 0.5
+        V[1, L // 2, 3] = float("inf")
+    elif what == "a query NaN":
+        q[1, 1, 3] = float("nan")
+    elif what == "only the last key finite":
+        K[1, :L - 1, 4] = float("-inf")
+    got = ops.attention_block(q, K, V, heads, torch.full((n,), L, device="cuda"))
+    for j in range(n):
+        for h in range(heads):
+            c = slice(h * hd, (h + 1) * hd)
+            ref = _attention_ref(q[j, :, c], K[j, :, c], V[j, :, c], hd ** -0.5)
+            torch.testing.assert_close(got[j, :, c].double(), ref, atol=2e-3, rtol=2e-3, equal_nan=True)
