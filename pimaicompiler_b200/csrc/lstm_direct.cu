@@ -6,7 +6,8 @@
 // them, a flag, polling, an acquire, and a bulk copy into shared memory, three L2 round trips and four CTA barriers.  Here
 // the records validate themselves and travel straight into the registers that multiply them:
 //   * a CTA owns 8 hidden units (32 gate rows).  Its record of a sequence is the 8 new hidden values, 16 bytes.  A record
-//     that has not arrived holds a sentinel, the fp16 pattern 0xffff, which no hidden value has (NaN is stored as 0x7fff);
+//     that has not arrived holds a sentinel, the fp16 pattern 0xffff, which no hidden value has (NaN is stored as 0x7fff,
+//     those of the initial states too);
 //     every 32-bit word is checked, so nothing is assumed about a record arriving in one piece.  There is no flag and no
 //     release: one L2 trip from the writer's store to the reader's load;
 //   * four buffers are used in turn.  At step s a warp of its own writes sentinels into the CTA's records of buffer
@@ -117,7 +118,8 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_direct_kernel(const __grid_c
         long g_step = 0;
         if (live) {
             if (a.c0[layer]) c = __half2float(a.c0[layer][(size_t)gn * H + u]);
-            if (a.h0[layer]) hh = a.h0[layer][(size_t)gn * H + u];
+            // (through fp32, which leaves a NaN as 0x7fff: layer B's first records are the caller's own bits otherwise)
+            if (a.h0[layer]) hh = __float2half_rn(__half2float(a.h0[layer][(size_t)gn * H + u]));
             bias4 = *reinterpret_cast<const float4*>(a.bias[layer] + (size_t)u * 4);
             if (layer == 0) {
                 gp = a.G + (size_t)(a.reverse ? T - 1 : 0) * a.g_tstride + (size_t)gn * a.g_bstride + (size_t)u * 4;

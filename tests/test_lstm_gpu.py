@@ -283,6 +283,24 @@ def test_recurrence_kernels_at_the_edges_of_their_ranges(B, L, H):
         assert_close(y[:, keep], ref[0][:, keep], LSTM_ATOL, LSTM_RTOL, f"beside a NaN sequence, B {B} H {H}")
 
 
+@pytest.mark.parametrize("B,L", [(3, 2), (8, 2), (3, 1), (9, 1), (20, 1), (70, 1)])
+def test_initial_state_of_nans_with_every_bit_set(B, L):
+    # 0xffff is a NaN and the exchange's mark of a record that has not arrived
+    ops = _ops()
+    g = torch.Generator().manual_seed(B)
+    T, I, H = 12, 24, 256
+    m = ops.Lstm([to_dev(p) for p in lstm_params(L, 1, I, H, g)], L, False, I, H, True)
+    x, h0, c0 = (to_dev(torch.randn(*s, generator=g)) for s in ((T, B, I), (L, B, H), (L, B, H)))
+    want = [t.clone() for t in m.forward(x, h0, c0)]
+    h0.view(torch.int16)[L - 1, 1] = -1
+    got = m.forward(x, h0, c0)
+    torch.cuda.synchronize()
+    assert m.last_status() == 0
+    assert torch.isnan(got[0][:, 1]).all() and torch.isnan(got[1][L - 1, 1]).all()
+    keep = [b for b in range(B) if b != 1]
+    assert all(torch.equal(a[:, keep], b[:, keep]) for a, b in zip(got, want))
+
+
 @pytest.mark.parametrize("T,B,I,H", [(6, 64, 64, 1024), (9, 23, 32, 256), (5, 40, 16, 128)])
 def test_tcgen05_recurrence_variant_matches_oracle(T, B, I, H):
     # the opt-in tensor-memory variant of the batched recurrence must give the same results as the default kernels
