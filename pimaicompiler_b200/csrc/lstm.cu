@@ -1853,6 +1853,17 @@ __global__ void __launch_bounds__(kPersistThreads, 1) lstm_persistent_tc_kernel(
 // ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
+// The record buffers of a kernel whose launches start on sentinels: a launch finds them in one set, and fills the other one
+// for the launch behind it.  That holds for launches that run once, one after the other.  A captured one runs whenever its
+// graph is replayed, so it is preceded by a fill of its own (2 us), and from the first capture on so is every other launch of
+// the handle, which may find any number of replays, or none, between itself and the call before it.
+struct RecordSets {
+    uint4* buf = nullptr;      // two sets
+    size_t words = 0;          // records of a set
+    unsigned launches = 0;     // that the stream has taken
+    bool captured = false;
+};
+
 struct pimb200_lstm {
     int L = 0, D = 1, I = 0, H = 0, has_biases = 0, device = 0;
     int variant = PIMB200_LSTM_AUTO;
@@ -1880,10 +1891,7 @@ struct pimb200_lstm {
     int packed_lockstep = 1;   // 0: packed input runs timestep by timestep on the streamed kernels
     int wavefront = 1;         // 1: stacked layers of up to 8 sequences run in pairs, one step apart, in one launch
     uint4* xchg = nullptr;  // [kXchgCopies][2][kXchgWords]
-    uint4* direct_buf = nullptr;     // few sequences: two sets of four record buffers, used by alternate launches
-    unsigned direct_launches = 0;
-    uint4* pipe_buf = nullptr;       // the same for the pipelined kernel
-    unsigned pipe_launches = 0;
+    RecordSets direct_sets, pipe_sets;   // of the kernels for few sequences and of the pipelined kernel
     uint4* bulk_data = nullptr;      // batched variant: [2][n_cta][32] records
     uint32_t* bulk_flags = nullptr;  // [2][n_cta]
     uint32_t bulk_tag = 0;
@@ -1978,8 +1986,10 @@ extern "C" int pimb200_lstm_create(const void* const* params, int n_params, int 
     h->d_status = reinterpret_cast<int*>(h->arena + o_status);
     h->xchg = reinterpret_cast<uint4*>(h->arena + o_xchg);
     h->bulk_flags = reinterpret_cast<uint32_t*>(h->arena + o_flags);
-    h->direct_buf = reinterpret_cast<uint4*>(h->arena + o_direct);
-    h->pipe_buf = reinterpret_cast<uint4*>(h->arena + o_pipe);
+    h->direct_sets.buf = reinterpret_cast<uint4*>(h->arena + o_direct);
+    h->direct_sets.words = kDirectSetWords;
+    h->pipe_sets.buf = reinterpret_cast<uint4*>(h->arena + o_pipe);
+    h->pipe_sets.words = kPipeSetWords;
     h->bulk_data = reinterpret_cast<uint4*>(h->arena + o_data);
     for (int l = 0; l < num_layers; ++l) {
         for (int d = 0; d < D; ++d) {
@@ -2158,14 +2168,25 @@ struct SeqLayout {
     long x_seq_rows = 0;            // batch-first input: rows from one sequence to the next (0 = T)
 };
 
+// The set that the next launch finds sentinels in, and the one that it fills; the caller counts the launch once the stream has taken it
+static int next_set(RecordSets& r, uint4** set, uint4** other, cudaStream_t st) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    PIMB200_CUDA_TRY(cudaStreamIsCapturing(st, &status));
+    if (status != cudaStreamCaptureStatusNone) r.captured = true;
+    *set = r.buf + (r.launches & 1) * r.words;
+    *other = r.buf + ((r.launches & 1) ^ 1) * r.words;
+    if (r.captured) PIMB200_CUDA_TRY(cudaMemsetAsync(*set, 0xff, r.words * sizeof(uint4), st));
+    return PIMB200_OK;
+}
+
 // the launch on a handle's next set of record buffers; `steps` of `layers` recurrences for the profile
 static int run_direct(pimb200_lstm* h, DirectArgs& a, int layers, int steps, cudaStream_t st) {
-    const unsigned n = h->direct_launches++;
-    a.set = h->direct_buf + (n & 1) * kDirectSetWords;
-    a.other_set = h->direct_buf + ((n & 1) ^ 1) * kDirectSetWords;
+    int rc = next_set(h->direct_sets, &a.set, &a.other_set, st);
+    if (rc != PIMB200_OK) return rc;
     a.status = h->d_status; a.gen = next_gen(h); a.H = h->H; a.poll_limit = h->poll_limit;
     if (h->prof) prof_mark(h, st);
-    const int rc = launch_lstm_direct(a, layers, st);
+    rc = launch_lstm_direct(a, layers, st);
+    if (rc == PIMB200_OK) ++h->direct_sets.launches;
     if (h->prof) {
         prof_mark(h, st);
         h->prof_bytes += (double)layers * steps * 4.0 * h->H * h->H * 2.0;
@@ -2241,10 +2262,10 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
             PipeArgs a;
             a.Whh = h->w_hh[ld]; a.bias = h->bias[ld]; a.G = G; a.g_tstride = g_tstride; a.g_bstride = g_bstride;
             a.h0 = h0; a.c0 = c0; a.y = y; a.y_tstride = y_tstride; a.y_bstride = y_bstride; a.hn = hn; a.cn = cn;
-            const unsigned turn = h->pipe_launches++ & 1;
+            const int rc = next_set(h->pipe_sets, &a.set, &a.other_set, st);
+            if (rc != PIMB200_OK) return rc;
             a.flags = h->bulk_flags; a.tag_base = h->bulk_tag;
             h->bulk_tag += (uint32_t)T + 1u;
-            a.set = h->pipe_buf + turn * kPipeSetWords; a.other_set = h->pipe_buf + (turn ^ 1) * kPipeSetWords;
             a.status = h->d_status; a.gen = next_gen(h);
             a.H = H; a.T = T; a.B = B; a.halves = halves; a.reverse = reverse ? 1 : 0; a.poll_limit = h->poll_limit;
             a.trace = h->trace;
@@ -2267,6 +2288,7 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
             void* kargs[] = {&a};
             if (h->prof) prof_mark(h, st);
             PIMB200_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(halves * H / upc), dim3(kPipeThreads), kargs, smem, st));
+            ++h->pipe_sets.launches;
             if (h->prof) {
                 prof_mark(h, st);
                 // each batch half is a recurrence of its own on its own CTAs, with its own register-resident copy of W_hh

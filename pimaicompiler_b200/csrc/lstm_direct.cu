@@ -14,7 +14,7 @@
 //     (s + 2) % 4 and fences; the next step's barrier orders that before the CTA publishes step s + 1.  A reader looks at that
 //     buffer only after it has read the same CTA's record of step s + 1, and its old contents (step s - 2) have been read
 //     by everyone, since every CTA has published step s - 1.  A launch starts on buffers that the previous launch of the
-//     handle has filled with sentinels (two sets, alternating);
+//     handle has filled with sentinels (two sets, alternating; in a captured call a fill of its own does that);
 //   * the eight warps split K into blocks of 32 columns, and a lane polls exactly the records that are its B fragments: the
 //     contraction index is only a summation order, so lane (sequence g, t) of a block takes units 8t .. 8t+7 of it as one
 //     16-byte record, and W_hh lies in registers (or shared memory) in the same order.  No staging, no barrier between

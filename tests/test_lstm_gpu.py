@@ -301,6 +301,43 @@ def test_initial_state_of_nans_with_every_bit_set(B, L):
     assert all(torch.equal(a[:, keep], b[:, keep]) for a, b in zip(got, want))
 
 
+@pytest.mark.parametrize("L,B,T", [(1, 1, 10), (1, 1, 11), (1, 8, 12), (1, 16, 13), (2, 1, 8), (2, 3, 9), (2, 8, 10), (3, 2, 11),
+                                   (1, 20, 8), (1, 40, 10), (2, 70, 11), (1, 128, 9)])
+def test_captured_recurrence_replayed_among_eager_calls(L, B, T):
+    # a call that was captured and never run, and replays of graphs with one, two or three recurrences of a handle between
+    # eager calls: always what a handle of its own gives, bit for bit
+    ops = _ops()
+    g = torch.Generator().manual_seed(L * 100 + B)
+    I, H = 24, 256
+    ps = [to_dev(p) for p in lstm_params(L, 1, I, H, g)]
+    m = ops.Lstm(ps, L, False, I, H, True)
+    xs = [to_dev(torch.randn(T, B, I, generator=g)) for _ in range(7)]
+    want = [[t.clone() for t in ops.Lstm(ps, L, False, I, H, True).forward(x)] for x in xs]
+
+    def check(i, got):
+        torch.cuda.synchronize()
+        assert m.last_status() == 0
+        assert all(torch.equal(a, b) for a, b in zip(got, want[i])), f"input {i}"
+
+    check(0, m.forward(xs[0]))                                   # (workspaces grow outside a capture)
+    x = xs[1].clone()
+    graphs = []
+    for calls in (1, 2):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(calls):
+                got = m.forward(x)
+        graphs.append((graph, got))
+        check(2, m.forward(xs[2]))
+    for i in (3, 4, 5, 6, 0, 1):
+        for graph, got in graphs:
+            x.copy_(xs[i])
+            graph.replay()
+            check(i, got)
+        if i % 2:
+            check(i - 1, m.forward(xs[i - 1]))
+
+
 @pytest.mark.parametrize("T,B,I,H", [(6, 64, 64, 1024), (9, 23, 32, 256), (5, 40, 16, 128)])
 def test_tcgen05_recurrence_variant_matches_oracle(T, B, I, H):
     # the opt-in tensor-memory variant of the batched recurrence must give the same results as the default kernels
