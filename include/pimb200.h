@@ -341,8 +341,8 @@ int pimb200_lstm_set_use_tc(pimb200_lstm* h, int on);
  * pipelined kernel for 17..128 sequences (W_hh slice in registers; the sequences advance as independent groups, so
  * one group's hidden-state exchange runs under the other groups' arithmetic; 65..128 sequences as two batch halves)
  * and, for 1..16 sequences, the kernel that polls the other CTAs' records straight into registers; 3 = the pipelined
- * kernel for every batch size; 1 = the kernel with the exchange on the compute warps for
- * 1..64 sequences; 0 = the K-split kernel with W_hh in shared memory (up to 32 sequences; also what H > 1024 falls
+ * kernel for every batch size; 1 = the kernel with the exchange on the compute warps for 1..64 sequences (neither with
+ * the wavefront below); 0 = the K-split kernel with W_hh in shared memory (up to 32 sequences; also what H > 1024 falls
  * back to).  Results agree within the LSTM tolerance; within one kernel they do not depend on the batch size.  No
  * counterpart in the reference. */
 int pimb200_lstm_set_bulk_wide(pimb200_lstm* h, int on);

@@ -2300,7 +2300,7 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
     // up to 16 sequences: records polled straight into the registers that multiply them (1.3 to 2.0 us per step against
     // 2.8 with flags and bulk copies); beyond that the polling loads themselves cost more than the flags
     const bool direct_fits = wide_ok && !packed && B <= kDirectMaxSlots && H / 8 <= h->sm_count && H / 8 <= kDirectMaxCtas &&
-                             (h->bulk_wide == 1 || h->bulk_wide == 2) && (int)direct_smem(H, 1) <= h->max_smem_optin;
+                             h->bulk_wide == 2 && (int)direct_smem(H, 1) <= h->max_smem_optin;
     if (direct_fits && (h->variant == PIMB200_LSTM_PERSISTENT || (h->variant == PIMB200_LSTM_AUTO && T >= 8))) {
         DirectArgs a = {};
         a.Whh[0] = h->w_hh[ld]; a.bias[0] = h->bias[ld]; a.G = G; a.g_tstride = g_tstride; a.g_bstride = g_bstride;
@@ -2557,7 +2557,7 @@ static int lstm_forward_packed_lockstep(pimb200_lstm* h, const __half* data, con
 static bool wave_fits(const pimb200_lstm* h, int l, int T, int B, bool packed) {
     const int H = h->H;
     return h->wavefront && !packed && h->D == 1 && l + 1 < h->L && T >= 8 && B >= 1 && B <= 8 && H % 16 == 0 &&
-           H / 8 <= kDirectMaxCtas && H / 8 <= h->sm_count && h->bulk_wide >= 1 &&
+           H / 8 <= kDirectMaxCtas && H / 8 <= h->sm_count && h->bulk_wide == 2 &&
            (h->variant == PIMB200_LSTM_AUTO || h->variant == PIMB200_LSTM_PERSISTENT) && (int)direct_smem(H, 2) <= h->max_smem_optin;
 }
 static int run_wave(pimb200_lstm* h, int l, int T, int B, const float* G, long g_tstride, long g_bstride, const __half* h0,

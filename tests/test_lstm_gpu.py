@@ -338,6 +338,22 @@ def test_captured_recurrence_replayed_among_eager_calls(L, B, T):
             check(i - 1, m.forward(xs[i - 1]))
 
 
+@pytest.mark.parametrize("bulk_wide", [1, 3])
+@pytest.mark.parametrize("L", [1, 2])
+def test_a_chosen_recurrence_kernel_runs_at_every_batch_size(bulk_wide, L):
+    # within one kernel a sequence's result does not depend on how many share the launch; another kernel sums in another order
+    ops = _ops()
+    g = torch.Generator().manual_seed(L)
+    T, I, H = 40, 24, 1024
+    ps = lstm_params(L, 1, I, H, g)
+    x = h16(torch.randn(T, 32, I, generator=g))
+    run = lambda b, bw: [t.clone() for t in _run(ops, ps, x[:, :b], None, None, L, False, True, False, ops.LSTM_AUTO, bw)]  # noqa: E731
+    many = run(32, bulk_wide)
+    for b in (1, 4, 16):
+        assert all(torch.equal(f, m[:, :b]) for f, m in zip(run(b, bulk_wide), many)), f"{b} sequences"
+    assert not torch.equal(run(4, None)[0], many[0][:, :4])          # (the default kernel's differ, so the above means something)
+
+
 @pytest.mark.parametrize("T,B,I,H", [(6, 64, 64, 1024), (9, 23, 32, 256), (5, 40, 16, 128)])
 def test_tcgen05_recurrence_variant_matches_oracle(T, B, I, H):
     # the opt-in tensor-memory variant of the batched recurrence must give the same results as the default kernels
