@@ -1519,7 +1519,8 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
             uint4* const group0 = a.set + ((size_t)half * NG + g) * group_words;
             uint4* const mine = group0 + (size_t)slice * OCT * BPG;
             bool dead = false;
-            for (int s = 0; s + 1 < T && !dead; ++s) {
+            int s = 0;
+            for (; s + 1 < T; ++s) {
                 const int par = s & 1;
                 const uint32_t tag = a.tag_base + (uint32_t)s + 1u;
                 long long* tr = a.trace ? a.trace + ((size_t)blockIdx.x * T + s) * 8 : nullptr;
@@ -1528,7 +1529,11 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
                 for (int i = lane; i < OCT * BPG; i += 32)
                     asm volatile("st.relaxed.gpu.global.v4.b32 [%0], {%1,%1,%1,%1};" ::"l"(mine + (size_t)((s + 2) & 3) * buf_words + i), "r"(~0u) : "memory");
                 __threadfence();
-                if (!mbar_wait_polls(done0 + 8u * g, (uint32_t)(s & 1), a.status, a.gen, wait_limit)) break;
+                if (!mbar_wait_polls(done0 + 8u * g, (uint32_t)(s & 1), a.status, a.gen, wait_limit)) {
+                    --s;                       // the copies of the step before are out
+                    dead = s >= 0;
+                    break;
+                }
                 // ---- publish: raise this CTA's step flag in every replica, right behind the records (no release: the tensor
                 //      warps look for sentinels).  The records are read by the other CTAs' bulk copies (async proxy): the
                 //      cross-proxy fence sits on the writer's side (in front of the copy it costs several thousand cycles)
@@ -1600,12 +1605,11 @@ __global__ void __launch_bounds__(kPipeThreads, 1) lstm_persistent_pipe_kernel(P
                     }
                 }
                 if (tr && lane == 0 && g == 0) tr[7] = clock64();
-                if (dead) {
-                    // before the CTA hands its shared memory back, give the copies in flight a bounded chance to land
-                    for (uint32_t i = 0; i < (1u << 20); ++i)
-                        if (pimb200::tc::mbar_try_wait(fbar, (uint32_t)(s & 1))) break;
-                }
+                if (dead) break;
             }
+            // before the CTA hands its shared memory back, give the copies in flight, those of step s, a bounded chance to land
+            for (uint32_t i = 0; dead && i < (1u << 20); ++i)
+                if (pimb200::tc::mbar_try_wait(fbar, (uint32_t)(s & 1))) break;
         }
     }
     }

@@ -230,7 +230,8 @@ def test_persistent_bounded_wait_reports_timeout_and_context_survives(B, L):
     assert m.last_status() == _lib.ERR_TIMEOUT
 
 
-@pytest.mark.parametrize("B,L,H", [(1, 1, 1024), (8, 1, 320), (16, 1, 1024), (1, 2, 1024), (8, 2, 256)])
+@pytest.mark.parametrize("B,L,H", [(1, 1, 1024), (8, 1, 320), (16, 1, 1024), (1, 2, 1024), (8, 2, 256), (20, 1, 1024), (64, 1, 320),
+                                   (70, 1, 256), (128, 1, 1024)])
 def test_waits_that_run_out_in_different_steps(B, L, H):
     # limits of a few polls, which some warps of a CTA reach a step or two before others: every launch returns, a launch that
     # lost a wait says so, one that did not is right, and so is the next one with the normal limit
