@@ -20,12 +20,6 @@ namespace {
 // chunk).  The lanes of a row share its score after a shuffle reduction and hold the same columns of V, so weights need no
 // exchange either; the row groups' partial outputs meet in the end.
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint4 ldg_once(const __half* p) {
-    uint4 r;
-    asm("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
-    return r;
-}
-
 struct DecodeState {
     float m, sum, acc[8];
 };
@@ -39,8 +33,8 @@ __device__ __forceinline__ void decode_chunk(DecodeState& st, const float* qf, c
 #pragma unroll
     for (int i = 0; i < CL; ++i) {
         const long t = c0 + i * RPL + grp, at = (t < L ? t : L - 1) * kv_stride;
-        kr[i] = ldg_once(Ks + at);
-        vr[i] = ldg_once(Vs + at);
+        kr[i] = ld_stream_v4(Ks + at);
+        vr[i] = ld_stream_v4(Vs + at);
     }
     float s[CL], cm = -CUDART_INF_F;
 #pragma unroll
@@ -73,8 +67,8 @@ __device__ __forceinline__ void decode_chunk(DecodeState& st, const float* qf, c
 }
 
 template <int HD, int CL>
-__global__ void __launch_bounds__(128) attention_decode_kernel(const __half* __restrict__ q, const __half* __restrict__ K,
-                                                               const __half* __restrict__ V, const long long* row0, const long long* len_dev,
+__global__ void __launch_bounds__(128) attention_decode_kernel(const __half* q, const __half* K,
+                                                               const __half* V, const long long* row0, const long long* len_dev,
                                                                long len_inc, long len_add, long max_len, __half* __restrict__ out,
                                                                int heads, int n_seq, long kv_stride, long seq_stride, long q_stride,
                                                                long out_stride, float scale) {
@@ -176,8 +170,8 @@ __device__ __forceinline__ uint32_t finite_or_zero(uint32_t w) {
 
 template <int HD, int KT>   // KT: tiles of 16 positions
 __global__ void __launch_bounds__(kBlockWarps * 32) attention_block_mma_kernel(
-    const __half* __restrict__ Q, const __half* __restrict__ K, const __half* __restrict__ V, const long long* __restrict__ lengths,
-    const long long* __restrict__ row0, __half* __restrict__ out, long max_len, long row_stride, long seq_stride, long out_row_stride,
+    const __half* Q, const __half* K, const __half* V, const long long* lengths,
+    const long long* row0, __half* __restrict__ out, long max_len, long row_stride, long seq_stride, long out_row_stride,
     long out_seq_stride, float scale) {
     constexpr int PITCH = HD * 2 + 16;                  // bytes per shared row
     constexpr int CPR = HD / 8;                         // 16-byte chunks per row
@@ -196,9 +190,9 @@ __global__ void __launch_bounds__(kBlockWarps * 32) attention_block_mma_kernel(
         const size_t at = base + (size_t)r * row_stride + c * 8;
         uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a, d = a;
         if (r < L) {
-            a = ldg_once(Q + at);
-            b = ldg_once(K + at);
-            d = ldg_once(V + at);
+            a = ld_stream_v4(Q + at);
+            b = ld_stream_v4(K + at);
+            d = ld_stream_v4(V + at);
             infinite = infinite || has_infinity(d.x) || has_infinity(d.y) || has_infinity(d.z) || has_infinity(d.w);
         }
         *reinterpret_cast<uint4*>(sQ + r * PITCH + c * 16) = a;

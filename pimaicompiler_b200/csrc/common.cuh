@@ -52,7 +52,8 @@ DeviceCtx* current_ctx();  // nullptr when pimb200_init was not called for the c
 // A launch that may start while the kernel before it on the stream is still running (programmatic dependent launch): its
 // CTAs are scheduled and set up as soon as that kernel's CTAs have all called pdl_launch_dependents(), and block in
 // pdl_wait() until it has completed and its writes are visible.  Every kernel launched this way calls pdl_wait() before
-// it touches global memory.  It saves the gap between two short kernels, about a microsecond.
+// it touches global memory, but for constants that no launch writes.  It saves the gap between two short kernels, about a
+// microsecond.
 // CLUSTER: CTAs per thread-block cluster.
 template <int CLUSTER = 1, typename... P, typename... A>
 inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
@@ -72,8 +73,25 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_
 }
 
 // ---- device side -----------------------------------------------------------
+// A kernel ahead on the stream may still be writing when this one starts, so what it writes is not read-only for the duration
+// of this one, and is read behind the wait by plain loads: no ld.global.nc, which is defined for memory that nobody writes
+// meanwhile (__ldg is one, and a const __restrict__ parameter may become one), and no asm load that is not volatile, which the
+// compiler may move ahead of the wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// 16 bytes by a plain load behind a wait (ld_stream_v4: read once per launch, kept out of L1).  Volatile, so it stays there,
+// but without a memory clobber: products and stores move freely around it
+__device__ __forceinline__ uint4 ld_v4(const void* p) {
+    uint4 r;
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ uint4 ld_stream_v4(const void* p) {
+    uint4 r;
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+    return r;
+}
 
 __device__ __forceinline__ uint4 ldg_stream_v4(const void* p) {
     // weights are read once per launch: keep them out of L1

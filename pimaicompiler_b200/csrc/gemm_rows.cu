@@ -97,11 +97,6 @@ __device__ __forceinline__ void load_half16(const __half* p, float* f) {     // 
     widen8(q[0], f);
     widen8(q[1], f + 8);
 }
-__device__ __forceinline__ uint4 ldg_early(const uint4* p) {      // stays ahead of the volatile statements behind it
-    uint4 r;
-    asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
-    return r;
-}
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
     const __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&h);
@@ -355,7 +350,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
                     uint4 bb[CH / 8];                                  // under way while the accumulator is read
                     if (bias_vec) {
 #pragma unroll
-                        for (int i = 0; i < CH / 8; ++i) bb[i] = ldg_early(bias4 + c / 8 + i);
+                        for (int i = 0; i < CH / 8; ++i) bb[i] = ld_v4(bias4 + c / 8 + i);
                     }
                     uint32_t v[CH];
                     tmem_ld32_nowait(acc + (uint32_t)c, v);
@@ -374,7 +369,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
                         }
                     } else if (a.bias) {
 #pragma unroll
-                        for (int i = 0; i < CH; ++i) f[i] += (n0 + c + i < n_end) ? __half2float(__ldg(a.bias + n0 + c + i)) : 0.f;
+                        for (int i = 0; i < CH; ++i) f[i] += (n0 + c + i < n_end) ? __half2float(a.bias[n0 + c + i]) : 0.f;
                     }
                     if (a.direct) {                                    // rows of Y that no tensor map takes
                         if (row_ok) {
@@ -439,7 +434,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
                     uint4 bb[4];
                     if (bias_vec) {
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) bb[i] = ldg_early(bias4 + c / 8 + i);
+                        for (int i = 0; i < 4; ++i) bb[i] = ld_v4(bias4 + c / 8 + i);
                     }
                     uint32_t v[32];
                     tmem_ld32(acc + (uint32_t)c, v);
@@ -450,7 +445,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
                         for (int i = 0; i < 4; ++i) widen8(bb[i], b + 8 * i);
                     } else {
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) b[i] = (a.bias && i < lim) ? __half2float(__ldg(a.bias + nb + i)) : 0.f;
+                        for (int i = 0; i < 32; ++i) b[i] = (a.bias && i < lim) ? __half2float(a.bias[nb + i]) : 0.f;
                     }
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
@@ -483,7 +478,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
                     const float4* b4 = reinterpret_cast<const float4*>(a.cell_bias) + u0;
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
-                        const float4 b = __ldg(b4 + i);
+                        const float4 b = __ldg(b4 + i);        // (a constant of the handle)
                         const float zi = __uint_as_float(v[4 * i]) + b.x, zf = __uint_as_float(v[4 * i + 1]) + b.y,
                                     zg = __uint_as_float(v[4 * i + 2]) + b.z, zo = __uint_as_float(v[4 * i + 3]) + b.w;
                         cp[i] = sigmoidf_(zf) * cp[i] + sigmoidf_(zi) * tanhf_(zg);

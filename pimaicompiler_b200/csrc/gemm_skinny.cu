@@ -28,13 +28,14 @@ constexpr size_t kSkinnyMaxBlockedNK = (size_t)8 << 20;     // ... and 16 MB
 constexpr int kSkinnyMaxBlockedCtas = kNumSmB200;           // ... in one wave of CTAs: 3.5 us at 512 x 512, 128 rows (tcgen05
                                                             // 4.1), but 7.9 at 2048 x 512, 160 rows (4.2)
 
-// not volatile: the compiler may move these loads and products freely (volatile asm statements keep their order, which
-// would put every block's loads behind the previous block's products and serialise the HBM round trips)
+// not volatile: the compiler may move these products freely (volatile asm statements keep their order, which would put every
+// block's loads, which are, behind the previous block's products and serialise the HBM round trips)
 __device__ __forceinline__ void mma16816(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+// 16 bytes of a handle's weights, which no launch writes: may be loaded ahead of a wait
 __device__ __forceinline__ uint4 ldg_w(const __half* p) {
     uint4 r;
     asm("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
@@ -98,11 +99,11 @@ __global__ void __launch_bounds__(kSkinnyThreads) gemm_skinny_kernel(SkinnyArgs 
             const bool in = b < b_hi && b * 32 + 8 * t < K;
 #pragma unroll
             for (int m = 0; m < MTW; ++m) {
-                w[u][m][0] = in ? ldg_w(wrow[m][0] + (size_t)b * 32) : zero;
-                w[u][m][1] = in ? ldg_w(wrow[m][1] + (size_t)b * 32) : zero;
+                w[u][m][0] = in ? ld_stream_v4(wrow[m][0] + (size_t)b * 32) : zero;
+                w[u][m][1] = in ? ld_stream_v4(wrow[m][1] + (size_t)b * 32) : zero;
             }
 #pragma unroll
-            for (int j = 0; j < NT; ++j) x[u][j] = in ? __ldg(reinterpret_cast<const uint4*>(xrow[j] + (size_t)b * 32)) : zero;
+            for (int j = 0; j < NT; ++j) x[u][j] = in ? ld_v4(xrow[j] + (size_t)b * 32) : zero;
         }
     };
     auto multiply = [&](const uint4 (&w)[UB][MTW][2], const uint4 (&x)[UB][NT]) {
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(kSkinnyThreads) lstm_cell_skinny_kernel(const 
             for (int j = 0; j < NT; ++j) {
                 const int row = min(j * 8 + g, a.J - 1);           // rows past J repeat the last one
                 const __half* p = first ? a.x + (size_t)row * a.x_ld + b * 32 : a.h0 + (size_t)row * a.H + (b - bx) * 32;
-                x[u][j] = in ? __ldg(reinterpret_cast<const uint4*>(p + 8 * t)) : zero;
+                x[u][j] = in ? ld_v4(p + 8 * t) : zero;
             }
         }
     };
@@ -296,10 +297,10 @@ __global__ void __launch_bounds__(kSkinnyThreads) gemm_skinny_grouped_kernel(con
         for (int u = 0; u < UB; ++u) {
             const int b = b0 + u;
             const bool in = b < b_hi && b * 32 + 8 * t < K;
-            w[u][0] = in ? ldg_w(w_lo + (size_t)b * 32) : zero;
-            w[u][1] = in ? ldg_w(w_hi + (size_t)b * 32) : zero;
+            w[u][0] = in ? ld_stream_v4(w_lo + (size_t)b * 32) : zero;
+            w[u][1] = in ? ld_stream_v4(w_hi + (size_t)b * 32) : zero;
 #pragma unroll
-            for (int j = 0; j < NT; ++j) x[u][j] = in ? __ldg(reinterpret_cast<const uint4*>(xrow[j] + (size_t)b * 32)) : zero;
+            for (int j = 0; j < NT; ++j) x[u][j] = in ? ld_v4(xrow[j] + (size_t)b * 32) : zero;
         }
     };
     auto multiply = [&](const uint4 (&w)[UB][2], const uint4 (&x)[UB][NT]) {
@@ -384,8 +385,8 @@ __global__ void __launch_bounds__(kSkinnyThreads, 2) gemm_skinny_rows_kernel(Ski
 #pragma unroll
         for (int u = 0; u < UB; ++u)
             if (FULL || grp * UB + u < blocks) {
-                w[u][0] = ldg_w(p_lo + u * 32);
-                w[u][1] = ldg_w(p_hi + u * 32);
+                w[u][0] = ld_stream_v4(p_lo + u * 32);
+                w[u][1] = ld_stream_v4(p_hi + u * 32);
             }
     };
     float acc[NT][4];

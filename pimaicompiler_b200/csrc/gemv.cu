@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(256) dot_vv_kernel(const __half* __restrict__ 
 // =============================================================================================
 // fp16 add, same-shape or row-broadcast, any n
 // =============================================================================================
-__global__ void __launch_bounds__(256) add_f16_vec_kernel(const uint4* A, const uint4* __restrict__ B,
+__global__ void __launch_bounds__(256) add_f16_vec_kernel(const uint4* A, const uint4* B,
                                                           uint4* C, size_t total8, int n8, int bcast) {
     pdl_launch_dependents();
     pdl_wait();
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(256) add_f16_scalar_kernel(const __half* A, co
 // =============================================================================================
 template <typename V>
 __global__ void __launch_bounds__(256) copy_2d_kernel(unsigned char* __restrict__ dst, size_t dpitch,
-                                                      const unsigned char* __restrict__ src, size_t spitch,
+                                                      const unsigned char* src, size_t spitch,
                                                       size_t row_elems, size_t rows) {
     pdl_launch_dependents();
     pdl_wait();

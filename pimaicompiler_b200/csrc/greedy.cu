@@ -17,9 +17,9 @@ constexpr int kMaxParts = 2 * kNumSmB200;   // of the few-row projection: its CT
 
 // SLICES threads share a row's pieces: 32 for many rows, 128 for few (all their loads in flight at once)
 template <int SLICES>
-__global__ void __launch_bounds__(kRows * SLICES) greedy_token_kernel(const float* __restrict__ best_v, const int* __restrict__ best_i,
+__global__ void __launch_bounds__(kRows * SLICES) greedy_token_kernel(const float* best_v, const int* best_i,
                                                                        int parts, int J, int N, long long* __restrict__ idx,
-                                                                       const __half* __restrict__ emb, const __half* __restrict__ pos,
+                                                                       const __half* emb, const __half* pos,
                                                                        __half* __restrict__ x_next, int d) {
     constexpr int WARPS = kRows * SLICES / 32;
     __shared__ float sv[WARPS][kRows];

@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(256) lstm_cell_kernel(CellArgs a) {
                 for (int j = 0; j < BT; ++j) {
                     const int b = min(b0 + j, a.B - 1);
                     float xf[8];
-                    widen8(__ldg(reinterpret_cast<const uint4*>(first ? a.x + (size_t)b * a.x_bstride : a.h0 + (size_t)b * H) + c), xf);
+                    widen8(ld_v4((first ? a.x + (size_t)b * a.x_bstride : a.h0 + (size_t)b * H) + c * 8), xf);
 #pragma unroll
                     for (int g = 0; g < 4; ++g) acc[g][j] = dot8f(w[k][g], xf, acc[g][j]);
                 }

@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(T) softmax_rows_kernel(const __half* __restric
 }
 
 template <int T, bool VEC>
-__global__ void __launch_bounds__(T) argmax_rows_kernel(const __half* __restrict__ x, long long* __restrict__ idx,
+__global__ void __launch_bounds__(T) argmax_rows_kernel(const __half* x, long long* __restrict__ idx,
                                                                   long cols) {
     __shared__ float red_v[T / 32];
     __shared__ long long red_i[T / 32];
@@ -210,7 +210,7 @@ __global__ void masked_fill_f16_kernel(const __half* __restrict__ x, const unsig
 }
 
 // out[i, :] = table[idx[i], :], rows of row_bytes bytes; an index outside [0, n_table) yields a zero row
-__global__ void gather_rows_kernel(const unsigned char* __restrict__ table, const long long* __restrict__ idx,
+__global__ void gather_rows_kernel(const unsigned char* table, const long long* idx,
                                    unsigned char* __restrict__ out, size_t row_bytes, long n_table, int vec16) {
     pdl_launch_dependents();
     pdl_wait();
@@ -229,8 +229,8 @@ __global__ void gather_rows_kernel(const unsigned char* __restrict__ table, cons
 
 // table[idx[i], :] = src[i, :]: the write-side twin of the gather (a KV-cache append at a position that lives on the
 // device); an index outside [0, n_table) is skipped
-__global__ void scatter_rows_kernel(unsigned char* __restrict__ table, const long long* __restrict__ idx,
-                                    const unsigned char* __restrict__ src, size_t row_bytes, long n_table, int vec16) {
+__global__ void scatter_rows_kernel(unsigned char* __restrict__ table, const long long* idx,
+                                    const unsigned char* src, size_t row_bytes, long n_table, int vec16) {
     pdl_launch_dependents();
     pdl_wait();
     const long long r = idx[blockIdx.x];
@@ -363,8 +363,8 @@ constexpr int kAddAttnThreads = 256;
 constexpr int kAddAttnSlice = 256;       // context elements per CTA of the second launch (two per thread, 128 threads)
 
 __global__ void __launch_bounds__(kAddAttnThreads) additive_scores_kernel(
-    const __half* __restrict__ q, const __half* __restrict__ keys_proj, const long long* __restrict__ lengths,
-    const __half* __restrict__ v, const __half* __restrict__ bias, float* __restrict__ scores, int n_seq, long max_len,
+    const __half* q, const __half* keys_proj, const long long* lengths,
+    const __half* v, const __half* bias, float* __restrict__ scores, int n_seq, long max_len,
     int H, long row_stride, long seq_stride) {
     pdl_launch_dependents();
     pdl_wait();
@@ -385,10 +385,10 @@ __global__ void __launch_bounds__(kAddAttnThreads) additive_scores_kernel(
     if (vec) {
         for (int c = lane; c < (H >> 3); c += 32) {
             float kf[8], qf[8], vf[8], bf[8];
-            widen8(__ldg(reinterpret_cast<const uint4*>(kr) + c), kf);
-            widen8(__ldg(reinterpret_cast<const uint4*>(qr) + c), qf);
-            widen8(__ldg(reinterpret_cast<const uint4*>(v) + c), vf);
-            if (bias) widen8(__ldg(reinterpret_cast<const uint4*>(bias) + c), bf);
+            widen8(ld_v4(reinterpret_cast<const uint4*>(kr) + c), kf);
+            widen8(ld_v4(reinterpret_cast<const uint4*>(qr) + c), qf);
+            widen8(ld_v4(reinterpret_cast<const uint4*>(v) + c), vf);
+            if (bias) widen8(ld_v4(reinterpret_cast<const uint4*>(bias) + c), bf);
 #pragma unroll
             for (int i = 0; i < 8; ++i) a = fmaf(vf[i], tanhf_(kf[i] + (qf[i] + (bias ? bf[i] : 0.f))), a);
         }
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(kAddAttnThreads) additive_scores_kernel(
 }
 
 __global__ void __launch_bounds__(kAddAttnSlice / 2) additive_context_kernel(
-    const float* __restrict__ scores, const __half* __restrict__ values, const long long* __restrict__ lengths,
+    const float* scores, const __half* values, const long long* lengths,
     __half* __restrict__ ctx, long max_len, int H, long row_stride, long seq_stride, long ctx_stride, int copies, long copy_stride) {
     pdl_launch_dependents();
     pdl_wait();
@@ -475,8 +475,8 @@ __device__ __forceinline__ float ex2_(float x) {
 
 template <int C>
 __global__ void __launch_bounds__(kBahdanauThreads) bahdanau_kernel(
-    const __half* __restrict__ q, const __half* __restrict__ keys_proj, const __half* __restrict__ values,
-    const long long* __restrict__ lengths, const __half* __restrict__ v, const __half* __restrict__ bias, __half* __restrict__ ctx,
+    const __half* q, const __half* keys_proj, const __half* values,
+    const long long* lengths, const __half* v, const __half* bias, __half* __restrict__ ctx,
     float* __restrict__ scores, long max_len, int H, long row_stride, long seq_stride, long ctx_stride, int copies, long copy_stride) {
     constexpr int WARPS = kBahdanauThreads / 32;
     constexpr float kScale = 2.885390082f;                  // 2 / ln 2: e^2x = 2^(kScale x)
@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(kBahdanauThreads) bahdanau_kernel(
 #pragma unroll
     for (int i = 0; i < kBahdanauAhead; ++i) {
         const int s = grp + i * groups;
-        va[i] = s < L ? __ldg(reinterpret_cast<const uint4*>(vals + (size_t)s * row_stride)) : make_uint4(0u, 0u, 0u, 0u);
+        va[i] = s < L ? ld_v4(vals + (size_t)s * row_stride) : make_uint4(0u, 0u, 0u, 0u);
     }
     float my_v = 0.f;
     for (int h = tid; h < H; h += kBahdanauThreads) {
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(kBahdanauThreads) bahdanau_kernel(
 #pragma unroll 4
         for (int c = lane; c < n8; c += 32) {
             float k[8];
-            widen8(__ldg(kr + c), k);
+            widen8(ld_v4(kr + c), k);
 #pragma unroll
             for (int o = 0; o < 8; o += 4) {
                 const float4 b = *reinterpret_cast<const float4*>(qb + c * 8 + o), w = *reinterpret_cast<const float4*>(vs + c * 8 + o);
@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(kBahdanauThreads) bahdanau_kernel(
 #pragma unroll
         for (int i = 0; i < kBahdanauAhead; ++i) {
             const int s = s0 + (i + kBahdanauAhead) * groups;
-            va[i] = s < L ? __ldg(reinterpret_cast<const uint4*>(vals + (size_t)s * row_stride)) : make_uint4(0u, 0u, 0u, 0u);   // (0 x inf is a NaN)
+            va[i] = s < L ? ld_v4(vals + (size_t)s * row_stride) : make_uint4(0u, 0u, 0u, 0u);   // (0 x inf is a NaN)
         }
     }
     if (groups > 1) {
@@ -627,8 +627,8 @@ __global__ void __launch_bounds__(T) add_layer_norm_rows_kernel(const __half* __
 // 16-byte pieces per lane), no shared memory and no block-wide barrier.  Many rows: bound by HBM (131072 rows of 512: 155 us
 // with a CTA per row, 4 passes of 2-byte accesses); few rows: by latency, so one warp per CTA.
 template <int NV>
-__global__ void __launch_bounds__(256) add_layer_norm_warp_kernel(const __half* __restrict__ x, const __half* __restrict__ r,
-                                                                  const __half* __restrict__ gamma, const __half* __restrict__ beta,
+__global__ void __launch_bounds__(256) add_layer_norm_warp_kernel(const __half* x, const __half* r,
+                                                                  const __half* gamma, const __half* beta,
                                                                   __half* __restrict__ y, long rows, int cols, float eps) {
     pdl_launch_dependents();
     pdl_wait();
