@@ -267,6 +267,11 @@ int pimb200_additive_attention_copies(const void* q, const void* keys_proj, cons
 size_t pimb200_greedy_token_workspace(int N, int J);
 int pimb200_greedy_token(const void* W, const void* X, const void* bias, int N, int K, int J, int ldx, void* workspace,
                          long long* idx, const void* emb, const void* pos, void* x_next, int d, void* stream);
+/* The same for a step that is replayed from a graph: idx is a table of rows of J, the tokens go to row *step (int64 in DEVICE
+ * memory), and *next_step = *step + 1 is stored for the step behind it; two different words, used in turn. */
+int pimb200_greedy_token_step(const void* W, const void* X, const void* bias, int N, int K, int J, int ldx, void* workspace,
+                              long long* idx, const long long* step, long long* next_step, const void* emb, const void* pos,
+                              void* x_next, int d, void* stream);
 
 typedef struct pimb200_lstm pimb200_lstm;
 

@@ -65,6 +65,7 @@ SIGNATURES = {
     "pimb200_scatter_rows": (_i, [_vp, _vp, _vp, C.c_long, _sz, C.c_long, _vp]),
     "pimb200_greedy_token_workspace": (_sz, [_i, _i]),
     "pimb200_greedy_token": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp]),
+    "pimb200_greedy_token_step": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _vp]),
     "pimb200_masked_fill_f16": (_i, [_vp, _vp, C.c_float, _vp, _sz, _sz, _vp]),
     "pimb200_topk_rows": (_i, [_vp, _vp, _vp, C.c_long, C.c_long, _i, _i, _vp]),
     "pimb200_lstm_create": (_i, [C.POINTER(_vp), _i, _i, _i, _i, _i, _i, C.POINTER(_vp)]),

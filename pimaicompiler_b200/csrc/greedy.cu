@@ -20,13 +20,15 @@ template <int SLICES>
 __global__ void __launch_bounds__(kRows * SLICES) greedy_token_kernel(const float* best_v, const int* best_i,
                                                                        int parts, int J, int N, long long* __restrict__ idx,
                                                                        const __half* emb, const __half* pos,
-                                                                       __half* __restrict__ x_next, int d) {
+                                                                       __half* __restrict__ x_next, int d, const long long* step,
+                                                                       long long* next_step) {
     constexpr int WARPS = kRows * SLICES / 32;
     __shared__ float sv[WARPS][kRows];
     __shared__ int si[WARPS][kRows];
     __shared__ int tok[kRows];
     pdl_launch_dependents();
     pdl_wait();
+    const long long at_step = step ? *step : 0;
     const int r = threadIdx.x % kRows, slice = threadIdx.x / kRows, j = blockIdx.x * kRows + r;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float v = -INFINITY;
@@ -53,8 +55,9 @@ __global__ void __launch_bounds__(kRows * SLICES) greedy_token_kernel(const floa
             if (sv[w][r] > v || (sv[w][r] == v && si[w][r] < i)) { v = sv[w][r]; i = si[w][r]; }
         i = i < N ? i : 0;           // a row without a comparable logit: index 0, as arg max has it
         tok[r] = i;
-        if (j < J) idx[j] = i;
+        if (j < J) idx[(size_t)at_step * J + j] = i;
     }
+    if (next_step && blockIdx.x == 0 && threadIdx.x == 0) *next_step = at_step + 1;   // (nobody reads it before this kernel has ended)
     if (!emb) return;
     __syncthreads();
     const int chunks = d >> 3;
@@ -86,6 +89,13 @@ extern "C" size_t pimb200_greedy_token_workspace(int N, int J) {
 
 extern "C" int pimb200_greedy_token(const void* W, const void* X, const void* bias, int N, int K, int J, int ldx, void* workspace,
                                     long long* idx, const void* emb, const void* pos, void* x_next, int d, void* stream) {
+    return pimb200_greedy_token_step(W, X, bias, N, K, J, ldx, workspace, idx, nullptr, nullptr, emb, pos, x_next, d, stream);
+}
+
+extern "C" int pimb200_greedy_token_step(const void* W, const void* X, const void* bias, int N, int K, int J, int ldx, void* workspace,
+                                         long long* idx, const long long* step, long long* next_step, const void* emb,
+                                         const void* pos, void* x_next, int d, void* stream) {
+    if ((step != nullptr) != (next_step != nullptr) || (step && step == next_step)) return PIMB200_ERR_BAD_ARG;
     if (!W || !X || !workspace || !idx || N <= 0 || K <= 0 || J <= 0 || ldx < K || (emb && (!x_next || d <= 0))) return PIMB200_ERR_BAD_ARG;
     if (emb && (d % 8 != 0 || !aligned16(emb) || !aligned16(x_next) || (pos && !aligned16(pos)))) return PIMB200_ERR_UNSUPPORTED;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -98,7 +108,8 @@ extern "C" int pimb200_greedy_token(const void* W, const void* X, const void* bi
     if (rc != PIMB200_OK) return rc;
     auto run = [&](auto kernel, int slices) {
         return cuda_status(launch_pdl(kernel, dim3(ceil_div(J, kRows)), dim3(kRows * slices), 0, st, best_v, best_i, parts, J, N, idx,
-                                      static_cast<const __half*>(emb), static_cast<const __half*>(pos), static_cast<__half*>(x_next), d));
+                                      static_cast<const __half*>(emb), static_cast<const __half*>(pos), static_cast<__half*>(x_next), d, step,
+                                      next_step));
     };
     return J <= 256 ? run(greedy_token_kernel<128>, 128) : run(greedy_token_kernel<32>, 32);
 }

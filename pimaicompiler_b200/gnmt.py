@@ -12,13 +12,15 @@ hundreds of them runs `group` sentences in lock step instead:
   * decoder: one step for the whole group is four cells (each one launch: both products and the gate math; the output, for
     the last two with the residual added, goes straight into the next cell's concatenated input), the query projection, one
     attention launch (which writes the context into the other halves of those inputs), and the vocabulary projection with
-    its arg max and the next token's embedding (two launches, no logits in memory).  All steps are captured into one CUDA
-    graph; the chosen tokens stay on the device until the group is done.
+    its arg max and the next token's embedding (two launches, no logits in memory).  Eight, two and one steps are captured
+    into CUDA graphs when they are first needed, and any number of steps is made of their replays: the step's number lives
+    on the device.  The chosen tokens stay there until the group is done.
 
 `GnmtTranslator.translate` is the user call; `bench.py --workload c4` times it.
 """
 from __future__ import annotations
 
+import gc
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -98,10 +100,13 @@ class GnmtTranslator:
         self.cats = torch.zeros(G, 3, 2 * H, **f16)                     # inputs [previous output | context] of the last three cells
         self.cat = [self.cats[:, i] for i in range(3)]
         self.state = [[torch.zeros(1, G, H, **f16) for _ in range(8)] for _ in range(2)]   # h0..3, c0..3, two sets
+        self.step_no = torch.zeros(2, **i64)                            # the step's number: word t & 1 for step t, which sets the other
         self.token_ws = ops.greedy_token_workspace(V, G, self.dev)
-        self.toks = torch.zeros(cfg.max_steps + 1, G, **i64)            # row 0: start tokens, row t+1: choice of step t
+        self.start = torch.zeros(G, **i64)
+        self.toks = torch.zeros(max(cfg.max_steps, 1), G, **i64)        # row t: choice of step t
         self.forced = torch.zeros(cfg.max_steps + 1, G, **i64)          # row t: token fed to step t
-        self.logits = None                                              # [G, V], where the arg max needs them in memory
+        self.tok = torch.zeros(1, G, **i64)                             # a step's tokens, where the arg max is a launch of its own
+        self.logits = None                                              # [G, V], there
         self.logits_out = None
         self._graphs = {}
         self.launches_per_step = 0
@@ -132,14 +137,17 @@ class GnmtTranslator:
 
     # ------------------------------------------------------------------------------------------------ decoder
     def _step(self, t: int, forced: bool, want_logits: bool) -> int:
-        """One decode step of the whole group.  Returns its launch count."""
-        H, G, w, cfg = self.H, self.G, self.w, self.cfg
+        """A decode step of the whole group; of its number t only the last bit matters, so that replays of a graph can stand
+        for any step.  Returns its launch count."""
+        H, G, w = self.H, self.G, self.w
         src, dst = self.state[t & 1], self.state[1 - (t & 1)]
+        step, next_step = self.step_no[t & 1:(t & 1) + 1], self.step_no[1 - (t & 1):2 - (t & 1)]
         row, half = 3 * 2 * H * 2, H * 2        # bytes from row to row of a concatenated input, of half of it
         n = 0
         cat = self.cat
-        if t == 0 or forced or want_logits or self.logits is not None:
-            ops.gather_rows(w["emb_tgt"], (self.forced if forced else self.toks)[t], out=self.x); n += 1
+        if forced:                              # teacher forcing: the token comes from a table
+            ops.gather_rows(self.forced, step, out=self.tok)
+            ops.gather_rows(w["emb_tgt"], self.tok[0], out=self.x); n += 2
         # groups of 8 or more sentences: every cell writes its output (the last two with their residual added) straight
         # into the first half of the next cell's concatenated input, as the reference's labelled GNMT graph does
         fused = self.lstm["dec0"].forward_step(self.x, src[0][0], src[4][0], cat[0][:, :H], dst[0][0], dst[4][0])
@@ -167,53 +175,81 @@ class GnmtTranslator:
             ops.add_f16(cell(2), y1, out=self.r2)
             ops.copy_2d(self.cats, 4 * half, row, self.r2, 0, half, half, G)
             ops.add_f16(cell(3), self.r2, out=self.r3); n += 10
+        nxt = (None, None) if forced else (w["emb_tgt"], self.x)
         if not want_logits and self.logits is None:
-            last = forced or t + 1 >= cfg.max_steps
-            if ops.greedy_token(w["Wc"], self.r3, w["bc"], self.token_ws, self.toks[t + 1], None if last else w["emb_tgt"], None,
-                                None if last else self.x):
+            if ops.greedy_token(w["Wc"], self.r3, w["bc"], self.token_ws, self.toks, nxt[0], None, nxt[1], step, next_step):
                 return n + 2
+        if self.logits is None:
             self.logits = torch.zeros(G, self.V, dtype=torch.float16, device=self.dev)
-        lg = self.logits_out[t] if want_logits else self.logits
-        ops.gemm_wx(w["Wc"], self.r3, w["bc"], out=lg)
-        ops.argmax(lg, out=self.toks[t + 1])
-        return n + 2
+        ops.gemm_wx(w["Wc"], self.r3, w["bc"], out=self.logits)
+        ops.argmax(self.logits, out=self.tok[0])
+        ops.scatter_rows(self.toks, step, self.tok); n += 3
+        if want_logits:
+            ops.scatter_rows(self.logits_out.view(self.logits_out.shape[0], -1), step, self.logits.view(1, -1)); n += 1
+        if not forced:
+            ops.gather_rows(w["emb_tgt"], self.tok[0], out=self.x); n += 1
+        torch.add(step, 1, out=next_step)
+        return n + 1
+
+    CHUNKS = (8, 2, 1)       # steps per graph: of the last one, if any, the state ends up in the other set
 
     def _graph(self, steps: int, forced: bool, want_logits: bool):
-        """All steps, captured once per (steps, forced, logits) mode."""
+        """`steps` steps, captured once per (steps, forced, logits) mode."""
         key = (steps, forced, want_logits)
         if key in self._graphs:
             return self._graphs[key]
         side = torch.cuda.Stream(device=self.dev)
         side.wait_stream(torch.cuda.current_stream(self.dev))
-        with torch.cuda.stream(side):          # warm-up outside capture: buffers of the LSTM handles grow here
-            self._step(0, forced, want_logits)
+        with torch.cuda.stream(side):
+            if not any(k[1:] == key[1:] for k in self._graphs):
+                self.step_no.zero_()
+                self._step(0, forced, want_logits)   # outside the capture: buffers of the LSTM handles grow here
+            side.synchronize()
+            g = torch.cuda.CUDAGraph()
+            collecting = gc.isenabled()
+            gc.disable()                             # (a handle of some garbage would free device memory inside the capture)
+            try:
+                g.capture_begin()
+                try:
+                    for t in range(steps):
+                        self.launches_per_step = self._step(t, forced, want_logits)
+                finally:
+                    g.capture_end()
+            finally:
+                if collecting:
+                    gc.enable()
         torch.cuda.current_stream(self.dev).wait_stream(side)
-        torch.cuda.synchronize(self.dev)
-        g = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(g):
-            for t in range(steps):
-                self.launches_per_step = self._step(t, forced, want_logits)
         self._graphs[key] = g
         return g
 
     def decode(self, steps: int, forced: Optional[torch.Tensor] = None, want_logits: bool = False):
-        """Greedy decode of the encoded group for `steps` steps (one graph launch).  Returns the token table [steps, G]
-        (device, int64) and, when asked, the logits [steps, G, V]."""
+        """Greedy decode of the encoded group for `steps` steps.  Returns the token table [steps, G] (device, int64) and,
+        when asked, the logits [steps, G, V]."""
         cfg, G = self.cfg, self.G
         if steps > cfg.max_steps:
             raise ValueError("more steps than the configuration's maximum")
-        if want_logits and (self.logits_out is None or self.logits_out.shape[0] < steps):
+        if not want_logits:
+            if self.logits_out is not None:          # 2.6 GB for 512 sentences
+                self.logits_out = None
+                self._graphs = {k: v for k, v in self._graphs.items() if not k[2]}
+        elif self.logits_out is None or self.logits_out.shape[0] < steps:
             self.logits_out = torch.zeros(steps, G, self.V, dtype=torch.float16, device=self.dev)
             self._graphs = {k: v for k, v in self._graphs.items() if not k[2]}
         if forced is not None:
             self.forced[0].fill_(cfg.bos)
-            self.forced[1:steps].copy_(forced[:steps - 1].to(self.dev))          # step t is fed the token forced at t - 1
-        g = self._graph(steps, forced is not None, want_logits)
+            self.forced[1:max(steps, 1)].copy_(forced[:max(steps - 1, 0)].to(self.dev))   # step t is fed the token forced at t - 1
+        graphs, left = [], max(steps, 0)
+        for c in self.CHUNKS:
+            graphs += [self._graph(c, forced is not None, want_logits)] * (left // c) if left >= c else []
+            left %= c
         for s in self.state[0]:
             s.zero_()
-        self.toks[0].fill_(cfg.bos)
-        g.replay()
-        toks = self.toks[1:steps + 1]
+        self.step_no.zero_()
+        self.start.fill_(cfg.bos)
+        ops.gather_rows(self.w["emb_tgt"], self.start, out=self.x)
+        for g in graphs:
+            g.replay()
+        toks = self.toks[:steps]
         return (toks, self.logits_out[:steps]) if want_logits else (toks, None)
 
     # ------------------------------------------------------------------------------------------------ user call

@@ -365,20 +365,26 @@ def greedy_token_workspace(N: int, J: int, device) -> torch.Tensor:
 
 def greedy_token(W: torch.Tensor, X: torch.Tensor, bias: Optional[torch.Tensor], workspace: torch.Tensor, idx: torch.Tensor,
                  emb: Optional[torch.Tensor] = None, pos: Optional[torch.Tensor] = None,
-                 x_next: Optional[torch.Tensor] = None) -> bool:
+                 x_next: Optional[torch.Tensor] = None, step: Optional[torch.Tensor] = None,
+                 next_step: Optional[torch.Tensor] = None) -> bool:
     """idx[j] = arg max of the row W @ X[j] + bias, and x_next[j] = emb[idx[j]] (+ pos): the end of a greedy decode step and
-    the input of the next one, without the logits in memory.  Returns False when the shape has no kernel (use gemm_wx,
-    argmax, gather_rows)."""
+    the input of the next one, without the logits in memory.  With `step` and `next_step` (int64 [1] on the device, not the
+    same), idx is a table [rows, J]: the tokens go to row step, which has to exist, and next_step = step + 1.  Returns False
+    when the shape has no kernel (use gemm_wx, argmax, gather_rows)."""
     _req_half_cuda(W, bias, emb, pos, x_next)
     _req_half_cuda_rows(X)
     N, K = W.shape
     J = X.shape[0]
-    if idx.dtype != torch.int64 or not idx.is_cuda or not idx.is_contiguous() or idx.numel() != J:
+    if idx.dtype != torch.int64 or not idx.is_cuda or not idx.is_contiguous() or (idx.numel() != J if step is None else idx.shape[-1] != J):
         raise TypeError("expected a contiguous CUDA int64 index tensor with one element per row of X")
+    for t in (step, next_step):
+        if t is not None and (t.dtype != torch.int64 or not t.is_cuda or t.numel() != 1):
+            raise TypeError("a step is one CUDA int64 element")
     if workspace.numel() * workspace.element_size() < _lib.lib().pimb200_greedy_token_workspace(N, J):
         raise ValueError("workspace too small")
-    rc = _lib.lib().pimb200_greedy_token(_ptr(W), _ptr(X), _ptr(bias), N, K, J, X.stride(0), _ptr(workspace), _ptr(idx), _ptr(emb),
-                                         _ptr(pos), _ptr(x_next), emb.shape[1] if emb is not None else 0, _stream())
+    rc = _lib.lib().pimb200_greedy_token_step(_ptr(W), _ptr(X), _ptr(bias), N, K, J, X.stride(0), _ptr(workspace), _ptr(idx),
+                                              _ptr(step), _ptr(next_step), _ptr(emb), _ptr(pos), _ptr(x_next),
+                                              emb.shape[1] if emb is not None else 0, _stream())
     if rc == _lib.ERR_UNSUPPORTED:
         return False
     check(rc, "greedy_token")

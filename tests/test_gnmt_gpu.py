@@ -95,3 +95,40 @@ def test_gnmt_results_independent_of_group_and_repeatable():
     cut = tr.translate(sentences)
     for full, c in zip(a, cut):
         assert c == (full[:full.index(cfg.eos) + 1] if cfg.eos in full else full)
+
+
+@pytest.mark.parametrize("group,hidden", [(8, 64), (4, 40)])
+def test_gnmt_any_number_of_steps_from_few_graphs(group, hidden):
+    # every step count gives the same tokens as far as it goes, whatever was decoded before, and no count has graphs of its own
+    cfg = to.GnmtConfig(vocab=300, hidden=hidden, max_steps=27, min_len=3, max_len=17)
+    w = to.make_gnmt_weights(cfg, seed=9, gain=2.0, logit_gain=8.0)
+    sentences = to.make_sentences(7, cfg, seed=10)
+    forced = [[(5 * i + t) % 300 for t in range(27)] for i in range(7)]
+    tr = _translator(cfg, w, group)
+    full = tr.translate(sentences, steps=27)
+    ftoks, flogits = tr.translate(sentences, steps=27, forced=forced, want_logits=True)
+    for steps in (1, 2, 3, 7, 8, 9, 11, 16, 25, 26, 27, 5):
+        assert tr.translate(sentences, steps=steps) == [t[:steps] for t in full]
+        if steps % 3 == 0:
+            toks, logits = tr.translate(sentences, steps=steps, forced=forced, want_logits=True)
+            assert toks == [t[:steps] for t in ftoks]
+            assert all(torch.equal(a, b[:steps]) for a, b in zip(logits, flogits))
+    assert len([k for k in tr._graphs if not k[1]]) <= 3
+    assert tr.logits_out is None                     # given back by the first decode that does not ask for it
+
+
+@pytest.mark.parametrize("J", [5, 40])
+def test_greedy_token_rows_of_a_table(J):
+    from pimaicompiler_b200 import ops
+    g = torch.Generator().manual_seed(J)
+    W, X, emb = (torch.randn(*s, generator=g).half().cuda() for s in ((500, 64), (J, 64), (500, 72)))
+    ws = ops.greedy_token_workspace(500, J, "cuda")
+    want, x = torch.zeros(J, dtype=torch.int64, device="cuda"), torch.zeros(J, 72, dtype=torch.float16, device="cuda")
+    assert ops.greedy_token(W, X, None, ws, want, emb, None, x)
+    table, step, y = torch.full((5, J), -1, device="cuda"), torch.zeros(2, dtype=torch.int64, device="cuda"), torch.empty_like(x)
+    for t in range(4):
+        assert ops.greedy_token(W, X, None, ws, table, emb, None, y, step[t & 1:(t & 1) + 1], step[1 - (t & 1):2 - (t & 1)])
+    assert bool((table[:4] == want).all()) and bool((table[4] == -1).all()) and torch.equal(x, y)
+    assert step.tolist() == [4, 3]
+    with pytest.raises(Exception):
+        ops.greedy_token(W, X, None, ws, table, emb, None, y, step[:1], step[:1])
