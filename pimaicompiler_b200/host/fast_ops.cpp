@@ -34,6 +34,7 @@ inline const at::Tensor& half_contiguous(PyObject* o) {
     if (!t.is_contiguous()) fail(PyExc_ValueError, "expected a contiguous tensor");
     return t;
 }
+// (the address of a tensor without storage, such as a tracer's, is a C++ exception: asked for while Python's lock is held)
 inline const void* half_or_null(PyObject* o) { return o == Py_None ? nullptr : half_contiguous(o).data_ptr(); }
 inline void require(bool ok, const char* msg) {
     if (!ok) fail(PyExc_AssertionError, msg);
@@ -63,13 +64,15 @@ void check(int status, const char* where) {
     throw PyError();
 }
 
-// a call of the C ABI: other Python threads run meanwhile (it may allocate, or wait for another thread's call)
+// a call of the C ABI: other Python threads run meanwhile (it may allocate, or wait for another thread's call).  `call` takes
+// addresses and numbers only
 template <typename F>
 int abi(F call) {
-    PyThreadState* state = PyEval_SaveThread();
-    const int status = call();
-    PyEval_RestoreThread(state);
-    return status;
+    struct Unlocked {
+        PyThreadState* state = PyEval_SaveThread();
+        ~Unlocked() { PyEval_RestoreThread(state); }
+    } unlocked;
+    return call();
 }
 
 // runs f and turns C++ exceptions into Python ones
@@ -120,8 +123,9 @@ PyObject* gemv_mv(PyObject*, PyObject* const* a, Py_ssize_t n) {
         require(x.numel() == K, "x does not have one element per column of W");
         const int act = (int)as_long(a[3]);
         Out y = output(a[4], {N}, at::kHalf, W);
-        check(abi([&] { return pimb200_gemv_mv(W.data_ptr(), x.data_ptr(), bias, y.get().data_ptr(), (int)N, (int)K, act, stream()); }),
-              "gemv_mv");
+        const void *wp = W.data_ptr(), *xp = x.data_ptr();
+        void *yp = y.get().data_ptr(), *st = stream();
+        check(abi([&] { return pimb200_gemv_mv(wp, xp, bias, yp, (int)N, (int)K, act, st); }), "gemv_mv");
         return y.release();
     });
 }
@@ -137,8 +141,9 @@ PyObject* gemv_vm(PyObject*, PyObject* const* a, Py_ssize_t n) {
         require(x.numel() == K, "x does not have one element per row of A");
         const int act = (int)as_long(a[3]);
         Out y = output(a[4], {N}, at::kHalf, A);
-        check(abi([&] { return pimb200_gemv_vm(x.data_ptr(), A.data_ptr(), bias, y.get().data_ptr(), (int)K, (int)N, act, stream()); }),
-              "gemv_vm");
+        const void *xp = x.data_ptr(), *ap = A.data_ptr();
+        void *yp = y.get().data_ptr(), *st = stream();
+        check(abi([&] { return pimb200_gemv_vm(xp, ap, bias, yp, (int)K, (int)N, act, st); }), "gemv_vm");
         return y.release();
     });
 }
@@ -159,9 +164,10 @@ PyObject* gemm_wx(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const int act = (int)as_long(a[3]);
         Out y = output(a[5], {J, N}, as_bool(a[4]) ? at::kFloat : at::kHalf, W);
         const at::Tensor& Y = y.get();
-        check(abi([&] { return pimb200_gemm_wx(W.data_ptr(), X.data_ptr(), bias, Y.data_ptr(), (int)N, (int)K, (int)J, (int)X.stride(0),
-                              (int)Y.stride(0), act, Y.scalar_type() == at::kFloat ? 1 : 0, stream()); }),
-              "gemm_wx");
+        const void *wp = W.data_ptr(), *xp = X.data_ptr();
+        void *yp = Y.data_ptr(), *st = stream();
+        const int ldx = (int)X.stride(0), ldy = (int)Y.stride(0), f32 = Y.scalar_type() == at::kFloat ? 1 : 0;
+        check(abi([&] { return pimb200_gemm_wx(wp, xp, bias, yp, (int)N, (int)K, (int)J, ldx, ldy, act, f32, st); }), "gemm_wx");
         return y.release();
     });
 }
@@ -202,8 +208,9 @@ PyObject* lstm_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
             }
             Py_DECREF(given);
             if (!three) fail(PyExc_ValueError, "out holds y, hn and cn");
-            check(abi([&] { return pimb200_lstm_forward(h, x.data_ptr(), (int)T, (int)B, h0, c0, p[0], p[1], p[2], bf ? 1 : 0, stream()); }),
-                  "lstm_forward");
+            const void* xp = x.data_ptr();
+            void* st = stream();
+            check(abi([&] { return pimb200_lstm_forward(h, xp, (int)T, (int)B, h0, c0, p[0], p[1], p[2], bf ? 1 : 0, st); }), "lstm_forward");
             Py_INCREF(a[8]);
             return a[8];
         }
@@ -211,9 +218,9 @@ PyObject* lstm_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         o.y.own = empty({x.size(0), x.size(1), D * H}, at::kHalf, x);
         o.hn.own = empty({LD, B, H}, at::kHalf, x);
         o.cn.own = empty({LD, B, H}, at::kHalf, x);
-        check(abi([&] { return pimb200_lstm_forward(h, x.data_ptr(), (int)T, (int)B, h0, c0, o.y.own.data_ptr(), o.hn.own.data_ptr(),
-                                                    o.cn.own.data_ptr(), bf ? 1 : 0, stream()); }),
-              "lstm_forward");
+        const void* xp = x.data_ptr();
+        void *yp = o.y.own.data_ptr(), *hp = o.hn.own.data_ptr(), *cp = o.cn.own.data_ptr(), *st = stream();
+        check(abi([&] { return pimb200_lstm_forward(h, xp, (int)T, (int)B, h0, c0, yp, hp, cp, bf ? 1 : 0, st); }), "lstm_forward");
         return o.release();
     });
 }
@@ -234,9 +241,11 @@ PyObject* lstm_forward_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
         o.y.own = empty({x.size(0), D * H}, at::kHalf, x);
         o.hn.own = empty({LD, B, H}, at::kHalf, x);
         o.cn.own = empty({LD, B, H}, at::kHalf, x);
-        check(abi([&] { return pimb200_lstm_forward_packed(h, x.data_ptr(), sizes.data_ptr<int64_t>(), (int)sizes.numel(), h0, c0,
-                                          o.y.own.data_ptr(), o.hn.own.data_ptr(), o.cn.own.data_ptr(), stream()); }),
-              "lstm_forward_packed");
+        const void* xp = x.data_ptr();
+        const int64_t* sp = sizes.data_ptr<int64_t>();
+        const int steps = (int)sizes.numel();
+        void *yp = o.y.own.data_ptr(), *hp = o.hn.own.data_ptr(), *cp = o.cn.own.data_ptr(), *st = stream();
+        check(abi([&] { return pimb200_lstm_forward_packed(h, xp, sp, steps, h0, c0, yp, hp, cp, st); }), "lstm_forward_packed");
         return o.release();
     });
 }
