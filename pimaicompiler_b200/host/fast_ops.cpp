@@ -159,7 +159,7 @@ PyObject* gemm_wx(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (X.dim() && X.stride(-1) != 1) fail(PyExc_ValueError, "expected a contiguous last dimension");
         if (W.dim() != 2) fail(PyExc_ValueError, "expected a 2-D weight matrix");
         const int64_t N = W.size(0), K = W.size(1);
-        require(X.dim() == 2 && X.size(1) == K, "X does not have the columns of W");
+        require(X.dim() >= 2 && X.size(1) == K && X.stride(1) == 1, "X does not have the columns of W");
         const int64_t J = X.size(0);
         const int act = (int)as_long(a[3]);
         Out y = output(a[5], {J, N}, as_bool(a[4]) ? at::kFloat : at::kHalf, W);
@@ -185,7 +185,7 @@ struct LstmOut {
     }
 };
 
-// lstm_forward(handle, layers * directions, directions, hidden, x, h0, c0, batch_first, out)
+// lstm_forward(handle, layers * directions, directions, hidden, x, h0, c0, batch_first, out): out is None or a tuple (y, hn, cn)
 PyObject* lstm_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
         if (n != 9) fail(PyExc_TypeError, "lstm_forward takes 9 arguments");
@@ -198,16 +198,12 @@ PyObject* lstm_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (x.dim() != 3) fail(PyExc_ValueError, "expected a 3-D input");
         const int64_t B = x.size(bf ? 0 : 1), T = x.size(bf ? 1 : 0);
         if (a[8] != Py_None) {
-            PyObject* given = PySequence_Fast(a[8], "out holds y, hn and cn");
-            if (!given) throw PyError();
-            void* p[3] = {nullptr, nullptr, nullptr};
-            const bool three = PySequence_Fast_GET_SIZE(given) == 3;
-            for (int i = 0; three && i < 3; ++i) {
-                PyObject* t = PySequence_Fast_GET_ITEM(given, i);
-                if (t != Py_None && THPVariable_Check(t)) p[i] = THPVariable_Unpack(t).data_ptr();
+            if (!PyTuple_Check(a[8]) || PyTuple_GET_SIZE(a[8]) != 3) fail(PyExc_ValueError, "out holds y, hn and cn");
+            void* p[3];
+            for (int i = 0; i < 3; ++i) {
+                PyObject* t = PyTuple_GET_ITEM(a[8], i);
+                p[i] = t == Py_None ? nullptr : tensor(t).data_ptr();
             }
-            Py_DECREF(given);
-            if (!three) fail(PyExc_ValueError, "out holds y, hn and cn");
             const void* xp = x.data_ptr();
             void* st = stream();
             check(abi([&] { return pimb200_lstm_forward(h, xp, (int)T, (int)B, h0, c0, p[0], p[1], p[2], bf ? 1 : 0, st); }), "lstm_forward");

@@ -454,6 +454,9 @@ class Lstm:
 
     def forward(self, x: torch.Tensor, h0: Optional[torch.Tensor] = None, c0: Optional[torch.Tensor] = None,
                 batch_first: bool = False, out=None):
+        if out is not None:
+            y, hn, cn = out
+            out = (y, hn, cn)
         return (_lib._native or _lib.native()).lstm_forward(self._handle, self.L * self.D, self.D, self.H, x, h0, c0,
                                                             batch_first, out)
 
@@ -474,5 +477,7 @@ class Lstm:
 
     def forward_packed(self, data: torch.Tensor, batch_sizes: torch.Tensor, h0: Optional[torch.Tensor] = None,
                        c0: Optional[torch.Tensor] = None):
+        if not isinstance(batch_sizes, torch.Tensor):
+            batch_sizes = torch.tensor([int(v) for v in batch_sizes.tolist()], dtype=torch.int64)
         return (_lib._native or _lib.native()).lstm_forward_packed(self._handle, self.L * self.D, self.D, self.H, data,
                                                                    batch_sizes, h0, c0)

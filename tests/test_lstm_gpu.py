@@ -516,3 +516,28 @@ def test_lstm_layer_wavefront_matches_oracle_and_sequential_layers(T, B, I, H, L
         ref = co.lstm(x.numpy(), [p.numpy() for p in ps], L, False, True, h0.numpy(), c0.numpy(), bf)
         for name, a, b in zip(("y", "hn", "cn"), (y, hn, cn), ref):
             assert_close(a, b, LSTM_ATOL, LSTM_RTOL, f"wavefront {name}")
+
+
+def test_outputs_given_in_any_sequence_and_batch_sizes_of_any_array():
+    ops = _ops()
+    g = torch.Generator().manual_seed(2)
+    T, B, I, H = 4, 3, 16, 32
+    m = ops.Lstm([to_dev(p) for p in lstm_params(1, 1, I, H, g)], 1, False, I, H, True)
+    x = to_dev(torch.randn(T, B, I, generator=g))
+    want = m.forward(x)
+    fresh = lambda: [torch.empty_like(t) for t in want]  # noqa: E731
+    for given in (tuple, list, iter, lambda ts: (t for t in ts)):
+        ts = fresh()
+        got = m.forward(x, out=given(ts))
+        assert isinstance(got, tuple) and all(a is b for a, b in zip(got, ts))
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    y, hn, cn = fresh()
+    assert m.forward(x, out=(y, None, None)) == (y, None, None) and torch.equal(y, want[0])
+    for wrong in ((y, 5, cn), (y, hn), (y, "cn", None)):
+        with pytest.raises(Exception):
+            m.forward(x, out=wrong)
+    data = to_dev(torch.randn(7, I, generator=g))
+    sizes = np.array([3, 2, 2])
+    want = m.forward_packed(data, torch.from_numpy(sizes))
+    for given in (sizes, sizes.astype(np.int32), torch.from_numpy(sizes).int(), torch.from_numpy(sizes).cuda(), torch.from_numpy(sizes).float()):
+        assert all(torch.equal(a, b) for a, b in zip(m.forward_packed(data, given), want))
