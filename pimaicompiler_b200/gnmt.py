@@ -29,6 +29,17 @@ import torch
 from . import ops
 
 
+def flat_tokens(sentences: Sequence[torch.Tensor]) -> torch.Tensor:
+    """The sentences' tokens one behind the other, as int64 on the host, whatever type and device each sentence has."""
+    try:
+        flat = torch.cat(list(sentences)) if len(sentences) else torch.zeros(0, dtype=torch.int64)
+    except RuntimeError:             # not on one device
+        flat = None
+    if flat is None or flat.dtype != torch.int64:     # (of several types it would hold them all in a common one)
+        flat = torch.cat([s.to("cpu", torch.int64) for s in sentences])
+    return flat.cpu()
+
+
 def stage_groups(sentences: Sequence[torch.Tensor], G: int, enc_batch: int, max_len: int, pin: bool = False):
     """Host-side packing of sentences into lock-step groups of G.  A group is a dict: `idx` (sentence indices, longest
     first), `S` (longest sentence), `lengths` [G] int64, and `slices`: per `enc_batch` sentences the packed token ids
@@ -40,7 +51,7 @@ def stage_groups(sentences: Sequence[torch.Tensor], G: int, enc_batch: int, max_
     lens = np.fromiter((s.shape[0] for s in sentences), np.int64, n)
     if n and (lens.max() > max_len or lens.min() < 1):
         raise ValueError("sentence length outside 1..max_len")
-    flat = torch.cat(list(sentences)).numpy() if n else np.zeros(0, np.int64)
+    flat = flat_tokens(sentences).numpy()
     start = np.cumsum(lens) - lens
     order = np.argsort(-lens, kind="stable")
     groups = []
@@ -282,7 +293,7 @@ class GnmtTranslator:
 
     def translate(self, sentences: Sequence[torch.Tensor], steps: Optional[int] = None,
                   forced: Optional[Sequence[Sequence[int]]] = None, want_logits: bool = False):
-        """sentences: 1-D int64 CPU tensors of source token ids.  Returns one token list per sentence (cut behind the
+        """sentences: 1-D tensors of source token ids.  Returns one token list per sentence (cut behind the
         first end-of-sentence token unless `steps` is given, which decodes exactly that many steps) and, when asked,
         the logits [steps, V] of each."""
         cfg, G = self.cfg, self.G

@@ -26,6 +26,31 @@ import numpy as np
 import torch
 
 from . import ops
+from .gnmt import flat_tokens
+
+
+def stage_groups(sequences: Sequence[torch.Tensor], G: int, max_len: int, pin: bool = False):
+    """Lock-step groups, longest sequences first: dicts of `idx` (sequence indices), `S` (longest length) and the tensors
+    `ids` and `pos` (token and position of every row, one sequence behind the other), `lengths` [G] and `row0` [G] (first row
+    of every sequence), with `pin` in pinned host memory.  A ragged last group is filled with one-token dummies."""
+    n = len(sequences)
+    lens = np.fromiter((s.shape[0] for s in sequences), np.int64, n)
+    if n and (lens.max() > max_len or lens.min() < 1):
+        raise ValueError("sequence length outside 1..max_len")
+    order = np.argsort(-lens, kind="stable").tolist()
+    keep = (lambda t: t.pin_memory()) if pin else (lambda t: t)
+    dummy = torch.full((1,), 4, dtype=torch.int64)
+    groups = []
+    for g0 in range(0, n, G):
+        idx = order[g0:g0 + G]
+        lens_g = np.ones(G, np.int64)
+        lens_g[:len(idx)] = lens[idx]
+        row0 = np.cumsum(lens_g) - lens_g
+        ids = torch.cat([flat_tokens([sequences[i] for i in idx])] + [dummy] * (G - len(idx)))
+        pos = np.arange(ids.numel()) - np.repeat(row0, lens_g)
+        groups.append({"idx": idx, "S": int(lens_g[0]), "ids": keep(ids), "pos": keep(torch.from_numpy(pos)),
+                       "lengths": keep(torch.from_numpy(lens_g)), "row0": keep(torch.from_numpy(row0))})
+    return groups
 
 
 class TransformerTranslator:
@@ -160,27 +185,8 @@ class TransformerTranslator:
 
     # ------------------------------------------------------------------------------------------------ user call
     def stage(self, sequences: Sequence[torch.Tensor]):
-        """Packs lock-step groups, longest sequences first: dicts of `idx` (sequence indices), `S` (longest length) and, in
-        pinned host memory, `ids` and `pos` (token and position of every row, one sequence behind the other), `lengths` [G]
-        and `row0` [G] (first row of every sequence).  A ragged last group is filled with one-token dummies."""
-        G, n = self.G, len(sequences)
-        lens = np.fromiter((s.shape[0] for s in sequences), np.int64, n)
-        if n and (lens.max() > self.cfg.max_len or lens.min() < 1):
-            raise ValueError("sequence length outside 1..max_len")
-        order = np.argsort(-lens, kind="stable").tolist()
-        pin = lambda t: t.pin_memory()
-        dummy = torch.full((1,), 4, dtype=torch.int64)
-        groups = []
-        for g0 in range(0, n, G):
-            idx = order[g0:g0 + G]
-            lens_g = np.ones(G, np.int64)
-            lens_g[:len(idx)] = lens[idx]
-            row0 = np.cumsum(lens_g) - lens_g
-            ids = torch.cat([sequences[i] for i in idx] + [dummy] * (G - len(idx)))
-            pos = np.arange(ids.numel()) - np.repeat(row0, lens_g)
-            groups.append({"idx": idx, "S": int(lens_g[0]), "ids": pin(ids), "pos": pin(torch.from_numpy(pos)),
-                           "lengths": pin(torch.from_numpy(lens_g)), "row0": pin(torch.from_numpy(row0))})
-        return groups
+        """Packs the sequences into lock-step groups (see stage_groups)."""
+        return stage_groups(sequences, self.G, self.cfg.max_len, pin=True)
 
     def to_device(self, group: dict) -> dict:
         return {k: v.to(self.dev, non_blocking=True) if isinstance(v, torch.Tensor) else v for k, v in group.items()}
@@ -197,7 +203,7 @@ class TransformerTranslator:
 
     def translate(self, sequences: Sequence[torch.Tensor], steps: Optional[int] = None,
                   forced: Optional[Sequence[Sequence[int]]] = None, want_logits: bool = False):
-        """sequences: 1-D int64 CPU tensors of source token ids.  Returns one token list per sequence (cut behind the first
+        """sequences: 1-D tensors of source token ids.  Returns one token list per sequence (cut behind the first
         end-of-sequence token unless `steps` is given) and, when asked, each one's logits [steps, V]."""
         cfg, G = self.cfg, self.G
         n = len(sequences)

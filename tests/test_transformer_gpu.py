@@ -71,3 +71,16 @@ def test_transformer_benchmark_configuration_full_length():
     seqs = to.make_sentences(5, cfg, seed=2)
     decided, total = _follow(cfg, w, seqs, 32, cfg.max_steps, 3e-2, 2e-2, 0.1)
     assert decided > total // 5
+
+
+def test_translators_take_tokens_of_any_type_and_device():
+    from pimaicompiler_b200.gnmt import GnmtTranslator
+    from pimaicompiler_b200.transformer import TransformerTranslator
+    gc, tc = to.GnmtConfig(vocab=300, hidden=64, max_steps=5, min_len=3, max_len=17), to.TransformerConfig(
+        vocab=300, d_model=128, heads=2, layers=1, ffn=256, max_steps=5, min_len=3, max_len=17)
+    for tr, cfg in ((GnmtTranslator(gc, to.make_gnmt_weights(gc, seed=3), group=4), gc),
+                    (TransformerTranslator(tc, to.make_transformer_weights(tc, seed=3), group=4), tc)):
+        sents = to.make_sentences(6, cfg, seed=5)
+        want = tr.translate(sents, steps=5)
+        for other in ([s.int() for s in sents], [s.cuda() for s in sents], [s.cuda() if i % 2 else s.short() for i, s in enumerate(sents)]):
+            assert tr.translate(other, steps=5) == want

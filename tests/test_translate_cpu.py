@@ -49,3 +49,19 @@ def test_round_robin_shards_partition_the_streams():
             for k, s in enumerate(sh):
                 back[r + k * world] = s
         assert all(torch.equal(a, b) for a, b in zip(back, seqs))
+
+
+def test_tokens_of_any_type_are_staged_as_int64():
+    # the device takes 64-bit token ids only
+    from pimaicompiler_b200 import transformer
+    cfg = syn.GnmtConfig(vocab=300, hidden=64, max_steps=12, min_len=3, max_len=17)
+    sents = syn.make_sentences(8, cfg, 5)
+    for types in ([torch.int32], [torch.int16], [torch.uint8, torch.int64], [torch.int64, torch.int32], [torch.float16, torch.int64, torch.int32]):
+        src = [s.remainder(250) for s in sents]
+        other = [s.to(types[i % len(types)]) for i, s in enumerate(src)]
+        for G in (4, 5, 8):
+            for a, b in ((stage_groups(src, G, 3, 17), stage_groups(other, G, 3, 17)),
+                         (transformer.stage_groups(src, G, 17), transformer.stage_groups(other, G, 17))):
+                for ga, gb in zip(a, b):
+                    for xa, xb in zip(ga.get("slices", [ga]), gb.get("slices", [gb])):
+                        assert xb["ids"].dtype == torch.int64 and torch.equal(xa["ids"], xb["ids"])
