@@ -294,7 +294,24 @@ __global__ void __launch_bounds__(256) lstm_cell_kernel(CellArgs a) {
 // H = 1024: 27.6 us as two products and this kernel, 15.4 us as one).
 constexpr int kCellGemmMinB = 8;
 constexpr int kCellRowsMinB = 33;
+// Do rows of two views share elements?  Rows equally far apart: compared column by column, around the row, so that halves of
+// the same buffer do not; otherwise by the range of their addresses.
+static bool rows_overlap(const __half* a, long a_ld, int a_cols, const __half* b, long b_ld, int b_cols, int rows) {
+    if (!a || !b) return false;
+    const uintptr_t a0 = reinterpret_cast<uintptr_t>(a), b0 = reinterpret_cast<uintptr_t>(b);
+    const uintptr_t a1 = a0 + ((uintptr_t)(rows - 1) * a_ld + a_cols) * 2, b1 = b0 + ((uintptr_t)(rows - 1) * b_ld + b_cols) * 2;
+    if (a1 <= b0 || b1 <= a0) return false;
+    if (a_ld != b_ld) return true;
+    const uintptr_t row = (uintptr_t)a_ld * 2, off = b0 >= a0 ? (b0 - a0) % row : (row - (a0 - b0) % row) % row;   // of b behind a
+    return off < (uintptr_t)a_cols * 2 || off + (uintptr_t)b_cols * 2 > row;
+}
 static int launch_cell(const RowsCell& c, cudaStream_t st) {
+    // its CTAs read all inputs while others write their outputs: a step whose outputs lie over its inputs takes two products
+    // and the gate kernel, which are done with the inputs by then
+    const struct { const __half* p; long ld; } outs[] = {{c.y, c.y_ld}, {c.hn, c.H}, {c.cn, c.H}};
+    for (const auto& o : outs)
+        if (rows_overlap(c.x, c.x_ld, c.I, o.p, o.ld, c.H, c.J) || rows_overlap(c.h0, c.H, c.H, o.p, o.ld, c.H, c.J))
+            return PIMB200_ERR_UNSUPPORTED;
     return c.J < kCellRowsMinB ? launch_lstm_cell_skinny(c, st) : launch_gemm_rows_cell(c, st);
 }
 struct CellPointArgs {

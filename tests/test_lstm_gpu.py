@@ -541,3 +541,21 @@ def test_outputs_given_in_any_sequence_and_batch_sizes_of_any_array():
     want = m.forward_packed(data, torch.from_numpy(sizes))
     for given in (sizes, sizes.astype(np.int32), torch.from_numpy(sizes).int(), torch.from_numpy(sizes).cuda(), torch.from_numpy(sizes).float()):
         assert all(torch.equal(a, b) for a, b in zip(m.forward_packed(data, given), want))
+
+
+@pytest.mark.parametrize("B,H", [(8, 1024), (32, 1024), (130, 512), (2048, 1024)])
+def test_decode_step_whose_output_lies_over_its_input(B, H):
+    ops = _ops()
+    g = torch.Generator().manual_seed(B)
+    I = H
+    m = ops.Lstm([to_dev(p) for p in lstm_params(1, 1, I, H, g)], 1, False, I, H, True)
+    rows = to_dev(torch.randn(B, 2 * H, generator=g))
+    h0, c0 = (to_dev(torch.randn(B, H, generator=g) * 0.5) for _ in range(2))
+    y, hn, cn = (torch.empty(B, H, dtype=torch.float16, device="cuda") for _ in range(3))
+    assert m.forward_step(rows[:, :I], h0, c0, y, hn, cn)
+    for _ in range(10):
+        for at in (0, 8, H // 2, H):                # H: the other half of the same rows, which overlaps nothing
+            buf, hb, cb = rows.clone(), torch.empty_like(hn), torch.empty_like(cn)
+            assert m.forward_step(buf[:, :I], h0, c0, buf[:, at:at + H], hb, cb)
+            for got, want in ((buf[:, at:at + H], y), (hb, hn), (cb, cn)):
+                assert_close(got, want, LSTM_ATOL, LSTM_RTOL, f"output {at} columns behind the input")
