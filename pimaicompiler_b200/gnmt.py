@@ -12,7 +12,7 @@ hundreds of them runs `group` sentences in lock step instead:
   * decoder: one step for the whole group is four cells (each one launch: both products and the gate math; the output, for
     the last two with the residual added, goes straight into the next cell's concatenated input), the query projection, one
     attention launch (which writes the context into the other halves of those inputs), and the vocabulary projection with
-    its arg max and the next token's embedding (two launches, no logits in memory).  Eight, two and one steps are captured
+    its arg max and the next token's embedding (two launches, no logits in memory).  Sixteen, four, two and one steps are captured
     into CUDA graphs when they are first needed, and any number of steps is made of their replays: the step's number lives
     on the device.  The chosen tokens stay there until the group is done.
 
@@ -202,7 +202,7 @@ class GnmtTranslator:
         torch.add(step, 1, out=next_step)
         return n + 1
 
-    CHUNKS = (8, 2, 1)       # steps per graph: of the last one, if any, the state ends up in the other set
+    CHUNKS = (16, 4, 2, 1)   # steps per graph: of the last one, if any, the state ends up in the other set
 
     def _graph(self, steps: int, forced: bool, want_logits: bool):
         """`steps` steps, captured once per (steps, forced, logits) mode."""
