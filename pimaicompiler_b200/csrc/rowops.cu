@@ -474,7 +474,7 @@ __device__ __forceinline__ float ex2_(float x) {
 }
 
 template <int C>
-__global__ void __launch_bounds__(kBahdanauThreads) bahdanau_kernel(
+__global__ void __launch_bounds__(kBahdanauThreads, C == 1 ? 4 : 3) bahdanau_kernel(
     const __half* q, const __half* keys_proj, const __half* values,
     const long long* lengths, const __half* v, const __half* bias, __half* __restrict__ ctx,
     float* __restrict__ scores, long max_len, int H, long row_stride, long seq_stride, long ctx_stride, int copies, long copy_stride) {
