@@ -1111,6 +1111,10 @@ __global__ void __launch_bounds__(kWideThreads, 1) lstm_persistent_wide_kernel(B
 // hidden value has (see lstm_direct.cu: four buffers in turn, this CTA's records of buffer (s + 2) % 4 made sentinels in step
 // s, two sets of buffers for alternate launches).  It is a NaN, so a copy that was too early shows in the tensor warps' sums,
 // without any instruction in their product; they then wait for the records themselves (seen in 1 of 10^4 phases).
+// Observed rather than given by the memory model: sentinels are fenced for the async proxy by the lanes that raise the flag
+// only, and the reader's copy has no proxy fence (in front of the copy it costs several thousand cycles), so a copy could in
+// principle bring a record that is older than the sentinel over it, of step s - 2.  L2 serves both proxies from one copy, the
+// sentinel has been there for a whole step by then, and no wrong value has been seen.
 // Measured at H = 1024, us per step: 48 sequences 3.89 -> 2.94, 64 4.13 -> 3.14, 128 4.82 -> 3.91, together with the gate
 // warps' shorter phase (running addresses, 32-bit record stores: 1660 -> 900 cycles at 128) and the tensor warps' (operands
 // by ldmatrix, the barriers' state asked for ahead of its use, one arrival per warp: 4 x 1500 cycles at 128, of which the
@@ -2574,7 +2578,7 @@ static int lstm_forward_packed_lockstep(pimb200_lstm* h, const __half* data, con
     return PIMB200_OK;
 }
 
-// Layers l and l + 1 (one direction) as a wavefront: true when the shape is the wave kernel's
+// Layers l and l + 1 (one direction) as a wavefront: true when the shape is that of lstm_direct.cu
 static bool wave_fits(const pimb200_lstm* h, int l, int T, int B, bool packed) {
     const int H = h->H;
     return h->wavefront && !packed && h->D == 1 && l + 1 < h->L && T >= 8 && B >= 1 && B <= 8 && H % 16 == 0 &&

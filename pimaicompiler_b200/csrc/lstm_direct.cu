@@ -30,6 +30,11 @@
 // made from the registers that hold h_A, while the gates work and the records are on their way, and stays in the
 // accumulators that W_hh(B) . h_B then continues.
 // Measured at H = 1024, one sequence: 2.80 -> 1.30 us per step for one layer, 2.72 -> 1.81 for a wavefront.
+// What the memory model gives and what is observed: a record's words are relaxed stores and loads, and every word is looked at,
+// so nothing hangs on their order.  That a lane which has seen a CTA's record of step s + 1 finds that CTA's sentinels of
+// buffer (s + 2) % 4, fenced ahead of it, and not the older record, rests on its own two loads staying in order: they are
+// relaxed loads of different addresses, ordered by control flow only (an acquire would invalidate L1 and cost 380 cycles a
+// step).  An SM issues them in order and L2 answers from one copy; no wrong value has been seen.
 // Every wait is bounded; a CTA that gives up raises the status word, and the others, polling, see it.  Giving up keeps the
 // handover exact, or the gates would wait at a barrier for ever: a product warp that gives up in step s notes the step
 // (dead_step keeps the smallest), arrives at that step's barrier and leaves.  The gates pass the barrier of the smallest
