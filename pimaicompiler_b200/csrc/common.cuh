@@ -182,5 +182,16 @@ __device__ __forceinline__ float tanhf_(float x) {
     // tanh(x) = 2*sigmoid(2x) - 1
     return fmaf(2.0f, rcp_approx(1.0f + __expf(-2.0f * x)), -1.0f);
 }
+// The update of one LSTM cell from the sums of its four gates, with three reciprocals instead of five (the special-function unit
+// bounds the gate phase of the batched kernels): sigmoid(a) tanh(b) = (1 - B) / ((1 + A)(1 + B)) for A = e^-a, B = e^-2b.  -2b is
+// capped at 40, where tanh is -1 in fp32, so that 1 - B stays finite; an A without bound makes the quotient 0.  NaNs stay NaNs.
+__device__ __forceinline__ float sigmoid_tanh(float a, float b) {
+    const float A = __expf(-a), B = __expf(min_nan(-2.0f * b, 40.f));
+    return (1.f - B) * rcp_approx((1.f + A) * (1.f + B));
+}
+__device__ __forceinline__ float lstm_cell(float zi, float zf, float zg, float zo, float& c) {
+    c = fmaf(sigmoidf_(zf), c, sigmoid_tanh(zi, zg));
+    return sigmoid_tanh(zo, c);
+}
 
 }  // namespace pimb200

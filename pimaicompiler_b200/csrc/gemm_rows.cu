@@ -107,85 +107,7 @@ __device__ __forceinline__ void store_half16(__half* p, const uint32_t* w) {
     q[1] = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
-// The producer's and the issuer's loops run with all 32 lanes, and only the instructions themselves are predicated on one
-// elected lane (`el`).  Inside an `if (lane == 0)` the compiler keeps addresses and descriptors in per-thread registers and
-// moves each to the uniform ones that these instructions take: the issuer then needed 600 cycles per K block and the
-// producer 510, more than the MMAs and the loads themselves.
-__device__ __forceinline__ uint32_t elect_one() {
-    uint32_t r;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void expect_tx_if(uint32_t el, uint32_t bar, uint32_t bytes) {
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar),
-                 "r"(bytes), "r"(el)
-                 : "memory");
-}
-// the address of a barrier in the CTA of a given rank of the pair
-__device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-// cta_group::2 forms: loads that count their bytes at the pair leader's barrier, the MMA over both CTAs' operands, and a
-// commit that arrives in both
-template <int CG>
-__device__ __forceinline__ void load_2d(uint32_t el, uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
-    if (CG == 1)
-        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}" ::"r"(dst),
-                     "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(el)
-                     : "memory");
-    else
-        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}" ::"r"(dst),
-                     "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(el)
-                     : "memory");
-}
-template <int CG>
-__device__ __forceinline__ void load_3d(uint32_t el, uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
-    if (CG == 1)
-        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}" ::"r"(dst),
-                     "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(el)
-                     : "memory");
-    else
-        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t@q cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}" ::"r"(dst),
-                     "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(el)
-                     : "memory");
-}
-template <int CG>
-__device__ __forceinline__ void mma(uint32_t el, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    if (CG == 1)
-        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-                     "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-                     "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(el)
-                     : "memory");
-    else
-        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-                     "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-                     "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(el)
-                     : "memory");
-}
-template <int CG>
-__device__ __forceinline__ void commit(uint32_t el, uint32_t bar) {
-    if (CG == 1)
-        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
-                     "r"(el)
-                     : "memory");
-    else
-        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(bar),
-                     "h"((uint16_t)3), "r"(el)
-                     : "memory");
-}
-
 }  // namespace
-
-template <int CG>
-__device__ __forceinline__ void pair_sync() {
-    if (CG == 1) __syncthreads();
-    else {
-        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    }
-}
 
 template <int BN, int EPI, int CG>
 __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Args a) {

@@ -14,6 +14,8 @@ bool encode_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
                int elem_bytes);
 bool encode_x_time_major(CUtensorMap* map, const void* base, uint64_t batch, uint64_t steps, uint64_t seq_rows, uint64_t cols,
                          uint64_t ldx_bytes, uint32_t box_t);
+bool encode_3d(CUtensorMap* map, const void* base, uint64_t cols, uint64_t batch, uint64_t steps, uint64_t row_stride_bytes,
+               uint64_t step_stride_bytes, uint32_t box_b);
 int tc_prepare(int* dev, int** status, int* gen);
 int tc_sm_count(int dev);
 

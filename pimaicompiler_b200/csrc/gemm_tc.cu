@@ -63,6 +63,18 @@ bool encode_x_time_major(CUtensorMap* map, const void* base, uint64_t batch, uin
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// [steps][batch][cols] halves, boxes of box_b rows of one step x 64 columns
+bool encode_3d(CUtensorMap* map, const void* base, uint64_t cols, uint64_t batch, uint64_t steps, uint64_t row_stride_bytes,
+               uint64_t step_stride_bytes, uint32_t box_b) {
+    const cuuint64_t dims[3] = {cols, batch, steps};
+    const cuuint64_t strides[2] = {row_stride_bytes, step_stride_bytes};
+    const cuuint32_t box[3] = {64, box_b, 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    return g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // the device's status block and a fresh launch generation; PIMB200_ERR_UNSUPPORTED without the tensor-map encoder
 int tc_prepare(int* dev, int** status, int* gen) {
     PIMB200_CUDA_TRY(cudaGetDevice(dev));

@@ -34,6 +34,7 @@
 #include "tc_common.cuh"
 
 #include "gemm_rows.cuh"
+#include "lstm_batch.cuh"
 #include "lstm_direct.cuh"
 
 namespace pimb200 {
@@ -1920,6 +1921,10 @@ struct pimb200_lstm {
     uint4* bulk_data = nullptr;      // batched variant: [2][n_cta][32] records
     uint32_t* bulk_flags = nullptr;  // [2][n_cta]
     uint32_t bulk_tag = 0;
+    // recurrence for many sequences: counters of its CTA pairs, time-major copy of a batch-first input's steps
+    uint32_t* batch_counters = nullptr;
+    __half* batch_x = nullptr;
+    size_t batch_x_cap = 0;
     int* d_status = nullptr;         // {sticky error code, generation of the launch that gave up}
     int launch_gen = 0;              // generation handed to the last persistent launch (never 0)
     uint32_t tag_counter = 0;
@@ -1965,6 +1970,7 @@ extern "C" int pimb200_lstm_destroy(pimb200_lstm* h) {
     cudaFree(h->pk_row0);
     cudaFree(h->pk_x);
     cudaFree(h->pk_run);
+    cudaFree(h->batch_x);
     cudaFree(h->ybuf[0]);
     cudaFree(h->ybuf[1]);
     cudaFree(h->cstate);
@@ -1997,7 +2003,7 @@ extern "C" int pimb200_lstm_create(const void* const* params, int n_params, int 
     const size_t o_flags = take(std::max((size_t)kBulkFlagCopies * 2, (size_t)kPipeFlagCopies * 2 * 2 * kPipeMaxGroups) * ncta * kPipeFlagWords * 4);
     const size_t zeros = at;
     const size_t o_direct = take(kDirectBytes), o_pipe = take(kPipeBytes), sentinels = at - o_direct;
-    const size_t o_data = take(2 * ncta * kBulkMaxB * 16);
+    const size_t o_data = take(2 * ncta * kBulkMaxB * 16), o_batch = take(kBatchFlagBytes);
     std::vector<size_t> o_w;
     for (int l = 0; l < num_layers; ++l)
         for (int d = 0; d < D; ++d) {
@@ -2016,6 +2022,7 @@ extern "C" int pimb200_lstm_create(const void* const* params, int n_params, int 
     h->pipe_sets.buf = reinterpret_cast<uint4*>(h->arena + o_pipe);
     h->pipe_sets.words = kPipeSetWords;
     h->bulk_data = reinterpret_cast<uint4*>(h->arena + o_data);
+    h->batch_counters = reinterpret_cast<uint32_t*>(h->arena + o_batch);
     for (int l = 0; l < num_layers; ++l) {
         for (int d = 0; d < D; ++d) {
             const int ld = l * D + d, Il = in_size(h, l);
@@ -2604,6 +2611,104 @@ static int run_wave(pimb200_lstm* h, int l, int T, int B, const float* G, long g
     return run_direct(h, a, 2, T, st);
 }
 
+// ---------------------------------------------------------------------------------------------
+// many sequences: the recurrence of lstm_batch.cu over chunks of steps
+//
+// The projection of a chunk's input rows, then the recurrence over its steps: the fp32 gate terms of a thousand sequences by a
+// thousand steps would take 17 GB.  Everything between the layers is time-major (with the sequences' own order, the rows of
+// one step lie a page apart).
+// ---------------------------------------------------------------------------------------------
+constexpr int kBatchMinB = 129;              // fewer sequences: the kernels above
+constexpr long kBatchChunkRows = 131072;     // rows of gate terms per chunk (2 GB at H = 1024)
+
+// dst[t, b, :] <- src[t * t_rows + b * b_rows, :] of `cols` halves, t < T, b < B; a warp per row
+__global__ void lstm_time_major_kernel(const __half* __restrict__ src, long t_rows, long b_rows, __half* __restrict__ dst, int B,
+                                       long rows, int cols, int vec) {
+    const int lane = threadIdx.x & 31;
+    for (long row = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += (long)gridDim.x * (blockDim.x >> 5)) {
+        const __half* s = src + (row / B * t_rows + row % B * b_rows) * cols;
+        __half* d = dst + row * cols;
+        if (vec)
+            for (int i = lane; i < cols / 8; i += 32) reinterpret_cast<uint4*>(d)[i] = __ldg(reinterpret_cast<const uint4*>(s) + i);
+        else
+            for (int i = lane; i < cols; i += 32) d[i] = s[i];
+    }
+}
+
+// strides of a [T, B, features] tensor in rows
+struct RowStrides { long t, b; };
+
+static bool batch_fits(const pimb200_lstm* h, int T, int B) {
+    return B >= kBatchMinB && T >= 8 && h->bulk_wide == 2 && !h->use_tc &&
+           (h->variant == PIMB200_LSTM_AUTO || h->variant == PIMB200_LSTM_PERSISTENT) && lstm_batch_capacity(h->H, h->D) > 0;
+}
+
+// All layers for up to lstm_batch_capacity sequences.  Output row (t, b) at y + (t / y_fold) * y_t + (t % y_fold) * H + b * y_b
+// (in halves; y_fold 1 when bidirectional).  h0, c0, hn, cn: [L * D][total][H], of which these are the B behind the pointers.
+static int forward_batch(pimb200_lstm* h, const __half* x, RowStrides xs, int T, int B, int total, const __half* h0, const __half* c0,
+                         __half* y, long y_t, long y_b, int y_fold, __half* hn, __half* cn, cudaStream_t st) {
+    const int H = h->H, D = h->D, L = h->L;
+    int chunk = (int)std::max(1L, kBatchChunkRows / ((long)B * D));
+    if (chunk > T) chunk = T;
+    else chunk = ceil_div(T, ceil_div(T, chunk));
+    int rc;
+    const long rows = (long)chunk * B;
+    const bool copy = xs.b != 1 || xs.t != B;
+    if ((rc = grow(&h->G, &h->G_cap, (size_t)rows * D * 4 * H)) != PIMB200_OK) return rc;
+    if ((rc = grow(&h->cstate, &h->c_cap, (size_t)D * B * H)) != PIMB200_OK) return rc;
+    if (copy && (rc = grow(&h->batch_x, &h->batch_x_cap, (size_t)rows * h->I)) != PIMB200_OK) return rc;
+    for (int l = 0; l + 1 < L && l < 2; ++l)
+        if ((rc = grow(&h->ybuf[l], &h->y_cap[l], (size_t)T * B * D * H)) != PIMB200_OK) return rc;
+    for (int l = 0; l < L; ++l) {
+        const int Il = in_size(h, l);
+        const bool last = l == L - 1;
+        const __half* X = l == 0 ? x : h->ybuf[(l - 1) & 1];
+        BatchArgs a = {};
+        a.dirs = D;
+        a.g_tstride = (long)B * 4 * H; a.g_bstride = 4L * H;
+        a.y_tstride = last ? y_t : (long)B * D * H; a.y_bstride = last ? y_b : (long)D * H; a.y_fold = last ? y_fold : 1;
+        a.H = H; a.T = T; a.B = B;
+        a.counters = h->batch_counters; a.status = h->d_status; a.poll_limit = h->poll_limit; a.trace = h->trace;
+        for (int d = 0; d < D; ++d) {
+            BatchDir& r = a.dir[d];
+            const int ld = l * D + d;
+            const size_t off = (size_t)ld * total * H;
+            r.Whh = h->w_hh[ld]; r.bias = h->bias[ld]; r.G = h->G + (size_t)d * rows * 4 * H;
+            r.h0 = h0 ? h0 + off : nullptr; r.c0 = c0 ? c0 + off : nullptr;
+            r.y = (last ? y : h->ybuf[l & 1]) + (size_t)d * H;
+            r.hn = hn ? hn + off : nullptr; r.cn = cn ? cn + off : nullptr;
+            r.reverse = d;
+            a.c_state[d] = h->cstate + (size_t)d * B * H;
+        }
+        for (a.begin = 0; a.begin < T; a.begin += a.steps) {
+            a.steps = std::min(chunk, T - a.begin);
+            const int n = a.steps * B;
+            for (int d = 0; d < D; ++d) {
+                const int t0 = d ? T - a.begin - a.steps : a.begin;      // the chunk's first timestep
+                const __half* Xc = X + (size_t)t0 * B * Il;
+                if (l == 0 && copy) {
+                    const __half* src = x + t0 * xs.t * (long)Il;
+                    const int vec = Il % 8 == 0 && aligned16(src);
+                    lstm_time_major_kernel<<<std::min(ceil_div(n, 8), 8 * h->sm_count), 256, 0, st>>>(src, xs.t, xs.b, h->batch_x, B, n, Il, vec);
+                    if ((rc = launch_status()) != PIMB200_OK) return rc;
+                    Xc = h->batch_x;
+                }
+                if ((rc = launch_gemm_wx(h->w_ih[l * D + d], Xc, nullptr, h->G + (size_t)d * rows * 4 * H, 4 * H, Il, n, Il, 4 * H,
+                                         PIMB200_ACT_NONE, 1, st)) != PIMB200_OK)
+                    return rc;
+            }
+            a.gen = next_gen(h);
+            if (h->prof) prof_mark(h, st);
+            if ((rc = launch_lstm_batch(a, st)) != PIMB200_OK) return rc;
+            if (h->prof) {
+                prof_mark(h, st);
+                h->prof_bytes += (double)D * a.steps * 4.0 * H * H * 2.0;
+            }
+        }
+    }
+    return PIMB200_OK;
+}
+
 static int lstm_forward_impl(pimb200_lstm* h, const __half* x, const SeqLayout& sq, const __half* h0,
                              const __half* c0, __half* y, __half* hn, __half* cn, int batch_first,
                              cudaStream_t st) {
@@ -2620,6 +2725,19 @@ static int lstm_forward_impl(pimb200_lstm* h, const __half* x, const SeqLayout& 
     // path for the padded rows; the streamed kernels below take every other case)
     if (packed && h->packed_lockstep && h->variant != PIMB200_LSTM_STREAMED && T > 1 && H % 16 == 0 && B <= kPipeMaxB)
         return lstm_forward_packed_lockstep(h, x, sq, h0, c0, y, hn, cn, st);
+    // many sequences, in equal parts of what a launch takes
+    if (!packed && batch_fits(h, T, B) && aligned16(y) && (!h0 || aligned16(h0)) && (!hn || aligned16(hn))) {
+        const int parts = ceil_div(B, lstm_batch_capacity(H, D)), per = ceil_div(B, parts);
+        const RowStrides xs = batch_first ? RowStrides{1, x_seq} : RowStrides{B, 1};
+        const long y_t = (batch_first ? 1L : B) * D * H, y_b = (batch_first ? (long)T : 1L) * D * H;
+        for (int b = 0; b < B; b += per) {
+            const size_t off = (size_t)b * H;
+            if ((rc = forward_batch(h, x + b * xs.b * h->I, xs, T, std::min(per, B - b), B, h0 ? h0 + off : nullptr, c0 ? c0 + off : nullptr,
+                                    y + b * y_b, y_t, y_b, 1, hn ? hn + off : nullptr, cn ? cn + off : nullptr, st)) != PIMB200_OK)
+                return rc;
+        }
+        return PIMB200_OK;
+    }
     // decode form: seq_len 1, every extent a multiple of 8 and 16-byte aligned -> one fused cell launch per layer
     bool cell = !packed && T == 1 && h->variant != PIMB200_LSTM_PERSISTENT && h->variant != PIMB200_LSTM_PERSISTENT_TAGGED &&
                 H % 8 == 0 && h->I % 8 == 0 && aligned16(x) && aligned16(y) && (!h0 || aligned16(h0)) && (!batch_first || x_seq == T);
@@ -2736,6 +2854,18 @@ int lstm_forward_batch_first(pimb200_lstm* h, const __half* x, long x_seq_rows, 
     SeqLayout sq;
     sq.T = T; sq.B = B; sq.batch_sizes = nullptr; sq.x_seq_rows = x_seq_rows;
     return lstm_forward_impl(h, x, sq, nullptr, nullptr, y, nullptr, nullptr, 1, st);
+}
+
+// How many batch-first sequences lstm_forward_folded takes at once (0: the sizes are not its own, or too few sequences).
+int lstm_folded_capacity(const pimb200_lstm* h, int T, int B) {
+    return h->D == 1 && batch_fits(h, T, B) ? lstm_batch_capacity(h->H, 1) : 0;
+}
+// Forward of x [.., B, T, I] (sequences x_seq_rows apart when batch_first, else time-major) into the time-major
+// y [T / fold][B][fold * H]: `fold` consecutive steps of a sequence side by side.
+int lstm_forward_folded(pimb200_lstm* h, const __half* x, int batch_first, long x_seq_rows, int T, int B, int fold, __half* y, cudaStream_t st) {
+    std::lock_guard<std::mutex> lk(h->mu);
+    return forward_batch(h, x, batch_first ? RowStrides{1, x_seq_rows} : RowStrides{B, 1}, T, B, B, nullptr, nullptr, y,
+                         (long)B * fold * h->H, (long)fold * h->H, fold, nullptr, nullptr, st);
 }
 
 // Decode step of a one-layer, one-direction handle for B >= 8 sequences with strided rows: x rows x_ld halves apart, the

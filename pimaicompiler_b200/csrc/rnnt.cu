@@ -17,6 +17,8 @@
 //   joint: Linear(EH+PH -> JH) -> ReLU -> Linear(JH -> V); greedy, at most one symbol per frame
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include <mutex>
 #include <vector>
 
@@ -34,6 +36,8 @@ namespace pimb200 {
 void lstm_pack_matrix(const __half* src, __half* dst, int H, int cols, cudaStream_t st);
 void lstm_pack_bias(const __half* b_ih, const __half* b_hh, float* dst, int H, cudaStream_t st);
 }
+int lstm_folded_capacity(const pimb200_lstm* h, int T, int B);
+int lstm_forward_folded(pimb200_lstm* h, const __half* x, int batch_first, long x_seq_rows, int T, int B, int fold, __half* y, cudaStream_t st);
 int lstm_forward_batch_first(pimb200_lstm* h, const __half* x, long x_seq_rows, int T, int B, __half* y, cudaStream_t st);
 
 __global__ void rnnt_add_bias_rows_kernel(float* __restrict__ P0, const float* __restrict__ bias, int n, int rows) {
@@ -66,7 +70,8 @@ __global__ void rnnt_widen_kernel(const __half* __restrict__ src, float* __restr
 
 struct GreedyArgs {
     // per-utterance inputs/outputs
-    const float* E;        // [n_utts][Tp][JH]  encoder half of the joint, bias b1 included
+    const float* E;        // encoder half of the joint, bias b1 included: JH floats of utterance u and frame t at
+    long e_utt, e_frame;   // E + u * e_utt + t * e_frame
     int* tokens;           // [n_utts][Tp]
     int* n_tokens;         // [n_utts]
     float* logits;         // optional [n_utts][Tp][V]
@@ -370,7 +375,7 @@ __global__ void __launch_bounds__(kGreedyThreads, 1) rnnt_greedy_kernel(GreedyAr
     };
 
     for (int utt = cluster_id; utt < a.n_utts; utt += n_clusters) {
-        const float* E = a.E + (size_t)utt * a.Tp * JH;
+        const float* E = a.E + utt * a.e_utt;
         int* tokens = a.tokens + (size_t)utt * a.Tp;
         float* logits = a.logits ? a.logits + (size_t)utt * a.Tp * V : nullptr;
         for (int i = tid; i < 2 * PH; i += nthr) {
@@ -398,8 +403,8 @@ __global__ void __launch_bounds__(kGreedyThreads, 1) rnnt_greedy_kernel(GreedyAr
                 if (trp && tid == 0) trp[0] = clock64();
                 const float e_cur0 = e_next[0], e_cur1 = e_next[1];
                 if (t + 1 < a.Tp) {
-                    if (tid < JH) e_next[0] = __ldcg(E + (size_t)(t + 1) * JH + tid);
-                    if (tid + nthr < JH) e_next[1] = __ldcg(E + (size_t)(t + 1) * JH + tid + nthr);
+                    if (tid < JH) e_next[0] = __ldcg(E + (t + 1) * a.e_frame + tid);
+                    if (tid + nthr < JH) e_next[1] = __ldcg(E + (t + 1) * a.e_frame + tid + nthr);
                 }
                 if (tid < JH) zs[tid] = __float2half_rn(fmaxf(e_cur0 + Pj[tid], 0.f));
                 if (tid + nthr < JH) zs[tid + nthr] = __float2half_rn(fmaxf(e_cur1 + Pj[tid + nthr], 0.f));
@@ -664,7 +669,7 @@ __global__ void __launch_bounds__(kGreedyThreads, 1) rnnt_greedy_multi_kernel(Gr
 #pragma unroll
             for (int m = 0; m < M; ++m) {
                 if (valid & (1u << m)) {
-                    const float* E = a.E + ((size_t)(utt0 + m) * a.Tp + t) * JH;
+                    const float* E = a.E + (utt0 + m) * a.e_utt + t * a.e_frame;
                     for (int i = tid; i < JH; i += nthr)
                         zs[m * JH + i] = __float2half_rn(fmaxf(__ldcg(E + i) + Pj[m * JH + i], 0.f));
                 }
@@ -1134,13 +1139,13 @@ __global__ void __launch_bounds__(kGreedyThreads, 1) rnnt_greedy_mma_kernel(Gree
         float4 e_lo = make_float4(0.f, 0.f, 0.f, 0.f), e_hi = e_lo;
         auto load_E = [&](int t) {
             if (zlive && t < a.Tp) {
-                const float4* ep = reinterpret_cast<const float4*>(a.E + ((size_t)(utt0 + zn) * a.Tp + t) * JH + zk);
+                const float4* ep = reinterpret_cast<const float4*>(a.E + (utt0 + zn) * a.e_utt + t * a.e_frame + zk);
                 e_lo = __ldcg(ep);
                 e_hi = __ldcg(ep + 1);
                 // E streams from HBM once; pull the rows of the frames after this one into L2 now, so that their loads
                 // (which the scheduler makes other phases wait for) return with L2 latency
-                if (t + 2 < a.Tp) asm volatile("prefetch.global.L2 [%0];" ::"l"(ep + (size_t)2 * (JH / 4)));
-                if (t + 1 < a.Tp && t == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(ep + (size_t)(JH / 4)));
+                if (t + 2 < a.Tp) asm volatile("prefetch.global.L2 [%0];" ::"l"(ep + 2 * (a.e_frame / 4)));
+                if (t + 1 < a.Tp && t == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(ep + a.e_frame / 4));
             }
         };
         if (square) load_E(0);
@@ -1170,7 +1175,7 @@ __global__ void __launch_bounds__(kGreedyThreads, 1) rnnt_greedy_mma_kernel(Gree
                     for (int i = tid; i < M * JH; i += nthr) {
                         const int n = i / JH, k = i - n * JH;
                         if (valid & (1u << n)) {
-                            const float e = __ldcg(a.E + ((size_t)(utt0 + n) * a.Tp + t) * JH + k);
+                            const float e = __ldcg(a.E + (utt0 + n) * a.e_utt + t * a.e_frame + k);
                             zs[(size_t)n * zp + k] = __float2half_rn(fmaxf(e + __half2float(Pj[i]), 0.f));
                         }
                     }
@@ -1279,6 +1284,8 @@ static GreedyFn pick_greedy_multi(int gate_rows, int joint_rows, int vocab) {
 // ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
+constexpr int kEncoderBatch = 128;   // utterances in lock step below the sizes of lstm_batch.cu
+
 struct pimb200_rnnt {
     pimb200_rnnt_config cfg;
     int device = 0;
@@ -1302,7 +1309,7 @@ struct pimb200_rnnt {
     int smem_mask_multi = 0;
     size_t smem_bytes_multi = 0;
     int greedy_multi = 1;   // 0 = always one utterance per cluster
-    int enc_batch = 128;    // utterances the encoder advances in lock step
+    int enc_batch = 0;      // utterances the encoder advances in lock step: 0 = as many as its kernels take
     int cluster = 0;        // CTAs per cluster
     int resident = 1;       // clusters of each greedy kernel that are co-resident on the device (occupancy query)
     int resident_mma = 1;
@@ -1589,6 +1596,44 @@ static int regrow(T** p, size_t elems) {
     return PIMB200_OK;
 }
 
+// The greedy loop over n_utts utterances of Tp frames, E as in GreedyArgs
+static int launch_greedy(pimb200_rnnt* h, const float* E, long e_utt, long e_frame, int n_utts, int Tp, int32_t* tokens,
+                         int32_t* n_tokens, float* logits, cudaStream_t st) {
+    const pimb200_rnnt_config& c = h->cfg;
+    auto next_gen = [h] { return h->gen = h->gen == 0x7fffffff ? 1 : h->gen + 1; };
+    GreedyArgs a;
+    a.E = E; a.e_utt = e_utt; a.e_frame = e_frame; a.tokens = tokens; a.n_tokens = n_tokens; a.logits = logits; a.n_utts = n_utts; a.Tp = Tp;
+    a.P0 = h->P0; a.Whh0 = h->Whh0; a.Wih1 = h->Wih1; a.Whh1 = h->Whh1; a.bias1 = h->bias1;
+    a.W1p = h->W1p; a.W1pf = h->W1pf; a.W2 = h->W2; a.b2 = h->b2;
+    a.trace = h->trace;
+    a.status = h->d_status; a.gen = next_gen(); a.poll_limit = h->poll_limit;
+    a.PH = c.pred_hidden; a.JH = c.joint_hidden; a.V = c.vocab; a.blank = c.blank; a.smem_mask = h->smem_mask;
+    const int C = h->cluster;
+    // more utterances than clusters: several utterances per cluster in lock step
+    // greedy_multi: 0 = one utterance per cluster, 1 = best available, 2 = FMA lock-step variant (4 per cluster)
+    const bool crowded = n_utts > h->resident;
+    const bool use_mma = h->mma_ok && h->greedy_multi == 1 && crowded;
+    const bool multi = !use_mma && h->fn_multi && h->greedy_multi >= 1 && crowded;
+    const int groups = use_mma ? ceil_div(n_utts, kMmaUtts) : (multi ? ceil_div(n_utts, kGreedyMulti) : n_utts);
+    // the grid holds as many clusters as are co-resident at this kernel's shared-memory footprint (the occupancy
+    // query of create time), each working through groups cluster, cluster + n_clusters, ...
+    const int max_clusters = use_mma ? h->resident_mma : (multi ? h->resident_multi : h->resident);
+    const int n_clusters = groups < max_clusters ? groups : max_clusters;
+    if (multi) a.smem_mask = h->smem_mask_multi;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(C * n_clusters);
+    lc.blockDim = dim3(512);
+    lc.dynamicSmemBytes = use_mma ? h->smem_bytes_mma : (multi ? h->smem_bytes_multi : h->smem_bytes);
+    lc.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    PIMB200_CUDA_TRY(cudaLaunchKernelEx(&lc, use_mma ? h->fn_mma : (multi ? h->fn_multi : h->fn), a));
+    return PIMB200_OK;
+}
+
 extern "C" int pimb200_rnnt_decode(pimb200_rnnt* h, const void* feats, int T, int n_utts, int32_t* tokens,
                                    int32_t* n_tokens, float* logits, void* stream) {
     if (!h || !feats || !tokens || !n_tokens || T <= 0 || n_utts <= 0) return PIMB200_ERR_BAD_ARG;
@@ -1614,49 +1659,38 @@ extern "C" int pimb200_rnnt_decode(pimb200_rnnt* h, const void* feats, int T, in
     // reach no output of the forward-only encoder, so they are left out and every length takes the lock-step path (37
     // utterances of 727 frames, one by one before: 149.0 -> 12.4 ms).
     const int Te = Tp * c.stack_factor;
-    const int group = h->enc_batch;
+    // Hundreds of utterances: all in lock step, as many as the recurrence of lstm_batch.cu takes, everything time-major; the
+    // first stack writes the frames that are stacked side by side.
+    int per = 0;
+    if (h->enc_batch == 0) {
+        const int cap = std::min(lstm_folded_capacity(h->pre, Te, n_utts), lstm_folded_capacity(h->post, Tp, n_utts));
+        if (cap > 0) per = ceil_div(n_utts, ceil_div(n_utts, cap));
+        if (per > 0 && n_utts % per != 0 && lstm_folded_capacity(h->post, Tp, n_utts % per) == 0) per = 0;
+    }
+    const int group = per > 0 ? per : (h->enc_batch > 0 ? h->enc_batch : kEncoderBatch);
+    int rc;
     for (int u = 0; u < n_utts; u += group) {
         const int g = (n_utts - u < group) ? (n_utts - u) : group;
         __half* y1 = h->y_pre + (size_t)u * Te * EH;
         __half* y2 = h->y_post + (size_t)u * Tp * EH;
-        int rc = lstm_forward_batch_first(h->pre, x + (size_t)u * T * c.feat_dim, T, Te, g, y1, st);
-        if (rc != PIMB200_OK) return rc;
-        rc = lstm_forward_batch_first(h->post, y1, Tp, Tp, g, y2, st);
-        if (rc != PIMB200_OK) return rc;
+        const __half* xu = x + (size_t)u * T * c.feat_dim;
+        if (per > 0) {
+            if ((rc = lstm_forward_folded(h->pre, xu, 1, T, Te, g, c.stack_factor, y1, st)) != PIMB200_OK) return rc;
+            if ((rc = lstm_forward_folded(h->post, y1, 0, 0, Tp, g, 1, y2, st)) != PIMB200_OK) return rc;
+        } else {
+            if ((rc = lstm_forward_batch_first(h->pre, xu, T, Te, g, y1, st)) != PIMB200_OK) return rc;
+            if ((rc = lstm_forward_batch_first(h->post, y1, Tp, Tp, g, y2, st)) != PIMB200_OK) return rc;
+        }
     }
     // encoder half of the joint for every frame of every utterance: one dense GEMM
-    int rc = launch_gemm_wx(h->W1e, h->y_post, h->b1, h->E, JH, EH, n_utts * Tp, EH, JH, PIMB200_ACT_NONE, 1, st);
+    rc = launch_gemm_wx(h->W1e, h->y_post, h->b1, h->E, JH, EH, n_utts * Tp, EH, JH, PIMB200_ACT_NONE, 1, st);
     if (rc != PIMB200_OK) return rc;
-    GreedyArgs a;
-    a.E = h->E; a.tokens = tokens; a.n_tokens = n_tokens; a.logits = logits; a.n_utts = n_utts; a.Tp = Tp;
-    a.P0 = h->P0; a.Whh0 = h->Whh0; a.Wih1 = h->Wih1; a.Whh1 = h->Whh1; a.bias1 = h->bias1;
-    a.W1p = h->W1p; a.W1pf = h->W1pf; a.W2 = h->W2; a.b2 = h->b2;
-    a.trace = h->trace;
-    h->gen = h->gen == 0x7fffffff ? 1 : h->gen + 1;
-    a.status = h->d_status; a.gen = h->gen; a.poll_limit = h->poll_limit;
-    a.PH = c.pred_hidden; a.JH = JH; a.V = c.vocab; a.blank = c.blank; a.smem_mask = h->smem_mask;
-    const int C = h->cluster;
-    // more utterances than clusters: several utterances per cluster in lock step
-    // greedy_multi: 0 = one utterance per cluster, 1 = best available, 2 = FMA lock-step variant (4 per cluster)
-    const bool crowded = n_utts > h->resident;
-    const bool use_mma = h->mma_ok && h->greedy_multi == 1 && crowded;
-    const bool multi = !use_mma && h->fn_multi && h->greedy_multi >= 1 && crowded;
-    const int groups = use_mma ? ceil_div(n_utts, kMmaUtts) : (multi ? ceil_div(n_utts, kGreedyMulti) : n_utts);
-    // the grid holds as many clusters as are co-resident at this kernel's shared-memory footprint (the occupancy
-    // query of create time), each working through groups cluster, cluster + n_clusters, ...
-    const int max_clusters = use_mma ? h->resident_mma : (multi ? h->resident_multi : h->resident);
-    const int n_clusters = groups < max_clusters ? groups : max_clusters;
-    if (multi) a.smem_mask = h->smem_mask_multi;
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(C * n_clusters);
-    lc.blockDim = dim3(512);
-    lc.dynamicSmemBytes = use_mma ? h->smem_bytes_mma : (multi ? h->smem_bytes_multi : h->smem_bytes);
-    lc.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = C; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    lc.attrs = at;
-    lc.numAttrs = 1;
-    PIMB200_CUDA_TRY(cudaLaunchKernelEx(&lc, use_mma ? h->fn_mma : (multi ? h->fn_multi : h->fn), a));
+    if (per == 0) return launch_greedy(h, h->E, (long)Tp * JH, JH, n_utts, Tp, tokens, n_tokens, logits, st);
+    for (int u = 0; u < n_utts; u += per) {
+        const int g = std::min(per, n_utts - u);
+        rc = launch_greedy(h, h->E + (size_t)u * Tp * JH, JH, (long)g * JH, g, Tp, tokens + (size_t)u * Tp, n_tokens + u,
+                           logits ? logits + (size_t)u * Tp * c.vocab : nullptr, st);
+        if (rc != PIMB200_OK) return rc;
+    }
     return PIMB200_OK;
 }

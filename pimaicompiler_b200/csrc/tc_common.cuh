@@ -106,5 +106,117 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// The producer's and the issuer's loops run with all 32 lanes, and only the instructions themselves are predicated on one
+// elected lane (`el`).  Inside an `if (lane == 0)` the compiler keeps addresses and descriptors in per-thread registers and
+// moves each to the uniform ones that these instructions take: the issuer then needed 600 cycles per K block and the
+// producer 510, more than the MMAs and the loads themselves.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void expect_tx_if(uint32_t el, uint32_t bar, uint32_t bytes) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar),
+                 "r"(bytes), "r"(el)
+                 : "memory");
+}
+// the address of a barrier in the CTA of a given rank of the pair
+__device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+// cta_group::2 forms: loads that count their bytes at the pair leader's barrier, the MMA over both CTAs' operands, and a
+// commit that arrives in both
+template <int CG>
+__device__ __forceinline__ void load_2d(uint32_t el, uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+    if (CG == 1)
+        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}" ::"r"(dst),
+                     "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(el)
+                     : "memory");
+    else
+        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}" ::"r"(dst),
+                     "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(el)
+                     : "memory");
+}
+template <int CG>
+__device__ __forceinline__ void load_3d(uint32_t el, uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
+    if (CG == 1)
+        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}" ::"r"(dst),
+                     "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(el)
+                     : "memory");
+    else
+        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t@q cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}" ::"r"(dst),
+                     "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(el)
+                     : "memory");
+}
+template <int CG>
+__device__ __forceinline__ void mma(uint32_t el, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    if (CG == 1)
+        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+                     "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+                     "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(el)
+                     : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+                     "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+                     "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(el)
+                     : "memory");
+}
+template <int CG>
+__device__ __forceinline__ void commit(uint32_t el, uint32_t bar) {
+    if (CG == 1)
+        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
+                     "r"(el)
+                     : "memory");
+    else
+        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(bar),
+                     "h"((uint16_t)3), "r"(el)
+                     : "memory");
+}
+template <int CG>
+__device__ __forceinline__ void pair_sync() {
+    if (CG == 1) __syncthreads();
+    else {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+}
+
+// A in tensor memory (fp16, two halves per column)
+template <int CG>
+__device__ __forceinline__ void mma_ta(uint32_t el, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    if (CG == 1)
+        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+                     "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+                     "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(el)
+                     : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+                     "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+                     "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(el)
+                     : "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
+        "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]),
+        "r"(r[31])
+        : "memory");
+}
+// 16 lanes x 8 columns: r[0], r[1] lane (lane base + thread / 4), columns 2 (thread % 4) and the next; r[2], r[3] eight lanes on
+__device__ __forceinline__ void tmem_ld_16x256(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ uint32_t tile_offset(int row, int chunk) {   // byte offset inside a [rows x 64 halves] tile, 128-byte swizzle
+    return (uint32_t)((row >> 3) * 1024 + (row & 7) * 128 + ((chunk ^ (row & 7)) << 4));
+}
+// gate rows as the M operand: TMEM lane 32 q + 8 g + u is gate g of unit 8 q + u of the CTA, so that tmem_ld_16x256 of both lane
+// halves gives one thread all gates of its cells.  The packed row (4 * unit + gate) in M row `row`
+__device__ __forceinline__ int packed_row(int row) { return ((row >> 5) * 8 + (row & 7)) * 4 + (row >> 3 & 3); }
+
 }  // namespace tc
 }  // namespace pimb200

@@ -194,7 +194,7 @@ def test_lstm_outputs_alias_slices_of_caller_buffers():
     assert (cat_buf[..., 1024:] == 5).all() and (state_buf[:2] == 5).all() and (state_buf[4:] == 5).all()
 
 
-@pytest.mark.parametrize("B,L", [(1, 1), (4, 1), (40, 1), (2, 2)])
+@pytest.mark.parametrize("B,L", [(1, 1), (4, 1), (40, 1), (2, 2), (150, 1)])
 def test_persistent_bounded_wait_reports_timeout_and_context_survives(B, L):
     # Fault handling without faulting anything: shrink the bounded wait to a single poll, so the hidden-state exchange
     # cannot complete in time; the kernel must give up, record ERR_TIMEOUT and return, and the next call (normal
@@ -231,7 +231,7 @@ def test_persistent_bounded_wait_reports_timeout_and_context_survives(B, L):
 
 
 @pytest.mark.parametrize("B,L,H", [(1, 1, 1024), (8, 1, 320), (16, 1, 1024), (1, 2, 1024), (8, 2, 256), (20, 1, 1024), (64, 1, 320),
-                                   (70, 1, 256), (128, 1, 1024)])
+                                   (70, 1, 256), (128, 1, 1024), (300, 1, 1024), (200, 1, 320)])
 def test_waits_that_run_out_in_different_steps(B, L, H):
     # limits of a few polls, which some warps of a CTA reach a step or two before others: every launch returns, a launch that
     # lost a wait says so, one that did not is right, and so is the next one with the normal limit
@@ -518,6 +518,32 @@ def test_lstm_layer_wavefront_matches_oracle_and_sequential_layers(T, B, I, H, L
         ref = co.lstm(x.numpy(), [p.numpy() for p in ps], L, False, True, h0.numpy(), c0.numpy(), bf)
         for name, a, b in zip(("y", "hn", "cn"), (y, hn, cn), ref):
             assert_close(a, b, LSTM_ATOL, LSTM_RTOL, f"wavefront {name}")
+
+
+def _libtorch(ps, x, h0, c0, L, bi, bf):
+    state = tuple(torch.zeros(L * (2 if bi else 1), x.shape[0 if bf else 1], ps[1].shape[1]) if s is None else s for s in (h0, c0))
+    return torch.lstm(x, state, ps, True, L, 0.0, False, bi, bf)
+
+
+# (T, B, I, H, L, bidirectional, batch_first, state): sub-batches of every width of the tensor-core recurrence (16 columns a step
+# at H = 1024: four groups of two), one sub-batch per group, several parts, several chunks of steps, a ragged last group
+@pytest.mark.parametrize("T,B,I,H,L,bi,bf,state", [
+    (8, 129, 24, 1024, 1, False, False, True), (9, 257, 8, 1024, 1, False, False, False), (8, 512, 8, 1024, 1, False, True, True),
+    (8, 520, 8, 1024, 1, False, False, True), (8, 700, 8, 1024, 1, False, False, True), (10, 897, 8, 1024, 1, False, False, True),
+    (8, 1025, 16, 1024, 1, False, False, True), (11, 150, 20, 320, 3, False, True, True), (12, 200, 64, 512, 2, True, True, True),
+    (9, 260, 64, 960, 1, True, False, True), (8, 130, 7, 64, 2, True, False, False), (130, 1024, 8, 64, 1, False, False, True),
+    (70, 1030, 8, 64, 1, True, True, True)])
+def test_many_sequences_on_the_tensor_core_recurrence_vs_libtorch(T, B, I, H, L, bi, bf, state):
+    ops = _ops()
+    g = torch.Generator().manual_seed(T * B + H)
+    ps = lstm_params(L, 2 if bi else 1, I, H, g)
+    x = h16(torch.randn(*((B, T, I) if bf else (T, B, I)), generator=g))
+    LD = L * (2 if bi else 1)
+    h0, c0 = (h16(torch.randn(LD, B, H, generator=g) * 0.5) for _ in range(2)) if state else (None, None)
+    y, hn, cn = _run(ops, ps, x, h0, c0, L, bi, True, bf, ops.LSTM_AUTO)
+    ref = _libtorch(ps, x, h0, c0, L, bi, bf)
+    for got, want, name in zip((y, hn, cn), ref, ("y", "hn", "cn")):
+        assert_close(got, want.numpy(), LSTM_ATOL, LSTM_RTOL, name)
 
 
 def test_outputs_given_in_any_sequence_and_batch_sizes_of_any_array():

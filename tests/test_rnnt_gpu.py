@@ -183,6 +183,23 @@ def test_rnnt_ragged_group_sizes_and_odd_frame_count():
             _check_utterance(cfg, w, feats[i], toks[i], logits[i].cpu().numpy(), co.rnnt_greedy)
 
 
+@pytest.mark.parametrize("n_utts,blank_bias", [(85, 1.0), (225, 3.0), (700, 2.0), (1030, 1.0)])
+def test_rnnt_many_utterances_in_lock_step(n_utts, blank_bias):
+    # the encoder's tensor-core recurrence (from 129 utterances), at 1030 in two parts; a few utterances of each call against the oracle
+    cfg = to.RnntConfig()
+    w = to.make_rnnt_weights(cfg, seed=5, gain=2.0, logit_gain=8.0)
+    w.b2[cfg.blank] += blank_bias              # the utterances emit in different frames
+    w.b2 = w.b2.to(torch.float16).to(torch.float32)
+    dec = _decoder(cfg, w)
+    g = torch.Generator().manual_seed(n_utts)
+    feats = torch.randn(n_utts, 33, cfg.feat_dim, generator=g).to(torch.float16)
+    toks, logits = dec.decode(feats.cuda(), want_logits=True)
+    for i in sorted({0, 17, n_utts // 2, n_utts - 1}):
+        _check_utterance(cfg, w, feats[i].float(), toks[i], logits[i].cpu().numpy(), to.rnnt_greedy)
+    again, logits2 = dec.decode(feats.cuda(), want_logits=True)
+    assert again == toks and torch.equal(logits2, logits)
+
+
 def test_rnnt_benchmark_scale_is_independent_of_batching():
     # The benchmark's configuration at full length (1000 frames): 72 utterances in one call (one encoder group of two
     # batch halves, nine greedy groups over two rounds of clusters) against the first 40 of them in a call of their own
