@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "rnnt_batch.cuh"
 #include "pimb200_rnnt.h"
 
 namespace cg = cooperative_groups;
@@ -1284,6 +1285,7 @@ static GreedyFn pick_greedy_multi(int gate_rows, int joint_rows, int vocab) {
 // ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
+constexpr int kGreedyBatchMin = 81;    // utterances from which rnnt_batch.cu takes the greedy loop
 constexpr int kEncoderBatch = 128;   // utterances in lock step below the sizes of lstm_batch.cu
 
 struct pimb200_rnnt {
@@ -1300,6 +1302,10 @@ struct pimb200_rnnt {
     __half *y_pre = nullptr, *y_post = nullptr;
     float* E = nullptr;
     size_t cap_frames = 0;  // frames*utts capacity of the three buffers above
+    // many utterances (rnnt_batch.cu): how many a launch takes, and what its CTAs exchange their values through
+    int batch_capacity = 0;
+    unsigned char* batch_work = nullptr;
+    size_t batch_partials = 0, batch_counters = 0;   // offsets
     long long* trace = nullptr;  // diagnostics buffer (not owned)
     GreedyFn fn = nullptr;
     bool mma_ok = false;           // tensor-core variant (kMmaUtts utterances per cluster) available
@@ -1349,7 +1355,7 @@ extern "C" int pimb200_rnnt_destroy(pimb200_rnnt* h) {
     pimb200_lstm_destroy(h->pre);
     pimb200_lstm_destroy(h->post);
     void* ptrs[] = {h->W1e, h->W1p, h->W2, h->b1, h->b2, h->Whh0, h->Wih1, h->Whh1, h->P0, h->bias1,
-                    h->y_pre, h->y_post, h->E, h->d_status, h->W1pf};
+                    h->y_pre, h->y_post, h->E, h->d_status, h->W1pf, h->batch_work};
     for (void* p : ptrs) cudaFree(p);
     delete h;
     return PIMB200_OK;
@@ -1500,6 +1506,13 @@ extern "C" int pimb200_rnnt_create(const pimb200_rnnt_config* cfg, const pimb200
         }
     }
     if (h->cluster == 0) return fail(PIMB200_ERR_UNSUPPORTED);
+    if ((h->batch_capacity = greedy_batch_capacity(PH, JH, V)) > 0) {
+        size_t state, partials, counters;
+        greedy_batch_workspace(PH, V, &state, &partials, &counters);
+        h->batch_partials = state;
+        h->batch_counters = state + partials;
+        if (cudaMalloc(&h->batch_work, state + partials + counters) != cudaSuccess) return fail(PIMB200_ERR_NO_MEMORY);
+    }
     *out = h;
     return PIMB200_OK;
 }
@@ -1601,6 +1614,24 @@ static int launch_greedy(pimb200_rnnt* h, const float* E, long e_utt, long e_fra
                          int32_t* n_tokens, float* logits, cudaStream_t st) {
     const pimb200_rnnt_config& c = h->cfg;
     auto next_gen = [h] { return h->gen = h->gen == 0x7fffffff ? 1 : h->gen + 1; };
+    if (h->greedy_multi == 1 && h->batch_capacity > 0 && n_utts >= kGreedyBatchMin) {
+        const int per = ceil_div(n_utts, ceil_div(n_utts, h->batch_capacity));
+        for (int u = 0; u < n_utts; u += per) {
+            GreedyBatchArgs b = {};
+            b.E = E + (size_t)u * e_utt; b.e_utt = e_utt; b.e_frame = e_frame;
+            b.tokens = tokens + (size_t)u * Tp; b.n_tokens = n_tokens + u; b.logits = logits ? logits + (size_t)u * Tp * c.vocab : nullptr;
+            b.n_utts = std::min(per, n_utts - u); b.Tp = Tp;
+            b.P0 = h->P0; b.Whh0 = h->Whh0; b.Wih1 = h->Wih1; b.Whh1 = h->Whh1; b.bias1 = h->bias1; b.W1p = h->W1p; b.W2 = h->W2; b.b2 = h->b2;
+            b.PH = c.pred_hidden; b.JH = c.joint_hidden; b.V = c.vocab; b.blank = c.blank;
+            b.state = reinterpret_cast<__half*>(h->batch_work);
+            b.partials = reinterpret_cast<float*>(h->batch_work + h->batch_partials);
+            b.counters = reinterpret_cast<uint32_t*>(h->batch_work + h->batch_counters);
+            b.trace = h->trace; b.status = h->d_status; b.gen = next_gen(); b.poll_limit = h->poll_limit;
+            const int rc = launch_greedy_batch(b, st);
+            if (rc != PIMB200_OK) return rc;
+        }
+        return PIMB200_OK;
+    }
     GreedyArgs a;
     a.E = E; a.e_utt = e_utt; a.e_frame = e_frame; a.tokens = tokens; a.n_tokens = n_tokens; a.logits = logits; a.n_utts = n_utts; a.Tp = Tp;
     a.P0 = h->P0; a.Whh0 = h->Whh0; a.Wih1 = h->Wih1; a.Whh1 = h->Whh1; a.bias1 = h->bias1;

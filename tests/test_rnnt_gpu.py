@@ -185,7 +185,8 @@ def test_rnnt_ragged_group_sizes_and_odd_frame_count():
 
 @pytest.mark.parametrize("n_utts,blank_bias", [(85, 1.0), (225, 3.0), (700, 2.0), (1030, 1.0)])
 def test_rnnt_many_utterances_in_lock_step(n_utts, blank_bias):
-    # the encoder's tensor-core recurrence (from 129 utterances), at 1030 in two parts; a few utterances of each call against the oracle
+    # the encoder's tensor-core recurrence (from 129 utterances) and the greedy loop of many utterances, one to five tiles of 16
+    # per group, a ragged last group and, at 1030, two parts; a few utterances of each call against the oracle
     cfg = to.RnntConfig()
     w = to.make_rnnt_weights(cfg, seed=5, gain=2.0, logit_gain=8.0)
     w.b2[cfg.blank] += blank_bias              # the utterances emit in different frames
@@ -198,6 +199,27 @@ def test_rnnt_many_utterances_in_lock_step(n_utts, blank_bias):
         _check_utterance(cfg, w, feats[i].float(), toks[i], logits[i].cpu().numpy(), to.rnnt_greedy)
     again, logits2 = dec.decode(feats.cuda(), want_logits=True)
     assert again == toks and torch.equal(logits2, logits)
+
+
+def test_rnnt_many_utterances_time_out_and_recover():
+    from pimaicompiler_b200 import _lib
+    cfg = to.RnntConfig(feat_dim=24, enc_hidden=64, pred_hidden=64, joint_hidden=128, vocab=11, blank=10)
+    w = to.make_rnnt_weights(cfg, seed=11, gain=2.0, logit_gain=6.0)
+    dec = _decoder(cfg, w)
+    feats = torch.stack([to.make_features(40, cfg, 900 + i) for i in range(140)]).to(torch.float16)
+    toks, logits = dec.decode(feats.cuda(), want_logits=True)
+    for i in (0, 70, 139):
+        _check_utterance(cfg, w, feats[i].float(), toks[i], logits[i].cpu().numpy(), co.rnnt_greedy)
+    for limit in (1, 2, 3, 5):
+        dec.set_poll_limit(limit)
+        try:
+            got = dec.decode(feats.cuda())
+            assert limit > 1 and got == toks
+        except _lib.Pimb200Error as e:
+            assert e.status == _lib.ERR_TIMEOUT
+        dec.set_poll_limit(1 << 21)
+        again, logits2 = dec.decode(feats.cuda(), want_logits=True)
+        assert again == toks and torch.equal(logits2, logits)
 
 
 def test_rnnt_benchmark_scale_is_independent_of_batching():
