@@ -3,8 +3,8 @@
 //     Z[4H, b] = W_hh[4H, H] h[H, b]        c, h <- gates(G + bias + Z)        one persistent launch for all steps
 //
 // Weights stay on the chip for the whole launch.  A CTA pair (cta_group::2) owns 64 hidden units, each CTA the 128 gate rows of
-// 32 of them as the M operand: 256 KB at H = 1024, one half in tensor memory (an A operand may lie there), the other in shared
-// memory.  H / 64 pairs hold the matrix, 16 at H = 1024, so 64 pairs make four groups that each walk their own sequences, up to
+// 32 of them as the M operand: 256 KB at H = 1024, half of them or more in tensor memory (an A operand may lie there), the others in
+// shared memory.  H / 64 pairs hold the matrix, 16 at H = 1024, so 64 pairs make four groups that each walk their own sequences, up to
 // 256, as two sub-batches: the products of one run under the gates and the exchange of the other.
 //
 // Hidden states are the N operand: a sub-batch's rows are fetched by TMA straight from the output tensor, each CTA of a pair
@@ -27,12 +27,8 @@ namespace pimb200 {
 namespace tc {
 namespace {
 
-constexpr int kThreads = 352;          // TMA, MMA, TMEM owner, eight gate warps
-constexpr int kFirstEpi = 3;
-constexpr int kEpiWarps = 8;
+constexpr int kFirstEpi = 3;            // warps: TMA, MMA, TMEM owner, then 8 or 16 for the gates
 constexpr int kUnits = 32;             // hidden units per CTA
-constexpr int kTmemBlocks = 8;         // K blocks of 64 whose weights lie in tensor memory
-constexpr int kACol = 256;             // their first TMEM column; accumulator of sub-batch b at column 128 b
 constexpr int kMaxBlocks = 16;         // H <= 1024
 constexpr int kBlockBytes = 128 * 128; // a K block of a CTA's weights
 constexpr int kRingBytes = 96 * 1024;
@@ -46,8 +42,12 @@ __host__ __device__ constexpr int blocks_per_stage(int nj) { return nj > 4 ? 2 :
 __host__ __device__ constexpr int stages_of(int nj) {
     return kRingBytes / (blocks_per_stage(nj) * nj * 1024) < kMaxStages ? kRingBytes / (blocks_per_stage(nj) * nj * 1024) : kMaxStages;
 }
-size_t smem_of(int H) {
-    const int blocks = H / 64, own = blocks > kTmemBlocks ? blocks - kTmemBlocks : 0;
+// TMEM: the accumulator of sub-batch b at column b * acc_cols, behind them as many K blocks of weights (32 columns each) as fit.
+// An MMA of few columns is bound by its A operand: 74 cycles from shared memory, 37 from tensor memory, at up to 64 columns.
+__host__ __device__ constexpr int acc_cols(int nj) { return (16 * nj + 31) / 32 * 32; }
+__host__ __device__ constexpr int tmem_blocks(int nj, int subs) { return (512 - subs * acc_cols(nj)) / 32; }
+size_t smem_of(int H, int nj, int subs) {
+    const int blocks = H / 64, t = tmem_blocks(nj, subs), own = blocks > t ? blocks - t : 0;
     return (size_t)own * kBlockBytes + kRingBytes + 1024 /*align*/ + 512 /*barriers*/;
 }
 
@@ -56,13 +56,21 @@ __device__ __forceinline__ float4 ldg_stream_f4(const float* p) {
     return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
 }
 
+// Gate warps: sixteen from 96 columns on (1024 sequences: a phase of 5.4 thousand cycles with eight), where a thread's share of
+// the cells still fits its registers.
+__host__ __device__ constexpr int gate_warps(int nj) { return nj >= 6 ? 16 : 8; }
+__host__ __device__ constexpr int threads_of(int nj) { return (kFirstEpi + gate_warps(nj)) * 32; }
+
 // NJ: eighths of the sequences of a CTA's half of a sub-batch (a sub-batch is 16 NJ columns); SUBS: sub-batches per group
 template <int NJ, int SUBS>
-__global__ void __launch_bounds__(kThreads, 1) lstm_batch_kernel(const __grid_constant__ BatchMaps maps, const __grid_constant__ BatchArgs a) {
+__global__ void __launch_bounds__(threads_of(NJ), 1) lstm_batch_kernel(const __grid_constant__ BatchMaps maps, const __grid_constant__ BatchArgs a) {
     constexpr int KPS = blocks_per_stage(NJ), BLOCK = NJ * 1024, STAGE = KPS * BLOCK, STAGES = stages_of(NJ);
-    constexpr int COLS = 16 * NJ;
+    constexpr int COLS = 16 * NJ, kThreads = threads_of(NJ), kEpiWarps = gate_warps(NJ);
+    constexpr int PARTS = kEpiWarps / 4, OCT = 2 * NJ / PARTS;         // column parts of the gate warps, octets of columns per part
+    static_assert(2 * NJ % PARTS == 0, "whole octets per warp");
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    constexpr int kTmemBlocks = tmem_blocks(NJ, SUBS), kACol = SUBS * acc_cols(NJ);
     const int blocks = a.H >> 6, tblocks = blocks < kTmemBlocks ? blocks : kTmemBlocks;
     unsigned char* ring = smem + (size_t)(blocks - tblocks) * kBlockBytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(ring + kRingBytes);
@@ -86,7 +94,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_batch_kernel(const __grid_co
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(accf0 + 8 * s, 1);
-            mbar_init(acce0 + 8 * s, 2 * kEpiWarps);
+            mbar_init(acce0 + 8 * s, 2 * (kEpiWarps + (s == 0 ? 1 : 0)));
         }
         mbar_init(done0, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -188,7 +196,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_batch_kernel(const __grid_co
 #pragma unroll 1
                 for (int b = 0; b < SUBS && !failed; ++b) {
                     if (!mbar_wait(acce0 + 8 * b, (uses & 1) ^ 1, abort_flag, a.gen)) { failed = true; break; }
-                    const uint32_t acc = tmem_base + 128 * b;
+                    const uint32_t acc = tmem_base + acc_cols(NJ) * b;
                     for (int k0 = 0; k0 < blocks; k0 += KPS) {
                         if (!mbar_wait(full0 + 8 * st, par, abort_flag, a.gen)) { failed = true; break; }
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -224,14 +232,33 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_batch_kernel(const __grid_co
         if (!mbar_wait(done0, 0, abort_flag, a.gen))
             for (uint32_t i = 0; i < (1u << 20); ++i)
                 if (mbar_try_wait(done0, 0)) break;
+    } else if (warp == 2) {
+        // ---------------- input terms of this CTA's units into L2, two steps ahead: 64 KB per sub-batch and CTA, wanted by all CTAs
+        //                  at once, take longer from HBM than the phase they are asked for in ----------------
+        const long g_step = dir.reverse ? -a.g_tstride : a.g_tstride;
+        const float* g = dir.G + (dir.reverse ? (long)(a.steps - 1) * a.g_tstride : 0) + 4 * u0 + (lane & 3) * 32;   // four lines per sequence
+        const int n = min(SUBS * COLS, a.B - seq0);
+        uint32_t par = 0;
+        for (int s = 0; s < a.steps; ++s) {
+            for (int ahead = s == 0 ? 1 : 2; ahead <= 2; ++ahead)
+                if (s + ahead < a.steps)
+                    for (int i = lane >> 2; i < n; i += 8)
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(g + ahead * g_step + (long)(seq0 + i) * a.g_bstride));
+            g += g_step;
+            if (s == 0 && !h_first) continue;
+            if (__any_sync(0xffffffffu, !mbar_wait(accf0, par, abort_flag, a.gen))) break;
+            par ^= 1;
+            // (never two steps behind: the next products wait for this)
+            if (lane == 0) asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapa(acce0, 0)) : "memory");
+        }
     } else if (warp >= kFirstEpi) {
-        // ---------------- gates: TMEM lane quarter = warp % 4, every second half of the columns ----------------
-        const int q = warp & 3, hf = (warp - kFirstEpi) >> 2;
+        // ---------------- gates: TMEM lane quarter = warp % 4, a part of the columns ----------------
+        const int q = warp & 3, part = (warp - kFirstEpi) >> 2;
         const int r = lane >> 2, cq = lane & 3;
         const int unit = u0 + 8 * q + r;
-        const int col = hf * (COLS / 2) + 2 * cq;                      // this thread's first column; the others 8 j + {0, 1} on
+        const int col = part * (COLS / PARTS) + 2 * cq;                      // this thread's first column; the others 8 j + {0, 1} on
         const float4 bias = __ldg(reinterpret_cast<const float4*>(dir.bias) + unit);
-        float c[SUBS][NJ][2];
+        float c[SUBS][OCT][2];
         const float* gp[SUBS];
         int left[SUBS];                                                // sequences from the thread's first column to the end
         const int t_low = dir.reverse ? a.steps - 1 : 0;
@@ -242,7 +269,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_batch_kernel(const __grid_co
             left[b] = a.B - seq;
             gp[b] = dir.G + (long)t_low * a.g_tstride + (long)seq * a.g_bstride + 4 * unit;
 #pragma unroll
-            for (int j = 0; j < NJ; ++j)
+            for (int j = 0; j < OCT; ++j)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     c[b][j][e] = 0.f;
@@ -254,9 +281,9 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_batch_kernel(const __grid_co
                 }
         }
         // input terms of the coming phase (a sub-batch's step), asked for behind the phase before
-        float4 g[NJ][2];
+        float4 g[OCT][2];
 #pragma unroll
-        for (int j = 0; j < NJ; ++j)
+        for (int j = 0; j < OCT; ++j)
 #pragma unroll
             for (int e = 0; e < 2; ++e)
                 g[j][e] = 8 * j + e < left[0] ? ldg_stream_f4(gp[0] + (long)(8 * j + e) * a.g_bstride) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -278,23 +305,23 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_batch_kernel(const __grid_co
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
                 if (a.trace && lane == 0 && warp == kFirstEpi) a.trace[((size_t)blockIdx.x * a.steps + s) * 8 + 2 + 2 * b] = clock64();
-                const uint32_t acc = tmem_base + ((uint32_t)(32 * q) << 16) + 128 * b + hf * (COLS / 2);
+                const uint32_t acc = tmem_base + ((uint32_t)(32 * q) << 16) + acc_cols(NJ) * b + part * (COLS / PARTS);
                 const int nb = b + 1 < SUBS ? b + 1 : 0;
                 const float* const gn = b + 1 < SUBS ? gp[nb] : gp[0] + g_step;
                 const int n_left = b + 1 < SUBS || !last ? left[nb] : 0;
-                uint32_t hv[NJ];
+                uint32_t hv[OCT];
                 // four column octets at a time: their cells' chains run side by side
 #pragma unroll
-                for (int j0 = 0; j0 < NJ; j0 += 4) {
+                for (int j0 = 0; j0 < OCT; j0 += 4) {
                     uint32_t v[4][8];
                     if (has) {
 #pragma unroll
-                        for (int j = j0; j < NJ && j < j0 + 4; ++j) {
+                        for (int j = j0; j < OCT && j < j0 + 4; ++j) {
                             tmem_ld_16x256(acc + 8 * j, v[j - j0]);
                             tmem_ld_16x256(acc + (16u << 16) + 8 * j, v[j - j0] + 4);
                         }
                         tmem_wait_ld();
-                        if (j0 + 4 >= NJ) {        // the accumulator may be written again
+                        if (j0 + 4 >= OCT) {        // the accumulator may be written again
                             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                             __syncwarp();
                             if (lane == 0) asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapa(acce0 + 8 * b, 0)) : "memory");
@@ -304,7 +331,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_batch_kernel(const __grid_co
                         for (int i = 0; i < 32; ++i) v[i >> 3][i & 7] = 0u;
                     }
 #pragma unroll
-                    for (int j = j0; j < NJ && j < j0 + 4; ++j) {
+                    for (int j = j0; j < OCT && j < j0 + 4; ++j) {
                         float hj[2];
 #pragma unroll
                         for (int e = 0; e < 2; ++e) {
@@ -320,35 +347,35 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_batch_kernel(const __grid_co
                 }
                 // eight lanes hold the eight units of an octet for the same two sequences per j: pairs of lanes swap, so that
                 // each has two units of one sequence, then four units, then all eight of one sequence per four j
-                uint32_t w[NJ];
+                uint32_t w[OCT];
 #pragma unroll
-                for (int j = 0; j < NJ; ++j) {
+                for (int j = 0; j < OCT; ++j) {
                     const uint32_t o = __shfl_xor_sync(0xffffffffu, hv[j], 4);
                     w[j] = b0 ? __byte_perm(o, hv[j], 0x7632) : __byte_perm(hv[j], o, 0x5410);
                 }
                 const int seq = seq0 + b * COLS + col + b0;
                 auto put = [&](__half* base, long pitch) {
-                    if constexpr (NJ % 2 != 0) {
+                    if constexpr (OCT % 2 != 0) {
 #pragma unroll
-                        for (int j = 0; j < NJ; ++j)
+                        for (int j = 0; j < OCT; ++j)
                             if (seq + 8 * j < a.B)
                                 *reinterpret_cast<uint32_t*>(base + (long)(seq + 8 * j) * pitch + u0 + 8 * q + 2 * (r >> 1)) = w[j];
                     } else {
-                        uint2 x[NJ / 2 > 0 ? NJ / 2 : 1];
+                        uint2 x[OCT / 2 > 0 ? OCT / 2 : 1];
 #pragma unroll
-                        for (int m = 0; m < NJ / 2; ++m) {
+                        for (int m = 0; m < OCT / 2; ++m) {
                             const uint32_t o = __shfl_xor_sync(0xffffffffu, b1 ? w[2 * m] : w[2 * m + 1], 8);
                             x[m] = b1 ? make_uint2(o, w[2 * m + 1]) : make_uint2(w[2 * m], o);
                         }
-                        if constexpr (NJ % 4 != 0) {
+                        if constexpr (OCT % 4 != 0) {
 #pragma unroll
-                            for (int m = 0; m < NJ / 2; ++m) {
+                            for (int m = 0; m < OCT / 2; ++m) {
                                 const int n = seq + 8 * (2 * m + b1);
                                 if (n < a.B) *reinterpret_cast<uint2*>(base + (long)n * pitch + u0 + 8 * q + 4 * b2) = x[m];
                             }
                         } else {
 #pragma unroll
-                            for (int m = 0; m < NJ / 4; ++m) {
+                            for (int m = 0; m < OCT / 4; ++m) {
                                 const uint2 keep = b2 ? x[2 * m + 1] : x[2 * m], give = b2 ? x[2 * m] : x[2 * m + 1];
                                 const uint32_t ox = __shfl_xor_sync(0xffffffffu, give.x, 16), oy = __shfl_xor_sync(0xffffffffu, give.y, 16);
                                 const int n = seq + 8 * (4 * m + 2 * b2 + b1);
@@ -369,7 +396,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_batch_kernel(const __grid_co
                 } else {
                     if (a.begin + a.steps == a.T && dir.hn) put(dir.hn, a.H);
 #pragma unroll
-                    for (int j = 0; j < NJ; ++j)
+                    for (int j = 0; j < OCT; ++j)
 #pragma unroll
                         for (int e = 0; e < 2; ++e) {
                             if (8 * j + e >= left[b]) continue;
@@ -382,7 +409,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_batch_kernel(const __grid_co
                 // the next phase's input terms: behind the fence, which would wait for them (they come from HBM)
                 const float* gq = gn;          // (a running address: the products of all cells would be kept in registers)
 #pragma unroll
-                for (int j = 0; j < NJ; ++j, gq += 8 * a.g_bstride) {
+                for (int j = 0; j < OCT; ++j, gq += 8 * a.g_bstride) {
                     if (8 * j < n_left) g[j][0] = ldg_stream_f4(gq);
                     if (8 * j + 1 < n_left) g[j][1] = ldg_stream_f4(gq + a.g_bstride);
                 }
@@ -411,16 +438,15 @@ BatchFn pick_nj(int nj) {
         case 4: return lstm_batch_kernel<4, SUBS>;
         case 5: return lstm_batch_kernel<5, SUBS>;
         case 6: return lstm_batch_kernel<6, SUBS>;
-        case 7: return lstm_batch_kernel<7, SUBS>;
         default: return lstm_batch_kernel<8, SUBS>;
     }
 }
 
-void launch_config(cudaLaunchConfig_t& lc, cudaLaunchAttribute* at, int H, int ctas, cudaStream_t st) {
+void launch_config(cudaLaunchConfig_t& lc, cudaLaunchAttribute* at, int H, int nj, int subs, int ctas, cudaStream_t st) {
     lc = {};
     lc.gridDim = dim3(ctas);
-    lc.blockDim = dim3(kThreads);
-    lc.dynamicSmemBytes = smem_of(H);
+    lc.blockDim = dim3(threads_of(nj));
+    lc.dynamicSmemBytes = smem_of(H, nj, subs);
     lc.stream = st;
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
@@ -438,10 +464,10 @@ int resident_pairs(int dev) {
     if (pairs[dev] == 0) {
         cudaLaunchConfig_t lc;
         cudaLaunchAttribute at[2];
-        launch_config(lc, at, 1024, 2, nullptr);
+        launch_config(lc, at, 1024, 8, 2, 2, nullptr);
         lc.numAttrs = 1;
         int n = 0;
-        if (cudaFuncSetAttribute(lstm_batch_kernel<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(1024)) != cudaSuccess ||
+        if (cudaFuncSetAttribute(lstm_batch_kernel<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(1024, 8, 2)) != cudaSuccess ||
             cudaOccupancyMaxActiveClusters(&n, lstm_batch_kernel<8, 2>, &lc) != cudaSuccess) {
             cudaGetLastError();
             n = 0;
@@ -479,7 +505,8 @@ int launch_lstm_batch(BatchArgs& a, cudaStream_t st) {
     // as many groups as there are, and two sub-batches where a group has more than the 32 columns that cost as much as 16
     groups = std::min(groups, ceil_div(a.B, 16));
     const int subs = ceil_div(a.B, groups) > 32 ? 2 : 1;
-    const int nj = ceil_div(ceil_div(a.B, groups * subs), 16);
+    int nj = ceil_div(ceil_div(a.B, groups * subs), 16);
+    if (nj == 7) nj = 8;                   // (sixteen gate warps share an even number of octets)
     groups = ceil_div(a.B, subs * nj * 16);
     BatchMaps m = {};
     for (int d = 0; d < a.dirs; ++d) {
@@ -490,11 +517,11 @@ int launch_lstm_batch(BatchArgs& a, cudaStream_t st) {
     }
     const BatchFn fn = subs == 2 ? pick_nj<2>(nj) : pick_nj<1>(nj);
     const int blocks = a.H / 64;
-    PIMB200_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(a.H)));
+    PIMB200_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(a.H, nj, subs)));
     PIMB200_CUDA_TRY(cudaMemsetAsync(a.counters, 0, (size_t)groups * a.dirs * subs * blocks * kBatchFlagWords * 4, st));
     cudaLaunchConfig_t lc;
     cudaLaunchAttribute at[2];
-    launch_config(lc, at, a.H, 2 * groups * a.dirs * blocks, st);
+    launch_config(lc, at, a.H, nj, subs, 2 * groups * a.dirs * blocks, st);
     return cuda_status(cudaLaunchKernelEx(&lc, fn, m, a));
 }
 
