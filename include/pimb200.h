@@ -322,6 +322,10 @@ int pimb200_lstm_forward_step(pimb200_lstm* h, const void* x, long x_ld, int B, 
 int pimb200_lstm_forward_packed(pimb200_lstm* h, const void* data, const int64_t* batch_sizes, int T,
                                 const void* h0, const void* c0, void* y, void* hn, void* cn, void* stream);
 
+/* How many sequences of a packed batch this handle walks in lock step, in one launch per layer (0: none; larger batches run
+ * timestep by timestep). */
+int pimb200_lstm_packed_capacity(const pimb200_lstm* h);
+
 /* The last device-side status of a handle's asynchronous work: call after synchronising the
  * stream; returns PIMB200_ERR_TIMEOUT when a bounded wait inside the persistent kernel gave up (the outputs of that
  * call are then undefined); reading clears it.  A launch that gave up does not affect the launches after it. */

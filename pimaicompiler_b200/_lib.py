@@ -78,6 +78,7 @@ SIGNATURES = {
     "pimb200_lstm_forward": (_i, [_vp, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp]),
     "pimb200_lstm_forward_packed": (_i, [_vp, _vp, C.POINTER(C.c_int64), _i, _vp, _vp, _vp, _vp, _vp, _vp]),
     "pimb200_lstm_last_status": (_i, [_vp]),
+    "pimb200_lstm_packed_capacity": (_i, [_vp]),
     "pimb200_lstm_profile_enable": (_i, [_vp, _i]),
     "pimb200_lstm_profile_read": (_i, [_vp, C.POINTER(C.c_double), C.POINTER(C.c_long), C.POINTER(C.c_double)]),
     "pimb200_lstm_set_poll_limit": (_i, [_vp, _i]),

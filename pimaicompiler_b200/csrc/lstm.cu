@@ -2470,10 +2470,30 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
 //     0 and 1, the cell state stays frozen, so the kernel's c_n is the state after the sequence's own last step;
 //     h_n is the output row of that step, picked up when the outputs are stored.
 // ---------------------------------------------------------------------------------------------
+constexpr int kBatchMinB = 129;              // fewer sequences: the kernels above
+constexpr long kBatchChunkRows = 131072;     // rows of gate terms per chunk (2 GB at H = 1024)
+constexpr int kBatchMinBothB = 33;           // two directions, which lstm_batch.cu walks in one launch
+constexpr long kBatchMaxPackedRows = 4 * kBatchChunkRows;
 struct PackedMeta {
     const int* lens;       // [B] device
     const long* row0;      // [T] device: first packed row of timestep t
 };
+
+// `n` halves by the threads of a block, 16 bytes at a time where both ends allow it
+__device__ __forceinline__ void copy_row(__half* d, const __half* s, int n) {
+    if (((reinterpret_cast<uintptr_t>(d) | reinterpret_cast<uintptr_t>(s)) & 15) == 0 && n % 8 == 0) {
+        for (int c = threadIdx.x; c < n / 8; c += blockDim.x) reinterpret_cast<uint4*>(d)[c] = reinterpret_cast<const uint4*>(s)[c];
+        return;
+    }
+    for (int c = threadIdx.x; c < n; c += blockDim.x) d[c] = s[c];
+}
+__device__ __forceinline__ void zero_row(__half* d, int n) {
+    if ((reinterpret_cast<uintptr_t>(d) & 15) == 0 && n % 8 == 0) {
+        for (int c = threadIdx.x; c < n / 8; c += blockDim.x) reinterpret_cast<uint4*>(d)[c] = make_uint4(0u, 0u, 0u, 0u);
+        return;
+    }
+    for (int c = threadIdx.x; c < n; c += blockDim.x) d[c] = __float2half_rn(0.f);
+}
 
 // dst[t, b, :] (padded, row t*B+b, `w` halves) <- row (ts, b) of src, ts = reverse ? len_b-1-t : t; zeros for t >= len_b.
 // src is packed (row0[ts] + b) when src_packed, else padded (ts*B + b), rows src_ld halves apart.
@@ -2484,12 +2504,11 @@ __global__ void lstm_to_padded_kernel(const __half* __restrict__ src, long src_l
     const int len = m.lens[b];
     __half* d = dst + row * (long)w;
     if (t >= len) {
-        for (int c = threadIdx.x; c < w; c += blockDim.x) d[c] = __float2half_rn(0.f);
+        zero_row(d, w);
         return;
     }
     const int ts = reverse ? len - 1 - t : t;
-    const __half* sp = src + (src_packed ? (m.row0[ts] + b) : ((long)ts * B + b)) * src_ld;
-    for (int c = threadIdx.x; c < w; c += blockDim.x) d[c] = sp[c];
+    copy_row(d, src + (src_packed ? (m.row0[ts] + b) : ((long)ts * B + b)) * src_ld, w);
 }
 
 // Behind each sequence's end: input gate off, forget gate on, the other two terms zero (packed gate order i, f, g, o).
@@ -2510,25 +2529,25 @@ __global__ void lstm_from_padded_kernel(const __half* __restrict__ src, __half* 
     const int t = (int)(row / B), b = (int)(row % B);
     const int len = m.lens[b];
     if (t >= len) {
-        if (!dst_packed) {
-            __half* d = dst + ((long)t * B + b) * dst_ld + col;
-            for (int c = threadIdx.x; c < H; c += blockDim.x) d[c] = __float2half_rn(0.f);
-        }
+        if (!dst_packed) zero_row(dst + ((long)t * B + b) * dst_ld + col, H);
         return;
     }
     const int ts = reverse ? len - 1 - t : t;
     const __half* sp = src + row * (long)H;
-    __half* d = dst + (dst_packed ? (m.row0[ts] + b) : ((long)ts * B + b)) * dst_ld + col;
-    for (int c = threadIdx.x; c < H; c += blockDim.x) d[c] = sp[c];
-    if (hn && t == len - 1) {
-        __half* hp = hn + (long)b * H;
-        for (int c = threadIdx.x; c < H; c += blockDim.x) hp[c] = sp[c];
-    }
+    copy_row(dst + (dst_packed ? (m.row0[ts] + b) : ((long)ts * B + b)) * dst_ld + col, sp, H);
+    if (hn && t == len - 1) copy_row(hn + (long)b * H, sp, H);
 }
 
 static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool reverse, const float* G, long g_tstride,
                           long g_bstride, const __half* h0, const __half* c0, __half* y, long y_tstride,
                           long y_bstride, __half* hn, __half* cn, cudaStream_t st);
+
+// the recurrence of lstm_batch.cu for a packed batch: more sequences than the kernels above take, or two directions at once
+static bool batch_fits_packed(const pimb200_lstm* h, int T, int B) {
+    return B >= (h->D == 2 ? kBatchMinBothB : kBatchMinB) && T >= 8 && h->bulk_wide == 2 && !h->use_tc &&
+           (h->variant == PIMB200_LSTM_AUTO || h->variant == PIMB200_LSTM_PERSISTENT) && (long)T * B * h->D <= kBatchMaxPackedRows &&
+           lstm_batch_capacity(h->H, h->D) >= B;
+}
 
 static int lstm_forward_packed_lockstep(pimb200_lstm* h, const __half* data, const SeqLayout& sq, const __half* h0,
                                         const __half* c0, __half* y, __half* hn, __half* cn, cudaStream_t st) {
@@ -2548,8 +2567,10 @@ static int lstm_forward_packed_lockstep(pimb200_lstm* h, const __half* data, con
     int max_in = h->I;
     if (L > 1 && D * H > max_in) max_in = D * H;
     if ((rc = grow(&h->pk_x, &h->pk_x_cap, (size_t)prow * max_in)) != PIMB200_OK) return rc;
-    if ((rc = grow(&h->pk_run, &h->pk_run_cap, (size_t)prow * H)) != PIMB200_OK) return rc;
-    if ((rc = grow(&h->G, &h->G_cap, (size_t)prow * 4 * H)) != PIMB200_OK) return rc;
+    const bool batch = batch_fits_packed(h, T, B) && (!h0 || aligned16(h0));
+    const size_t runs = batch ? D : 1;         // directions that are under way at once
+    if ((rc = grow(&h->pk_run, &h->pk_run_cap, runs * prow * H)) != PIMB200_OK) return rc;
+    if ((rc = grow(&h->G, &h->G_cap, runs * prow * 4 * H)) != PIMB200_OK) return rc;
     if (L > 1 && (rc = grow(&h->ybuf[0], &h->y_cap[0], (size_t)prow * D * H)) != PIMB200_OK) return rc;
     if (L > 2 && (rc = grow(&h->ybuf[1], &h->y_cap[1], (size_t)prow * D * H)) != PIMB200_OK) return rc;
     SeqLayout padded;
@@ -2560,29 +2581,54 @@ static int lstm_forward_packed_lockstep(pimb200_lstm* h, const __half* data, con
         const bool first = (l == 0), last = (l == L - 1);
         const __half* Xin = first ? data : h->ybuf[(l - 1) & 1];      // packed rows (layer 0) or padded rows
         __half* Yout = last ? y : h->ybuf[l & 1];
+        BatchArgs ba = {};
         for (int d = 0; d < D; ++d) {
             const int ld = l * D + d;
             const __half* X = Xin;
+            float* G = h->G + (batch ? (size_t)d * prow * 4 * H : 0);
+            __half* run = h->pk_run + (batch ? (size_t)d * prow * H : 0);
             if (first || d == 1) {   // padded (and, for the backward direction, per-sequence reversed) copy of the input
                 lstm_to_padded_kernel<<<grid, 128, 0, st>>>(Xin, Il, first ? 1 : 0, h->pk_x, meta, T, B, Il, d);
                 X = h->pk_x;
             }
-            if ((rc = launch_gemm_wx(h->w_ih[ld], X, nullptr, h->G, 4 * H, Il, (int)prow, Il, 4 * H, PIMB200_ACT_NONE, 1, st)) !=
+            if ((rc = launch_gemm_wx(h->w_ih[ld], X, nullptr, G, 4 * H, Il, (int)prow, Il, 4 * H, PIMB200_ACT_NONE, 1, st)) !=
                 PIMB200_OK)
                 return rc;
-            lstm_freeze_gates_kernel<<<grid, 128, 0, st>>>(h->G, meta, T, B, H);
+            lstm_freeze_gates_kernel<<<grid, 128, 0, st>>>(G, meta, T, B, H);
             const __half* h0_ld = h0 ? h0 + (size_t)ld * B * H : nullptr;
             const __half* c0_ld = c0 ? c0 + (size_t)ld * B * H : nullptr;
             __half* cn_ld = cn ? cn + (size_t)ld * B * H : nullptr;
-            if ((rc = run_recurrence(h, ld, padded, false, h->G, (long)B * 4 * H, 4L * H, h0_ld, c0_ld, h->pk_run, (long)B * H,
-                                     (long)H, nullptr, cn_ld, st)) != PIMB200_OK)
+            if (batch) {
+                ba.dir[d] = BatchDir{h->w_hh[ld], h->bias[ld], G, h0_ld, c0_ld, run, nullptr, cn_ld, 0};
+                if (d + 1 < D) continue;
+                ba.dirs = D;
+                ba.g_tstride = (long)B * 4 * H; ba.g_bstride = 4L * H;
+                ba.y_tstride = (long)B * H; ba.y_bstride = H; ba.y_fold = 1;
+                ba.H = H; ba.T = T; ba.B = B; ba.steps = T;
+                ba.counters = h->batch_counters; ba.status = h->d_status; ba.gen = next_gen(h); ba.poll_limit = h->poll_limit;
+                if (h->prof) prof_mark(h, st);
+                if ((rc = launch_lstm_batch(ba, st)) != PIMB200_OK) return rc;
+                if (h->prof) {
+                    prof_mark(h, st);
+                    h->prof_bytes += (double)D * T * 4.0 * H * H * 2.0;
+                }
+            } else if ((rc = run_recurrence(h, ld, padded, false, G, (long)B * 4 * H, 4L * H, h0_ld, c0_ld, run, (long)B * H, (long)H,
+                                            nullptr, cn_ld, st)) != PIMB200_OK) {
                 return rc;
-            lstm_from_padded_kernel<<<grid, 128, 0, st>>>(h->pk_run, Yout, (long)D * H, last ? 1 : 0, d * H,
-                                                          hn ? hn + (size_t)ld * B * H : nullptr, meta, T, B, H, d);
+            }
+            for (int e = batch ? 0 : d; e <= d; ++e)      // (with both directions at once, behind the second one)
+                lstm_from_padded_kernel<<<grid, 128, 0, st>>>(h->pk_run + (batch ? (size_t)e * prow * H : 0), Yout, (long)D * H, last ? 1 : 0,
+                                                              e * H, hn ? hn + (size_t)(l * D + e) * B * H : nullptr, meta, T, B, H, e);
             if ((rc = launch_status()) != PIMB200_OK) return rc;
         }
     }
     return PIMB200_OK;
+}
+
+extern "C" int pimb200_lstm_packed_capacity(const pimb200_lstm* h) {
+    if (!h) return 0;
+    const bool batch = h->bulk_wide == 2 && !h->use_tc && (h->variant == PIMB200_LSTM_AUTO || h->variant == PIMB200_LSTM_PERSISTENT);
+    return std::max(h->H % 16 == 0 ? kPipeMaxB : 0, batch ? lstm_batch_capacity(h->H, h->D) : 0);
 }
 
 // Layers l and l + 1 (one direction) as a wavefront: true when the shape is that of lstm_direct.cu
@@ -2618,8 +2664,6 @@ static int run_wave(pimb200_lstm* h, int l, int T, int B, const float* G, long g
 // thousand steps would take 17 GB.  Everything between the layers is time-major (with the sequences' own order, the rows of
 // one step lie a page apart).
 // ---------------------------------------------------------------------------------------------
-constexpr int kBatchMinB = 129;              // fewer sequences: the kernels above
-constexpr long kBatchChunkRows = 131072;     // rows of gate terms per chunk (2 GB at H = 1024)
 
 // dst[t, b, :] <- src[t * t_rows + b * b_rows, :] of `cols` halves, t < T, b < B; a warp per row
 __global__ void lstm_time_major_kernel(const __half* __restrict__ src, long t_rows, long b_rows, __half* __restrict__ dst, int B,
@@ -2639,7 +2683,7 @@ __global__ void lstm_time_major_kernel(const __half* __restrict__ src, long t_ro
 struct RowStrides { long t, b; };
 
 static bool batch_fits(const pimb200_lstm* h, int T, int B) {
-    return B >= kBatchMinB && T >= 8 && h->bulk_wide == 2 && !h->use_tc &&
+    return B >= (h->D == 2 ? kBatchMinBothB : kBatchMinB) && T >= 8 && h->bulk_wide == 2 && !h->use_tc &&
            (h->variant == PIMB200_LSTM_AUTO || h->variant == PIMB200_LSTM_PERSISTENT) && lstm_batch_capacity(h->H, h->D) > 0;
 }
 
@@ -2723,7 +2767,7 @@ static int lstm_forward_impl(pimb200_lstm* h, const __half* x, const SeqLayout& 
     int rc;
     // packed input of several steps: as a padded lock-step batch on the persistent recurrences (needs the 128-bit GEMM
     // path for the padded rows; the streamed kernels below take every other case)
-    if (packed && h->packed_lockstep && h->variant != PIMB200_LSTM_STREAMED && T > 1 && H % 16 == 0 && B <= kPipeMaxB)
+    if (packed && h->packed_lockstep && h->variant != PIMB200_LSTM_STREAMED && T > 1 && H % 16 == 0 && (B <= kPipeMaxB || batch_fits_packed(h, T, B)))
         return lstm_forward_packed_lockstep(h, x, sq, h0, c0, y, hn, cn, st);
     // many sequences, in equal parts of what a launch takes
     if (!packed && batch_fits(h, T, B) && aligned16(y) && (!h0 || aligned16(h0)) && (!hn || aligned16(hn))) {

@@ -6,7 +6,7 @@ projection a batch-1 addmm (runtime/source/executor/op_executor/aten_ops_executo
 inputs examples/runtime/source/pipeline_manager.cpp:143-151).  Sentences are independent, so a GPU that has to serve
 hundreds of them runs `group` sentences in lock step instead:
 
-  * encoder: the group's sentences, sorted by length, go through each layer as packed batches of up to 128 sentences
+  * encoder: the group's sentences, sorted by length, go through each layer as packed batches of up to 512 sentences
     (aten::lstm's packed overload, which the library runs as a padded lock-step batch on the persistent weight-stationary
     recurrence, the backward direction of the first layer on the sentences reversed one by one);
   * decoder: one step for the whole group is four cells (each one launch: both products and the gate math; the output, for
@@ -95,6 +95,7 @@ class GnmtTranslator:
         for name in ("enc1", "enc2", "enc3", "dec0", "dec1", "dec2", "dec3"):
             p = self.w[name]
             self.lstm[name] = ops.Lstm(p, 1, False, p[0].shape[1], H, True)
+        self.enc_batch = min(self.ENC_BATCH, max(128, min(self.lstm[f"enc{i}"].packed_capacity() for i in range(4))))
         f16 = dict(dtype=torch.float16, device=self.dev)
         i64 = dict(dtype=torch.int64, device=self.dev)
         # encoder outputs / attention keys of the current group, time-major, at their maximum size
@@ -123,10 +124,10 @@ class GnmtTranslator:
         self.launches_per_step = 0
 
     # ------------------------------------------------------------------------------------------------ encoder
-    ENC_BATCH = 128          # sequences per packed aten::lstm call (the lock-step recurrences take up to 128)
+    ENC_BATCH = 512          # sequences per packed aten::lstm call, where the lock-step recurrences take as many
 
     def encode(self, group: dict) -> int:
-        """One staged group (see stage(); tensors on the device).  Every slice of up to 128 sentences goes through the
+        """One staged group (see stage(); tensors on the device).  Every slice of up to 512 sentences goes through the
         encoder as a PACKED batch (the aten::lstm overload the reference's GNMT graph uses for its encoder): rows of
         padding never reach a GEMM or an add, and the library runs the packed batch on the lock-step recurrences.  The
         encoder states are scattered into the padded time-major buffer the attention kernel reads.  Returns S_g."""
@@ -266,7 +267,7 @@ class GnmtTranslator:
     # ------------------------------------------------------------------------------------------------ user call
     def stage(self, sentences: Sequence[torch.Tensor]):
         """Sorts the sentences by length and packs them into lock-step groups (see stage_groups)."""
-        return stage_groups(sentences, self.G, self.ENC_BATCH, self.S, pin=True)
+        return stage_groups(sentences, self.G, self.enc_batch, self.S, pin=True)
 
     def to_device(self, group: dict) -> dict:
         """The group's tensors copied to the device (batch_sizes stays on the host, as aten::lstm takes it)."""

@@ -449,6 +449,10 @@ class Lstm:
     def set_wavefront(self, on: bool) -> None:
         check(_lib.lib().pimb200_lstm_set_wavefront(self._h, 1 if on else 0), "lstm_set_wavefront")
 
+    def packed_capacity(self) -> int:
+        """Sequences of a packed batch that run in lock step, one launch per layer."""
+        return int(_lib.lib().pimb200_lstm_packed_capacity(self._h))
+
     def set_packed_lockstep(self, on: bool) -> None:
         check(_lib.lib().pimb200_lstm_set_packed_lockstep(self._h, 1 if on else 0), "lstm_set_packed_lockstep")
 

@@ -440,7 +440,8 @@ def test_lstm_benchmark_shape_batched_vs_libtorch():
 
 
 @pytest.mark.parametrize("B,I,H,L,bi,lo,hi", [(7, 24, 64, 2, True, 1, 9), (40, 1024, 1024, 1, True, 20, 50), (128, 48, 128, 2, False, 3, 30),
-                                             (33, 40, 256, 3, True, 2, 12), (5, 16, 48, 1, False, 4, 4)])
+                                             (33, 40, 256, 3, True, 2, 12), (5, 16, 48, 1, False, 4, 4),
+                                             (96, 64, 1024, 1, True, 8, 20), (200, 40, 256, 2, True, 3, 14), (300, 24, 320, 2, False, 5, 20)])
 def test_lstm_packed_sequences_on_the_lockstep_kernels_vs_libtorch(B, I, H, L, bi, lo, hi):
     # packed input (sequences of ragged length, sorted) runs as a padded lock-step batch on the persistent recurrences:
     # outputs, h_n and c_n against libtorch's packed overload, and against the timestep-by-timestep streamed path
