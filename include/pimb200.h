@@ -99,6 +99,10 @@ int pimb200_bmm_row(const void* x, const void* A, void* y, int k, int n, void* s
 int pimb200_gemm_wx(const void* W, const void* X, const void* bias, void* Y,
                     int N, int K, int J, int ldx, int ldy, int act, int y_is_f32, void* stream);
 
+/* The same for a W that no work ahead on the stream writes: the launch may read it before that work has ended. */
+int pimb200_gemm_wx_fixed(const void* W, const void* X, const void* bias, void* Y,
+                          int N, int K, int J, int ldx, int ldy, int act, int y_is_f32, void* stream);
+
 /* n independent products of the form above in ONE launch when their shapes allow it (each with at most 32 activation
  * rows, or at most 256 against a matrix of at most 2048 rows; up to 8 per launch, more are issued in launches of 8); any
  * other mix is issued product by product on the same stream, so the call is always complete.  The fan-out of a

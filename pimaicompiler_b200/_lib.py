@@ -47,6 +47,7 @@ SIGNATURES = {
     "pimb200_layer_norm_rows": (_i, [_vp, _vp, _vp, _vp, C.c_long, C.c_long, C.c_float, _vp]),
     "pimb200_tanh_f16": (_i, [_vp, _vp, _sz, _vp]),
     "pimb200_attention_row": (_i, [_vp, _vp, _vp, _vp, C.c_long, C.c_long, _vp, _i, _i, C.c_long, C.c_float, _vp]),
+    "pimb200_gemm_wx_fixed": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp]),
     "pimb200_gemm_wx_grouped": (_i, [_vp, _i, _vp]),
     "pimb200_attention_rows": (_i, [_vp, _vp, _vp, _vp, C.c_long, C.c_long, C.c_long, _vp, _i, _i, _i, C.c_long, C.c_long,
                                     C.c_long, C.c_long, C.c_float, _vp]),

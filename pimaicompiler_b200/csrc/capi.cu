@@ -6,7 +6,7 @@
 namespace pimb200 {
 
 int launch_gemm_wx(const __half* W, const __half* X, const __half* bias, void* Y, int N, int K, int J, int ldx,
-                   int ldy, int act, int y_is_f32, cudaStream_t st);
+                   int ldy, int act, int y_is_f32, cudaStream_t st, int fixed = 0);
 
 static std::mutex g_ctx_mutex;
 static DeviceCtx g_ctx[64];
@@ -87,6 +87,14 @@ extern "C" int pimb200_gemm_wx(const void* W, const void* X, const void* bias, v
     return launch_gemm_wx(static_cast<const __half*>(W), static_cast<const __half*>(X),
                           static_cast<const __half*>(bias), Y, N, K, J, ldx, ldy, act, y_is_f32,
                           static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int pimb200_gemm_wx_fixed(const void* W, const void* X, const void* bias, void* Y, int N, int K, int J, int ldx, int ldy,
+                                     int act, int y_is_f32, void* stream) {
+    if (!W || !X || !Y || N <= 0 || K <= 0 || J <= 0 || ldx < K || ldy < N) return PIMB200_ERR_BAD_ARG;
+    if (act != PIMB200_ACT_NONE && act != PIMB200_ACT_RELU) return PIMB200_ERR_BAD_ARG;
+    return launch_gemm_wx(static_cast<const __half*>(W), static_cast<const __half*>(X), static_cast<const __half*>(bias), Y, N, K, J,
+                          ldx, ldy, act, y_is_f32, static_cast<cudaStream_t>(stream), 1);
 }
 
 namespace pimb200 {

@@ -69,6 +69,7 @@ struct Args {
     void* Y;
     long ldy;
     int direct;               // 1: the outputs are stored element by element
+    int fixed;                // 1: no work ahead on the stream writes the weights (they may be read before that work has ended)
     int x_batch;              // > 0: rows are numbered time-major over batch-first sequences (map x is 3-D: K, b, t)
     int* status;
     int gen;
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
     const uint32_t tmem_base = *tmem_slot;
     bool failed = false;
     pdl_launch_dependents();
-    pdl_wait();
+    if (warp != 1 || !a.fixed) pdl_wait();
 
     if (warp < 2) {
         // ---------------- TMA producers: warp 0 the activation rows, warp 1 the weight rows, each one stream of K blocks
@@ -525,14 +526,14 @@ bool operands_ok(const void* W, const void* X, int K, long ldx) {
 }  // namespace tc
 
 int launch_gemm_rows(const __half* W, const __half* X, const __half* bias, void* Y, int N, int K, int J, int ldx, int ldy,
-                     int act, int y_is_f32, int x_batch, long x_seq_rows, cudaStream_t st) {
+                     int act, int y_is_f32, int x_batch, long x_seq_rows, cudaStream_t st, int fixed) {
     using namespace tc;
     if (!operands_ok(W, X, K, ldx)) return PIMB200_ERR_UNSUPPORTED;
     if (x_batch > 0 && (J % x_batch != 0 || x_batch > BM)) return PIMB200_ERR_UNSUPPORTED;
     Args a = {};
     int dev = 0, rc;
     if ((rc = tc_prepare(&dev, &a.status, &a.gen)) != PIMB200_OK) return rc;
-    a.bias = bias; a.N = N; a.J = J; a.act = act;
+    a.bias = bias; a.N = N; a.J = J; a.act = act; a.fixed = fixed;
     // whole timesteps, or no more rows than there are: a tile's other rows are never stored, and a load of rows past the end
     // of X costs more than one of rows that exist (32320 x 1024, 32 rows: 19.2 us with boxes of 128)
     a.jrows = x_batch > 0 ? BM / x_batch * x_batch : tile_rows(J);
@@ -560,13 +561,13 @@ int launch_gemm_rows(const __half* W, const __half* X, const __half* bias, void*
 int gemm_rows_max_parts(int N) { return 2 * ceil_div(N, 64); }
 
 int launch_gemm_rows_argmax(const __half* W, const __half* X, const __half* bias, float* best_v, int* best_i, int* parts, int N,
-                            int K, int J, int ldx, cudaStream_t st) {
+                            int K, int J, int ldx, cudaStream_t st, int fixed) {
     using namespace tc;
     if (!operands_ok(W, X, K, ldx)) return PIMB200_ERR_UNSUPPORTED;
     Args a = {};
     int dev = 0, rc;
     if ((rc = tc_prepare(&dev, &a.status, &a.gen)) != PIMB200_OK) return rc;
-    a.bias = bias; a.N = N; a.J = J; a.act = PIMB200_ACT_NONE;
+    a.bias = bias; a.N = N; a.J = J; a.act = PIMB200_ACT_NONE; a.fixed = fixed;
     a.jrows = tile_rows(J);
     a.kb1 = ceil_div(K, BK);
     const Plan p = pick(N, J, a.jrows, a.kb1, 32, tc_sm_count(dev));
@@ -588,7 +589,7 @@ int launch_gemm_rows_cell(const RowsCell& c, cudaStream_t st) {
     Args a = {};
     int dev = 0, rc;
     if ((rc = tc_prepare(&dev, &a.status, &a.gen)) != PIMB200_OK) return rc;
-    a.N = 4 * c.H; a.J = c.J; a.jrows = tile_rows(c.J);
+    a.N = 4 * c.H; a.J = c.J; a.jrows = tile_rows(c.J); a.fixed = 1;
     a.kb1 = ceil_div(c.I, BK);
     a.kb2 = c.h0 ? ceil_div(c.H, BK) : 0;
     a.cell_bias = c.bias; a.c0 = c.c0; a.y = c.y; a.y_ld = c.y_ld; a.hn = c.hn; a.cn = c.cn; a.res = c.res; a.res_ld = c.res_ld;

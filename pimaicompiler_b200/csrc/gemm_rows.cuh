@@ -26,12 +26,12 @@ int tc_sm_count(int dev);
 // Y[J, N] = act(X W^T + bias) as fp16 or fp32; x_batch > 0: X is batch-first [x_batch][x_seq_rows][K] and the rows of Y are
 // numbered time-major (row = t * x_batch + b)
 int launch_gemm_rows(const __half* W, const __half* X, const __half* bias, void* Y, int N, int K, int J, int ldx, int ldy,
-                     int act, int y_is_f32, int x_batch, long x_seq_rows, cudaStream_t st);
+                     int act, int y_is_f32, int x_batch, long x_seq_rows, cudaStream_t st, int fixed = 0);
 
 // The largest of fp16(X W^T + bias) of every row in pieces: best_v / best_i [*parts][J], *parts <= gemm_rows_max_parts(N).
 int gemm_rows_max_parts(int N);
 int launch_gemm_rows_argmax(const __half* W, const __half* X, const __half* bias, float* best_v, int* best_i, int* parts, int N,
-                            int K, int J, int ldx, cudaStream_t st);
+                            int K, int J, int ldx, cudaStream_t st, int fixed = 0);
 
 // One LSTM step of J sequences: gates = X Wx^T + H0 Wh^T + bias (H0 may be NULL), cell update, y = h (+ residual)
 struct RowsCell {

@@ -50,19 +50,21 @@ struct SkinnyArgs {
     int N, K, J, ldx, ldy, act, y_is_f32;
     float* best_v;        // arg max form: [CTAs][J] largest output of the CTA's rows and its index
     int* best_i;
+    int fixed;            // 1: no work ahead on the stream writes W (it may be read before that work has ended)
 };
 
 // NT: n-tiles of 8 activation rows; MTW: 16-row weight tiles per warp (1 or 2; they share the warp's X fragments).
 // The 8 warps of a CTA split K; a warp walks its K range in groups of UB 32-wide blocks, the loads of the next group
 // in flight while the current one is multiplied.
-template <int NT, int MTW>
-__global__ void __launch_bounds__(kSkinnyThreads) gemm_skinny_kernel(SkinnyArgs a) {
+// UB: 32-wide K blocks per register buffer.  One is all that a warp has at K <= 512, and leaves room for CTAs of the launches behind
+// this one on the same SM (20 rows: 250 registers with buffers of four).
+template <int NT, int MTW, int UB = 4 / MTW>
+__global__ void __launch_bounds__(kSkinnyThreads, UB == 1 ? 2 : 1) gemm_skinny_kernel(const __grid_constant__ SkinnyArgs a) {
     constexpr int KS = kSkinnyWarps;
     constexpr int ROWS = MTW * kSkinnyRows;
-    constexpr int UB = 4 / MTW;
     __shared__ float part[KS][ROWS][NT * 8 + 1];
     pdl_launch_dependents();
-    pdl_wait();
+    if (!a.fixed) pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int n0 = blockIdx.x * ROWS;
@@ -91,7 +93,7 @@ __global__ void __launch_bounds__(kSkinnyThreads) gemm_skinny_kernel(SkinnyArgs 
             for (int i = 0; i < 4; ++i) acc[m][j][i] = 0.f;
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     uint4 wc[UB][MTW][2], xc[UB][NT], wn[UB][MTW][2], xn[UB][NT];
-    auto load_group = [&](uint4 (&w)[UB][MTW][2], uint4 (&x)[UB][NT], int b0) {
+    auto load_w = [&](uint4 (&w)[UB][MTW][2], int b0) {
 #pragma unroll
         for (int u = 0; u < UB; ++u) {
             const int b = b0 + u;
@@ -102,6 +104,13 @@ __global__ void __launch_bounds__(kSkinnyThreads) gemm_skinny_kernel(SkinnyArgs 
                 w[u][m][0] = in ? ld_stream_v4(wrow[m][0] + (size_t)b * 32) : zero;
                 w[u][m][1] = in ? ld_stream_v4(wrow[m][1] + (size_t)b * 32) : zero;
             }
+        }
+    };
+    auto load_x = [&](uint4 (&x)[UB][NT], int b0) {
+#pragma unroll
+        for (int u = 0; u < UB; ++u) {
+            const int b = b0 + u;
+            const bool in = b < b_hi && b * 32 + 8 * t < K;
 #pragma unroll
             for (int j = 0; j < NT; ++j) x[u][j] = in ? ld_v4(xrow[j] + (size_t)b * 32) : zero;
         }
@@ -118,13 +127,32 @@ __global__ void __launch_bounds__(kSkinnyThreads) gemm_skinny_kernel(SkinnyArgs 
                     mma16816(acc[m][j], w[u][m][0].z, w[u][m][1].z, w[u][m][0].w, w[u][m][1].w, x[u][j].z, x[u][j].w);
                 }
     };
-    // two register buffers used alternately (no copies between them: a move would wait for the load it moves)
-    load_group(wc, xc, b_lo);
-    for (int b0 = b_lo; b0 < b_hi; b0 += 2 * UB) {
-        load_group(wn, xn, b0 + UB);
+    // two register buffers used alternately (no copies between them: a move would wait for the load it moves); weights that
+    // nobody writes are on their way before the predecessor has ended
+    load_w(wc, b_lo);
+    if (a.fixed) {
+        load_w(wn, b_lo + UB);
+        pdl_wait();
+        load_x(xc, b_lo);
+        load_x(xn, b_lo + UB);
         multiply(wc, xc);
-        load_group(wc, xc, b0 + 2 * UB);
+        load_w(wc, b_lo + 2 * UB); load_x(xc, b_lo + 2 * UB);
         multiply(wn, xn);
+        if (b_lo + 2 * UB < b_hi) { load_w(wn, b_lo + 3 * UB); load_x(xn, b_lo + 3 * UB); }
+        for (int b0 = b_lo + 2 * UB; b0 < b_hi; b0 += 2 * UB) {
+            multiply(wc, xc);
+            load_w(wc, b0 + 2 * UB); load_x(xc, b0 + 2 * UB);
+            multiply(wn, xn);
+            load_w(wn, b0 + 3 * UB); load_x(xn, b0 + 3 * UB);
+        }
+    } else {
+        load_x(xc, b_lo);
+        for (int b0 = b_lo; b0 < b_hi; b0 += 2 * UB) {
+            load_w(wn, b0 + UB); load_x(xn, b0 + UB);
+            multiply(wc, xc);
+            load_w(wc, b0 + 2 * UB); load_x(xc, b0 + 2 * UB);
+            multiply(wn, xn);
+        }
     }
     // accumulator layout: (row g, cols 2t, 2t+1), (row g+8, same cols) of each n-tile
 #pragma unroll
@@ -354,14 +382,14 @@ __global__ void __launch_bounds__(kSkinnyThreads, 2) gemm_skinny_rows_kernel(Ski
     constexpr int UB = 4;                                            // 32-wide K blocks per register buffer
     extern __shared__ __align__(16) unsigned char sk_smem[];
     pdl_launch_dependents();
-    pdl_wait();
+    if (!a.fixed) pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int K = a.K;                                               // K % 64 == 0 (checked by the launcher)
     const int xs = K * 2;                                            // bytes per X row, a multiple of 128
     const int blocks = K >> 5;
     const int gpt = (blocks + UB - 1) / UB;                          // groups of K blocks per tile
-    {
+    auto copy_x = [&] {
         const int chunks = K >> 3;                                   // 16-byte chunks per row
         for (int row = warp; row < NT * 8; row += kSkinnyWarps) {
             const __half* src = a.X + (size_t)min(row, a.J - 1) * a.ldx;   // rows past J repeat the last one
@@ -372,7 +400,7 @@ __global__ void __launch_bounds__(kSkinnyThreads, 2) gemm_skinny_rows_kernel(Ski
                              "l"(src + c * 8) : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
-    }
+    };
     // tile i of the launch belongs to CTA i % gridDim.x, warp (i / gridDim.x) % 8; a warp walks its tiles as one stream of
     // (tile, group) pairs, so the loads of a tile's first group are in flight during the previous tile's last products
     const int stride = kSkinnyWarps * gridDim.x;
@@ -444,7 +472,12 @@ __global__ void __launch_bounds__(kSkinnyThreads, 2) gemm_skinny_rows_kernel(Ski
     };
     int lt = blockIdx.x + warp * gridDim.x, lg = 0;                  // load cursor
     int ct = lt, cg = 0;                                             // compute cursor
+    if (!a.fixed) copy_x();
     load_group(w0, lt, lg); advance(lt, lg);
+    if (a.fixed) {                                                   // the weights are on their way before the predecessor has ended
+        pdl_wait();
+        copy_x();
+    }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();                                                 // reached by every warp, with or without a tile
     while (ct < tiles) {
@@ -515,7 +548,7 @@ int launch_skinny_rows(const SkinnyArgs& a, cudaStream_t st) {
 
 // PIMB200_ERR_UNSUPPORTED when the shape is not this kernel's (the caller then takes the tensor-core or SIMT path)
 int launch_gemm_wx_skinny(const __half* W, const __half* X, const __half* bias, void* Y, int N, int K, int J, int ldx,
-                          int ldy, int act, int y_is_f32, cudaStream_t st) {
+                          int ldy, int act, int y_is_f32, cudaStream_t st, int fixed) {
     if (J < 1 || K % 8 != 0 || ldx % 8 != 0 || !aligned16(W) || !aligned16(X)) return PIMB200_ERR_UNSUPPORTED;
     // More than 32 activation rows run as column blocks of 32 (grid.y) when the weight matrix is small: W then comes
     // from L2 for all but the first block, and a matrix of a few 128-row tiles would leave most SMs of the tcgen05
@@ -523,7 +556,7 @@ int launch_gemm_wx_skinny(const __half* W, const __half* X, const __half* bias, 
     if (J > kSkinnyMaxJ && (J > kSkinnyMaxBlockedJ || N > kSkinnyMaxBlockedN || (size_t)N * K > kSkinnyMaxBlockedNK ||
                             ceil_div(N, kSkinnyRows) * ceil_div(J, kSkinnyMaxJ) > kSkinnyMaxBlockedCtas))
         return PIMB200_ERR_UNSUPPORTED;
-    SkinnyArgs a{W, X, bias, Y, N, K, J, ldx, ldy, act, y_is_f32, nullptr, nullptr};
+    SkinnyArgs a{W, X, bias, Y, N, K, J, ldx, ldy, act, y_is_f32, nullptr, nullptr, fixed};
     const int nt = J > kSkinnyMaxJ ? 4 : ceil_div(J, 8);
     const int jblocks = ceil_div(J, kSkinnyMaxJ);
     if (nt >= 2 && N >= 16384 && jblocks == 1) {
@@ -532,24 +565,14 @@ int launch_gemm_wx_skinny(const __half* W, const __half* X, const __half* bias, 
                                                                     : launch_skinny_rows<4, false>(a, st);
         if (rc != PIMB200_ERR_UNSUPPORTED) return rc;
     }
-    cudaError_t rc = cudaSuccess;
-    if (N >= 2048) {
-        const dim3 grid(ceil_div(N, 2 * kSkinnyRows), jblocks);
-        switch (nt) {
-            case 1: rc = launch_pdl(gemm_skinny_kernel<1, 2>, grid, dim3(kSkinnyThreads), 0, st, a); break;
-            case 2: rc = launch_pdl(gemm_skinny_kernel<2, 2>, grid, dim3(kSkinnyThreads), 0, st, a); break;
-            case 3: rc = launch_pdl(gemm_skinny_kernel<3, 2>, grid, dim3(kSkinnyThreads), 0, st, a); break;
-            default: rc = launch_pdl(gemm_skinny_kernel<4, 2>, grid, dim3(kSkinnyThreads), 0, st, a); break;
-        }
-    } else {
-        const dim3 grid(ceil_div(N, kSkinnyRows), jblocks);
-        switch (nt) {
-            case 1: rc = launch_pdl(gemm_skinny_kernel<1, 1>, grid, dim3(kSkinnyThreads), 0, st, a); break;
-            case 2: rc = launch_pdl(gemm_skinny_kernel<2, 1>, grid, dim3(kSkinnyThreads), 0, st, a); break;
-            case 3: rc = launch_pdl(gemm_skinny_kernel<3, 1>, grid, dim3(kSkinnyThreads), 0, st, a); break;
-            default: rc = launch_pdl(gemm_skinny_kernel<4, 1>, grid, dim3(kSkinnyThreads), 0, st, a); break;
-        }
-    }
+    const bool wide = N >= 2048;
+    const dim3 grid(ceil_div(N, wide ? 2 * kSkinnyRows : kSkinnyRows), jblocks);
+    static void (*const kernels[2][2][4])(SkinnyArgs) = {      // [K <= 512][32 weight rows per CTA][tiles of 8 activation rows]
+        {{gemm_skinny_kernel<1, 1>, gemm_skinny_kernel<2, 1>, gemm_skinny_kernel<3, 1>, gemm_skinny_kernel<4, 1>},
+         {gemm_skinny_kernel<1, 2>, gemm_skinny_kernel<2, 2>, gemm_skinny_kernel<3, 2>, gemm_skinny_kernel<4, 2>}},
+        {{gemm_skinny_kernel<1, 1, 1>, gemm_skinny_kernel<2, 1, 1>, gemm_skinny_kernel<3, 1, 1>, gemm_skinny_kernel<4, 1, 1>},
+         {gemm_skinny_kernel<1, 2, 1>, gemm_skinny_kernel<2, 2, 1>, gemm_skinny_kernel<3, 2, 1>, gemm_skinny_kernel<4, 2, 1>}}};
+    const cudaError_t rc = launch_pdl(kernels[K <= 512][wide][nt - 1], grid, dim3(kSkinnyThreads), 0, st, a);
     return cuda_status(rc);
 }
 
@@ -567,9 +590,9 @@ int launch_lstm_cell_skinny(const RowsCell& c, cudaStream_t st) {
 
 // The arg max form for up to 32 activation rows: best_v / best_i [*parts][J]
 int launch_skinny_argmax(const __half* W, const __half* X, const __half* bias, float* best_v, int* best_i, int* parts, int N, int K,
-                         int J, int ldx, cudaStream_t st) {
+                         int J, int ldx, cudaStream_t st, int fixed) {
     if (J < 1 || J > kSkinnyMaxJ || K % 64 != 0 || ldx % 8 != 0 || !aligned16(W) || !aligned16(X)) return PIMB200_ERR_UNSUPPORTED;
-    const SkinnyArgs a{W, X, bias, nullptr, N, K, J, ldx, 0, PIMB200_ACT_NONE, 0, best_v, best_i};
+    const SkinnyArgs a{W, X, bias, nullptr, N, K, J, ldx, 0, PIMB200_ACT_NONE, 0, best_v, best_i, fixed};
     const int nt = ceil_div(J, 8);
     *parts = skinny_rows_grid(N, (size_t)nt * 8 * K * 2);
     switch (nt) {
@@ -591,7 +614,7 @@ int launch_gemm_wx_grouped(const GemmProblem* pr, int n, cudaStream_t st) {
         if (q.J < 1 || q.J > kSkinnyMaxBlockedJ || q.K % 8 != 0 || q.ldx % 8 != 0 || !aligned16(q.W) || !aligned16(q.X))
             return PIMB200_ERR_UNSUPPORTED;
         if (q.J > kSkinnyMaxJ && (q.N > kSkinnyMaxBlockedN || (size_t)q.N * q.K > kSkinnyMaxBlockedNK)) return PIMB200_ERR_UNSUPPORTED;
-        ga.p[i] = SkinnyArgs{q.W, q.X, q.bias, q.Y, q.N, q.K, q.J, q.ldx, q.ldy, q.act, q.y_is_f32, nullptr, nullptr};
+        ga.p[i] = SkinnyArgs{q.W, q.X, q.bias, q.Y, q.N, q.K, q.J, q.ldx, q.ldy, q.act, q.y_is_f32, nullptr, nullptr, 0};
         max_tiles = max(max_tiles, ceil_div(q.N, kSkinnyRows));
         max_jb = max(max_jb, ceil_div(q.J, kSkinnyMaxJ));
         max_j = max(max_j, min(q.J, kSkinnyMaxJ));

@@ -105,16 +105,17 @@ int tc_sm_count(int dev) {
 static int g_force_simt = 0;
 
 int launch_gemm_wx_skinny(const __half* W, const __half* X, const __half* bias, void* Y, int N, int K, int J, int ldx,
-                          int ldy, int act, int y_is_f32, cudaStream_t st);
+                          int ldy, int act, int y_is_f32, cudaStream_t st, int fixed);
 
 // Router of the dense contraction: up to 32 activation rows stream W on every SM (HBM-bound, like the GEMV); more rows
-// go to the tcgen05 kernel; shapes neither takes (unaligned operands, K not a multiple of 8) to the SIMT kernel.
+// go to the tcgen05 kernel; shapes neither takes (unaligned operands, K not a multiple of 8) to the SIMT kernel.  `fixed`: no
+// work ahead on the stream writes W, so it may be read before that work has ended.
 int launch_gemm_wx(const __half* W, const __half* X, const __half* bias, void* Y, int N, int K, int J, int ldx,
-                   int ldy, int act, int y_is_f32, cudaStream_t st) {
+                   int ldy, int act, int y_is_f32, cudaStream_t st, int fixed) {
     if (!g_force_simt) {
-        const int rs = launch_gemm_wx_skinny(W, X, bias, Y, N, K, J, ldx, ldy, act, y_is_f32, st);
+        const int rs = launch_gemm_wx_skinny(W, X, bias, Y, N, K, J, ldx, ldy, act, y_is_f32, st, fixed);
         if (rs != PIMB200_ERR_UNSUPPORTED) return rs;
-        const int rc = launch_gemm_rows(W, X, bias, Y, N, K, J, ldx, ldy, act, y_is_f32, 0, 0, st);
+        const int rc = launch_gemm_rows(W, X, bias, Y, N, K, J, ldx, ldy, act, y_is_f32, 0, 0, st, fixed);
         if (rc != PIMB200_ERR_UNSUPPORTED) return rc;
     }
     return launch_gemm_wx_simt(W, X, bias, Y, N, K, J, ldx, ldy, act, y_is_f32, st);
@@ -126,7 +127,7 @@ int launch_gemm_wx(const __half* W, const __half* X, const __half* bias, void* Y
 int launch_gemm_wx_time_major(const __half* W, const __half* X, void* Y, int N, int K, int J, int ldx, int ldy, int batch,
                               long seq_rows, cudaStream_t st) {
     if (g_force_simt || batch <= 0) return PIMB200_ERR_UNSUPPORTED;
-    return launch_gemm_rows(W, X, nullptr, Y, N, K, J, ldx, ldy, PIMB200_ACT_NONE, 1, batch, seq_rows, st);
+    return launch_gemm_rows(W, X, nullptr, Y, N, K, J, ldx, ldy, PIMB200_ACT_NONE, 1, batch, seq_rows, st, 1);   // (a handle's weights)
 }
 
 }  // namespace pimb200

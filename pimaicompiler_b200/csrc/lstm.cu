@@ -41,7 +41,7 @@ namespace pimb200 {
 int launch_gemm_wx_simt(const __half* W, const __half* X, const __half* bias, void* Y, int N, int K, int J, int ldx,
                         int ldy, int act, int y_is_f32, cudaStream_t st);
 int launch_gemm_wx(const __half* W, const __half* X, const __half* bias, void* Y, int N, int K, int J, int ldx,
-                   int ldy, int act, int y_is_f32, cudaStream_t st);
+                   int ldy, int act, int y_is_f32, cudaStream_t st, int fixed = 0);
 int launch_gemm_wx_time_major(const __half* W, const __half* X, void* Y, int N, int K, int J, int ldx, int ldy, int batch,
                               long seq_rows, cudaStream_t st);
 }  // namespace pimb200

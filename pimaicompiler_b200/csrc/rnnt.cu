@@ -31,7 +31,7 @@ using namespace pimb200;
 
 namespace pimb200 {
 int launch_gemm_wx(const __half* W, const __half* X, const __half* bias, void* Y, int N, int K, int J, int ldx,
-                   int ldy, int act, int y_is_f32, cudaStream_t st);
+                   int ldy, int act, int y_is_f32, cudaStream_t st, int fixed = 0);
 }
 namespace pimb200 {
 void lstm_pack_matrix(const __half* src, __half* dst, int H, int cols, cudaStream_t st);

@@ -168,7 +168,7 @@ class GnmtTranslator:
         if not fused:
             self.lstm["dec0"].forward(self.x.view(1, G, H), src[0], src[4], out=(self.y[0], dst[0], dst[4]))
             ops.copy_2d(self.cats, 0, row, self.y[0], 0, half, half, G); n += 1
-        ops.gemm_wx(w["Wq"], y0, out=self.q); n += 1
+        ops.gemm_wx_fixed(w["Wq"], y0, out=self.q); n += 1
         ops.additive_attention(self.q, self.keys_proj, self.enc_out, self.lengths, self.v_norm, w["att_b"],
                                out=cat[0][:, H:], scores=self.scores, copies=3, copy_stride=2 * H); n += 1
         if fused:

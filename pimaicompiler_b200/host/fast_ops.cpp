@@ -148,7 +148,8 @@ PyObject* gemv_vm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     });
 }
 
-// gemm_wx(W, X, bias, act, out_f32, out): rows of X and of out may be strided
+// gemm_wx(W, X, bias, act, out_f32, out): rows of X and of out may be strided.  FIXED: gemm_wx_fixed
+template <bool FIXED>
 PyObject* gemm_wx(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
         if (n != 6) fail(PyExc_TypeError, "gemm_wx takes 6 arguments");
@@ -167,7 +168,7 @@ PyObject* gemm_wx(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const void *wp = W.data_ptr(), *xp = X.data_ptr();
         void *yp = Y.data_ptr(), *st = stream();
         const int ldx = (int)X.stride(0), ldy = (int)Y.stride(0), f32 = Y.scalar_type() == at::kFloat ? 1 : 0;
-        check(abi([&] { return pimb200_gemm_wx(wp, xp, bias, yp, (int)N, (int)K, (int)J, ldx, ldy, act, f32, st); }), "gemm_wx");
+        check(abi([&] { return (FIXED ? pimb200_gemm_wx_fixed : pimb200_gemm_wx)(wp, xp, bias, yp, (int)N, (int)K, (int)J, ldx, ldy, act, f32, st); }), "gemm_wx");
         return y.release();
     });
 }
@@ -255,7 +256,8 @@ PyObject* set_check(PyObject*, PyObject* f) {
 PyMethodDef kMethods[] = {
     {"gemv_mv", (PyCFunction)(void (*)(void))gemv_mv, METH_FASTCALL, nullptr},
     {"gemv_vm", (PyCFunction)(void (*)(void))gemv_vm, METH_FASTCALL, nullptr},
-    {"gemm_wx", (PyCFunction)(void (*)(void))gemm_wx, METH_FASTCALL, nullptr},
+    {"gemm_wx", (PyCFunction)(void (*)(void))gemm_wx<false>, METH_FASTCALL, nullptr},
+    {"gemm_wx_fixed", (PyCFunction)(void (*)(void))gemm_wx<true>, METH_FASTCALL, nullptr},
     {"lstm_forward", (PyCFunction)(void (*)(void))lstm_forward, METH_FASTCALL, nullptr},
     {"lstm_forward_packed", (PyCFunction)(void (*)(void))lstm_forward_packed, METH_FASTCALL, nullptr},
     {"set_check", set_check, METH_O, nullptr},

@@ -101,6 +101,12 @@ def gemm_wx(W: torch.Tensor, X: torch.Tensor, bias: Optional[torch.Tensor] = Non
     return (_lib._native or _lib.native()).gemm_wx(W, X, bias, act, out_f32, out)
 
 
+def gemm_wx_fixed(W: torch.Tensor, X: torch.Tensor, bias: Optional[torch.Tensor] = None, act: int = ACT_NONE,
+                  out_f32: bool = False, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """gemm_wx for a W that no work ahead on the stream writes: the launch may read it before that work has ended."""
+    return (_lib._native or _lib.native()).gemm_wx_fixed(W, X, bias, act, out_f32, out)
+
+
 def gemm_wx_grouped(problems: Sequence[tuple], act: int = ACT_NONE) -> list:
     """[(W [N,K], X [J,K], bias or None), ...] -> [Y [J,N], ...]: independent products in one launch when their shapes allow
     it (the branches of a MULTISTREAM node), else one launch each."""

@@ -98,6 +98,7 @@ class TransformerTranslator:
         self.logits_all = None
         self._graphs = {}
         self.launches_per_step = 0
+        torch.cuda.current_stream(self.dev).synchronize()            # weights are in place before a launch reads them ahead of its turn
 
     # ------------------------------------------------------------------------------------------------ encoder
     def encode(self, group: dict) -> None:
@@ -109,12 +110,12 @@ class TransformerTranslator:
         self.row0.copy_(group["row0"])
         x = ops.add_f16(ops.gather_rows(self.emb_src, group["ids"]), ops.gather_rows(self.pe, group["pos"]))    # [n, d]
         for L in self.enc:
-            qkv = ops.gemm_wx(L["qkv"], x, L["qkv_b"])
+            qkv = ops.gemm_wx_fixed(L["qkv"], x, L["qkv_b"])
             a = ops.attention_block_packed(qkv[:, :d], qkv[:, d:2 * d], qkv[:, 2 * d:], cfg.heads, self.row0, self.lengths, group["S"])
-            x = ops.add_layer_norm(x, ops.gemm_wx(L["so"], a, L["so_b"]))
-            f = ops.gemm_wx(L["f2"], ops.gemm_wx(L["f1"], x, L["f1_b"], ops.ACT_RELU), L["f2_b"])
+            x = ops.add_layer_norm(x, ops.gemm_wx_fixed(L["so"], a, L["so_b"]))
+            f = ops.gemm_wx_fixed(L["f2"], ops.gemm_wx_fixed(L["f1"], x, L["f1_b"], ops.ACT_RELU), L["f2_b"])
             x = ops.add_layer_norm(x, f)
-        ops.gemm_wx(self.ckv, x, self.ckv_b, out=self.cross[:n])
+        ops.gemm_wx_fixed(self.ckv, x, self.ckv_b, out=self.cross[:n])
 
     # ------------------------------------------------------------------------------------------------ decoder
     def _step(self, t: int, forced: bool, want_logits: bool) -> int:
@@ -127,16 +128,16 @@ class TransformerTranslator:
             x = self.x0                                                          # left there by the previous step
         for i, L in enumerate(self.dec):
             row = self.cache[i][:, t]                                            # [G, 3d]: q, k, v of step t
-            ops.gemm_wx(L["qkv"], x, L["qkv_b"], out=row); n += 1
+            ops.gemm_wx_fixed(L["qkv"], x, L["qkv_b"], out=row); n += 1
             a = ops.attention_rows(row[:, :d], self.cache[i][:, :, d:2 * d], self.cache[i][:, :, 2 * d:], cfg.heads,
                                    len_add=t + 1); n += 1
-            x = ops.add_layer_norm(x, ops.gemm_wx(L["so"], a, L["so_b"])); n += 2
-            cq = ops.gemm_wx(L["cq"], x, L["cq_b"]); n += 1
+            x = ops.add_layer_norm(x, ops.gemm_wx_fixed(L["so"], a, L["so_b"])); n += 2
+            cq = ops.gemm_wx_fixed(L["cq"], x, L["cq_b"]); n += 1
             ck = self.cross[:, (2 * i) * d:(2 * i + 1) * d]
             cv = self.cross[:, (2 * i + 1) * d:(2 * i + 2) * d]
             ca = ops.attention_rows_packed(cq, ck, cv, cfg.heads, self.row0, self.lengths, cfg.max_len); n += 1
-            x = ops.add_layer_norm(x, ops.gemm_wx(L["co"], ca, L["co_b"])); n += 2
-            f = ops.gemm_wx(L["f2"], ops.gemm_wx(L["f1"], x, L["f1_b"], ops.ACT_RELU), L["f2_b"]); n += 2
+            x = ops.add_layer_norm(x, ops.gemm_wx_fixed(L["co"], ca, L["co_b"])); n += 2
+            f = ops.gemm_wx_fixed(L["f2"], ops.gemm_wx_fixed(L["f1"], x, L["f1_b"], ops.ACT_RELU), L["f2_b"]); n += 2
             x = ops.add_layer_norm(x, f); n += 1
         if not want_logits and self.logits is None:
             nxt = None if forced or t + 1 >= cfg.max_steps else self.pe[t + 1]
@@ -145,7 +146,7 @@ class TransformerTranslator:
                 return n + 2
             self.logits = torch.zeros(G, cfg.vocab, dtype=torch.float16, device=self.dev)
         lg = self.logits_all[t] if want_logits else self.logits
-        ops.gemm_wx(self.Wo, x, out=lg); n += 1
+        ops.gemm_wx_fixed(self.Wo, x, out=lg); n += 1
         ops.argmax(lg, out=self.toks[t + 1]); n += 1
         return n
 
