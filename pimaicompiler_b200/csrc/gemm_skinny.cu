@@ -58,7 +58,7 @@ struct SkinnyArgs {
 // in flight while the current one is multiplied.
 // UB: 32-wide K blocks per register buffer.  One is all that a warp has at K <= 512, and leaves room for CTAs of the launches behind
 // this one on the same SM (20 rows: 250 registers with buffers of four).
-template <int NT, int MTW, int UB = 4 / MTW>
+template <int NT, int MTW, int UB>
 __global__ void __launch_bounds__(kSkinnyThreads, UB == 1 ? 2 : 1) gemm_skinny_kernel(const __grid_constant__ SkinnyArgs a) {
     constexpr int KS = kSkinnyWarps;
     constexpr int ROWS = MTW * kSkinnyRows;
@@ -93,27 +93,26 @@ __global__ void __launch_bounds__(kSkinnyThreads, UB == 1 ? 2 : 1) gemm_skinny_k
             for (int i = 0; i < 4; ++i) acc[m][j][i] = 0.f;
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     uint4 wc[UB][MTW][2], xc[UB][NT], wn[UB][MTW][2], xn[UB][NT];
+    // K % 8 == 0: a thread's 8 consecutive k are all inside or all outside
+    auto inside = [&](int b) { return b < b_hi && b * 32 + 8 * t < K; };
+    auto load_w1 = [&](uint4 (&w)[MTW][2], int b) {
+#pragma unroll
+        for (int m = 0; m < MTW; ++m) {
+            w[m][0] = inside(b) ? ld_stream_v4(wrow[m][0] + (size_t)b * 32) : zero;
+            w[m][1] = inside(b) ? ld_stream_v4(wrow[m][1] + (size_t)b * 32) : zero;
+        }
+    };
+    auto load_x1 = [&](uint4 (&x)[NT], int b) {
+#pragma unroll
+        for (int j = 0; j < NT; ++j) x[j] = inside(b) ? ld_v4(xrow[j] + (size_t)b * 32) : zero;
+    };
     auto load_w = [&](uint4 (&w)[UB][MTW][2], int b0) {
 #pragma unroll
-        for (int u = 0; u < UB; ++u) {
-            const int b = b0 + u;
-            // K % 8 == 0: a thread's 8 consecutive k are all inside or all outside
-            const bool in = b < b_hi && b * 32 + 8 * t < K;
-#pragma unroll
-            for (int m = 0; m < MTW; ++m) {
-                w[u][m][0] = in ? ld_stream_v4(wrow[m][0] + (size_t)b * 32) : zero;
-                w[u][m][1] = in ? ld_stream_v4(wrow[m][1] + (size_t)b * 32) : zero;
-            }
-        }
+        for (int u = 0; u < UB; ++u) load_w1(w[u], b0 + u);
     };
     auto load_x = [&](uint4 (&x)[UB][NT], int b0) {
 #pragma unroll
-        for (int u = 0; u < UB; ++u) {
-            const int b = b0 + u;
-            const bool in = b < b_hi && b * 32 + 8 * t < K;
-#pragma unroll
-            for (int j = 0; j < NT; ++j) x[u][j] = in ? ld_v4(xrow[j] + (size_t)b * 32) : zero;
-        }
+        for (int u = 0; u < UB; ++u) load_x1(x[u], b0 + u);
     };
     auto multiply = [&](const uint4 (&w)[UB][MTW][2], const uint4 (&x)[UB][NT]) {
 #pragma unroll
@@ -129,30 +128,21 @@ __global__ void __launch_bounds__(kSkinnyThreads, UB == 1 ? 2 : 1) gemm_skinny_k
     };
     // two register buffers used alternately (no copies between them: a move would wait for the load it moves); weights that
     // nobody writes are on their way before the predecessor has ended
-    load_w(wc, b_lo);
     if (a.fixed) {
+        load_w(wc, b_lo);
         load_w(wn, b_lo + UB);
         pdl_wait();
         load_x(xc, b_lo);
         load_x(xn, b_lo + UB);
-        multiply(wc, xc);
-        load_w(wc, b_lo + 2 * UB); load_x(xc, b_lo + 2 * UB);
-        multiply(wn, xn);
-        if (b_lo + 2 * UB < b_hi) { load_w(wn, b_lo + 3 * UB); load_x(xn, b_lo + 3 * UB); }
-        for (int b0 = b_lo + 2 * UB; b0 < b_hi; b0 += 2 * UB) {
-            multiply(wc, xc);
-            load_w(wc, b0 + 2 * UB); load_x(xc, b0 + 2 * UB);
-            multiply(wn, xn);
-            load_w(wn, b0 + 3 * UB); load_x(xn, b0 + 3 * UB);
-        }
     } else {
-        load_x(xc, b_lo);
-        for (int b0 = b_lo; b0 < b_hi; b0 += 2 * UB) {
-            load_w(wn, b0 + UB); load_x(xn, b0 + UB);
-            multiply(wc, xc);
-            load_w(wc, b0 + 2 * UB); load_x(xc, b0 + 2 * UB);
-            multiply(wn, xn);
-        }
+        load_w(wc, b_lo); load_x(xc, b_lo);
+        load_w(wn, b_lo + UB); load_x(xn, b_lo + UB);
+    }
+    for (int b0 = b_lo; b0 < b_hi; b0 += 2 * UB) {
+        multiply(wc, xc);
+        load_w(wc, b0 + 2 * UB); load_x(xc, b0 + 2 * UB);
+        multiply(wn, xn);
+        load_w(wn, b0 + 3 * UB); load_x(xn, b0 + 3 * UB);
     }
     // accumulator layout: (row g, cols 2t, 2t+1), (row g+8, same cols) of each n-tile
 #pragma unroll
@@ -567,12 +557,19 @@ int launch_gemm_wx_skinny(const __half* W, const __half* X, const __half* bias, 
     }
     const bool wide = N >= 2048;
     const dim3 grid(ceil_div(N, wide ? 2 * kSkinnyRows : kSkinnyRows), jblocks);
-    static void (*const kernels[2][2][4])(SkinnyArgs) = {      // [K <= 512][32 weight rows per CTA][tiles of 8 activation rows]
-        {{gemm_skinny_kernel<1, 1>, gemm_skinny_kernel<2, 1>, gemm_skinny_kernel<3, 1>, gemm_skinny_kernel<4, 1>},
-         {gemm_skinny_kernel<1, 2>, gemm_skinny_kernel<2, 2>, gemm_skinny_kernel<3, 2>, gemm_skinny_kernel<4, 2>}},
-        {{gemm_skinny_kernel<1, 1, 1>, gemm_skinny_kernel<2, 1, 1>, gemm_skinny_kernel<3, 1, 1>, gemm_skinny_kernel<4, 1, 1>},
-         {gemm_skinny_kernel<1, 2, 1>, gemm_skinny_kernel<2, 2, 1>, gemm_skinny_kernel<3, 2, 1>, gemm_skinny_kernel<4, 2, 1>}}};
-    const cudaError_t rc = launch_pdl(kernels[K <= 512][wide][nt - 1], grid, dim3(kSkinnyThreads), 0, st, a);
+    // K blocks per buffer (two buffers per warp).  16 weight rows: as few as hold the warp's share of K, at most four.  32: one at
+    // K <= 512, and where a second CTA per SM has work (8192 x 2048, 1 / 20 / 32 rows: 5.1 / 7.4 / 9.0 us with two, 3.9 / 6.4 / 8.0
+    // with one), else two (4096 x 1024, 20 rows: 2.8 us, 4.0 with one).
+    static void (*const narrow[3][4])(SkinnyArgs) = {
+        {gemm_skinny_kernel<1, 1, 1>, gemm_skinny_kernel<2, 1, 1>, gemm_skinny_kernel<3, 1, 1>, gemm_skinny_kernel<4, 1, 1>},
+        {gemm_skinny_kernel<1, 1, 2>, gemm_skinny_kernel<2, 1, 2>, gemm_skinny_kernel<3, 1, 2>, gemm_skinny_kernel<4, 1, 2>},
+        {gemm_skinny_kernel<1, 1, 4>, gemm_skinny_kernel<2, 1, 4>, gemm_skinny_kernel<3, 1, 4>, gemm_skinny_kernel<4, 1, 4>}};
+    static void (*const broad[2][4])(SkinnyArgs) = {
+        {gemm_skinny_kernel<1, 2, 1>, gemm_skinny_kernel<2, 2, 1>, gemm_skinny_kernel<3, 2, 1>, gemm_skinny_kernel<4, 2, 1>},
+        {gemm_skinny_kernel<1, 2, 2>, gemm_skinny_kernel<2, 2, 2>, gemm_skinny_kernel<3, 2, 2>, gemm_skinny_kernel<4, 2, 2>}};
+    const bool one_wave = grid.x * grid.y <= kNumSmB200;
+    void (*const kernel)(SkinnyArgs) = wide ? broad[K > 512 ? one_wave || nt == 1 : one_wave && nt == 3][nt - 1] : narrow[K <= 512 ? 0 : K <= 1024 ? 1 : 2][nt - 1];
+    const cudaError_t rc = launch_pdl(kernel, grid, dim3(kSkinnyThreads), 0, st, a);
     return cuda_status(rc);
 }
 
