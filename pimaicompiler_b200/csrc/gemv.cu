@@ -18,14 +18,16 @@ namespace pimb200 {
 // first costs a barrier before the first weight load and measured slower.  R*unroll independent
 // 16-byte loads are in flight per lane.
 // =============================================================================================
+// The launch may start while its predecessor is still running: it then asks for its rows of W to be brought into L2 (which is
+// coherent, so it does not matter whether anyone still writes them) and reads everything behind the wait.
 template <int R>
-__global__ void __launch_bounds__(256) gemv_mv_vec_kernel(const __half* __restrict__ W, const __half* __restrict__ x,
-                                                          const __half* __restrict__ bias, __half* __restrict__ y,
-                                                          int N, int K, int act) {
+__global__ void __launch_bounds__(256) gemv_mv_vec_kernel(const __half* W, const __half* x, const __half* bias, __half* y, int N, int K, int act) {
+    pdl_launch_dependents();
     const int K8 = K >> 3;
-    const uint4* x4 = reinterpret_cast<const uint4*>(x);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row0 = (blockIdx.x * (blockDim.x >> 5) + warp) * R;
+    if (lane < R && row0 + lane < N) prefetch_l2(W + (size_t)(row0 + lane) * K, (uint32_t)K * 2);
+    pdl_wait();
     if (row0 >= N) return;
 
     const uint4* wrow[R];
@@ -39,9 +41,9 @@ __global__ void __launch_bounds__(256) gemv_mv_vec_kernel(const __half* __restri
 #pragma unroll 4
     for (int c = lane; c < K8; c += 32) {
         float xf[8];
-        widen8(__ldg(x4 + c), xf);
+        widen8(ld_v4(x + 8 * c), xf);
 #pragma unroll
-        for (int r = 0; r < R; ++r) acc[r] = dot8f(ldg_stream_v4(wrow[r] + c), xf, acc[r]);
+        for (int r = 0; r < R; ++r) acc[r] = dot8f(ld_stream_v4(wrow[r] + c), xf, acc[r]);
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) acc[r] = warp_sum(acc[r]);
@@ -88,10 +90,9 @@ static int launch_gemv_mv(const __half* W, const __half* x, const __half* bias, 
     const long want = (long)kNumSmB200 * 8 * 2;
     const int R = warps4 >= want ? 4 : (warps2 >= want ? 2 : 1);
     const int grid = ceil_div(N, 8 * R);
-    if (R == 4) gemv_mv_vec_kernel<4><<<grid, 256, 0, st>>>(W, x, bias, y, N, K, act);
-    else if (R == 2) gemv_mv_vec_kernel<2><<<grid, 256, 0, st>>>(W, x, bias, y, N, K, act);
-    else gemv_mv_vec_kernel<1><<<grid, 256, 0, st>>>(W, x, bias, y, N, K, act);
-    return launch_status();
+    void (*const kernel)(const __half*, const __half*, const __half*, __half*, int, int, int) =
+        R == 4 ? gemv_mv_vec_kernel<4> : R == 2 ? gemv_mv_vec_kernel<2> : gemv_mv_vec_kernel<1>;
+    return cuda_status(launch_pdl(kernel, dim3(grid), dim3(256), 0, st, W, x, bias, y, N, K, act));
 }
 
 // =============================================================================================

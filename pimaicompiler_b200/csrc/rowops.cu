@@ -474,7 +474,7 @@ __device__ __forceinline__ float ex2_(float x) {
 }
 
 template <int C>
-__global__ void __launch_bounds__(kBahdanauThreads, C == 1 ? 4 : 3) bahdanau_kernel(
+__global__ void __launch_bounds__(kBahdanauThreads, C == 8 ? 3 : 4) bahdanau_kernel(
     const __half* q, const __half* keys_proj, const __half* values,
     const long long* lengths, const __half* v, const __half* bias, __half* __restrict__ ctx,
     float* __restrict__ scores, long max_len, int H, long row_stride, long seq_stride, long ctx_stride, int copies, long copy_stride) {
@@ -930,7 +930,10 @@ extern "C" int pimb200_additive_attention_copies(const void* q, const void* keys
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (H % 8 == 0 && row_stride % 8 == 0 && seq_stride % 8 == 0 && ctx_stride % 8 == 0 && copy_stride % 8 == 0 && aligned16(keys_proj) &&
         aligned16(values) && aligned16(ctx) && ((size_t)2 * H + 8 * kBahdanauThreads + max_len) * sizeof(float) + 64 <= 48 * 1024) {
-        // CTAs per sentence: as many as keep the grid within two CTAs per SM, if the pieces of a row split evenly
+        // CTAs per sentence: as many as are resident at once, if the pieces of a row split evenly: a CTA's own chain is what takes the
+        // time (256 sentences with one CTA each took 24 us, 512 26).  Four per SM with 64 registers a thread; eight CTAs per sentence,
+        // which only few sentences have, take more registers (16 sentences: 6.2 us, 7.0 with 64).
+        // 128 sentences: 12.5 us with two, 10.6 with four; 256: 23.9 with one, 16.4 with two
         auto run = [&](auto f) {
             return f(static_cast<const __half*>(q), static_cast<const __half*>(keys_proj), static_cast<const __half*>(values), lengths,
                      static_cast<const __half*>(v), static_cast<const __half*>(bias), static_cast<__half*>(ctx), scores, n_seq, max_len, H,
@@ -938,7 +941,7 @@ extern "C" int pimb200_additive_attention_copies(const void* q, const void* keys
         };
         auto fits = [&](int c) { return (H / 8) % c == 0 && H / 8 / c <= kBahdanauThreads && kBahdanauThreads % (H / 8 / c) == 0; };
         for (int c = 8; c >= 1; c /= 2) {
-            if (!fits(c) || (c > 1 && (long)n_seq * c > 2 * kNumSmB200)) continue;
+            if (!fits(c) || (c > 1 && (long)n_seq * c > (c == 8 ? 2 : 4) * kNumSmB200)) continue;
             return c == 8 ? run(launch_bahdanau<8>) : c == 4 ? run(launch_bahdanau<4>) : c == 2 ? run(launch_bahdanau<2>) : run(launch_bahdanau<1>);
         }
     }
