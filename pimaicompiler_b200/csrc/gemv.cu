@@ -18,15 +18,17 @@ namespace pimb200 {
 // first costs a barrier before the first weight load and measured slower.  R*unroll independent
 // 16-byte loads are in flight per lane.
 // =============================================================================================
-// The launch may start while its predecessor is still running: it then asks for its rows of W to be brought into L2 (which is
+// The launch may start while its predecessor is still running: unless the matrix is large it then asks for its rows of W to be brought into L2 (which is
 // coherent, so it does not matter whether anyone still writes them) and reads everything behind the wait.
+constexpr size_t kMvAheadMax = (size_t)12 << 20;     // elements
 template <int R>
-__global__ void __launch_bounds__(256) gemv_mv_vec_kernel(const __half* W, const __half* x, const __half* bias, __half* y, int N, int K, int act) {
+__global__ void __launch_bounds__(256) gemv_mv_vec_kernel(const __half* W, const __half* x, const __half* bias, __half* y, int N, int K, int act,
+                                                          int ahead) {
     pdl_launch_dependents();
     const int K8 = K >> 3;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row0 = (blockIdx.x * (blockDim.x >> 5) + warp) * R;
-    if (lane < R && row0 + lane < N) prefetch_l2(W + (size_t)(row0 + lane) * K, (uint32_t)K * 2);
+    if (ahead && lane < R && row0 + lane < N) prefetch_l2(W + (size_t)(row0 + lane) * K, (uint32_t)K * 2);
     pdl_wait();
     if (row0 >= N) return;
 
@@ -90,9 +92,11 @@ static int launch_gemv_mv(const __half* W, const __half* x, const __half* bias, 
     const long want = (long)kNumSmB200 * 8 * 2;
     const int R = warps4 >= want ? 4 : (warps2 >= want ? 2 : 1);
     const int grid = ceil_div(N, 8 * R);
-    void (*const kernel)(const __half*, const __half*, const __half*, __half*, int, int, int) =
+    void (*const kernel)(const __half*, const __half*, const __half*, __half*, int, int, int, int) =
         R == 4 ? gemv_mv_vec_kernel<4> : R == 2 ? gemv_mv_vec_kernel<2> : gemv_mv_vec_kernel<1>;
-    return cuda_status(launch_pdl(kernel, dim3(grid), dim3(256), 0, st, W, x, bias, y, N, K, act));
+    // (larger matrices take several waves of CTAs, whose rows would be asked for twice at once: 32768 x 4096 43.7 -> 56.7 us)
+    const int ahead = (size_t)N * K <= kMvAheadMax;
+    return cuda_status(launch_pdl(kernel, dim3(grid), dim3(256), 0, st, W, x, bias, y, N, K, act, ahead));
 }
 
 // =============================================================================================
@@ -235,6 +239,100 @@ int launch_gemv_vm_with_scratch(const __half* x, const __half* A, const __half* 
     return launch_status();
 }
 
+// The same for moderate K, in one phase: the S <= 8 CTAs that share a column tile are a cluster, whose partial sums
+// meet in its first CTA's shared memory.  Through global memory (partial sums, a fence, a ticket, another trip to L2) the
+// meeting took as long as the product itself, and the shared scratch needs an event behind every call.
+template <int LPR, int S>
+__global__ void __launch_bounds__(256) gemv_vm_cluster_kernel(const __half* x, const __half* A, const __half* bias, __half* y, int K, int N, int act,
+                                                              int rows_per_split) {
+    constexpr int TILE = LPR * 8, RPW = 32 / LPR, AHEAD = 8;
+    __shared__ float red[8][TILE];
+    __shared__ float parts[S][TILE];     // of the first CTA: every CTA's sums
+    pdl_launch_dependents();
+    if (S > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int sub = lane / LPR, cl = lane % LPR;
+    const int rank = blockIdx.x % S, tile = blockIdx.x / S;
+    const int col = tile * TILE + cl * 8;
+    const int k0 = rank * rows_per_split, k1 = min(K, k0 + rows_per_split);
+    // the first rows on their way into L2 while the predecessor finishes (coherent: it does not matter who still writes them)
+    if ((cl & 7) == 0 && col < N)
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+            const int k = k0 + warp * RPW + sub + i * 8 * RPW;
+            if (k < k1) asm volatile("prefetch.global.L2 [%0];" ::"l"(A + (size_t)k * N + col));
+        }
+    pdl_wait();
+    float acc[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+    if (col < N) {
+#pragma unroll 8
+        for (int k = k0 + warp * RPW + sub; k < k1; k += 8 * RPW) {
+            const uint4 a = ld_stream_v4(A + (size_t)k * N + col);
+            const float xk = __half2float(x[k]);
+            float2 f;
+            f = h2f2(a.x); acc[0] = fmaf(xk, f.x, acc[0]); acc[1] = fmaf(xk, f.y, acc[1]);
+            f = h2f2(a.y); acc[2] = fmaf(xk, f.x, acc[2]); acc[3] = fmaf(xk, f.y, acc[3]);
+            f = h2f2(a.z); acc[4] = fmaf(xk, f.x, acc[4]); acc[5] = fmaf(xk, f.y, acc[5]);
+            f = h2f2(a.w); acc[6] = fmaf(xk, f.x, acc[6]); acc[7] = fmaf(xk, f.y, acc[7]);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o >= LPR; o >>= 1) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+    }
+    if (sub == 0) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) red[warp][cl * 8 + j] = acc[j];
+    }
+    __syncthreads();
+    const int t = threadIdx.x, ocol = tile * TILE + t;
+    float v = 0.f;
+    if (t < TILE) {
+#pragma unroll
+        for (int w = 0; w < 8; ++w) v += red[w][t];
+    }
+    if (S > 1) {
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");    // every CTA of the cluster has started
+        if (t < TILE) {
+            uint32_t at;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(&parts[rank][t])));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (rank > 0) return;
+        v = 0.f;
+        if (t < TILE) {
+#pragma unroll
+            for (int s = 0; s < S; ++s) v += parts[s][t];
+        }
+    }
+    if (t < TILE && ocol < N) {
+        v += bias ? __half2float(bias[ocol]) : 0.f;
+        if (act == PIMB200_ACT_RELU) v = fmaxf(v, 0.f);
+        y[ocol] = __float2half_rn(v);
+    }
+}
+
+// S: about four CTAs per SM, at least four passes over the rows per CTA
+template <int LPR>
+static int launch_gemv_vm_cluster(const __half* x, const __half* A, const __half* bias, __half* y, int K, int N, int act, cudaStream_t st) {
+    const int tiles = ceil_div(N, LPR * 8), passes = K / (8 * (32 / LPR));
+    int S = 1;
+    while (S < 8 && tiles * S * 2 <= 6 * kNumSmB200 && passes / (2 * S) >= 4) S *= 2;
+    const dim3 grid(tiles * S), block(256);
+    const int rows = ceil_div(K, S);
+    switch (S) {
+        case 1: return cuda_status(launch_pdl<1>(gemv_vm_cluster_kernel<LPR, 1>, grid, block, 0, st, x, A, bias, y, K, N, act, rows));
+        case 2: return cuda_status(launch_pdl<2>(gemv_vm_cluster_kernel<LPR, 2>, grid, block, 0, st, x, A, bias, y, K, N, act, rows));
+        case 4: return cuda_status(launch_pdl<4>(gemv_vm_cluster_kernel<LPR, 4>, grid, block, 0, st, x, A, bias, y, K, N, act, rows));
+        default: return cuda_status(launch_pdl<8>(gemv_vm_cluster_kernel<LPR, 8>, grid, block, 0, st, x, A, bias, y, K, N, act, rows));
+    }
+}
+
 static std::mutex g_vm_mutex;
 static cudaStream_t g_vm_last_stream[64];
 static bool g_vm_used[64];
@@ -275,13 +373,18 @@ static int launch_gemv_vm(const __half* x, const __half* A, const __half* bias, 
         gemv_vm_generic_kernel<<<ceil_div(N, 32), 256, 0, st>>>(x, A, bias, y, K, N, act);
         return launch_status();
     }
+    DeviceCtx* ctx = allow_split ? current_ctx() : nullptr;
+    if (allow_split && !ctx) return PIMB200_ERR_NOT_INIT;
+    // one phase up to K = 4096, and up to 8192 where eight CTAs per tile fill the SMs twice (1024 columns: 12.1 us, 10.5 with the split
+    // through memory; 4096 columns: 15.2, 22.6)
+    const bool wide = ceil_div(N, 256) >= kNumSmB200 / 4;
+    if (K <= 4096 || (K <= 8192 && ceil_div(N, wide ? 256 : 64) * 8 >= 2 * kNumSmB200))
+        return wide ? launch_gemv_vm_cluster<32>(x, A, bias, y, K, N, act, st) : launch_gemv_vm_cluster<8>(x, A, bias, y, K, N, act, st);
     float* partials = nullptr;
     unsigned int* tickets = nullptr;
     VmPlan p;
     int dev = -1;
     if (allow_split) {
-        DeviceCtx* ctx = current_ctx();
-        if (!ctx) return PIMB200_ERR_NOT_INIT;
         p = plan_gemv_vm(K, N, kSplitKMaxFloats, kSplitKMaxTiles);
         if (p.splits > 1) {
             PIMB200_CUDA_TRY(cudaGetDevice(&dev));
