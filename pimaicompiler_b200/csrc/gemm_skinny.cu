@@ -183,6 +183,7 @@ __global__ void __launch_bounds__(kSkinnyThreads) lstm_cell_skinny_kernel(const 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int n0 = blockIdx.x * ROWS;                              // 4H is a multiple of 32
+    const int j_base = blockIdx.y * kSkinnyMaxJ, J = min(a.J - j_base, kSkinnyMaxJ);   // this CTA's sequences
     const int bx = a.I >> 5, blocks = bx + (a.h0 ? a.H >> 5 : 0);  // 32-wide K blocks of both products
     const int per = (blocks + KS - 1) / KS;
     const int b_lo = min(blocks, warp * per), b_hi = min(blocks, b_lo + per);
@@ -215,7 +216,7 @@ __global__ void __launch_bounds__(kSkinnyThreads) lstm_cell_skinny_kernel(const 
             const bool in = b < b_hi, first = b < bx;
 #pragma unroll
             for (int j = 0; j < NT; ++j) {
-                const int row = min(j * 8 + g, a.J - 1);           // rows past J repeat the last one
+                const int row = j_base + min(j * 8 + g, J - 1);    // rows past J repeat the last one
                 const __half* p = first ? a.x + (size_t)row * a.x_ld + b * 32 : a.h0 + (size_t)row * a.H + (b - bx) * 32;
                 x[u][j] = in ? ld_v4(p + 8 * t) : zero;
             }
@@ -233,7 +234,8 @@ __global__ void __launch_bounds__(kSkinnyThreads) lstm_cell_skinny_kernel(const 
                 }
     };
     // the CTA's rows of both matrices, 128 to 256 KB, on their way into L2 while the predecessor finishes
-    if (threadIdx.x < 32) prefetch_l2(a.Wx + (size_t)(n0 + lane) * a.I, (uint32_t)a.I * 2);
+    if (blockIdx.y > 0) {
+    } else if (threadIdx.x < 32) prefetch_l2(a.Wx + (size_t)(n0 + lane) * a.I, (uint32_t)a.I * 2);
     else if (threadIdx.x < 64 && a.h0) prefetch_l2(a.Wh + (size_t)(n0 + lane) * a.H, (uint32_t)a.H * 2);
     load_w(wc, b_lo);
     pdl_wait();
@@ -252,19 +254,20 @@ __global__ void __launch_bounds__(kSkinnyThreads) lstm_cell_skinny_kernel(const 
             for (int e = 0; e < 4; ++e) part[warp][m * 16 + g + (e >> 1) * 8][j * 8 + 2 * t + (e & 1)] = acc[m][j][e];
     __syncthreads();
     const int ul = threadIdx.x & 7, u = (n0 >> 2) + ul;            // a thread per (sequence, unit)
-    for (int j = threadIdx.x >> 3; j < a.J; j += kSkinnyThreads / 8) {
+    for (int j = threadIdx.x >> 3; j < J; j += kSkinnyThreads / 8) {
+        const size_t row = j_base + j;
         const float4 b4 = *reinterpret_cast<const float4*>(a.bias + (size_t)u * 4);
         float z[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int w = 0; w < KS; ++w)
 #pragma unroll
             for (int q = 0; q < 4; ++q) z[q] += part[w][ul * 4 + q][j];
-        const float cprev = a.c0 ? __half2float(a.c0[(size_t)j * a.H + u]) : 0.f;
+        const float cprev = a.c0 ? __half2float(a.c0[row * a.H + u]) : 0.f;
         const float cnew = sigmoidf_(z[1] + b4.y) * cprev + sigmoidf_(z[0] + b4.x) * tanhf_(z[2] + b4.z);
         const __half hh = __float2half_rn(sigmoidf_(z[3] + b4.w) * tanhf_(cnew));
-        a.y[(size_t)j * a.y_ld + u] = a.res ? __float2half_rn(__half2float(hh) + __half2float(a.res[(size_t)j * a.res_ld + u])) : hh;
-        if (a.hn) a.hn[(size_t)j * a.H + u] = hh;
-        if (a.cn) a.cn[(size_t)j * a.H + u] = __float2half_rn(cnew);
+        a.y[row * a.y_ld + u] = a.res ? __float2half_rn(__half2float(hh) + __half2float(a.res[row * a.res_ld + u])) : hh;
+        if (a.hn) a.hn[row * a.H + u] = hh;
+        if (a.cn) a.cn[row * a.H + u] = __float2half_rn(cnew);
     }
 }
 
@@ -574,10 +577,10 @@ int launch_gemm_wx_skinny(const __half* W, const __half* X, const __half* bias, 
 }
 
 int launch_lstm_cell_skinny(const RowsCell& c, cudaStream_t st) {
-    if (c.J < 1 || c.J > kSkinnyMaxJ || c.I % 32 != 0 || c.H % 32 != 0 || c.x_ld % 8 != 0 || !aligned16(c.x) || (c.h0 && !aligned16(c.h0)))
+    if (c.J < 1 || c.J > 65535 * kSkinnyMaxJ || c.I % 32 != 0 || c.H % 32 != 0 || c.x_ld % 8 != 0 || !aligned16(c.x) || (c.h0 && !aligned16(c.h0)))
         return PIMB200_ERR_UNSUPPORTED;
-    const dim3 grid(4 * c.H / (2 * kSkinnyRows)), block(kSkinnyThreads);
-    switch (ceil_div(c.J, 8)) {
+    const dim3 grid(4 * c.H / (2 * kSkinnyRows), ceil_div(c.J, kSkinnyMaxJ)), block(kSkinnyThreads);
+    switch (grid.y > 1 ? 4 : ceil_div(c.J, 8)) {
         case 1: return cuda_status(launch_pdl(lstm_cell_skinny_kernel<1>, grid, block, 0, st, c));
         case 2: return cuda_status(launch_pdl(lstm_cell_skinny_kernel<2>, grid, block, 0, st, c));
         case 3: return cuda_status(launch_pdl(lstm_cell_skinny_kernel<3>, grid, block, 0, st, c));

@@ -313,7 +313,15 @@ static int launch_cell(const RowsCell& c, cudaStream_t st) {
     for (const auto& o : outs)
         if (rows_overlap(c.x, c.x_ld, c.I, o.p, o.ld, c.H, c.J) || rows_overlap(c.h0, c.H, c.H, o.p, o.ld, c.H, c.J))
             return PIMB200_ERR_UNSUPPORTED;
-    return c.J < kCellRowsMinB ? launch_lstm_cell_skinny(c, st) : launch_gemm_rows_cell(c, st);
+    // few rows, or few enough that the blocks of 32 of them are one wave of CTAs: the tensor-core kernel's tiles of 64 gate rows would
+    // leave most SMs idle (H = 320, 2048 inputs, 33..96 sequences: 10.5..10.9 us, 8.6..8.9 in blocks; H = 512, 33..64: 11.1, 9.0).
+    // In more than one wave the blocks lose (H = 1024, 33 sequences: 13.0, 17.9 in blocks)
+    const long blocks = (long)ceil_div(4 * c.H, 32) * ceil_div(c.J, 32);
+    if (c.J < kCellRowsMinB || blocks <= kNumSmB200) {
+        const int rc = launch_lstm_cell_skinny(c, st);
+        if (rc != PIMB200_ERR_UNSUPPORTED || c.J < kCellRowsMinB) return rc;
+    }
+    return launch_gemm_rows_cell(c, st);
 }
 struct CellPointArgs {
     const float* Gx;     // [B, 4H]  W_ih x, packed gate order (unit-major)

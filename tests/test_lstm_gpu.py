@@ -470,7 +470,7 @@ def test_lstm_packed_sequences_on_the_lockstep_kernels_vs_libtorch(B, I, H, L, b
     assert_close(cn, cns, LSTM_ATOL, LSTM_RTOL, "lock-step vs streamed c_n")
 
 
-@pytest.mark.parametrize("B,I,H", [(8, 64, 32), (33, 256, 128), (128, 2048, 1024)])
+@pytest.mark.parametrize("B,I,H", [(8, 64, 32), (33, 256, 128), (128, 2048, 1024), (96, 512, 320), (97, 96, 320), (64, 2048, 512), (65, 240, 64)])
 def test_lstm_decode_step_with_strided_rows_and_residual(B, I, H):
     # the decode step that writes into one half of the next cell's concatenated input: equal to forward() with T = 1 bit
     # for bit, and to the fp16 add of a residual row
