@@ -68,7 +68,7 @@ struct Args {
     int j_tiles, n_tiles;     // tiles along the activation rows (of one CTA or a pair) and along the weight rows
     void* Y;
     long ldy;
-    int direct;               // 1: the outputs are stored element by element
+    int direct;               // 1: the outputs are stored by the warps, row by row; 2: and rows start at multiples of 4 bytes
     int fixed;                // 1: no work ahead on the stream writes the weights (they may be read before that work has ended)
     int x_batch;              // > 0: rows are numbered time-major over batch-first sequences (map x is 3-D: K, b, t)
     int* status;
@@ -294,19 +294,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
 #pragma unroll
                         for (int i = 0; i < CH; ++i) f[i] += (n0 + c + i < n_end) ? __half2float(a.bias[n0 + c + i]) : 0.f;
                     }
-                    if (a.direct) {                                    // rows of Y that no tensor map takes
-                        if (row_ok) {
-#pragma unroll
-                            for (int i = 0; i < CH; ++i) {
-                                if (n0 + c + i >= n_end) break;
-                                const size_t at = (size_t)j * a.ldy + n0 + c + i;
-                                if (EPI == kRowsHalf) static_cast<__half*>(a.Y)[at] = __float2half_rn(max_nan(f[i], lo));
-                                else static_cast<float*>(a.Y)[at] = max_nan(f[i], lo);
-                            }
-                        }
-                        __syncwarp();
-                        continue;
-                    }
                     uint4 o[8];
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
@@ -318,6 +305,38 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
                             o[i] = make_uint4(__float_as_uint(max_nan(f[4 * i], lo)), __float_as_uint(max_nan(f[4 * i + 1], lo)),
                                               __float_as_uint(max_nan(f[4 * i + 2], lo)), __float_as_uint(max_nan(f[4 * i + 3], lo)));
                         }
+                    }
+                    if (a.direct) {
+                        // rows of Y that no tensor map takes: through shared memory too, but stored by the warp, a row at a time (a
+                        // thread's own stores touch 32 rows at once: 656 rows of 8823 x 128 took 75 us)
+                        unsigned char* buf = stg + (chunks & 1) * CHUNK_BYTES;
+                        uint4* row = reinterpret_cast<uint4*>(buf + lane * 128);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) row[i ^ (lane & 7)] = o[i];
+                        __syncwarp();
+                        const int cols = min(CH, n_end - n0 - c), first_row = j0 + q * 32, rows = min(min(32, rows_left), a.J - first_row);
+#pragma unroll 4
+                        for (int rr = 0; rr < rows; ++rr) {
+                            const unsigned char* src = buf + rr * 128;
+                            const size_t at = (size_t)(first_row + rr) * a.ldy + n0 + c;
+                            // 4 bytes per lane: piece lane / 4 of the row, which lies at (lane / 4) ^ (rr & 7)
+                            const uint32_t w = *reinterpret_cast<const uint32_t*>(src + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
+                            if (EPI == kRowsFloat) {
+                                if (lane < cols) static_cast<float*>(a.Y)[at + lane] = __uint_as_float(w);
+                            } else if (a.direct == 2) {                // every row starts at a multiple of 4 bytes
+                                __half* y = static_cast<__half*>(a.Y) + at + 2 * lane;
+                                if (2 * lane + 1 < cols) *reinterpret_cast<uint32_t*>(y) = w;
+                                else if (2 * lane < cols) *reinterpret_cast<uint16_t*>(y) = (uint16_t)w;
+                            } else {
+                                // 2-byte stores of neighbours: lane l takes elements l and 32 + l
+                                const uint32_t lo = __shfl_sync(0xffffffffu, w, lane >> 1), hi = __shfl_sync(0xffffffffu, w, 16 + (lane >> 1));
+                                uint16_t* y = reinterpret_cast<uint16_t*>(static_cast<__half*>(a.Y) + at);
+                                if (lane < cols) y[lane] = (uint16_t)(lane & 1 ? lo >> 16 : lo);
+                                if (32 + lane < cols) y[32 + lane] = (uint16_t)(lane & 1 ? hi >> 16 : hi);
+                            }
+                        }
+                        ++chunks;
+                        continue;
                     }
                     if (n0 + c + CH > n_end && n_end < a.N) {          // half a chunk left of this tile: the map's boxes are whole ones
                         if (row_ok) {
@@ -551,6 +570,7 @@ int launch_gemm_rows(const __half* W, const __half* X, const __half* bias, void*
     const int es = y_is_f32 ? 4 : 2, tail = a.jrows % 32, whole = a.jrows < 32 ? a.jrows : 32;
     a.Y = Y; a.ldy = ldy;
     a.direct = !aligned16(Y) || (long)ldy * es % 16 != 0;
+    if (a.direct && ((long)ldy * es | (long)(reinterpret_cast<uintptr_t>(Y))) % 4 == 0) a.direct = 2;
     if (a.direct) m.y = m.x;   // (prefetched only)
     else if (!encode_2d(&m.y, Y, J, N, (uint64_t)ldy * es, whole, es) ||
         (tail && !encode_2d(&m.y_tail, Y, J, N, (uint64_t)ldy * es, tail, es)))

@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(kGreedyThreads, 1) rnnt_greedy_kernel(GreedyAr
     };
 
     for (int utt = cluster_id; utt < a.n_utts; utt += n_clusters) {
-        const float* E = a.E + utt * a.e_utt;
+        const float* E = a.E + utt * a.e_utt;      // the next frame's (a running address)
         int* tokens = a.tokens + (size_t)utt * a.Tp;
         float* logits = a.logits ? a.logits + (size_t)utt * a.Tp * V : nullptr;
         for (int i = tid; i < 2 * PH; i += nthr) {
@@ -393,6 +393,7 @@ __global__ void __launch_bounds__(kGreedyThreads, 1) rnnt_greedy_kernel(GreedyAr
         if (a.Tp > 0) {
             if (tid < JH) e_next[0] = __ldcg(E + tid);
             if (tid + nthr < JH) e_next[1] = __ldcg(E + tid + nthr);
+            E += a.e_frame;
         }
         // iteration -1 is the start of sequence: the blank row of the embedding, zero state (one inlined copy of the
         // evaluation serves both: the loop body is the kernel's instruction footprint)
@@ -404,8 +405,9 @@ __global__ void __launch_bounds__(kGreedyThreads, 1) rnnt_greedy_kernel(GreedyAr
                 if (trp && tid == 0) trp[0] = clock64();
                 const float e_cur0 = e_next[0], e_cur1 = e_next[1];
                 if (t + 1 < a.Tp) {
-                    if (tid < JH) e_next[0] = __ldcg(E + (t + 1) * a.e_frame + tid);
-                    if (tid + nthr < JH) e_next[1] = __ldcg(E + (t + 1) * a.e_frame + tid + nthr);
+                    if (tid < JH) e_next[0] = __ldcg(E + tid);
+                    if (tid + nthr < JH) e_next[1] = __ldcg(E + tid + nthr);
+                    E += a.e_frame;
                 }
                 if (tid < JH) zs[tid] = __float2half_rn(fmaxf(e_cur0 + Pj[tid], 0.f));
                 if (tid + nthr < JH) zs[tid + nthr] = __float2half_rn(fmaxf(e_cur1 + Pj[tid + nthr], 0.f));
