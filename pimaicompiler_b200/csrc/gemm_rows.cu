@@ -108,6 +108,31 @@ __device__ __forceinline__ void store_half16(__half* p, const uint32_t* w) {
     q[1] = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
+// Rows of a warp's staged chunk (128 bytes each, 16-byte pieces swapped by row) to rows of Y that start at `at`, `ldy` elements apart.
+// pairs: every row starts at a multiple of 4 bytes.  Not inlined: the kernel's loop has no registers for it
+template <bool F32>
+__device__ __noinline__ void store_rows(const unsigned char* buf, void* Y, size_t at, long ldy, int rows, int cols, bool pairs) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 4
+    for (int rr = 0; rr < rows; ++rr, at += ldy) {
+        // 4 bytes per lane: piece lane / 4 of the row, which lies at (lane / 4) ^ (rr & 7)
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(buf + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
+        if (F32) {
+            if (lane < cols) static_cast<float*>(Y)[at + lane] = __uint_as_float(w);
+        } else if (pairs) {
+            __half* y = static_cast<__half*>(Y) + at + 2 * lane;
+            if (2 * lane + 1 < cols) *reinterpret_cast<uint32_t*>(y) = w;
+            else if (2 * lane < cols) *reinterpret_cast<uint16_t*>(y) = (uint16_t)w;
+        } else {
+            // 2-byte stores of neighbours: lane l takes elements l and 32 + l
+            const uint32_t lo = __shfl_sync(0xffffffffu, w, lane >> 1), hi = __shfl_sync(0xffffffffu, w, 16 + (lane >> 1));
+            uint16_t* y = static_cast<uint16_t*>(Y) + at;
+            if (lane < cols) y[lane] = (uint16_t)(lane & 1 ? lo >> 16 : lo);
+            if (32 + lane < cols) y[32 + lane] = (uint16_t)(lane & 1 ? hi >> 16 : hi);
+        }
+    }
+}
+
 }  // namespace
 
 template <int BN, int EPI, int CG>
@@ -315,26 +340,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_kernel(const __grid_cons
                         for (int i = 0; i < 8; ++i) row[i ^ (lane & 7)] = o[i];
                         __syncwarp();
                         const int cols = min(CH, n_end - n0 - c), first_row = j0 + q * 32, rows = min(min(32, rows_left), a.J - first_row);
-#pragma unroll 4
-                        for (int rr = 0; rr < rows; ++rr) {
-                            const unsigned char* src = buf + rr * 128;
-                            const size_t at = (size_t)(first_row + rr) * a.ldy + n0 + c;
-                            // 4 bytes per lane: piece lane / 4 of the row, which lies at (lane / 4) ^ (rr & 7)
-                            const uint32_t w = *reinterpret_cast<const uint32_t*>(src + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
-                            if (EPI == kRowsFloat) {
-                                if (lane < cols) static_cast<float*>(a.Y)[at + lane] = __uint_as_float(w);
-                            } else if (a.direct == 2) {                // every row starts at a multiple of 4 bytes
-                                __half* y = static_cast<__half*>(a.Y) + at + 2 * lane;
-                                if (2 * lane + 1 < cols) *reinterpret_cast<uint32_t*>(y) = w;
-                                else if (2 * lane < cols) *reinterpret_cast<uint16_t*>(y) = (uint16_t)w;
-                            } else {
-                                // 2-byte stores of neighbours: lane l takes elements l and 32 + l
-                                const uint32_t lo = __shfl_sync(0xffffffffu, w, lane >> 1), hi = __shfl_sync(0xffffffffu, w, 16 + (lane >> 1));
-                                uint16_t* y = reinterpret_cast<uint16_t*>(static_cast<__half*>(a.Y) + at);
-                                if (lane < cols) y[lane] = (uint16_t)(lane & 1 ? lo >> 16 : lo);
-                                if (32 + lane < cols) y[32 + lane] = (uint16_t)(lane & 1 ? hi >> 16 : hi);
-                            }
-                        }
+                        store_rows<EPI == kRowsFloat>(buf, a.Y, (size_t)first_row * a.ldy + n0 + c, a.ldy, rows, cols, a.direct == 2);
                         ++chunks;
                         continue;
                     }

@@ -10,6 +10,8 @@
 
 namespace pimb200 {
 
+int launch_gemm_wx_ragged(const __half* W, const __half* X, const __half* bias, void* Y, int N, int K, int J, int ldx, int ldy, int act,
+                          int y_is_f32, cudaStream_t st);
 int launch_gemm_wx_simt(const __half* W, const __half* X, const __half* bias, void* Y, int N, int K, int J, int ldx,
                         int ldy, int act, int y_is_f32, cudaStream_t st);
 
@@ -108,7 +110,7 @@ int launch_gemm_wx_skinny(const __half* W, const __half* X, const __half* bias, 
                           int ldy, int act, int y_is_f32, cudaStream_t st, int fixed);
 
 // Router of the dense contraction: up to 32 activation rows stream W on every SM (HBM-bound, like the GEMV); more rows
-// go to the tcgen05 kernel; shapes neither takes (unaligned operands, K not a multiple of 8) to the SIMT kernel.  `fixed`: no
+// go to the tcgen05 kernel; shapes neither takes (unaligned operands, K not a multiple of 8) to the ragged kernel.  `fixed`: no
 // work ahead on the stream writes W, so it may be read before that work has ended.
 int launch_gemm_wx(const __half* W, const __half* X, const __half* bias, void* Y, int N, int K, int J, int ldx,
                    int ldy, int act, int y_is_f32, cudaStream_t st, int fixed) {
@@ -117,6 +119,7 @@ int launch_gemm_wx(const __half* W, const __half* X, const __half* bias, void* Y
         if (rs != PIMB200_ERR_UNSUPPORTED) return rs;
         const int rc = launch_gemm_rows(W, X, bias, Y, N, K, J, ldx, ldy, act, y_is_f32, 0, 0, st, fixed);
         if (rc != PIMB200_ERR_UNSUPPORTED) return rc;
+        return launch_gemm_wx_ragged(W, X, bias, Y, N, K, J, ldx, ldy, act, y_is_f32, st);
     }
     return launch_gemm_wx_simt(W, X, bias, Y, N, K, J, ldx, ldy, act, y_is_f32, st);
 }

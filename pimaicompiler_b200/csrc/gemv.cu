@@ -490,9 +490,8 @@ static int launch_copy_2d(void* dst, size_t dpitch, const void* src, size_t spit
 }
 
 // =============================================================================================
-// SIMT GEMM fall-back:  Y[j,n] = act(sum_k X[j,k] W[n,k] + b[n]) — any shape, any alignment.
-// 64x64 output tile, 32-deep k slab, 256 threads with a 4x4 register tile each.
-// The tensor-core kernel in gemm_tc.cu takes the shapes it supports; this one takes the rest.
+// SIMT GEMM:  Y[j,n] = act(sum_k X[j,k] W[n,k] + b[n]) — any shape, any alignment, exact fp32 products and sums.
+// 64x64 output tile, 32-deep k slab, 256 threads with a 4x4 register tile each.  The A/B switch of the tensor-core kernels.
 // =============================================================================================
 template <bool OUT_F32>
 __global__ void __launch_bounds__(256) gemm_wx_simt_kernel(const __half* __restrict__ W, const __half* __restrict__ X,
@@ -558,6 +557,108 @@ int launch_gemm_wx_simt(const __half* W, const __half* X, const __half* bias, vo
         gemm_wx_simt_kernel<true><<<grid, 256, 0, st>>>(W, X, bias, Y, N, K, J, ldx, ldy, act);
     else
         gemm_wx_simt_kernel<false><<<grid, 256, 0, st>>>(W, X, bias, Y, N, K, J, ldx, ldy, act);
+    return launch_status();
+}
+
+// =============================================================================================
+// Ragged dense contraction: any shape, any alignment (K not a multiple of 8, rows off 16-byte boundaries), where neither TMA
+// nor 16-byte loads apply.  64 x 64 tiles by mma.sync, 64-deep slabs read with 2-byte loads along the rows (64 bytes per warp
+// and load), the next slab's loads in flight during this one's products.  The SIMT kernel above took 72 us for 517 rows of
+// 1280 x 761: eight strided 2-byte loads per thread and slab, nothing in flight meanwhile, and FMAs.
+// =============================================================================================
+template <bool OUT_F32>
+__global__ void __launch_bounds__(256) gemm_wx_ragged_kernel(const __half* __restrict__ W, const __half* __restrict__ X,
+                                                             const __half* __restrict__ bias, void* __restrict__ Yv, int N, int K,
+                                                             int J, int ldx, int ldy, int act) {
+    constexpr int T = 64, BK = 64, P = BK + 8;         // pitch of 144 bytes: ldmatrix rows fall in distinct banks
+    __shared__ __align__(16) __half ws[2][T][P], xs[2][T][P];
+    const int n0 = blockIdx.x * T, j0 = blockIdx.y * T;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int wn = warp & 3, wj = warp >> 2;           // this warp's 16 weight rows and 32 activation rows
+    const unsigned short* Wu = reinterpret_cast<const unsigned short*>(W);
+    const unsigned short* Xu = reinterpret_cast<const unsigned short*>(X);
+    uint32_t wv[8], xv[8];                             // rows 8 * warp + i of both tiles, columns lane and lane + 32 of the slab
+    auto load = [&](int kb) {
+        const int k = kb + lane;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int n = n0 + 8 * warp + i, j = j0 + 8 * warp + i;
+            const size_t wr = (size_t)n * K + k, xr = (size_t)j * ldx + k;
+            uint32_t w0 = 0, w1 = 0, x0 = 0, x1 = 0;
+            if (n < N && k < K) w0 = __ldg(Wu + wr);
+            if (n < N && k + 32 < K) w1 = __ldg(Wu + wr + 32);
+            if (j < J && k < K) x0 = __ldg(Xu + xr);
+            if (j < J && k + 32 < K) x1 = __ldg(Xu + xr + 32);
+            wv[i] = w0 | w1 << 16;
+            xv[i] = x0 | x1 << 16;
+        }
+    };
+    auto store = [&](int b) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            unsigned short* w = reinterpret_cast<unsigned short*>(ws[b][8 * warp + i]) + lane;
+            unsigned short* x = reinterpret_cast<unsigned short*>(xs[b][8 * warp + i]) + lane;
+            w[0] = (unsigned short)wv[i];
+            w[32] = (unsigned short)(wv[i] >> 16);
+            x[0] = (unsigned short)xv[i];
+            x[32] = (unsigned short)(xv[i] >> 16);
+        }
+    };
+    auto ldm = [](uint32_t (&r)[4], const __half* p) {
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"((uint32_t)__cvta_generic_to_shared(p))
+                     : "memory");
+    };
+    float acc[4][4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
+    load(0);
+    store(0);
+    __syncthreads();
+    int b = 0;
+    for (int kb = 0; kb < K; kb += BK, b ^= 1) {
+        if (kb + BK < K) load(kb + BK);
+        float slab[4][4];              // summed apart and added in fp32: the tensor unit's own sums are cut off, not rounded
+#pragma unroll
+        for (int t = 0; t < 4; ++t) slab[t][0] = slab[t][1] = slab[t][2] = slab[t][3] = 0.f;
+#pragma unroll
+        for (int k = 0; k < BK; k += 16) {
+            uint32_t a[4], x[2][4];
+            ldm(a, &ws[b][wn * 16 + (lane & 7) + (lane >> 3 & 1) * 8][k + (lane >> 4) * 8]);
+#pragma unroll
+            for (int p = 0; p < 2; ++p) ldm(x[p], &xs[b][wj * 32 + p * 16 + (lane & 7) + (lane >> 4) * 8][k + (lane >> 3 & 1) * 8]);
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                             : "+f"(slab[t][0]), "+f"(slab[t][1]), "+f"(slab[t][2]), "+f"(slab[t][3])
+                             : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(x[t >> 1][2 * (t & 1)]), "r"(x[t >> 1][2 * (t & 1) + 1]));
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[t][e] += slab[t][e];
+        if (kb + BK < K) store(b ^ 1);                 // (everyone read that buffer before the last barrier)
+        __syncthreads();
+    }
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int n = n0 + wn * 16 + (lane >> 2) + (e >> 1) * 8, j = j0 + wj * 32 + t * 8 + 2 * (lane & 3) + (e & 1);
+            if (n >= N || j >= J) continue;
+            float v = acc[t][e] + (bias ? __half2float(bias[n]) : 0.f);
+            if (act == PIMB200_ACT_RELU) v = fmaxf(v, 0.f);
+            if (OUT_F32) static_cast<float*>(Yv)[(size_t)j * ldy + n] = v;
+            else static_cast<__half*>(Yv)[(size_t)j * ldy + n] = __float2half_rn(v);
+        }
+}
+
+int launch_gemm_wx_ragged(const __half* W, const __half* X, const __half* bias, void* Y, int N, int K, int J, int ldx, int ldy, int act,
+                          int y_is_f32, cudaStream_t st) {
+    const dim3 grid(ceil_div(N, 64), ceil_div(J, 64));
+    if (y_is_f32) gemm_wx_ragged_kernel<true><<<grid, 256, 0, st>>>(W, X, bias, Y, N, K, J, ldx, ldy, act);
+    else gemm_wx_ragged_kernel<false><<<grid, 256, 0, st>>>(W, X, bias, Y, N, K, J, ldx, ldy, act);
     return launch_status();
 }
 

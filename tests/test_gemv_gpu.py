@@ -185,6 +185,26 @@ def test_gemm_row_tiles(N, K, J, f32):
     assert _lib.lib().pimb200_gemm_last_status() == 0
 
 
+@pytest.mark.parametrize("N,K,J", [(1, 1, 2), (63, 9, 3), (64, 63, 64), (65, 65, 65), (129, 127, 2), (1280, 761, 130), (333, 2047, 40), (70, 130, 300)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_ragged_gemm(N, K, J, shift):
+    # shapes and alignments that neither TMA nor 16-byte loads take: edges of the 64 x 64 tiles and of the 64-deep slabs, and
+    # operands that start at an odd element inside wider rows
+    ops = _ops()
+    W, b, X = _c2_inputs(N, K, J, seed=N + K + J)
+    wide = torch.zeros(J, K + 2 + shift, dtype=torch.float16, device="cuda")
+    wide[:, shift:K + shift] = X.cuda()
+    Wd = torch.zeros(N * K + shift, dtype=torch.float16, device="cuda")[shift:].view(N, K)
+    Wd.copy_(W)
+    ref = X.double() @ W.double().T + b.double()
+    out = torch.full((J, N + 3), 7.0, dtype=torch.float32, device="cuda")
+    got = ops.gemm_wx(Wd, wide[:, shift:K + shift], to_dev(b), ops.ACT_NONE, out=out[:, :N])
+    assert_close(got, ref.numpy(), 1e-3, 1e-4, f"ragged gemm f32 {N}x{K}x{J}")
+    assert bool((out[:, N:] == 7.0).all())
+    got = ops.gemm_wx(Wd, wide[:, shift:K + shift], None, ops.ACT_RELU)
+    assert_close(got, np.maximum((X.double() @ W.double().T).numpy(), 0), GEMV_ATOL, GEMV_RTOL, f"ragged gemm f16 {N}x{K}x{J}")
+
+
 @pytest.mark.parametrize("N,K,J", [(4096, 240, 200), (512, 1024, 500), (4096, 2048, 130), (130, 72, 17), (128, 64, 16),
                                    (256, 8, 3), (1280, 320, 29)])
 def test_dense_gemm_tensor_core_and_simt_agree_with_oracle(N, K, J):
