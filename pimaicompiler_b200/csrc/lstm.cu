@@ -2478,9 +2478,13 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
 //     0 and 1, the cell state stays frozen, so the kernel's c_n is the state after the sequence's own last step;
 //     h_n is the output row of that step, picked up when the outputs are stored.
 // ---------------------------------------------------------------------------------------------
-constexpr int kBatchMinB = 129;              // fewer sequences: the kernels above
 constexpr long kBatchChunkRows = 131072;     // rows of gate terms per chunk (2 GB at H = 1024)
-constexpr int kBatchMinBothB = 33;           // two directions, which lstm_batch.cu walks in one launch
+// Sequences from which lstm_batch.cu takes the recurrence (fewer: the kernels above).  Its step is one chain, nearly as long for 17
+// sequences as for 256, and shorter for smaller matrices, of which more lies in tensor memory; the pipelined kernel's grows with
+// the groups of 16 that it walks.  100 steps with their projection, us, pipelined / batched: H = 256 at 64 sequences 345 / 328, 65:
+// 383 / 328; H = 512 at 64: 370 / 394, 65: 402 / 396, 128: 536 / 412; H = 768 at 96: 431 / 477, 112: 557 / 531; H = 1024 at 128:
+// 469 / 611.  Two directions share one launch of it (H = 1024, 33: 660 / 586; 24: 597 for both by the kernels above)
+static int batch_min(int H, int dirs) { return dirs == 2 ? 33 : H <= 512 ? 65 : H <= 768 ? 112 : kPipeMaxB + 1; }
 constexpr long kBatchMaxPackedRows = 4 * kBatchChunkRows;
 struct PackedMeta {
     const int* lens;       // [B] device
@@ -2552,7 +2556,7 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
 
 // the recurrence of lstm_batch.cu for a packed batch: more sequences than the kernels above take, or two directions at once
 static bool batch_fits_packed(const pimb200_lstm* h, int T, int B) {
-    return B >= (h->D == 2 ? kBatchMinBothB : kBatchMinB) && T >= 8 && h->bulk_wide == 2 && !h->use_tc &&
+    return B >= batch_min(h->H, h->D) && T >= 8 && h->bulk_wide == 2 && !h->use_tc &&
            (h->variant == PIMB200_LSTM_AUTO || h->variant == PIMB200_LSTM_PERSISTENT) && (long)T * B * h->D <= kBatchMaxPackedRows &&
            lstm_batch_capacity(h->H, h->D) >= B;
 }
@@ -2691,7 +2695,7 @@ __global__ void lstm_time_major_kernel(const __half* __restrict__ src, long t_ro
 struct RowStrides { long t, b; };
 
 static bool batch_fits(const pimb200_lstm* h, int T, int B) {
-    return B >= (h->D == 2 ? kBatchMinBothB : kBatchMinB) && T >= 8 && h->bulk_wide == 2 && !h->use_tc &&
+    return B >= batch_min(h->H, h->D) && T >= 8 && h->bulk_wide == 2 && !h->use_tc &&
            (h->variant == PIMB200_LSTM_AUTO || h->variant == PIMB200_LSTM_PERSISTENT) && lstm_batch_capacity(h->H, h->D) > 0;
 }
 
