@@ -5,7 +5,7 @@ features, batch 1 per stream, random-init weights of the benchmark architecture)
     python bench.py [--gpus N] [--steps K] [--warmup W] [--streams-total S] [--impl reference]
 
 One "step" = the benchmark configuration's 1024 utterance streams, sharded over the N ranks (1024 / N per rank,
-decoded in one call per rank: encoder groups of 128 utterances, one greedy launch).  Utterances are independent, so ranks share nothing on the data path
+decoded in one call per rank: all of them in lock step, one greedy launch).  Utterances are independent, so ranks share nothing on the data path
 ("strong" scaling: the total is fixed; no collective); torch.distributed is used only for the barrier and the
 max-over-ranks of the device time.  The same line carries the stand-alone LSTM (C1) and GEMV (C2) figures of the
 baseline metric under the keys `lstm_c1` and `gemv`.  Prints ONE JSON line on rank 0.
@@ -44,7 +44,19 @@ def base_config(streams_total: int) -> dict:
                   "features + activations) also exceeds the 126 MB L2"}
 
 
-RECURRENCE_KERNEL = "lstm_persistent_pipe_kernel<16,2,4> (W_hh recurrence, all T steps of 128 sequences per launch)"
+ENCODER_MAX = 1024      # utterances that the encoder advances in lock step on one GPU (128 where a call has no more)
+
+
+def recurrence_kernel(eb: int) -> str:
+    return ("lstm_batch_kernel (W_hh recurrence of up to 1024 sequences on tcgen05, a chunk of steps per launch)" if eb > 128 else
+            "lstm_persistent_pipe_kernel<16,2,4> (W_hh recurrence, all T steps of 128 sequences per launch)")
+
+
+def encoder_batch(asked: int, chunk: int) -> int:
+    """Utterances per recurrence launch, as RnntDecoder splits a call of `chunk`."""
+    if asked or chunk <= 128:
+        return min(asked or 128, chunk)
+    return -(-chunk // -(-chunk // ENCODER_MAX))
 
 
 def load_tensor_peak():
@@ -313,14 +325,20 @@ def run_gpu(args, rank, world, local):
     rec_s = prof["ms"] * 1e-3
     achieved = prof["bytes"] / rec_s / 1e9 if rec_s > 0 else 0.0
     share = prof["ms"] / sum(step_ms) if sum(step_ms) > 0 else 0.0
-    eb = min(args.encoder_batch or 128, chunk)
+    eb = encoder_batch(args.encoder_batch, chunk)
+    # (a launch of 65..128 sequences is two recurrences side by side, each with its own copy of W_hh)
+    timesteps = prof["bytes"] / (4.0 * cfg.enc_hidden * cfg.enc_hidden * 2.0 * (2 if 64 < eb <= 128 else 1))
     # the same launches as a contraction: 2 flop per weight element and sequence and timestep
-    flops = prof["bytes"] / 2.0 * 2.0 * eb
+    flops = 2.0 * 4.0 * cfg.enc_hidden * cfg.enc_hidden * eb * timesteps
     tflops = flops / rec_s / 1e12 if rec_s > 0 else 0.0
-    # per call of `chunk` utterances: per group of encoder-batch utterances (projection GEMM + recurrence) per LSTM
-    # layer; then the joint's encoder-half GEMM and one greedy kernel for the whole call
+    # per recurrence launch (all steps of a layer, or a chunk of them) one projection GEMM, and for many utterances a time-major
+    # copy of the features; then per call of `chunk` utterances the joint's encoder-half GEMM and one greedy kernel
     calls = (S + chunk - 1) // chunk
-    launches_per_step = calls * (((chunk + eb - 1) // eb) * 2 * (cfg.pre_layers + cfg.post_layers) + 2)
+    per_layer = prof["recurrences"] / args.steps / (cfg.pre_layers + cfg.post_layers / cfg.stack_factor)
+    launches_per_step = int(2 * prof["recurrences"] / args.steps + (per_layer if eb > 128 else 0) + 2 * calls)
+    # fp32 gate terms read once and fp16 outputs written once per timestep; captured for the 128-sequence kernel, counted for the other
+    # (ncu does not profile a cooperative launch of clusters)
+    traffic = (TRAFFIC_PER_TIMESTEP_128 * (eb / 128.0) if eb <= 128 else (4 * 4 + 2) * cfg.enc_hidden * eb) * timesteps / max(prof["recurrences"], 1)
 
     extras = {}
     if rank == 0 and world == 1 and not args.no_extras:        # the op sweeps ride on the one-GPU line only
@@ -349,15 +367,12 @@ def run_gpu(args, rank, world, local):
                 "h2d_bytes_per_step": int(feats_host.numel() * 2),
                 "d2h_bytes_per_step": int(tokens_host.numel() * 4 + n_tokens_host.numel() * 4)},
         "gpu_launches": launches_per_step * args.steps,
-        "roofline": {"bound": "hbm", "kernel": RECURRENCE_KERNEL,
+        "roofline": {"bound": "hbm", "kernel": recurrence_kernel(eb),
                      "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_source": peak_src,
-                     # DRAM bytes of an average launch, scaled from the committed ncu capture by its timesteps (a launch of
-                     # fewer than 128 sequences moves proportionally less; the capture is the 128-sequence case)
-                     "traffic": TRAFFIC_PER_TIMESTEP_128 * (eb / 128.0) * prof["bytes"] / max(prof["recurrences"], 1) /
-                                (4.0 * cfg.enc_hidden * cfg.enc_hidden * 2.0 * (2 if eb > 64 else 1)),
+                     "traffic": traffic,      # DRAM bytes of an average launch
                      "launches": prof["recurrences"], "avg_launch_ms": prof["ms"] / max(prof["recurrences"], 1),
-                     "us_per_timestep": prof["ms"] * 1e3 / max(prof["bytes"] / (4.0 * cfg.enc_hidden * cfg.enc_hidden * 2.0), 1.0),
+                     "us_per_timestep": prof["ms"] * 1e3 / max(timesteps, 1.0),
                      "sequences_per_launch": eb,
                      # what batch-1-per-stream execution would have to stream: every sequence its own W_hh per step
                      "per_stream_equivalent_gbs": achieved * eb,
@@ -366,9 +381,9 @@ def run_gpu(args, rank, world, local):
                      # the same launches as flops against the measured dense bf16 peak, and the pipe's active share
                      # from the committed ncu capture
                      "tensor": {"achieved_tflops": tflops, "peak_tflops": tpeak, "frac": tflops / tpeak,
-                                "peak_source": tpeak_src, "pipe_active_pct_ncu": TENSOR_PIPE_ACTIVE_PCT_NCU},
+                                "peak_source": tpeak_src, "pipe_active_pct_ncu": TENSOR_PIPE_ACTIVE_PCT_NCU if eb <= 128 else None},
                      "note": "algorithmic bytes = T * 4H*H * 2 per launch (W_hh once per timestep, the streamed "
-                             "formulation); the kernel keeps them in registers as mma fragments"},
+                             "formulation); the kernel keeps them on the chip"},
         "clocks": clocks,
     }
     line.update(extras)
@@ -751,8 +766,7 @@ def main():
     ap.add_argument("--streams-per-gpu", type=int, default=0,
                     help="overrides --streams-total with a per-rank count (profiling runs on small cases)")
     ap.add_argument("--streams-per-call", type=int, default=0,
-                    help="utterances per decode call (0 = the rank's whole shard in one call: the encoder still advances "
-                         "groups of up to 128 utterances, the greedy kernel takes all of them at once)")
+                    help="utterances per decode call (0 = the rank's whole shard in one call)")
     ap.add_argument("--no-extras", action="store_true", help="skip the C1 / C2 figures of the default line")
     ap.add_argument("--c2-shape", default="", help="with --workload c2: only this NxK shape (plus the headline shape), e.g. 4096x1024")
     ap.add_argument("--c2-batches", default="", help="with --c2-shape: the batched-stream sizes to time, e.g. 8,32")

@@ -55,12 +55,12 @@ int pimb200_rnnt_destroy(pimb200_rnnt* h);
 int pimb200_rnnt_decode(pimb200_rnnt* h, const void* feats, int T, int n_utts, int32_t* tokens,
                         int32_t* n_tokens, float* logits, void* stream);
 
-/* How many utterances the encoder advances in lock step (1..128, default 128); each is one column of the
- * recurrence's tensor-core tiles.  1 reproduces strict batch-1 execution. */
+/* How many utterances the encoder advances in lock step (1..128; by default as many as its recurrences take: 128, or where there
+ * are more and the sizes allow it, up to 1024).  1 reproduces strict batch-1 execution. */
 int pimb200_rnnt_set_encoder_batch(pimb200_rnnt* h, int n);
 
 /* Which greedy kernel a crowded call (more utterances than clusters) uses: 1 (default) = the best available
- * (tensor-core kernel, 8 utterances per cluster in lock step, when the shapes allow), 2 = the FMA lock-step kernel
+ * (from 81 utterances groups of CTAs with up to 80 each, below that 8 utterances per cluster in lock step, when the shapes allow), 2 = the FMA lock-step kernel
  * (4 per cluster), 0 = always one utterance per cluster.  For A/B measurements. */
 int pimb200_rnnt_set_greedy_multi(pimb200_rnnt* h, int mode);
 
