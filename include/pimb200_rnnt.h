@@ -60,7 +60,7 @@ int pimb200_rnnt_decode(pimb200_rnnt* h, const void* feats, int T, int n_utts, i
 int pimb200_rnnt_set_encoder_batch(pimb200_rnnt* h, int n);
 
 /* Which greedy kernel a crowded call (more utterances than clusters) uses: 1 (default) = the best available
- * (from 81 utterances groups of CTAs with up to 80 each, below that 8 utterances per cluster in lock step, when the shapes allow), 2 = the FMA lock-step kernel
+ * (from 113 utterances groups of CTAs with up to 80 each, below that 8 utterances per cluster in lock step, when the shapes allow), 2 = the FMA lock-step kernel
  * (4 per cluster), 0 = always one utterance per cluster.  For A/B measurements. */
 int pimb200_rnnt_set_greedy_multi(pimb200_rnnt* h, int mode);
 

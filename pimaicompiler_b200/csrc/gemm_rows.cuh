@@ -48,6 +48,6 @@ struct RowsCell {
     int I, H, J;
 };
 int launch_gemm_rows_cell(const RowsCell& c, cudaStream_t st);
-int launch_lstm_cell_skinny(const RowsCell& c, cudaStream_t st);   // up to 32 sequences (gemm_skinny.cu)
+int launch_lstm_cell_skinny(const RowsCell& c, cudaStream_t st);   // blocks of up to 32 sequences (gemm_skinny.cu)
 
 }  // namespace pimb200

@@ -18,35 +18,8 @@ namespace pimb200 {
 // first costs a barrier before the first weight load and measured slower.  R*unroll independent
 // 16-byte loads are in flight per lane.
 // =============================================================================================
-// The launch may start while its predecessor is still running: unless the matrix is large it then asks for its rows of W to be brought into L2 (which is
-// coherent, so it does not matter whether anyone still writes them) and reads everything behind the wait.
-constexpr size_t kMvAheadMax = (size_t)12 << 20;     // elements
 template <int R>
-__global__ void __launch_bounds__(256) gemv_mv_vec_kernel(const __half* W, const __half* x, const __half* bias, __half* y, int N, int K, int act,
-                                                          int ahead) {
-    pdl_launch_dependents();
-    const int K8 = K >> 3;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row0 = (blockIdx.x * (blockDim.x >> 5) + warp) * R;
-    if (ahead && lane < R && row0 + lane < N) prefetch_l2(W + (size_t)(row0 + lane) * K, (uint32_t)K * 2);
-    pdl_wait();
-    if (row0 >= N) return;
-
-    const uint4* wrow[R];
-    float acc[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        int row = min(row0 + r, N - 1);  // clamp: rows past N re-read the last row, never stored
-        wrow[r] = reinterpret_cast<const uint4*>(W + (size_t)row * K);
-        acc[r] = 0.f;
-    }
-#pragma unroll 4
-    for (int c = lane; c < K8; c += 32) {
-        float xf[8];
-        widen8(ld_v4(x + 8 * c), xf);
-#pragma unroll
-        for (int r = 0; r < R; ++r) acc[r] = dot8f(ld_stream_v4(wrow[r] + c), xf, acc[r]);
-    }
+__device__ __forceinline__ void mv_finish(float (&acc)[R], const __half* bias, __half* y, int row0, int N, int act, int lane) {
 #pragma unroll
     for (int r = 0; r < R; ++r) acc[r] = warp_sum(acc[r]);
     if (lane == 0) {
@@ -60,6 +33,70 @@ __global__ void __launch_bounds__(256) gemv_mv_vec_kernel(const __half* W, const
             }
         }
     }
+}
+
+template <int R>
+__global__ void __launch_bounds__(256) gemv_mv_vec_kernel(const __half* __restrict__ W, const __half* __restrict__ x,
+                                                          const __half* __restrict__ bias, __half* __restrict__ y,
+                                                          int N, int K, int act) {
+    const int K8 = K >> 3;
+    const uint4* x4 = reinterpret_cast<const uint4*>(x);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int row0 = (blockIdx.x * (blockDim.x >> 5) + warp) * R;
+    if (row0 >= N) return;
+
+    const uint4* wrow[R];
+    float acc[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        int row = min(row0 + r, N - 1);  // clamp: rows past N re-read the last row, never stored
+        wrow[r] = reinterpret_cast<const uint4*>(W + (size_t)row * K);
+        acc[r] = 0.f;
+    }
+#pragma unroll 4
+    for (int c = lane; c < K8; c += 32) {
+        float xf[8];
+        widen8(__ldg(x4 + c), xf);
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[r] = dot8f(ldg_stream_v4(wrow[r] + c), xf, acc[r]);
+    }
+    mv_finish<R>(acc, bias, y, row0, N, act, lane);
+}
+
+// The same for small matrices, where start and ramp are half the time.  The launch may start while its predecessor is still
+// running: it then asks for its rows of W to be brought into L2 (which is coherent, so it does not matter whether anyone still
+// writes them) and reads everything behind the wait, by plain loads.  In a loop of launches with cold weights, former kernel /
+// this one: 1024 x 1024 2.57 / 2.50 us, 4096 x 1024 3.42 / 3.18.  From 8 M elements on the read-only path of the former counts
+// for more: 16384 x 1024 7.40 / 7.66, 32320 x 1024 12.7 / 13.5, 32768 x 4096 42.5 / 45.9.
+// (The rows of W are asked for on a switch that is an argument and always set.  Without it the kernel needs 32 registers instead
+// of 34, eight CTAs fit an SM instead of six, and 4096 x 1024 takes 3.41: launches two ahead then ask for their rows too.)
+constexpr size_t kMvEarlyMax = (size_t)8 << 20;     // elements
+template <int R>
+__global__ void __launch_bounds__(256) gemv_mv_early_kernel(const __half* W, const __half* x, const __half* bias, __half* y, int N, int K, int act,
+                                                            int ahead) {
+    pdl_launch_dependents();
+    const int K8 = K >> 3;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int row0 = (blockIdx.x * (blockDim.x >> 5) + warp) * R;
+    if (ahead && lane < R && row0 + lane < N) prefetch_l2(W + (size_t)(row0 + lane) * K, (uint32_t)K * 2);
+    pdl_wait();
+    if (row0 >= N) return;
+
+    const uint4* wrow[R];
+    float acc[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        wrow[r] = reinterpret_cast<const uint4*>(W + (size_t)min(row0 + r, N - 1) * K);
+        acc[r] = 0.f;
+    }
+#pragma unroll 4
+    for (int c = lane; c < K8; c += 32) {
+        float xf[8];
+        widen8(ld_v4(x + 8 * c), xf);
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[r] = dot8f(ld_stream_v4(wrow[r] + c), xf, acc[r]);
+    }
+    mv_finish<R>(acc, bias, y, row0, N, act, lane);
 }
 
 // any K, any alignment: one warp per row, scalar half loads
@@ -92,11 +129,14 @@ static int launch_gemv_mv(const __half* W, const __half* x, const __half* bias, 
     const long want = (long)kNumSmB200 * 8 * 2;
     const int R = warps4 >= want ? 4 : (warps2 >= want ? 2 : 1);
     const int grid = ceil_div(N, 8 * R);
-    void (*const kernel)(const __half*, const __half*, const __half*, __half*, int, int, int, int) =
-        R == 4 ? gemv_mv_vec_kernel<4> : R == 2 ? gemv_mv_vec_kernel<2> : gemv_mv_vec_kernel<1>;
-    // (larger matrices take several waves of CTAs, whose rows would be asked for twice at once: 32768 x 4096 43.7 -> 56.7 us)
-    const int ahead = (size_t)N * K <= kMvAheadMax;
-    return cuda_status(launch_pdl(kernel, dim3(grid), dim3(256), 0, st, W, x, bias, y, N, K, act, ahead));
+    if ((size_t)N * K < kMvEarlyMax) {
+        const auto early = R == 4 ? gemv_mv_early_kernel<4> : R == 2 ? gemv_mv_early_kernel<2> : gemv_mv_early_kernel<1>;
+        return cuda_status(launch_pdl(early, dim3(grid), dim3(256), 0, st, W, x, bias, y, N, K, act, 1));
+    }
+    if (R == 4) gemv_mv_vec_kernel<4><<<grid, 256, 0, st>>>(W, x, bias, y, N, K, act);
+    else if (R == 2) gemv_mv_vec_kernel<2><<<grid, 256, 0, st>>>(W, x, bias, y, N, K, act);
+    else gemv_mv_vec_kernel<1><<<grid, 256, 0, st>>>(W, x, bias, y, N, K, act);
+    return launch_status();
 }
 
 // =============================================================================================
