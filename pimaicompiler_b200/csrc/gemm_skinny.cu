@@ -571,7 +571,12 @@ int launch_gemm_wx_skinny(const __half* W, const __half* X, const __half* bias, 
         {gemm_skinny_kernel<1, 2, 1>, gemm_skinny_kernel<2, 2, 1>, gemm_skinny_kernel<3, 2, 1>, gemm_skinny_kernel<4, 2, 1>},
         {gemm_skinny_kernel<1, 2, 2>, gemm_skinny_kernel<2, 2, 2>, gemm_skinny_kernel<3, 2, 2>, gemm_skinny_kernel<4, 2, 2>}};
     const bool one_wave = grid.x * grid.y <= kNumSmB200;
-    void (*const kernel)(SkinnyArgs) = wide ? broad[K > 512 ? one_wave || nt == 1 : one_wave && nt == 3][nt - 1] : narrow[K <= 512 ? 0 : K <= 1024 ? 1 : 2][nt - 1];
+    // up to 8 rows against several waves of CTAs: two where weights are loaded ahead of the wait or the waves are many (32320 x 1024,
+    // 2 rows: 11.9 / 13.4 us with two / one ahead of it, 13.2 / 13.8 behind), else one (16384 x 1024: 8.2 / 7.75).  17..24 rows
+    // at K <= 1024: two ahead of the wait (1024 x 1024: 2.5 / 3.1), one behind (512 x 768: 3.3 / 3.1)
+    const bool ahead = fixed || grid.x > 4 * kNumSmB200;
+    void (*const kernel)(SkinnyArgs) = wide ? broad[K > 512 ? one_wave || (nt == 1 && ahead) : one_wave && nt == 3][nt - 1]
+                                              : narrow[K <= 512 || (nt == 3 && K <= 1024 && !fixed) ? 0 : K <= 1024 ? 1 : 2][nt - 1];
     const cudaError_t rc = launch_pdl(kernel, grid, dim3(kSkinnyThreads), 0, st, a);
     return cuda_status(rc);
 }
