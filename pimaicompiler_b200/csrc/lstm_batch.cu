@@ -15,6 +15,11 @@
 // Ordering between CTAs: a warp writes its cells' h, fences for the async proxy and counts up its pair's counter with a
 // release; the TMA warps watch the counters (one lane each), acquire, and load K block k (the 64 units of pair k) as soon as
 // pair k's sixteen warps have counted.  K blocks are multiplied in the same order whoever comes first.
+// What bounds it: the chain of a step (states from L2, products, gates on the special-function unit, counters), of which two
+// sub-batches hide a half.  A step at H = 1024 takes 5.5 us for 129 sequences, 6.3 for 512, 8.2 for 768 and 9.5 for 1024, where
+// lstm_persistent_pipe_kernel takes 3.9 for every 128 (31 at 1024); the cycles of a step at 256..1024 sequences: states 1.1 k,
+// products 3.3..6 k, commit 1.2 k, gates 2.6..5.4 k, counters 1.5..2.5 k.
+//
 // Every wait is bounded; on giving up a CTA records the error, lets its copies land and frees its tensor memory.
 #include "lstm_batch.cuh"
 

@@ -12,7 +12,8 @@
 //
 // What bounds it: four exchanges through L2 per frame (write, fence, counter, poll, TMA load), and the special-function unit
 // in the gates.  The 8-utterance clusters of rnnt_greedy_mma_kernel exchange faster (through distributed shared memory), but
-// seven of them take 56 utterances a round.
+// seven of them take 56 utterances a round: 4.9 us per frame and round, 19 rounds for 1024 utterances.  A frame of all of them
+// takes 16.7 us here, of 448 utterances 15, of 112..224 8.9..9.6.
 //
 // Buffers are written again only after an exchange that every CTA joins later: h0 of the next evaluation follows the
 // partial logits, which every CTA sends after it has loaded h0 and h1; the partial logits of the next frame follow the labels.  Utterances without a label keep their states.
