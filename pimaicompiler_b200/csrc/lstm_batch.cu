@@ -20,11 +20,14 @@
 // lstm_persistent_pipe_kernel takes 3.9 for every 128 (31 at 1024); the cycles of a step at 256..1024 sequences: states 1.1 k,
 // products 3.3..6 k, commit 1.2 k, gates 2.6..5.4 k, counters 1.5..2.5 k.
 //
-// Every wait is bounded; on giving up a CTA records the error, lets its copies land and frees its tensor memory.
+// Every wait of the loops is bounded; on giving up a CTA records the error, lets its copies land and frees its tensor memory.
+// What has no bound waits for no other CTA's progress: the allocation of tensor memory finds it free (a CTA has its SM's shared
+// memory for itself), and both CTAs of a pair reach the barriers at either end.
 #include "lstm_batch.cuh"
 
 #include <algorithm>
 
+#include "batch_plan.h"
 #include "gemm_rows.cuh"
 #include "tc_common.cuh"
 
@@ -35,26 +38,10 @@ namespace {
 constexpr int kFirstEpi = 3;            // warps: TMA, MMA, TMEM owner, then 8 or 16 for the gates
 constexpr int kUnits = 32;             // hidden units per CTA
 constexpr int kMaxBlocks = 16;         // H <= 1024
-constexpr int kBlockBytes = 128 * 128; // a K block of a CTA's weights
-constexpr int kRingBytes = 96 * 1024;
-constexpr int kMaxStages = 8;
 
 struct BatchMaps {
     CUtensorMap h[2], h0[2];           // boxes of 64 units x 8 NJ sequences
 };
-
-__host__ __device__ constexpr int blocks_per_stage(int nj) { return nj > 4 ? 2 : 4; }
-__host__ __device__ constexpr int stages_of(int nj) {
-    return kRingBytes / (blocks_per_stage(nj) * nj * 1024) < kMaxStages ? kRingBytes / (blocks_per_stage(nj) * nj * 1024) : kMaxStages;
-}
-// TMEM: the accumulator of sub-batch b at column b * acc_cols, behind them as many K blocks of weights (32 columns each) as fit.
-// An MMA of few columns is bound by its A operand: 74 cycles from shared memory, 37 from tensor memory, at up to 64 columns.
-__host__ __device__ constexpr int acc_cols(int nj) { return (16 * nj + 31) / 32 * 32; }
-__host__ __device__ constexpr int tmem_blocks(int nj, int subs) { return (512 - subs * acc_cols(nj)) / 32; }
-size_t smem_of(int H, int nj, int subs) {
-    const int blocks = H / 64, t = tmem_blocks(nj, subs), own = blocks > t ? blocks - t : 0;
-    return (size_t)own * kBlockBytes + kRingBytes + 1024 /*align*/ + 512 /*barriers*/;
-}
 
 __device__ __forceinline__ float4 ldg_stream_f4(const float* p) {
     const uint4 v = ldg_stream_v4(p);
@@ -451,7 +438,7 @@ void launch_config(cudaLaunchConfig_t& lc, cudaLaunchAttribute* at, int H, int n
     lc = {};
     lc.gridDim = dim3(ctas);
     lc.blockDim = dim3(threads_of(nj));
-    lc.dynamicSmemBytes = smem_of(H, nj, subs);
+    lc.dynamicSmemBytes = lstm_batch_smem(H, nj, subs);
     lc.stream = st;
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
@@ -472,7 +459,7 @@ int resident_pairs(int dev) {
         launch_config(lc, at, 1024, 8, 2, 2, nullptr);
         lc.numAttrs = 1;
         int n = 0;
-        if (cudaFuncSetAttribute(lstm_batch_kernel<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(1024, 8, 2)) != cudaSuccess ||
+        if (cudaFuncSetAttribute(lstm_batch_kernel<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lstm_batch_smem(1024, 8, 2)) != cudaSuccess ||
             cudaOccupancyMaxActiveClusters(&n, lstm_batch_kernel<8, 2>, &lc) != cudaSuccess) {
             cudaGetLastError();
             n = 0;
@@ -522,7 +509,7 @@ int launch_lstm_batch(BatchArgs& a, cudaStream_t st) {
     }
     const BatchFn fn = subs == 2 ? pick_nj<2>(nj) : pick_nj<1>(nj);
     const int blocks = a.H / 64;
-    PIMB200_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(a.H, nj, subs)));
+    PIMB200_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lstm_batch_smem(a.H, nj, subs)));
     PIMB200_CUDA_TRY(cudaMemsetAsync(a.counters, 0, (size_t)groups * a.dirs * subs * blocks * kBatchFlagWords * 4, st));
     cudaLaunchConfig_t lc;
     cudaLaunchAttribute at[2];

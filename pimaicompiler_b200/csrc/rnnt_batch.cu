@@ -17,11 +17,13 @@
 //
 // Buffers are written again only after an exchange that every CTA joins later: h0 of the next evaluation follows the
 // partial logits, which every CTA sends after it has loaded h0 and h1; the partial logits of the next frame follow the labels.  Utterances without a label keep their states.
-// Every wait is bounded; on giving up a CTA records the error, lets its copies land and frees its tensor memory.
+// Every wait of the loops is bounded; on giving up a CTA records the error, lets its copies land and frees its tensor memory.
+// The allocation of tensor memory has no bound and finds it free: a CTA has its SM's shared memory for itself.
 #include "rnnt_batch.cuh"
 
 #include <algorithm>
 
+#include "batch_plan.h"
 #include "gemm_rows.cuh"
 #include "pimb200_rnnt.h"
 #include "tc_common.cuh"
@@ -37,7 +39,7 @@ constexpr int kUnits = 32;
 constexpr int kMaxBlocks = 5;          // PH <= 320: two matrices of 32 TMEM columns per K block of 64
 constexpr int kMaxUtts = 80;           // per group
 constexpr int kMaxJointRows = 64;      // per CTA: one K block of the product with W2
-constexpr int kVocab = 32;
+constexpr int kVocab = kGreedyVocab;
 constexpr int kACol = 192;             // TMEM: accumulators of layer 0 and of everything else at 0 and 96, Whh0, Whh1 from here
 constexpr int kCounterWords = 32;      // a counter has a 128-byte line
 constexpr int kExchanges = 3;          // h0, h1, partial logits
@@ -46,26 +48,6 @@ constexpr int kMaxCtas = 148;
 struct GreedyMaps {
     CUtensorMap h[2];                  // [utterances of all groups][PH], boxes of 64 units x one group
 };
-
-struct Smem {                          // offsets behind the 1024-byte boundary
-    int wih1, w1p, w2, h[2], bars, total;
-};
-__host__ __device__ inline int joint_rows(int JH, int ctas) { return ((JH + ctas - 1) / ctas + 3) / 4 * 4; }
-__host__ __device__ inline Smem layout(int PH, int jrows, int utts) {
-    Smem s;
-    const int blocks = PH / 64, jpad = (jrows + 7) / 8 * 8;
-    s.wih1 = 0;
-    s.w1p = s.wih1 + blocks * 128 * 128;
-    s.w2 = s.w1p + blocks * jpad * 128;
-    s.h[0] = s.w2 + kVocab * 128;
-    s.h[1] = s.h[0] + blocks * utts * 128;
-    s.bars = s.h[1] + blocks * utts * 128;
-    // an A operand has 128 rows: what lies behind the joint's and W2's is multiplied too, into lanes that nobody reads
-    const int last = s.w1p + (blocks - 1) * jpad * 128, reach = (last > s.w2 ? last : s.w2) + 128 * 128;
-    if (s.bars < reach) s.bars = reach;
-    s.total = s.bars + 1024;
-    return s;
-}
 
 __device__ __forceinline__ void count_up(uint32_t* p) { asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory"); }
 __device__ __forceinline__ void mbar_arrive_one(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
@@ -105,7 +87,7 @@ __global__ void __launch_bounds__(kThreads, 1) rnnt_greedy_batch_kernel(const __
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int PH = a.PH, blocks = PH >> 6, C = a.ctas;
     const int jpad = (a.jrows + 7) / 8 * 8;
-    const Smem at = layout(PH, a.jrows, UTTS);
+    const GreedySmem at = greedy_layout(PH, a.jrows, UTTS);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + at.bars);
     // h0 arrived [blocks], h1 arrived [blocks], then: layer-0 sums, layer-1 sums, joint sums, logits sums ready; layer-0 sums read,
     // layer-1 sums read, z written, partial logits read, labels known, seen by the TMA warp, labels
@@ -540,7 +522,7 @@ Plan plan_for(int PH, int JH, int V) {
     if (p.jrows > kMaxJointRows) return p;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    while (p.max_nj < kMaxUtts / 16 && layout(PH, p.jrows, 16 * (p.max_nj + 1)).total + 1024 <= smem) ++p.max_nj;
+    while (p.max_nj < kMaxUtts / 16 && (int)greedy_batch_smem(PH, p.jrows, 16 * (p.max_nj + 1)) <= smem) ++p.max_nj;
     if (p.max_nj > 0) p.groups = std::min(sms, kMaxCtas) / p.ctas;
     return p;
 }
@@ -578,7 +560,7 @@ int launch_greedy_batch(GreedyBatchArgs& a, cudaStream_t st) {
     for (int x = 0; x < 2; ++x)
         if (!encode_2d(&m.h[x], a.state + x * rows * a.PH, rows, a.PH, (uint64_t)a.PH * 2, 16 * nj, 2)) return PIMB200_ERR_UNSUPPORTED;
     const GreedyBatchFn fn = pick_nj(nj);
-    const int smem = layout(a.PH, a.jrows, 16 * nj).total + 1024;
+    const int smem = (int)greedy_batch_smem(a.PH, a.jrows, 16 * nj);
     PIMB200_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     a.labels = a.counters + (size_t)groups * p.ctas * kExchanges * kCounterWords;
     PIMB200_CUDA_TRY(cudaMemsetAsync(a.counters, 0, (size_t)groups * (p.ctas * kExchanges * kCounterWords + kMaxUtts) * 4, st));
