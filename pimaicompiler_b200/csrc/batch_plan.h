@@ -37,6 +37,24 @@ inline size_t lstm_batch_smem(int H, int nj, int subs) {
     return alone_on_sm((size_t)own * kBlockBytes + kRingBytes + 1024 /*align*/ + 512 /*barriers*/);
 }
 
+// Stage uses of a CTA pair, numbered from 0: each CTA asks for its half of use q's copies, and the bytes of both count at the
+// leader's barrier of stage q % STAGES, where the leader expects them when it asks for its own half.  A pair that gave up may
+// have asked for different numbers of uses.  What the leader then adds to the barrier of use q, so that its phase completes
+// when every copy that was asked for has landed: bytes to expect (with the arrival), or bytes to count as landed that will
+// never come.  (A use is asked for once the use STAGES before it was multiplied, so only the last STAGES can be incomplete.)
+struct StageDebt {
+    uint32_t expect, credit;
+};
+PIMB200_HD inline StageDebt stage_debt(uint32_t q, uint32_t leader_uses, uint32_t other_uses, uint32_t half_bytes) {
+    return StageDebt{q >= leader_uses ? half_bytes : 0u, q >= other_uses ? half_bytes : 0u};
+}
+PIMB200_HD inline uint32_t first_open_use(uint32_t uses, uint32_t stages) { return uses > stages ? uses - stages : 0; }
+// K blocks in use q: a sub-batch's step takes its `blocks` in uses of `per_use`
+PIMB200_HD inline uint32_t blocks_of_use(uint32_t q, uint32_t blocks, uint32_t per_use) {
+    const uint32_t k0 = q % ((blocks + per_use - 1) / per_use) * per_use;
+    return blocks - k0 < per_use ? blocks - k0 : per_use;
+}
+
 // ---- greedy loop of many utterances ----
 constexpr int kGreedyVocab = 32;
 struct GreedySmem {                    // offsets behind the 1024-byte boundary

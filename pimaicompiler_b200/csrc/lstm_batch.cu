@@ -66,9 +66,10 @@ __global__ void __launch_bounds__(threads_of(NJ), 1) lstm_batch_kernel(const __g
     const int blocks = a.H >> 6, tblocks = blocks < kTmemBlocks ? blocks : kTmemBlocks;
     unsigned char* ring = smem + (size_t)(blocks - tblocks) * kBlockBytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(ring + kRingBytes);
-    // full[STAGES], empty[STAGES], accumulator full[2], accumulator read[2], all products done; then the TMEM base
+    // full[STAGES], empty[STAGES], accumulator full[2], accumulator read[2], all products done; then the TMEM base and a count
     const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * STAGES, accf0 = empty0 + 8 * STAGES, acce0 = accf0 + 16, done0 = acce0 + 16;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 5);
+    uint32_t* other_uses = tmem_slot + 1;         // of the leader: stage uses that the other CTA asked for
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = (int)(blockIdx.x & 1), pair = (int)(blockIdx.x >> 1) % blocks, grp = (int)(blockIdx.x >> 1) / blocks;
     const int dir_groups = (int)(gridDim.x >> 1) / blocks / a.dirs, d = grp / dir_groups;
@@ -125,11 +126,12 @@ __global__ void __launch_bounds__(threads_of(NJ), 1) lstm_batch_kernel(const __g
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     bool failed = false;
+    uint32_t asked = 0;                           // stage uses whose copies this CTA asked for (TMA warp)
     if (warp == 0) {
         // ---------------- TMA: this CTA's half of every sub-batch's rows ----------------
         const uint32_t el = elect_one();
         const uint32_t ring0 = smem_u32(ring), lead0 = mapa(full0, 0);
-        uint32_t st = 0, par = 1, issued = 0;
+        uint32_t st = 0, par = 1;
         for (int s = 0; s < a.steps && !failed; ++s) {
             if (s == 0 && !h_first) continue;
             const int tp = step_time(s - 1);                           // the step before
@@ -164,17 +166,14 @@ __global__ void __launch_bounds__(threads_of(NJ), 1) lstm_batch_kernel(const __g
                     if (rank == 0) expect_tx_if(el, full0 + 8 * st, 2u * (uint32_t)((k1 - k0) * BLOCK));
                     for (int k = k0; k < k1; ++k)
                         load_3d<2>(el, ring0 + st * STAGE + (k - k0) * BLOCK, map, lead0 + 8 * st, fold * a.H + k * 64, row, tc);
-                    ++issued;
+                    ++asked;
                     if (++st == STAGES) { st = 0; par ^= 1; }
                 }
             }
         }
-        if (failed && lane == 0) {
-            status_raise(a.status, a.gen, PIMB200_ERR_TIMEOUT);
-            if (rank == 0)      // let the copies already issued land (the leader's barriers count those of both CTAs)
-                for (uint32_t q = issued > STAGES ? issued - STAGES : 0; q < issued; ++q)
-                    for (uint32_t i = 0; i < (1u << 20); ++i)
-                        if (mbar_try_wait(full0 + 8 * (q % STAGES), (q / STAGES) & 1)) break;
+        if (lane == 0) {
+            if (failed) status_raise(a.status, a.gen, PIMB200_ERR_TIMEOUT);
+            if (rank == 1) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(mapa(smem_u32(other_uses), 0)), "r"(asked) : "memory");
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (the pair's leader) ----------------
@@ -413,7 +412,21 @@ __global__ void __launch_bounds__(threads_of(NJ), 1) lstm_batch_kernel(const __g
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncwarp();
-    pair_sync<2>();                               // neither CTA leaves while the other may still signal it
+    pair_sync<2>();                               // nobody multiplies or asks for copies any more
+    if (warp == 0 && rank == 0 && lane == 0) {
+        // let every copy of both CTAs land, whoever gave up and where (all have, if nobody did)
+        const uint32_t theirs = *other_uses, all = asked > theirs ? asked : theirs;
+        for (uint32_t q = first_open_use(all, STAGES); q < all; ++q) {
+            const uint32_t bar = full0 + 8 * (q % STAGES);
+            const StageDebt debt = stage_debt(q, asked, theirs, blocks_of_use(q, blocks, KPS) * BLOCK);
+            if (debt.expect) mbar_expect_tx(bar, debt.expect);
+            if (debt.credit) mbar_complete_tx(bar, debt.credit);
+            for (uint32_t i = 0; i < (1u << 20); ++i)
+                if (mbar_try_wait(bar, (q / STAGES) & 1)) break;
+        }
+    }
+    __syncwarp();
+    pair_sync<2>();                               // neither CTA leaves while copies of the other may still signal it
     if (warp == 2) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");

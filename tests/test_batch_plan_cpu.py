@@ -14,6 +14,15 @@ extern "C" {
 size_t smem_per_sm() { return kSmemPerSm; }
 size_t smem_per_cta() { return kSmemPerCta; }
 size_t lstm_smem(int H, int nj, int subs) { return lstm_batch_smem(H, nj, subs); }
+int stages(int nj) { return stages_of(nj); }
+int per_stage(int nj) { return blocks_per_stage(nj); }
+void debt(unsigned q, unsigned leader, unsigned other, unsigned bytes, unsigned* out) {
+    const StageDebt d = stage_debt(q, leader, other, bytes);
+    out[0] = d.expect;
+    out[1] = d.credit;
+}
+unsigned first_open(unsigned uses, unsigned stages) { return first_open_use(uses, stages); }
+unsigned use_blocks(unsigned q, unsigned blocks, unsigned per_use) { return blocks_of_use(q, blocks, per_use); }
 size_t greedy_smem(int PH, int JH, int utts) { return greedy_batch_smem(PH, joint_rows(JH, PH / 32), utts); }
 }
 """
@@ -38,3 +47,60 @@ def test_a_cta_of_the_batched_kernels_has_its_sm_for_itself(plan):
     for smem in sizes:
         assert 2 * (smem + reserved) > plan.smem_per_sm()
         assert smem <= plan.smem_per_cta()
+
+
+class _Barrier:
+    """A barrier of one arrival per phase that also counts bytes: a phase ends when neither is outstanding."""
+
+    def __init__(self):
+        self.phase, self.arrivals, self.bytes = 0, 1, 0
+
+    def add(self, arrivals=0, expect=0, landed=0):
+        self.bytes += expect - landed
+        self.arrivals -= arrivals
+        assert self.arrivals >= 0
+        if self.arrivals == 0 and self.bytes == 0:
+            self.phase, self.arrivals = self.phase + 1, 1
+
+
+@pytest.mark.parametrize("nj", [1, 2, 4, 5, 8])
+@pytest.mark.parametrize("blocks", [1, 3, 5, 16])
+def test_a_pair_that_gave_up_waits_for_every_copy_of_both_ctas(plan, nj, blocks):
+    # whichever CTA got further, and whichever copies had landed before: behind the leader's drain all have
+    stages, per = plan.stages(nj), plan.per_stage(nj)
+    block_bytes, steps = nj * 1024, 4
+    sizes = [min(per, blocks - k) for _ in range(steps) for k in range(0, blocks, per)]
+    assert [plan.use_blocks(q, blocks, per) for q in range(len(sizes))] == sizes
+    debt = (ctypes.c_uint * 2)()
+    for leader in range(len(sizes) + 1):
+        for other in range(max(0, leader - stages), min(len(sizes), leader + stages) + 1):
+            done = max(0, max(leader, other) - stages)        # uses that were multiplied: all their copies have landed
+            if done > min(leader, other):
+                continue
+            for early in range(4):                            # copies of the open uses that land ahead of the drain: of whom
+                bars = [_Barrier() for _ in range(stages)]
+                late = []
+                for q in range(max(leader, other)):
+                    half, bar = sizes[q] * block_bytes, bars[q % stages]
+                    if q < other and (q < done or early & 1):
+                        bar.add(landed=half)                  # (may come before the leader expects it)
+                    elif q < other:
+                        late.append((q, half))
+                    if q < leader:
+                        bar.add(arrivals=1, expect=2 * half)
+                        if q < done or early & 2:
+                            bar.add(landed=half)
+                        else:
+                            late.append((q, half))
+                for q in range(plan.first_open(max(leader, other), stages), max(leader, other)):
+                    half = sizes[q] * block_bytes
+                    plan.debt(q, leader, other, half, debt)
+                    if debt[0]:
+                        bars[q % stages].add(arrivals=1, expect=debt[0])
+                    if debt[1]:
+                        bars[q % stages].add(landed=debt[1])
+                    mine = [h for u, h in late if u == q]
+                    for h in mine:                            # not before the last one
+                        assert bars[q % stages].phase == q // stages
+                        bars[q % stages].add(landed=h)
+                    assert bars[q % stages].phase == q // stages + 1 and bars[q % stages].bytes == 0
