@@ -389,7 +389,9 @@ int pimb200_lstm_set_exchange_copies(pimb200_lstm* h, int copies);
 int pimb200_lstm_set_exchange_stride(pimb200_lstm* h, int stride16);
 
 /* Diagnostics: a device buffer of n_cta * T * 8 int64 that the persistent kernels fill with per-step clocks (NULL
- * switches it off).  Not owned by the handle.  No counterpart in the reference. */
+ * switches it off), n_cta being ceil(hidden_size / 8), or 148 for PIMB200_LSTM_PERSISTENT_TAGGED.  Directions, layers and
+ * the chunks of a long sequence overwrite one another; the recurrence for many sequences, which has more CTAs, records the
+ * first n_cta of them.  Not owned by the handle.  No counterpart in the reference. */
 int pimb200_lstm_set_trace(pimb200_lstm* h, long long* device_buffer);
 
 #ifdef __cplusplus

@@ -2724,7 +2724,8 @@ static int forward_batch(pimb200_lstm* h, const __half* x, RowStrides xs, int T,
         a.g_tstride = (long)B * 4 * H; a.g_bstride = 4L * H;
         a.y_tstride = last ? y_t : (long)B * D * H; a.y_bstride = last ? y_b : (long)D * H; a.y_fold = last ? y_fold : 1;
         a.H = H; a.T = T; a.B = B;
-        a.counters = h->batch_counters; a.status = h->d_status; a.poll_limit = h->poll_limit; a.trace = h->trace;
+        a.counters = h->batch_counters; a.status = h->d_status; a.poll_limit = h->poll_limit;
+        a.trace = h->trace; a.trace_ctas = ceil_div(H, 8);      // (its launches have up to 148: no more than the buffer was made for)
         for (int d = 0; d < D; ++d) {
             BatchDir& r = a.dir[d];
             const int ld = l * D + d;

@@ -78,6 +78,7 @@ __global__ void __launch_bounds__(threads_of(NJ), 1) lstm_batch_kernel(const __g
     const int seq0 = (grp - d * dir_groups) * SUBS * COLS;             // first sequence of this group
     const bool h_first = a.begin > 0 || dir.h0 != nullptr;             // the first step has a product
     const volatile int* abort_flag = a.status + 1;
+    long long* const trace = blockIdx.x < (unsigned)a.trace_ctas ? a.trace : nullptr;
     auto step_time = [&](int s) { return dir.reverse ? a.T - 1 - (a.begin + s) : a.begin + s; };
 
     if (threadIdx.x == 0) {
@@ -160,8 +161,8 @@ __global__ void __launch_bounds__(threads_of(NJ), 1) lstm_batch_kernel(const __g
                         __syncwarp();
                     }
                     if (failed) break;
-                    if (a.trace && lane == 0 && b == 0 && k0 == 0) a.trace[((size_t)blockIdx.x * a.steps + s) * 8] = clock64();
-                    if (a.trace && lane == 0 && b == 0 && k1 == blocks) a.trace[((size_t)blockIdx.x * a.steps + s) * 8 + 1] = clock64();
+                    if (trace && lane == 0 && b == 0 && k0 == 0) trace[((size_t)blockIdx.x * a.steps + s) * 8] = clock64();
+                    if (trace && lane == 0 && b == 0 && k1 == blocks) trace[((size_t)blockIdx.x * a.steps + s) * 8 + 1] = clock64();
                     if (__any_sync(0xffffffffu, !mbar_wait(empty0 + 8 * st, par, abort_flag, a.gen))) { failed = true; break; }
                     if (rank == 0) expect_tx_if(el, full0 + 8 * st, 2u * (uint32_t)((k1 - k0) * BLOCK));
                     for (int k = k0; k < k1; ++k)
@@ -191,8 +192,8 @@ __global__ void __launch_bounds__(threads_of(NJ), 1) lstm_batch_kernel(const __g
                     for (int k0 = 0; k0 < blocks; k0 += KPS) {
                         if (!mbar_wait(full0 + 8 * st, par, abort_flag, a.gen)) { failed = true; break; }
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        if (a.trace && lane == 0 && b == 0 && k0 == 0) a.trace[((size_t)blockIdx.x * a.steps + s) * 8 + 6] = clock64();
-                        if (a.trace && lane == 0 && b == 0 && k0 + KPS >= blocks) a.trace[((size_t)blockIdx.x * a.steps + s) * 8 + 7] = clock64();
+                        if (trace && lane == 0 && b == 0 && k0 == 0) trace[((size_t)blockIdx.x * a.steps + s) * 8 + 6] = clock64();
+                        if (trace && lane == 0 && b == 0 && k0 + KPS >= blocks) trace[((size_t)blockIdx.x * a.steps + s) * 8 + 7] = clock64();
 #pragma unroll
                         for (int i = 0; i < KPS; ++i) {
                             const int kb = k0 + i;
@@ -295,7 +296,7 @@ __global__ void __launch_bounds__(threads_of(NJ), 1) lstm_batch_kernel(const __g
                     if (__any_sync(0xffffffffu, failed)) { failed = true; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
-                if (a.trace && lane == 0 && warp == kFirstEpi) a.trace[((size_t)blockIdx.x * a.steps + s) * 8 + 2 + 2 * b] = clock64();
+                if (trace && lane == 0 && warp == kFirstEpi) trace[((size_t)blockIdx.x * a.steps + s) * 8 + 2 + 2 * b] = clock64();
                 const uint32_t acc = tmem_base + ((uint32_t)(32 * q) << 16) + acc_cols(NJ) * b + part * (COLS / PARTS);
                 const int nb = b + 1 < SUBS ? b + 1 : 0;
                 const float* const gn = b + 1 < SUBS ? gp[nb] : gp[0] + g_step;
@@ -396,7 +397,7 @@ __global__ void __launch_bounds__(threads_of(NJ), 1) lstm_batch_kernel(const __g
                             else if (dir.cn) dir.cn[at] = __float2half_rn(c[b][j][e]);
                         }
                 }
-                if (a.trace && lane == 0 && warp == kFirstEpi) a.trace[((size_t)blockIdx.x * a.steps + s) * 8 + 3 + 2 * b] = clock64();
+                if (trace && lane == 0 && warp == kFirstEpi) trace[((size_t)blockIdx.x * a.steps + s) * 8 + 3 + 2 * b] = clock64();
                 // the next phase's input terms: behind the fence, which would wait for them (they come from HBM)
                 const float* gq = gn;          // (a running address: the products of all cells would be kept in registers)
 #pragma unroll

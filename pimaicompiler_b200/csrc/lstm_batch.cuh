@@ -33,7 +33,8 @@ struct BatchArgs {
     int* status;
     int gen;
     int poll_limit;
-    long long* trace;              // optional: 8 clocks per CTA and step
+    long long* trace;              // optional: 8 clocks per CTA and step of the first trace_ctas CTAs
+    int trace_ctas;
 };
 
 // Sequences per direction that one launch takes (0: none of this size).

@@ -547,6 +547,23 @@ def test_many_sequences_on_the_tensor_core_recurrence_vs_libtorch(T, B, I, H, L,
         assert_close(got, want.numpy(), LSTM_ATOL, LSTM_RTOL, name)
 
 
+@pytest.mark.parametrize("H,B", [(320, 224), (512, 100), (64, 40), (1024, 300)])
+def test_trace_buffer_of_one_record_per_eight_units_is_not_overrun(H, B):
+    # the recurrence for many sequences has up to 148 CTAs at any hidden size; the buffer has room for H / 8
+    ops = _ops()
+    from pimaicompiler_b200 import _lib
+    g = torch.Generator().manual_seed(H)
+    T, I, bi = 9, 24, B == 40
+    m = ops.Lstm([to_dev(p) for p in lstm_params(1, 2 if bi else 1, I, H, g)], 1, bi, I, H, True)
+    words, guard = -(-H // 8) * T * 8, 148 * T * 8
+    trace = torch.full((words + guard,), -1, dtype=torch.int64, device="cuda")
+    assert _lib.lib().pimb200_lstm_set_trace(m._h, trace.data_ptr()) == 0
+    m.forward(to_dev(torch.randn(T, B, I, generator=g)))
+    torch.cuda.synchronize()
+    assert _lib.lib().pimb200_lstm_set_trace(m._h, None) == 0
+    assert bool((trace[words:] == -1).all()) and bool((trace[:words] != -1).any())
+
+
 def test_outputs_given_in_any_sequence_and_batch_sizes_of_any_array():
     ops = _ops()
     g = torch.Generator().manual_seed(2)
