@@ -2200,6 +2200,12 @@ static PersistPlan plan_persistent(const pimb200_lstm* h) {
     return p;
 }
 
+// The most that the device allows, at every launch: the limit belongs to the function, and a thread with a handle of another size
+// may be about to launch it
+static cudaError_t raise_smem_limit(const pimb200_lstm* h, const void* fn) {
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, h->max_smem_optin);
+}
+
 // one (layer, direction) recurrence over a padded batch or a packed sequence
 struct SeqLayout {
     int T, B;                       // B = batch_sizes[0] for packed input
@@ -2269,7 +2275,7 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
         h->bulk_tag += (uint32_t)T + 1u;
         int bp = tc_bp;
         const size_t smem = tc_smem(H, bp);
-        PIMB200_CUDA_TRY(cudaFuncSetAttribute(lstm_persistent_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PIMB200_CUDA_TRY(raise_smem_limit(h, (const void*)lstm_persistent_tc_kernel));
         void* kargs[] = {&a, &bp};
         if (h->prof) prof_mark(h, st);
         PIMB200_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)lstm_persistent_tc_kernel, dim3(H / 8),
@@ -2324,7 +2330,7 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
                     default: fn = (const void*)lstm_persistent_pipe_kernel<8, 4, 2>; break;
                 }
             }
-            PIMB200_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            PIMB200_CUDA_TRY(raise_smem_limit(h, fn));
             void* kargs[] = {&a};
             if (h->prof) prof_mark(h, st);
             PIMB200_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(halves * H / upc), dim3(kPipeThreads), kargs, smem, st));
@@ -2376,7 +2382,7 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
                                  : nt == 2 ? (const void*)lstm_persistent_bulk_kernel<2>
                                            : (const void*)lstm_persistent_bulk_kernel<4>);
         const size_t smem = bsmem;
-        PIMB200_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PIMB200_CUDA_TRY(raise_smem_limit(h, fn));
         void* kargs[] = {&a};
         if (h->prof) prof_mark(h, st);
         PIMB200_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(H / 8), dim3(wide ? kWideThreads : kPersistThreads), kargs, smem, st));
@@ -2406,7 +2412,7 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
         }
         h->tag_counter += (uint32_t)T + 1u;
         const void* fn = (const void*)lstm_persistent_kernel;
-        PIMB200_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pp.smem));
+        PIMB200_CUDA_TRY(raise_smem_limit(h, fn));
         void* kargs[] = {&a};
         if (h->prof) prof_mark(h, st);
         PIMB200_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(pp.ncta), dim3(pp.threads), kargs, pp.smem, st));

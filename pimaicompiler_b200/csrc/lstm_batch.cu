@@ -26,6 +26,7 @@
 #include "lstm_batch.cuh"
 
 #include <algorithm>
+#include <atomic>
 
 #include "batch_plan.h"
 #include "gemm_rows.cuh"
@@ -462,25 +463,31 @@ void launch_config(cudaLaunchConfig_t& lc, cudaLaunchAttribute* at, int H, int n
     lc.numAttrs = 2;
 }
 
+// The most shared memory that any launch asks for, at every launch: the limit belongs to the function, and a thread with a handle of
+// another size may be about to launch it
+int raise_smem_limit(BatchFn fn) {
+    return cuda_status(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemPerCta));
+}
+
 // pairs of CTAs that are resident at once
 int resident_pairs(int dev) {
     constexpr int kMaxDevices = 64;
-    static int pairs[kMaxDevices];     // written with the same value by whoever comes first
+    static std::atomic<int> pairs[kMaxDevices];     // (two threads that come first find the same)
     if (dev < 0 || dev >= kMaxDevices) return 0;
-    if (pairs[dev] == 0) {
+    int n = pairs[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
         cudaLaunchConfig_t lc;
         cudaLaunchAttribute at[2];
         launch_config(lc, at, 1024, 8, 2, 2, nullptr);
         lc.numAttrs = 1;
-        int n = 0;
-        if (cudaFuncSetAttribute(lstm_batch_kernel<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lstm_batch_smem(1024, 8, 2)) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, lstm_batch_kernel<8, 2>, &lc) != cudaSuccess) {
+        if (raise_smem_limit(lstm_batch_kernel<8, 2>) != PIMB200_OK || cudaOccupancyMaxActiveClusters(&n, lstm_batch_kernel<8, 2>, &lc) != cudaSuccess) {
             cudaGetLastError();
             n = 0;
         }
-        pairs[dev] = n > 0 ? std::min(n, kBatchMaxPairs) : -1;
+        n = n > 0 ? std::min(n, kBatchMaxPairs) : -1;
+        pairs[dev].store(n, std::memory_order_relaxed);
     }
-    return std::max(pairs[dev], 0);
+    return std::max(n, 0);
 }
 
 int groups_per_dir(int H, int dirs, int dev) {
@@ -523,7 +530,7 @@ int launch_lstm_batch(BatchArgs& a, cudaStream_t st) {
     }
     const BatchFn fn = subs == 2 ? pick_nj<2>(nj) : pick_nj<1>(nj);
     const int blocks = a.H / 64;
-    PIMB200_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lstm_batch_smem(a.H, nj, subs)));
+    if ((rc = raise_smem_limit(fn)) != PIMB200_OK) return rc;
     PIMB200_CUDA_TRY(cudaMemsetAsync(a.counters, 0, (size_t)groups * a.dirs * subs * blocks * kBatchFlagWords * 4, st));
     cudaLaunchConfig_t lc;
     cudaLaunchAttribute at[2];

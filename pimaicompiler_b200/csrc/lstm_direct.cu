@@ -351,7 +351,8 @@ int launch_lstm_direct(const DirectArgs& a, int layers, cudaStream_t st) {
     const void* fn = layers == 2 ? (const void*)lstm_direct_kernel<2, 1>
                                  : (a.B <= 8 ? (const void*)lstm_direct_kernel<1, 1> : (const void*)lstm_direct_kernel<1, 2>);
     const size_t smem = direct_smem(a.H, layers);
-    PIMB200_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // (always what the largest layer needs: the limit belongs to the function, and another thread may be about to launch it)
+    PIMB200_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)direct_smem(8 * kDirectMaxCtas, layers)));
     void* kargs[] = {const_cast<DirectArgs*>(&a)};
     PIMB200_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(a.H / 8), dim3(kThreads), kargs, smem, st));
     return PIMB200_OK;

@@ -561,7 +561,8 @@ int launch_greedy_batch(GreedyBatchArgs& a, cudaStream_t st) {
         if (!encode_2d(&m.h[x], a.state + x * rows * a.PH, rows, a.PH, (uint64_t)a.PH * 2, 16 * nj, 2)) return PIMB200_ERR_UNSUPPORTED;
     const GreedyBatchFn fn = pick_nj(nj);
     const int smem = (int)greedy_batch_smem(a.PH, a.jrows, 16 * nj);
-    PIMB200_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // (always the most that any launch asks for: the limit belongs to the function, and another thread may be about to launch it)
+    PIMB200_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemPerCta));
     a.labels = a.counters + (size_t)groups * p.ctas * kExchanges * kCounterWords;
     PIMB200_CUDA_TRY(cudaMemsetAsync(a.counters, 0, (size_t)groups * (p.ctas * kExchanges * kCounterWords + kMaxUtts) * 4, st));
     void* args[] = {&m, &a};

@@ -547,6 +547,39 @@ def test_many_sequences_on_the_tensor_core_recurrence_vs_libtorch(T, B, I, H, L,
         assert_close(got, want.numpy(), LSTM_ATOL, LSTM_RTOL, name)
 
 
+@pytest.mark.parametrize("sizes", [((1024, 150), (320, 520)), ((1024, 40), (256, 40)), ((1024, 1), (64, 1))])
+def test_threads_with_handles_of_different_sizes_launch_the_same_kernel(sizes):
+    # the same instance with different amounts of shared memory, whose limit belongs to the kernel: no thread takes it from another
+    import threading
+    ops = _ops()
+    from pimaicompiler_b200 import _lib
+    g = torch.Generator().manual_seed(5)
+    T, I, jobs, failed = 8, 24, [], []
+    for H, B in sizes:
+        m = ops.Lstm([to_dev(p) for p in lstm_params(1, 1, I, H, g)], 1, False, I, H, True)
+        x = to_dev(torch.randn(T, B, I, generator=g))
+        want = m.forward(x)[0].clone()
+        jobs.append((m, x, torch.empty_like(want), want))
+    stream = torch.cuda.Stream()               # one for both: the threads meet on the host only
+    torch.cuda.synchronize()
+
+    def loop(m, x, y, want):
+        torch.cuda.set_device(0)
+        for _ in range(150):
+            if rc := _lib.lib().pimb200_lstm_forward(m._h, x.data_ptr(), T, x.shape[1], None, None, y.data_ptr(), None, None, 0, stream.cuda_stream):
+                failed.append(rc)
+
+    threads = [threading.Thread(target=loop, args=j) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
+    torch.cuda.synchronize()
+    for m, _, y, want in jobs:
+        assert m.last_status() == 0 and torch.equal(y, want)
+
+
 @pytest.mark.parametrize("H,B", [(320, 224), (512, 100), (64, 40), (1024, 300)])
 def test_trace_buffer_of_one_record_per_eight_units_is_not_overrun(H, B):
     # the recurrence for many sequences has up to 148 CTAs at any hidden size; the buffer has room for H / 8
