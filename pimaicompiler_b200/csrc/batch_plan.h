@@ -76,7 +76,25 @@ PIMB200_HD inline GreedySmem greedy_layout(int PH, int jrows, int utts) {
     s.total = s.bars + 1024;
     return s;
 }
+constexpr int kGreedyMaxCtas = 148, kGreedyMaxUtts = 80, kGreedyMaxJointRows = 64;
+struct GreedyPlan {                    // of a model; groups 0: not one of this size, or not on this device
+    int ctas, jrows;                   // CTAs of a group, joint rows of each
+    int groups, max_nj;                // groups of a launch, sixteenths of the utterances of a group
+    int capacity() const { return groups * max_nj * 16; }
+};
 inline size_t greedy_batch_smem(int PH, int jrows, int utts) { return alone_on_sm((size_t)greedy_layout(PH, jrows, utts).total + 1024 /*align*/); }
+// What fits a CTA's shared memory; then, as many groups as have all their CTAs resident at once
+inline GreedyPlan greedy_plan(int PH, int JH, size_t smem) {
+    GreedyPlan p = {};
+    p.ctas = PH / 32;
+    p.jrows = joint_rows(JH, p.ctas);
+    if (p.jrows > kGreedyMaxJointRows) return p;
+    while (p.max_nj < kGreedyMaxUtts / 16 && greedy_batch_smem(PH, p.jrows, 16 * (p.max_nj + 1)) <= smem) ++p.max_nj;
+    return p;
+}
+inline int greedy_groups(const GreedyPlan& p, int resident_ctas) {
+    return p.max_nj == 0 ? 0 : (resident_ctas < kGreedyMaxCtas ? resident_ctas : kGreedyMaxCtas) / p.ctas;
+}
 
 }  // namespace tc
 }  // namespace pimb200

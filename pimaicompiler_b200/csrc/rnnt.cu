@@ -1307,8 +1307,8 @@ struct pimb200_rnnt {
     __half *y_pre = nullptr, *y_post = nullptr;
     float* E = nullptr;
     size_t cap_frames = 0;  // frames*utts capacity of the three buffers above
-    // many utterances (rnnt_batch.cu): how many a launch takes, and what its CTAs exchange their values through
-    int batch_capacity = 0;
+    // many utterances (rnnt_batch.cu): its plan, and what its CTAs exchange their values through
+    tc::GreedyPlan batch_plan = {};
     unsigned char* batch_work = nullptr;
     size_t batch_partials = 0, batch_counters = 0;   // offsets
     long long* trace = nullptr;  // diagnostics buffer (not owned)
@@ -1511,12 +1511,16 @@ extern "C" int pimb200_rnnt_create(const pimb200_rnnt_config* cfg, const pimb200
         }
     }
     if (h->cluster == 0) return fail(PIMB200_ERR_UNSUPPORTED);
-    if ((h->batch_capacity = greedy_batch_capacity(PH, JH, V)) > 0) {
+    h->batch_plan = greedy_batch_plan(PH, JH, V);
+    if (h->batch_plan.capacity() > 0) {
         size_t state, partials, counters;
-        greedy_batch_workspace(PH, V, &state, &partials, &counters);
+        greedy_batch_workspace(PH, &state, &partials, &counters);
         h->batch_partials = state;
         h->batch_counters = state + partials;
-        if (cudaMalloc(&h->batch_work, state + partials + counters) != cudaSuccess) return fail(PIMB200_ERR_NO_MEMORY);
+        if (cudaMalloc(&h->batch_work, state + partials + counters) != cudaSuccess) {
+            cudaGetLastError();
+            h->batch_plan.groups = 0;      // the clusters take every call
+        }
     }
     *out = h;
     return PIMB200_OK;
@@ -1619,8 +1623,9 @@ static int launch_greedy(pimb200_rnnt* h, const float* E, long e_utt, long e_fra
                          int32_t* n_tokens, float* logits, cudaStream_t st) {
     const pimb200_rnnt_config& c = h->cfg;
     auto next_gen = [h] { return h->gen = h->gen == 0x7fffffff ? 1 : h->gen + 1; };
-    if (h->greedy_multi == 1 && h->batch_capacity > 0 && n_utts >= kGreedyBatchMin) {
-        const int per = ceil_div(n_utts, ceil_div(n_utts, h->batch_capacity));
+    int rc = PIMB200_ERR_UNSUPPORTED;
+    if (h->greedy_multi == 1 && h->batch_plan.capacity() > 0 && n_utts >= kGreedyBatchMin) {
+        const int per = ceil_div(n_utts, ceil_div(n_utts, h->batch_plan.capacity()));
         for (int u = 0; u < n_utts; u += per) {
             GreedyBatchArgs b = {};
             b.E = E + (size_t)u * e_utt; b.e_utt = e_utt; b.e_frame = e_frame;
@@ -1632,11 +1637,11 @@ static int launch_greedy(pimb200_rnnt* h, const float* E, long e_utt, long e_fra
             b.partials = reinterpret_cast<float*>(h->batch_work + h->batch_partials);
             b.counters = reinterpret_cast<uint32_t*>(h->batch_work + h->batch_counters);
             b.trace = h->trace; b.status = h->d_status; b.gen = next_gen(); b.poll_limit = h->poll_limit;
-            const int rc = launch_greedy_batch(b, st);
-            if (rc != PIMB200_OK) return rc;
+            rc = launch_greedy_batch(b, h->batch_plan, st);
+            if (rc != PIMB200_OK) break;
         }
-        return PIMB200_OK;
     }
+    if (rc != PIMB200_ERR_UNSUPPORTED) return rc;      // (else the clusters take all of it)
     GreedyArgs a;
     a.E = E; a.e_utt = e_utt; a.e_frame = e_frame; a.tokens = tokens; a.n_tokens = n_tokens; a.logits = logits; a.n_utts = n_utts; a.Tp = Tp;
     a.P0 = h->P0; a.Whh0 = h->Whh0; a.Wih1 = h->Wih1; a.Whh1 = h->Whh1; a.bias1 = h->bias1;

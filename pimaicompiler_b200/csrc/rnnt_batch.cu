@@ -37,13 +37,13 @@ constexpr int kFirstEpi = 3;
 constexpr int kEpiWarps = 8;
 constexpr int kUnits = 32;
 constexpr int kMaxBlocks = 5;          // PH <= 320: two matrices of 32 TMEM columns per K block of 64
-constexpr int kMaxUtts = 80;           // per group
-constexpr int kMaxJointRows = 64;      // per CTA: one K block of the product with W2
+constexpr int kMaxUtts = kGreedyMaxUtts;   // per group
+static_assert(kGreedyMaxJointRows == 64, "a CTA's joint rows are one K block of the product with W2");
 constexpr int kVocab = kGreedyVocab;
 constexpr int kACol = 192;             // TMEM: accumulators of layer 0 and of everything else at 0 and 96, Whh0, Whh1 from here
 constexpr int kCounterWords = 32;      // a counter has a 128-byte line
 constexpr int kExchanges = 3;          // h0, h1, partial logits
-constexpr int kMaxCtas = 148;
+constexpr int kMaxCtas = kGreedyMaxCtas;
 
 struct GreedyMaps {
     CUtensorMap h[2];                  // [utterances of all groups][PH], boxes of 64 units x one group
@@ -512,48 +512,44 @@ GreedyBatchFn pick_nj(int nj) {
     }
 }
 
-struct Plan { int ctas, groups, jrows, max_nj; };      // groups 0: not a model of this size
-Plan plan_for(int PH, int JH, int V) {
-    Plan p = {};
-    int dev = 0, sms = 0, smem = 0;
-    if (PH <= 0 || PH % 64 != 0 || PH / 64 > kMaxBlocks || V > kVocab || cudaGetDevice(&dev) != cudaSuccess) return p;
-    p.ctas = PH / kUnits;
-    p.jrows = joint_rows(JH, p.ctas);
-    if (p.jrows > kMaxJointRows) return p;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    while (p.max_nj < kMaxUtts / 16 && (int)greedy_batch_smem(PH, p.jrows, 16 * (p.max_nj + 1)) <= smem) ++p.max_nj;
-    if (p.max_nj > 0) p.groups = std::min(sms, kMaxCtas) / p.ctas;
-    return p;
-}
-
 }  // namespace
 }  // namespace tc
 
-int greedy_batch_capacity(int PH, int JH, int V) {
-    const tc::Plan p = tc::plan_for(PH, JH, V);
-    return p.groups * p.max_nj * 16;
+tc::GreedyPlan greedy_batch_plan(int PH, int JH, int V) {
+    using namespace tc;
+    GreedyPlan p = {};
+    int dev = 0, sms = 0, smem = 0, per_sm = 0;
+    if (PH <= 0 || PH % 64 != 0 || PH / 64 > kMaxBlocks || V > kVocab || cudaGetDevice(&dev) != cudaSuccess) return p;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    p = greedy_plan(PH, JH, (size_t)smem);
+    if (p.max_nj == 0) return p;
+    const GreedyBatchFn fn = pick_nj(p.max_nj);
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemPerCta) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, greedy_batch_smem(PH, p.jrows, 16 * p.max_nj)) != cudaSuccess) {
+        cudaGetLastError();
+        return p;
+    }
+    p.groups = greedy_groups(p, sms * per_sm);
+    return p;
 }
 
-void greedy_batch_workspace(int PH, int V, size_t* state, size_t* partials, size_t* counters) {
+void greedy_batch_workspace(int PH, size_t* state, size_t* partials, size_t* counters) {
     using namespace tc;
-    (void)V;
     const int ctas = PH / kUnits, groups = kMaxCtas / ctas;
     *state = (size_t)2 * groups * kMaxUtts * PH * 2;
     *partials = (size_t)groups * ctas * kMaxUtts * kVocab * 4;
     *counters = (size_t)groups * (ctas * kExchanges * kCounterWords + kMaxUtts) * 4;
 }
 
-int launch_greedy_batch(GreedyBatchArgs& a, cudaStream_t st) {
+int launch_greedy_batch(GreedyBatchArgs& a, const tc::GreedyPlan& p, cudaStream_t st) {
     using namespace tc;
-    const Plan p = plan_for(a.PH, a.JH, a.V);
-    if (p.groups == 0 || a.n_utts > p.groups * p.max_nj * 16) return PIMB200_ERR_UNSUPPORTED;
+    if (a.n_utts > p.capacity()) return PIMB200_ERR_UNSUPPORTED;
     int dev = 0, rc, gen;
     int* status;
     if ((rc = tc_prepare(&dev, &status, &gen)) != PIMB200_OK) return rc;     // (the tensor-map encoder)
     const int nj = ceil_div(ceil_div(a.n_utts, p.groups), 16), groups = ceil_div(a.n_utts, 16 * nj);
     a.ctas = p.ctas;
-    a.group_utts = 16 * nj;
     a.jrows = p.jrows;
     GreedyMaps m = {};
     const size_t rows = (size_t)groups * 16 * nj;
@@ -566,7 +562,10 @@ int launch_greedy_batch(GreedyBatchArgs& a, cudaStream_t st) {
     a.labels = a.counters + (size_t)groups * p.ctas * kExchanges * kCounterWords;
     PIMB200_CUDA_TRY(cudaMemsetAsync(a.counters, 0, (size_t)groups * (p.ctas * kExchanges * kCounterWords + kMaxUtts) * 4, st));
     void* args[] = {&m, &a};
-    return cuda_status(cudaLaunchCooperativeKernel((const void*)fn, dim3(groups * p.ctas), dim3(kThreads), args, smem, st));
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void*)fn, dim3(groups * p.ctas), dim3(kThreads), args, smem, st);
+    if (e != cudaErrorCooperativeLaunchTooLarge) return cuda_status(e);
+    cudaGetLastError();                        // (fewer CTAs resident than when the plan was made)
+    return PIMB200_ERR_UNSUPPORTED;
 }
 
 }  // namespace pimb200

@@ -1,5 +1,6 @@
 // Interface of the RNN-T greedy loop for many utterances (rnnt_batch.cu).
 #pragma once
+#include "batch_plan.h"
 #include "common.cuh"
 
 namespace pimb200 {
@@ -18,7 +19,7 @@ struct GreedyBatchArgs {
     const __half* W2;          // [V, JH]
     const float* b2;           // [V]
     int PH, JH, V, blank;
-    __half* state;             // greedy_batch_state_bytes: hidden states of both layers, exchanged through here
+    __half* state;             // hidden states of both layers, exchanged through here (greedy_batch_workspace)
     float* partials;           // partial logits behind them
     uint32_t* counters;
     long long* trace;          // optional: 8 clocks per frame of the first CTA
@@ -28,13 +29,13 @@ struct GreedyBatchArgs {
     // filled in by launch_greedy_batch
     uint32_t* labels;          // (behind the counters)
     int ctas;                  // per group
-    int group_utts;
     int jrows;                 // joint rows per CTA
 };
 
-// Utterances that one launch takes (0: not a model of this size), and the bytes behind state / partials / counters.
-int greedy_batch_capacity(int PH, int JH, int V);
-void greedy_batch_workspace(int PH, int V, size_t* state, size_t* partials, size_t* counters);
-int launch_greedy_batch(GreedyBatchArgs& a, cudaStream_t st);
+// The plan of a model on the current device (capacity 0: not one of its own), and the bytes behind state / partials / counters.
+tc::GreedyPlan greedy_batch_plan(int PH, int JH, int V);
+void greedy_batch_workspace(int PH, size_t* state, size_t* partials, size_t* counters);
+// PIMB200_ERR_UNSUPPORTED, with nothing launched, where the plan's CTAs are not resident at once
+int launch_greedy_batch(GreedyBatchArgs& a, const tc::GreedyPlan& plan, cudaStream_t st);
 
 }  // namespace pimb200

@@ -23,6 +23,11 @@ void debt(unsigned q, unsigned leader, unsigned other, unsigned bytes, unsigned*
 }
 unsigned first_open(unsigned uses, unsigned stages) { return first_open_use(uses, stages); }
 unsigned use_blocks(unsigned q, unsigned blocks, unsigned per_use) { return blocks_of_use(q, blocks, per_use); }
+void greedy(int PH, int JH, size_t smem, int resident, int* out) {
+    GreedyPlan p = greedy_plan(PH, JH, smem);
+    p.groups = greedy_groups(p, resident);
+    out[0] = p.ctas, out[1] = p.jrows, out[2] = p.groups, out[3] = p.max_nj, out[4] = p.capacity();
+}
 size_t greedy_smem(int PH, int JH, int utts) { return greedy_batch_smem(PH, joint_rows(JH, PH / 32), utts); }
 }
 """
@@ -47,6 +52,22 @@ def test_a_cta_of_the_batched_kernels_has_its_sm_for_itself(plan):
     for smem in sizes:
         assert 2 * (smem + reserved) > plan.smem_per_sm()
         assert smem <= plan.smem_per_cta()
+
+
+def test_groups_of_the_greedy_loop_have_all_their_ctas_resident(plan):
+    out = (ctypes.c_int * 5)()
+
+    def of(PH, JH, resident, smem=227 * 1024):
+        plan.greedy(PH, JH, ctypes.c_size_t(smem), resident, out)
+        return tuple(out)
+
+    assert of(320, 512, 148) == (10, 52, 14, 5, 1120)
+    assert of(320, 512, 9)[4] == 0 and of(320, 512, 10)[2] == 1       # fewer than a group has: the clusters take the call
+    for resident in (0, 1, 9, 74, 132, 148, 296):
+        ctas, _, groups, max_nj, capacity = of(320, 512, resident)
+        assert groups * ctas <= min(resident, 148) and capacity == groups * max_nj * 16
+    assert of(320, 1000, 148)[4] == 0                                 # more joint rows per CTA than one K block
+    assert of(320, 512, 148, smem=150 * 1024)[3] < 5 and of(320, 512, 148, smem=100 * 1024)[4] == 0
 
 
 class _Barrier:
