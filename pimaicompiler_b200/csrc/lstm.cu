@@ -2157,9 +2157,30 @@ static int grow(T** p, size_t* cap, size_t need_elems) {
     if (*p) cudaFree(*p);
     *p = nullptr;
     *cap = 0;
-    PIMB200_CUDA_TRY(cudaMalloc(p, need_elems * sizeof(T)));
+    const cudaError_t e = cudaMalloc(p, need_elems * sizeof(T));
+    if (e != cudaSuccess) {
+        cudaGetLastError();                     // (the caller may go on with less)
+        return cuda_status(e);
+    }
     *cap = need_elems;
     return PIMB200_OK;
+}
+
+// Gives the workspaces back, for a route that needs less where a larger one was refused
+static void release_workspaces(pimb200_lstm* h) {
+    cudaDeviceSynchronize();
+    auto drop = [](auto** p, size_t* cap) {
+        cudaFree(*p);
+        *p = nullptr;
+        *cap = 0;
+    };
+    drop(&h->G, &h->G_cap);
+    drop(&h->pk_x, &h->pk_x_cap);
+    drop(&h->pk_run, &h->pk_run_cap);
+    drop(&h->batch_x, &h->batch_x_cap);
+    drop(&h->cstate, &h->c_cap);
+    drop(&h->ybuf[0], &h->y_cap[0]);
+    drop(&h->ybuf[1], &h->y_cap[1]);
 }
 
 static size_t wide_smem(int H, int nt) {
@@ -2561,8 +2582,8 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
                           long y_bstride, __half* hn, __half* cn, cudaStream_t st);
 
 // the recurrence of lstm_batch.cu for a packed batch: more sequences than the kernels above take, or two directions at once
-static bool batch_fits_packed(const pimb200_lstm* h, int T, int B) {
-    return B >= batch_min(h->H, h->D) && T >= 8 && h->bulk_wide == 2 && !h->use_tc &&
+static bool batch_fits_packed(const pimb200_lstm* h, int T, int B, const __half* h0) {
+    return B >= batch_min(h->H, h->D) && T >= 8 && (!h0 || aligned16(h0)) && h->bulk_wide == 2 && !h->use_tc &&
            (h->variant == PIMB200_LSTM_AUTO || h->variant == PIMB200_LSTM_PERSISTENT) && (long)T * B * h->D <= kBatchMaxPackedRows &&
            lstm_batch_capacity(h->H, h->D) >= B;
 }
@@ -2584,13 +2605,24 @@ static int lstm_forward_packed_lockstep(pimb200_lstm* h, const __half* data, con
     const PackedMeta meta{h->pk_lens, h->pk_row0};
     int max_in = h->I;
     if (L > 1 && D * H > max_in) max_in = D * H;
-    if ((rc = grow(&h->pk_x, &h->pk_x_cap, (size_t)prow * max_in)) != PIMB200_OK) return rc;
-    const bool batch = batch_fits_packed(h, T, B) && (!h0 || aligned16(h0));
-    const size_t runs = batch ? D : 1;         // directions that are under way at once
-    if ((rc = grow(&h->pk_run, &h->pk_run_cap, runs * prow * H)) != PIMB200_OK) return rc;
-    if ((rc = grow(&h->G, &h->G_cap, runs * prow * 4 * H)) != PIMB200_OK) return rc;
-    if (L > 1 && (rc = grow(&h->ybuf[0], &h->y_cap[0], (size_t)prow * D * H)) != PIMB200_OK) return rc;
-    if (L > 2 && (rc = grow(&h->ybuf[1], &h->y_cap[1], (size_t)prow * D * H)) != PIMB200_OK) return rc;
+    // `runs`: directions that are under way at once
+    auto room = [&](size_t runs) {
+        int r = grow(&h->pk_x, &h->pk_x_cap, (size_t)prow * max_in);
+        if (r == PIMB200_OK) r = grow(&h->pk_run, &h->pk_run_cap, runs * prow * H);
+        if (r == PIMB200_OK) r = grow(&h->G, &h->G_cap, runs * prow * 4 * H);
+        if (r == PIMB200_OK && L > 1) r = grow(&h->ybuf[0], &h->y_cap[0], (size_t)prow * D * H);
+        if (r == PIMB200_OK && L > 2) r = grow(&h->ybuf[1], &h->y_cap[1], (size_t)prow * D * H);
+        return r;
+    };
+    bool batch = batch_fits_packed(h, T, B, h0);
+    rc = room(batch ? D : 1);
+    if (rc == PIMB200_ERR_NO_MEMORY && batch) {
+        release_workspaces(h);
+        if (B > kPipeMaxB) return rc;          // (the caller goes on with packed rows)
+        batch = false;                         // one direction after the other, in half the space
+        rc = room(1);
+    }
+    if (rc != PIMB200_OK) return rc;
     SeqLayout padded;
     padded.T = T; padded.B = B; padded.batch_sizes = nullptr;
     const unsigned grid = (unsigned)prow;
@@ -2707,6 +2739,7 @@ static bool batch_fits(const pimb200_lstm* h, int T, int B) {
 
 // All layers for up to lstm_batch_capacity sequences.  Output row (t, b) at y + (t / y_fold) * y_t + (t % y_fold) * H + b * y_b
 // (in halves; y_fold 1 when bidirectional).  h0, c0, hn, cn: [L * D][total][H], of which these are the B behind the pointers.
+// PIMB200_ERR_NO_MEMORY, with nothing launched, where the workspaces are refused.
 static int forward_batch(pimb200_lstm* h, const __half* x, RowStrides xs, int T, int B, int total, const __half* h0, const __half* c0,
                          __half* y, long y_t, long y_b, int y_fold, __half* hn, __half* cn, cudaStream_t st) {
     const int H = h->H, D = h->D, L = h->L;
@@ -2716,11 +2749,12 @@ static int forward_batch(pimb200_lstm* h, const __half* x, RowStrides xs, int T,
     int rc;
     const long rows = (long)chunk * B;
     const bool copy = xs.b != 1 || xs.t != B;
-    if ((rc = grow(&h->G, &h->G_cap, (size_t)rows * D * 4 * H)) != PIMB200_OK) return rc;
-    if ((rc = grow(&h->cstate, &h->c_cap, (size_t)D * B * H)) != PIMB200_OK) return rc;
-    if (copy && (rc = grow(&h->batch_x, &h->batch_x_cap, (size_t)rows * h->I)) != PIMB200_OK) return rc;
-    for (int l = 0; l + 1 < L && l < 2; ++l)
-        if ((rc = grow(&h->ybuf[l], &h->y_cap[l], (size_t)T * B * D * H)) != PIMB200_OK) return rc;
+    rc = grow(&h->G, &h->G_cap, (size_t)rows * D * 4 * H);
+    if (rc == PIMB200_OK) rc = grow(&h->cstate, &h->c_cap, (size_t)D * B * H);
+    if (rc == PIMB200_OK && copy) rc = grow(&h->batch_x, &h->batch_x_cap, (size_t)rows * h->I);
+    for (int l = 0; l + 1 < L && l < 2 && rc == PIMB200_OK; ++l) rc = grow(&h->ybuf[l], &h->y_cap[l], (size_t)T * B * D * H);
+    if (rc == PIMB200_ERR_NO_MEMORY) release_workspaces(h);
+    if (rc != PIMB200_OK) return rc;
     for (int l = 0; l < L; ++l) {
         const int Il = in_size(h, l);
         const bool last = l == L - 1;
@@ -2786,20 +2820,23 @@ static int lstm_forward_impl(pimb200_lstm* h, const __half* x, const SeqLayout& 
     int rc;
     // packed input of several steps: as a padded lock-step batch on the persistent recurrences (needs the 128-bit GEMM
     // path for the padded rows; the streamed kernels below take every other case)
-    if (packed && h->packed_lockstep && h->variant != PIMB200_LSTM_STREAMED && T > 1 && H % 16 == 0 && (B <= kPipeMaxB || batch_fits_packed(h, T, B)))
-        return lstm_forward_packed_lockstep(h, x, sq, h0, c0, y, hn, cn, st);
+    if (packed && h->packed_lockstep && h->variant != PIMB200_LSTM_STREAMED && T > 1 && H % 16 == 0 &&
+        (B <= kPipeMaxB || batch_fits_packed(h, T, B, h0))) {
+        rc = lstm_forward_packed_lockstep(h, x, sq, h0, c0, y, hn, cn, st);
+        if (rc != PIMB200_ERR_NO_MEMORY || B <= kPipeMaxB) return rc;
+    }
     // many sequences, in equal parts of what a launch takes
     if (!packed && batch_fits(h, T, B) && aligned16(y) && (!h0 || aligned16(h0)) && (!hn || aligned16(hn))) {
         const int parts = ceil_div(B, lstm_batch_capacity(H, D)), per = ceil_div(B, parts);
         const RowStrides xs = batch_first ? RowStrides{1, x_seq} : RowStrides{B, 1};
         const long y_t = (batch_first ? 1L : B) * D * H, y_b = (batch_first ? (long)T : 1L) * D * H;
-        for (int b = 0; b < B; b += per) {
+        rc = PIMB200_OK;
+        for (int b = 0; b < B && rc == PIMB200_OK; b += per) {
             const size_t off = (size_t)b * H;
-            if ((rc = forward_batch(h, x + b * xs.b * h->I, xs, T, std::min(per, B - b), B, h0 ? h0 + off : nullptr, c0 ? c0 + off : nullptr,
-                                    y + b * y_b, y_t, y_b, 1, hn ? hn + off : nullptr, cn ? cn + off : nullptr, st)) != PIMB200_OK)
-                return rc;
+            rc = forward_batch(h, x + b * xs.b * h->I, xs, T, std::min(per, B - b), B, h0 ? h0 + off : nullptr, c0 ? c0 + off : nullptr,
+                               y + b * y_b, y_t, y_b, 1, hn ? hn + off : nullptr, cn ? cn + off : nullptr, st);
         }
-        return PIMB200_OK;
+        if (rc != PIMB200_ERR_NO_MEMORY) return rc;    // (refused by the first part, ahead of any launch)
     }
     // decode form: seq_len 1, every extent a multiple of 8 and 16-byte aligned -> one fused cell launch per layer
     bool cell = !packed && T == 1 && h->variant != PIMB200_LSTM_PERSISTENT && h->variant != PIMB200_LSTM_PERSISTENT_TAGGED &&

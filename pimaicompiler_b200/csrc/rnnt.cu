@@ -1708,21 +1708,30 @@ extern "C" int pimb200_rnnt_decode(pimb200_rnnt* h, const void* feats, int T, in
         if (cap > 0) per = ceil_div(n_utts, ceil_div(n_utts, cap));
         if (per > 0 && n_utts % per != 0 && lstm_folded_capacity(h->post, Tp, n_utts % per) == 0) per = 0;
     }
-    const int group = per > 0 ? per : (h->enc_batch > 0 ? h->enc_batch : kEncoderBatch);
-    int rc;
-    for (int u = 0; u < n_utts; u += group) {
-        const int g = (n_utts - u < group) ? (n_utts - u) : group;
-        __half* y1 = h->y_pre + (size_t)u * Te * EH;
-        __half* y2 = h->y_post + (size_t)u * Tp * EH;
-        const __half* xu = x + (size_t)u * T * c.feat_dim;
-        if (per > 0) {
-            if ((rc = lstm_forward_folded(h->pre, xu, 1, T, Te, g, c.stack_factor, y1, st)) != PIMB200_OK) return rc;
-            if ((rc = lstm_forward_folded(h->post, y1, 0, 0, Tp, g, 1, y2, st)) != PIMB200_OK) return rc;
-        } else {
-            if ((rc = lstm_forward_batch_first(h->pre, xu, T, Te, g, y1, st)) != PIMB200_OK) return rc;
-            if ((rc = lstm_forward_batch_first(h->post, y1, Tp, Tp, g, y2, st)) != PIMB200_OK) return rc;
+    auto encode = [&](int group) {
+        for (int u = 0; u < n_utts; u += group) {
+            const int g = (n_utts - u < group) ? (n_utts - u) : group;
+            __half* y1 = h->y_pre + (size_t)u * Te * EH;
+            __half* y2 = h->y_post + (size_t)u * Tp * EH;
+            const __half* xu = x + (size_t)u * T * c.feat_dim;
+            int r;
+            if (per > 0) {
+                if ((r = lstm_forward_folded(h->pre, xu, 1, T, Te, g, c.stack_factor, y1, st)) != PIMB200_OK) return r;
+                if ((r = lstm_forward_folded(h->post, y1, 0, 0, Tp, g, 1, y2, st)) != PIMB200_OK) return r;
+            } else {
+                if ((r = lstm_forward_batch_first(h->pre, xu, T, Te, g, y1, st)) != PIMB200_OK) return r;
+                if ((r = lstm_forward_batch_first(h->post, y1, Tp, Tp, g, y2, st)) != PIMB200_OK) return r;
+            }
         }
+        return (int)PIMB200_OK;
+    };
+    int rc = PIMB200_ERR_NO_MEMORY;
+    if (per > 0) rc = encode(per);
+    if (rc == PIMB200_ERR_NO_MEMORY) {         // (or refused for all in lock step: smaller groups need less)
+        per = 0;
+        rc = encode(h->enc_batch > 0 ? h->enc_batch : kEncoderBatch);
     }
+    if (rc != PIMB200_OK) return rc;
     // encoder half of the joint for every frame of every utterance: one dense GEMM
     rc = launch_gemm_wx(h->W1e, h->y_post, h->b1, h->E, JH, EH, n_utts * Tp, EH, JH, PIMB200_ACT_NONE, 1, st);
     if (rc != PIMB200_OK) return rc;

@@ -8,7 +8,7 @@ import pytest
 import torch
 
 from oracle import c_oracle as co
-from tests.util import CONTRACT_ATOL, CONTRACT_RTOL, assert_close, h16, lstm_params, to_dev
+from tests.util import CONTRACT_ATOL, CONTRACT_RTOL, assert_close, device_memory_left, h16, lstm_params, to_dev
 
 pytestmark = pytest.mark.gpu
 GOLD = os.path.join(os.path.dirname(__file__), "golden")
@@ -545,6 +545,30 @@ def test_many_sequences_on_the_tensor_core_recurrence_vs_libtorch(T, B, I, H, L,
     ref = _libtorch(ps, x, h0, c0, L, bi, bf)
     for got, want, name in zip((y, hn, cn), ref, ("y", "hn", "cn")):
         assert_close(got, want.numpy(), LSTM_ATOL, LSTM_RTOL, name)
+
+
+# (T, B, H, bidirectional, packed, MiB left): the recurrence for many sequences wants the gate terms of both directions, or padded
+# rows, where the kernels before it take one direction, or packed rows
+@pytest.mark.parametrize("T,B,H,bi,packed,left", [(400, 96, 1024, True, True, 1024), (300, 150, 1024, True, False, 1100)])
+def test_smaller_workspaces_where_memory_is_short(T, B, H, bi, packed, left):
+    ops = _ops()
+    g = torch.Generator().manual_seed(B)
+    I, D = 64, 2 if bi else 1
+    ps = [to_dev(p) for p in lstm_params(1, D, I, H, g)]
+    lens = torch.linspace(T, T // 2, B).long()
+    sizes = (lens[:, None] > torch.arange(T)).sum(0)
+    x = to_dev(torch.randn(*((int(sizes.sum()), I) if packed else (T, B, I)), generator=g))
+    call = (lambda m: m.forward_packed(x, sizes)) if packed else (lambda m: m.forward(x))
+    want = [t.clone() for t in call(ops.Lstm(ps, 1, bi, I, H, True))]
+    m = ops.Lstm(ps, 1, bi, I, H, True)
+    with device_memory_left(left << 20):
+        out = call(m)
+        torch.cuda.synchronize()
+    assert m.last_status() == 0
+    for got, ref, name in zip(out, want, ("y", "hn", "cn")):
+        assert_close(got, ref.float().cpu().numpy(), LSTM_ATOL, LSTM_RTOL, name)
+    for got, ref in zip(call(m), want):                       # and with room again
+        assert torch.equal(got, ref)
 
 
 @pytest.mark.parametrize("sizes", [((1024, 150), (320, 520)), ((1024, 40), (256, 40)), ((1024, 1), (64, 1))])

@@ -5,7 +5,7 @@ import torch
 
 from oracle import c_oracle as co
 from oracle import torch_oracle as to
-from tests.util import CONTRACT_ATOL, CONTRACT_RTOL, assert_close
+from tests.util import CONTRACT_ATOL, CONTRACT_RTOL, assert_close, device_memory_left
 
 pytestmark = pytest.mark.gpu
 MARGIN = 1e-2  # token ids must match wherever the oracle's top-2 logit margin exceeds this
@@ -199,6 +199,20 @@ def test_rnnt_many_utterances_in_lock_step(n_utts, blank_bias):
         _check_utterance(cfg, w, feats[i].float(), toks[i], logits[i].cpu().numpy(), to.rnnt_greedy)
     again, logits2 = dec.decode(feats.cuda(), want_logits=True)
     assert again == toks and torch.equal(logits2, logits)
+
+
+def test_rnnt_many_utterances_where_memory_is_short():
+    # room for the encoder in groups of 128 utterances, not for all in lock step
+    cfg = to.RnntConfig()
+    w = to.make_rnnt_weights(cfg, seed=5, gain=2.0, logit_gain=8.0)
+    dec = _decoder(cfg, w)
+    n, T = 256, 400
+    feats = torch.randn(n, T, cfg.feat_dim, generator=torch.Generator().manual_seed(n)).to(torch.float16)
+    dev = feats.cuda()
+    with device_memory_left(2300 << 20):
+        toks, logits = dec.decode(dev, want_logits=True)
+    for i in (0, 200):
+        _check_utterance(cfg, w, feats[i].float(), toks[i], logits[i].cpu().numpy(), to.rnnt_greedy)
 
 
 def test_rnnt_many_utterances_time_out_and_recover():

@@ -1,4 +1,6 @@
 """Shared helpers of the parity tests."""
+import contextlib
+
 import numpy as np
 import torch
 
@@ -42,3 +44,17 @@ def lstm_params(L, D, I, H, gen, scale=None, has_biases=True):
                 ps.append(h16((torch.rand(4 * H, generator=gen) * 2 - 1) * k))
                 ps.append(h16((torch.rand(4 * H, generator=gen) * 2 - 1) * k))
     return ps
+
+
+@contextlib.contextmanager
+def device_memory_left(free_bytes):
+    """All device memory but about `free_bytes` is taken."""
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    hold = torch.empty(max(0, torch.cuda.mem_get_info()[0] - free_bytes), dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        torch.cuda.synchronize()
+        del hold
+        torch.cuda.empty_cache()
