@@ -2501,8 +2501,9 @@ static int run_recurrence(pimb200_lstm* h, int ld, const SeqLayout& sq, bool rev
 //   * the input is scattered into padded time-major rows (zeros behind each sequence); the backward direction gets
 //     every sequence reversed on its own, so it too is a forward recurrence that starts at the sequence's first step
 //     with the caller's initial state, and its outputs are reversed back when they are stored;
-//   * behind a sequence's end the gate terms of its input and forget gates are set to -1e4 / +1e4: sigmoid gives exactly
-//     0 and 1, the cell state stays frozen, so the kernel's c_n is the state after the sequence's own last step;
+//   * behind a sequence's end the gate terms of its input and forget gates are set to -inf / +inf: sigmoid gives exactly
+//     0 and 1 whatever finite product is added, the cell state stays frozen, so the kernel's c_n is the state after the
+//     sequence's own last step;
 //     h_n is the output row of that step, picked up when the outputs are stored.
 // ---------------------------------------------------------------------------------------------
 constexpr long kBatchChunkRows = 131072;     // rows of gate terms per chunk (2 GB at H = 1024)
@@ -2556,7 +2557,7 @@ __global__ void lstm_freeze_gates_kernel(float* __restrict__ G, PackedMeta m, in
     const int t = (int)(row / B), b = (int)(row % B);
     if (t < m.lens[b]) return;
     float4* g = reinterpret_cast<float4*>(G + row * 4L * H);
-    for (int u = threadIdx.x; u < H; u += blockDim.x) g[u] = make_float4(-1.0e4f, 1.0e4f, 0.f, 0.f);
+    for (int u = threadIdx.x; u < H; u += blockDim.x) g[u] = make_float4(-INFINITY, INFINITY, 0.f, 0.f);
 }
 
 // Stores the outputs of one direction's padded run (src [T, B, H], contiguous): row (t, b) of the run is timestep

@@ -547,6 +547,32 @@ def test_many_sequences_on_the_tensor_core_recurrence_vs_libtorch(T, B, I, H, L,
         assert_close(got, want.numpy(), LSTM_ATOL, LSTM_RTOL, name)
 
 
+@pytest.mark.parametrize("B,H,bi", [(3, 64, False), (20, 64, False), (40, 64, True), (70, 256, False), (150, 256, False)])
+def test_packed_sequences_end_under_products_of_any_size(B, H, bi):
+    # recurrent weights whose products are far beyond the range of a gate: behind a sequence's end nothing reaches its cell state
+    ops = _ops()
+    g = torch.Generator().manual_seed(B)
+    T, I, D = 12, 16, 2 if bi else 1
+    ps = lstm_params(1, D, I, H, g)
+    for d in range(D):
+        ps[4 * d] = h16(ps[4 * d].abs() * 4)                         # positive states: gates fully open, c grows by one a step
+        ps[4 * d + 1] = torch.full((4 * H, H), 1000.0)
+    x = h16(torch.rand(T, B, I, generator=g) + 0.5)
+    lens = torch.randint(1, T + 1, (B,), generator=g).sort(descending=True).values
+    lens[0] = T
+    packed = torch.nn.utils.rnn.pack_padded_sequence(x, lens)
+    zero = torch.zeros(D, B, H)
+    with torch.backends.mkldnn.flags(enabled=False):
+        ref = torch.lstm(packed.data, packed.batch_sizes, [zero, zero], ps, True, 1, 0.0, False, bi)
+    assert float(ref[2].min()) < T - 3 and float(ref[2].max()) > T - 1
+    m = ops.Lstm([to_dev(p) for p in ps], 1, bi, I, H, True)
+    got = m.forward_packed(to_dev(packed.data), packed.batch_sizes)
+    torch.cuda.synchronize()
+    assert m.last_status() == 0
+    for a, b, name in zip(got, ref, ("y", "hn", "cn")):
+        assert_close(a, b.numpy(), LSTM_ATOL, LSTM_RTOL, name)
+
+
 # (T, B, H, bidirectional, packed, MiB left): the recurrence for many sequences wants the gate terms of both directions, or padded
 # rows, where the kernels before it take one direction, or packed rows
 @pytest.mark.parametrize("T,B,H,bi,packed,left", [(400, 96, 1024, True, True, 1024), (300, 150, 1024, True, False, 1100)])
