@@ -473,8 +473,8 @@ __device__ __forceinline__ float ex2_(float x) {
     return r;
 }
 
-template <int C>
-__global__ void __launch_bounds__(kBahdanauThreads, C == 8 ? 3 : 4) bahdanau_kernel(
+template <int C, int PER_SM>
+__global__ void __launch_bounds__(kBahdanauThreads, PER_SM) bahdanau_kernel(
     const __half* q, const __half* keys_proj, const __half* values,
     const long long* lengths, const __half* v, const __half* bias, __half* __restrict__ ctx,
     float* __restrict__ scores, long max_len, int H, long row_stride, long seq_stride, long ctx_stride, int copies, long copy_stride) {
@@ -899,12 +899,12 @@ extern "C" int pimb200_attention_rows_packed(const void* q, const void* K, const
 }
 
 namespace {
-template <int C>
+template <int C, int PER_SM>
 int launch_bahdanau(const __half* q, const __half* kp, const __half* values, const long long* lengths, const __half* v, const __half* bias,
                     __half* ctx, float* scores, int n_seq, long max_len, int H, long row_stride, long seq_stride, long ctx_stride, int copies,
                     long copy_stride, cudaStream_t st) {
     const size_t smem = ((size_t)2 * H + 8 * kBahdanauThreads + max_len) * sizeof(float);
-    return cuda_status(launch_pdl<C>(bahdanau_kernel<C>, dim3(C, n_seq), dim3(kBahdanauThreads), smem, st, q, kp, values, lengths, v, bias, ctx,
+    return cuda_status(launch_pdl<C>(bahdanau_kernel<C, PER_SM>, dim3(C, n_seq), dim3(kBahdanauThreads), smem, st, q, kp, values, lengths, v, bias, ctx,
                                      scores, max_len, H, row_stride, seq_stride, ctx_stride, copies, copy_stride));
 }
 }  // namespace
@@ -931,19 +931,22 @@ extern "C" int pimb200_additive_attention_copies(const void* q, const void* keys
     if (H % 8 == 0 && row_stride % 8 == 0 && seq_stride % 8 == 0 && ctx_stride % 8 == 0 && copy_stride % 8 == 0 && aligned16(keys_proj) &&
         aligned16(values) && aligned16(ctx) && ((size_t)2 * H + 8 * kBahdanauThreads + max_len) * sizeof(float) + 64 <= 48 * 1024) {
         // CTAs per sentence: as many as are resident at once, if the pieces of a row split evenly: a CTA's own chain is what takes the
-        // time (256 sentences with one CTA each took 24 us, 512 26).  Four per SM with 64 registers a thread; eight CTAs per sentence,
-        // which only few sentences have, take more registers (16 sentences: 6.2 us, 7.0 with 64).
-        // 128 sentences: 12.5 us with two, 10.6 with four; 256: 23.9 with one, 16.4 with two
+        // time.  Four per SM leave 64 registers a thread, which spills, so grids that three per SM hold have 80 (20 / 50 keys, us with
+        // three / four per SM: 64 sentences 6.4 / 7.4 and 8.9 / 10.7; 104: 6.8 / 7.8 and 9.3 / 11.3; 200: 8.3 / 10.1 and 14.0 / 18.0;
+        // 400: 11.4 / 14.3 and 23.0 / 29.6).  Clusters do not fill every SM: of four CTAs, 104 fit with three per SM (106: 10.8) and 141
+        // with four (144: 11.4), of two CTAs all of 222 and 296.  More CTAs than are resident cost more than fewer CTAs per sentence
+        // (128 sentences of 20 keys: 8.0 with four, 8.1 with two, 9.7 with one; 148: 12.7, 8.2, 7.0; 256: 10.4 with two, 11.0 with one)
         auto run = [&](auto f) {
             return f(static_cast<const __half*>(q), static_cast<const __half*>(keys_proj), static_cast<const __half*>(values), lengths,
                      static_cast<const __half*>(v), static_cast<const __half*>(bias), static_cast<__half*>(ctx), scores, n_seq, max_len, H,
                      row_stride, seq_stride, ctx_stride, copies, copy_stride, st);
         };
         auto fits = [&](int c) { return (H / 8) % c == 0 && H / 8 / c <= kBahdanauThreads && kBahdanauThreads % (H / 8 / c) == 0; };
-        for (int c = 8; c >= 1; c /= 2) {
-            if (!fits(c) || (c > 1 && (long)n_seq * c > (c == 8 ? 2 : 4) * kNumSmB200)) continue;
-            return c == 8 ? run(launch_bahdanau<8>) : c == 4 ? run(launch_bahdanau<4>) : c == 2 ? run(launch_bahdanau<2>) : run(launch_bahdanau<1>);
-        }
+        const long sms = kNumSmB200, n = n_seq, lost = 28;         // (CTAs that clusters of four leave out)
+        if (fits(8) && 8 * n <= 2 * sms) return run(launch_bahdanau<8, 3>);
+        if (fits(4) && 4 * n <= 4 * sms - lost) return 4 * n <= 3 * sms - lost ? run(launch_bahdanau<4, 3>) : run(launch_bahdanau<4, 4>);
+        if (fits(2) && 2 * n <= 4 * sms) return 2 * n <= 3 * sms ? run(launch_bahdanau<2, 3>) : run(launch_bahdanau<2, 4>);
+        if (fits(1)) return n <= 3 * sms ? run(launch_bahdanau<1, 3>) : run(launch_bahdanau<1, 4>);
     }
     const long rows = (long)n_seq * max_len;
     const int rc = cuda_status(launch_pdl(

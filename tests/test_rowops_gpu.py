@@ -281,6 +281,21 @@ def test_additive_attention_clusters_beside_other_work(n):
     assert all(torch.equal(o, ref) for o in outs)
 
 
+@pytest.mark.parametrize("n", [37, 38, 103, 104, 140, 141, 222, 223, 296, 297, 444, 445])
+def test_additive_attention_where_the_ctas_of_a_sentence_change(n):
+    # eight, four, two and one CTAs per sentence, three and four of them per SM: the first and the last of each
+    from pimaicompiler_b200 import ops
+    g = torch.Generator().manual_seed(n)
+    S, H = 21, 1024
+    q, v, b = (torch.randn(*s, generator=g).half().cuda() for s in ((n, H), (H,), (H,)))
+    kp, val = (torch.randn(S, n, H, generator=g).half().cuda() for _ in range(2))
+    ln = torch.randint(1, S + 1, (n,), generator=g).cuda()
+    got = ops.additive_attention(q, kp, val, ln, v * 0.05, b)
+    e = (torch.tanh(kp.float() + (q.float() + b.float())) * (v * 0.05).float()).sum(2)
+    e = e.masked_fill(torch.arange(S, device="cuda")[:, None] >= ln, float("-inf"))
+    assert_close(got, (torch.softmax(e, 0)[:, :, None] * val.float()).sum(0), 2e-3, 2e-3, "context")
+
+
 @pytest.mark.parametrize("n", [1, 20, 40, 80, 300])
 def test_additive_attention_copies(n):
     # one to eight CTAs per sentence, the context written three times
