@@ -4,8 +4,10 @@
 // HIP GEMV templates (runtime/include/executor/op_executor/custom_ops.h).  All of them are
 // HBM-bandwidth bound: 128-bit coalesced loads that bypass L1, fp32 accumulation, warp-shuffle
 // reductions and the bias / ReLU epilogue fused into the same kernel.
+#include <atomic>
 #include <mutex>
 
+#include "batch_plan.h"
 #include "common.cuh"
 
 namespace pimb200 {
@@ -65,20 +67,24 @@ __global__ void __launch_bounds__(256) gemv_mv_vec_kernel(const __half* __restri
 
 // The same for small matrices, where start and ramp are half the time.  The launch may start while its predecessor is still
 // running: it then asks for its rows of W to be brought into L2 (which is coherent, so it does not matter whether anyone still
-// writes them) and reads everything behind the wait, by plain loads.  In a loop of launches with cold weights, former kernel /
-// this one: 1024 x 1024 2.57 / 2.50 us, 4096 x 1024 3.42 / 3.18.  From 8 M elements on the read-only path of the former counts
-// for more: 16384 x 1024 7.40 / 7.66, 32320 x 1024 12.7 / 13.5, 32768 x 4096 42.5 / 45.9.
-// (The rows of W are asked for on a switch that is an argument and always set.  Without it the kernel needs 32 registers instead
-// of 34, eight CTAs fit an SM instead of six, and 4096 x 1024 takes 3.41: launches two ahead then ask for their rows too.)
+// writes them) and reads everything behind the wait, by plain loads.  The launcher leaves room on an SM for this launch's share of CTAs
+// and one more: where registers allow six and the grid is two per SM, CTAs that start as their predecessors leave pile up on some
+// SMs.  In a loop of launches, W in HBM / in L2, us, kernel above, this one with room for six, and as it is:
+//   1024 x 1024 2.78 / 2.19, 2.27 / 1.90, 1.95 / 1.74    2000 x 4096 6.6 / 4.3, 6.5 / 5.8, 5.3 / 4.0
+//   4096 x 1024 3.62 / 2.70, 3.09 / 2.66, 2.62 / 2.35    5000 x 1024 4.5 / 2.7, 4.0 / 3.4, 3.9 / 2.8
+// (Room for exactly its share is faster still in such a loop and slower among other launches, which find no room beside it: a cell's
+// step behind it 8.8 us in all, 10.1.)
+// From 8 M elements on the read-only path of the former counts for more: 16384 x 1024 7.40, 7.66 here; 32320 x 1024 12.7, 13.5;
+// 32768 x 4096 42.5, 45.9.
 constexpr size_t kMvEarlyMax = (size_t)8 << 20;     // elements
+constexpr int kMvMaxPerSm = 5;                      // (registers allow no more than six)
 template <int R>
-__global__ void __launch_bounds__(256) gemv_mv_early_kernel(const __half* W, const __half* x, const __half* bias, __half* y, int N, int K, int act,
-                                                            int ahead) {
+__global__ void __launch_bounds__(256) gemv_mv_early_kernel(const __half* W, const __half* x, const __half* bias, __half* y, int N, int K, int act) {
     pdl_launch_dependents();
     const int K8 = K >> 3;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row0 = (blockIdx.x * (blockDim.x >> 5) + warp) * R;
-    if (ahead && lane < R && row0 + lane < N) prefetch_l2(W + (size_t)(row0 + lane) * K, (uint32_t)K * 2);
+    if (lane < R && row0 + lane < N) prefetch_l2(W + (size_t)(row0 + lane) * K, (uint32_t)K * 2);
     pdl_wait();
     if (row0 >= N) return;
 
@@ -130,8 +136,23 @@ static int launch_gemv_mv(const __half* W, const __half* x, const __half* bias, 
     const int R = warps4 >= want ? 4 : (warps2 >= want ? 2 : 1);
     const int grid = ceil_div(N, 8 * R);
     if ((size_t)N * K < kMvEarlyMax) {
-        const auto early = R == 4 ? gemv_mv_early_kernel<4> : R == 2 ? gemv_mv_early_kernel<2> : gemv_mv_early_kernel<1>;
-        return cuda_status(launch_pdl(early, dim3(grid), dim3(256), 0, st, W, x, bias, y, N, K, act, 1));
+        static void (*const early[3])(const __half*, const __half*, const __half*, __half*, int, int, int) = {
+            gemv_mv_early_kernel<1>, gemv_mv_early_kernel<2>, gemv_mv_early_kernel<4>};
+        const auto fn = early[R / 2];
+        // CTAs per SM, by an amount of shared memory that nothing uses: this launch's share and one more
+        const int per_sm = ceil_div(grid, kNumSmB200) + 1;
+        size_t room = 0;
+        if (per_sm <= kMvMaxPerSm) {
+            room = tc::kSmemPerSm / per_sm - 1024;             // (1 KB of a CTA's share is the system's)
+            static std::atomic<bool> allowed[64][3];
+            int dev = 0;
+            PIMB200_CUDA_TRY(cudaGetDevice(&dev));
+            if (dev >= 64 || !allowed[dev][R / 2].load(std::memory_order_relaxed)) {
+                PIMB200_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(tc::kSmemPerSm / 2 - 1024)));
+                if (dev < 64) allowed[dev][R / 2].store(true, std::memory_order_relaxed);
+            }
+        }
+        return cuda_status(launch_pdl(fn, dim3(grid), dim3(256), room, st, W, x, bias, y, N, K, act));
     }
     if (R == 4) gemv_mv_vec_kernel<4><<<grid, 256, 0, st>>>(W, x, bias, y, N, K, act);
     else if (R == 2) gemv_mv_vec_kernel<2><<<grid, 256, 0, st>>>(W, x, bias, y, N, K, act);

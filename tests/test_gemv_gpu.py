@@ -63,6 +63,20 @@ def test_gemv_vm_matches_oracle(N, K):
     assert_close(y2, co.vm(x[0].numpy(), A.numpy()), GEMV_ATOL, GEMV_RTOL, f"vm {K}x{N} second call")
 
 
+# one, two and four rows per warp; two to five CTAs per SM by their shared memory, and more; the largest below 8 M elements and the
+# first at it
+@pytest.mark.parametrize("N,K", [(1, 8), (9, 40), (1184, 72), (2000, 520), (2369, 264), (3553, 136), (4736, 64), (4737, 64), (7105, 96),
+                                 (9473, 56), (14209, 40), (18945, 24), (40000, 8), (2, 1000000), (8191, 1024), (8192, 1024)])
+def test_matrix_vector_product_that_starts_early(N, K):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(K + N)
+    W, x, b = ((torch.randn(*s, generator=g, device="cuda") * f).half() for s, f in (((N, K), K ** -0.5), ((K,), 1.0), ((N,), 1.0)))
+    ref = torch.relu(W.double() @ x.double() + b.double()).cpu().numpy()
+    out = torch.full((N + 64,), 7.0, dtype=torch.float16, device="cuda")
+    assert_close(ops.gemv_mv(W, x, b, ops.ACT_RELU, out=out[:N]), ref, GEMV_ATOL, GEMV_RTOL, f"mv {N}x{K}")
+    assert bool((out[N:] == 7.0).all())
+
+
 @pytest.mark.parametrize("K,N", [(1024, 4096), (320, 1280)])
 def test_reference_unit_test_shapes_and_tolerance(K, N):
     # customGemvTest / pimCustomGemvTest (runtime/unit-tests/custom_op_ut.cpp:20-148): x~U[0,1) fp16,
