@@ -6,6 +6,7 @@
 // reductions and the bias / ReLU epilogue fused into the same kernel.
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 
 #include "batch_plan.h"
 #include "common.cuh"
@@ -378,19 +379,42 @@ __global__ void __launch_bounds__(256) gemv_vm_cluster_kernel(const __half* x, c
     }
 }
 
-// S: about four CTAs per SM, at least four passes over the rows per CTA
+// Column tile and slices of K: as many slices as keep every CTA resident at once (a second wave of a few CTAs costs as much as the
+// first: 20000 columns x 4096 36.7 us with eight slices of 256 columns, 27.6 with seven, 29.2 by the split through memory), with at
+// least four passes over the rows in each.  Narrow tiles hold 5.2 CTAs per SM, wide ones 4.  Wide tiles from where narrow ones would
+// have less than four slices (12000 columns x 4096: 17.3 us in narrow ones, 18.9 in wide ones; 14000: 25.6 and 20.4), and up to
+// K = 1024 from where they fill a quarter of the SMs (9480 x 512: 4.1 us, 5.1 in narrow ones).
+struct VmSplit {
+    bool wide;
+    int tiles, slices;
+};
+static VmSplit split_vm(int K, int N) {
+    const int narrow = ceil_div(N, 64);
+    const int narrow_most = kNumSmB200 * 26 / 5;
+    const bool wide = narrow * 4 > narrow_most || (K <= 1024 && ceil_div(N, 256) >= kNumSmB200 / 4);
+    VmSplit v{wide, wide ? ceil_div(N, 256) : narrow, 8};
+    const int passes = K / (wide ? 8 : 32), most = wide ? kNumSmB200 * 4 : narrow_most;
+    while (v.slices > 1 && (v.tiles * v.slices > most || passes < 4 * v.slices)) --v.slices;
+    return v;
+}
 template <int LPR>
-static int launch_gemv_vm_cluster(const __half* x, const __half* A, const __half* bias, __half* y, int K, int N, int act, cudaStream_t st) {
-    const int tiles = ceil_div(N, LPR * 8), passes = K / (8 * (32 / LPR));
-    int S = 1;
-    while (S < 8 && tiles * S * 2 <= 6 * kNumSmB200 && passes / (2 * S) >= 4) S *= 2;
-    const dim3 grid(tiles * S), block(256);
-    const int rows = ceil_div(K, S);
-    switch (S) {
-        case 1: return cuda_status(launch_pdl<1>(gemv_vm_cluster_kernel<LPR, 1>, grid, block, 0, st, x, A, bias, y, K, N, act, rows));
-        case 2: return cuda_status(launch_pdl<2>(gemv_vm_cluster_kernel<LPR, 2>, grid, block, 0, st, x, A, bias, y, K, N, act, rows));
-        case 4: return cuda_status(launch_pdl<4>(gemv_vm_cluster_kernel<LPR, 4>, grid, block, 0, st, x, A, bias, y, K, N, act, rows));
-        default: return cuda_status(launch_pdl<8>(gemv_vm_cluster_kernel<LPR, 8>, grid, block, 0, st, x, A, bias, y, K, N, act, rows));
+static int launch_gemv_vm_cluster(const __half* x, const __half* A, const __half* bias, __half* y, int K, int N, int act, const VmSplit& v,
+                                  cudaStream_t st) {
+    const dim3 grid(v.tiles * v.slices), block(256);
+    const int rows = ceil_div(K, v.slices);
+    auto run = [&](auto slices) {
+        constexpr int S = decltype(slices)::value;
+        return cuda_status(launch_pdl<S>(gemv_vm_cluster_kernel<LPR, S>, grid, block, 0, st, x, A, bias, y, K, N, act, rows));
+    };
+    switch (v.slices) {
+        case 1: return run(std::integral_constant<int, 1>());
+        case 2: return run(std::integral_constant<int, 2>());
+        case 3: return run(std::integral_constant<int, 3>());
+        case 4: return run(std::integral_constant<int, 4>());
+        case 5: return run(std::integral_constant<int, 5>());
+        case 6: return run(std::integral_constant<int, 6>());
+        case 7: return run(std::integral_constant<int, 7>());
+        default: return run(std::integral_constant<int, 8>());
     }
 }
 
@@ -436,11 +460,11 @@ static int launch_gemv_vm(const __half* x, const __half* A, const __half* bias, 
     }
     DeviceCtx* ctx = allow_split ? current_ctx() : nullptr;
     if (allow_split && !ctx) return PIMB200_ERR_NOT_INIT;
-    // one phase up to K = 4096, and up to 8192 where eight CTAs per tile fill the SMs twice (1024 columns: 12.1 us, 10.5 with the split
-    // through memory; 4096 columns: 15.2, 22.6)
-    const bool wide = ceil_div(N, 256) >= kNumSmB200 / 4;
-    if (K <= 4096 || (K <= 8192 && ceil_div(N, wide ? 256 : 64) * 8 >= 2 * kNumSmB200))
-        return wide ? launch_gemv_vm_cluster<32>(x, A, bias, y, K, N, act, st) : launch_gemv_vm_cluster<8>(x, A, bias, y, K, N, act, st);
+    // one phase up to K = 4096, and up to 8192 where its CTAs fill the SMs twice (1024 columns: 12.1 us, 10.5 with the split through
+    // memory; 4096 columns: 15.2, 22.6)
+    const VmSplit v = split_vm(K, N);
+    if (K <= 4096 || (K <= 8192 && v.tiles * v.slices >= 2 * kNumSmB200))
+        return v.wide ? launch_gemv_vm_cluster<32>(x, A, bias, y, K, N, act, v, st) : launch_gemv_vm_cluster<8>(x, A, bias, y, K, N, act, v, st);
     float* partials = nullptr;
     unsigned int* tickets = nullptr;
     VmPlan p;

@@ -63,6 +63,21 @@ def test_gemv_vm_matches_oracle(N, K):
     assert_close(y2, co.vm(x[0].numpy(), A.numpy()), GEMV_ATOL, GEMV_RTOL, f"vm {K}x{N} second call")
 
 
+# narrow column tiles with eight to four slices of K, wide ones with eight to four, first and last of each; rows that the slices do not
+# divide, columns that the tiles do not, few rows, and up to 8192 rows in one phase and through memory
+@pytest.mark.parametrize("K,N", [(1001, 72), (4095, 264), (1023, 6144), (997, 6152), (1025, 7048), (1003, 8200), (999, 9480), (1026, 9864),
+                                 (515, 12288), (515, 12296), (1003, 19008), (777, 24400), (643, 28200), (643, 33000), (65, 20000), (31, 40000),
+                                 (6000, 72), (6001, 4096), (8191, 1024), (8192, 9480), (8200, 520)])
+def test_vector_matrix_product_in_slices(K, N):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(K + N)
+    A, x, b = ((torch.randn(*s, generator=g, device="cuda") * f).half() for s, f in (((K, N), K ** -0.5), ((K,), 1.0), ((N,), 1.0)))
+    ref = torch.relu(x.double() @ A.double() + b.double()).cpu().numpy()
+    out = torch.full((N + 64,), 7.0, dtype=torch.float16, device="cuda")
+    assert_close(ops.gemv_vm(x, A, b, ops.ACT_RELU, out=out[:N]), ref, GEMV_ATOL, GEMV_RTOL, f"vm {K}x{N}")
+    assert bool((out[N:] == 7.0).all())
+
+
 # one, two and four rows per warp; two to five CTAs per SM by their shared memory, and more; the largest below 8 M elements and the
 # first at it
 @pytest.mark.parametrize("N,K", [(1, 8), (9, 40), (1184, 72), (2000, 520), (2369, 264), (3553, 136), (4736, 64), (4737, 64), (7105, 96),
