@@ -575,7 +575,8 @@ int launch_gemm_rows(const __half* W, const __half* X, const __half* bias, void*
     }
     const int es = y_is_f32 ? 4 : 2, tail = a.jrows % 32, whole = a.jrows < 32 ? a.jrows : 32;
     a.Y = Y; a.ldy = ldy;
-    a.direct = !aligned16(Y) || (long)ldy * es % 16 != 0;
+    // (a store through a map writes whole 16 bytes: the last of a row of another width would reach into what lies behind it)
+    a.direct = !aligned16(Y) || ((long)ldy * es | (long)N * es) % 16 != 0;
     if (a.direct && ((long)ldy * es | (long)(reinterpret_cast<uintptr_t>(Y))) % 4 == 0) a.direct = 2;
     if (a.direct) m.y = m.x;   // (prefetched only)
     else if (!encode_2d(&m.y, Y, J, N, (uint64_t)ldy * es, whole, es) ||

@@ -214,6 +214,21 @@ def test_gemm_row_tiles(N, K, J, f32):
     assert _lib.lib().pimb200_gemm_last_status() == 0
 
 
+# rows of Y that start at 16-byte boundaries and end between them: what lies behind them in a wider buffer stays
+@pytest.mark.parametrize("N", [65, 130, 2001, 2002, 2004])
+@pytest.mark.parametrize("J", [33, 130, 520])
+@pytest.mark.parametrize("f32", [False, True])
+def test_columns_behind_the_result_stay(N, J, f32):
+    ops = _ops()
+    K = 2056
+    g = torch.Generator(device="cuda").manual_seed(N + J)
+    W, X = ((torch.randn(*s, generator=g, device="cuda") * f).half() for s, f in (((N, K), K ** -0.5), ((J, K), 1.0)))
+    out = torch.full((J, (N + 39) // 8 * 8), 7.0, dtype=torch.float32 if f32 else torch.float16, device="cuda")
+    ref = (X.double() @ W.double().T).cpu().numpy()
+    assert_close(ops.gemm_wx(W, X, None, ops.ACT_NONE, out=out[:, :N]), ref, 1e-4 if f32 else GEMV_ATOL, 1e-4 if f32 else GEMV_RTOL, f"{N}x{K}x{J}")
+    assert bool((out[:, N:] == 7.0).all())
+
+
 @pytest.mark.parametrize("N,K,J", [(1, 1, 2), (63, 9, 3), (64, 63, 64), (65, 65, 65), (129, 127, 2), (1280, 761, 130), (333, 2047, 40), (70, 130, 300)])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_ragged_gemm(N, K, J, shift):
