@@ -109,26 +109,48 @@ __device__ __forceinline__ void store_half16(__half* p, const uint32_t* w) {
 }
 
 // Rows of a warp's staged chunk (128 bytes each, 16-byte pieces swapped by row) to rows of Y that start at `at`, `ldy` elements apart.
-// pairs: every row starts at a multiple of 4 bytes.  Not inlined: the kernel's loop has no registers for it
+// pairs: every row starts at a multiple of 4 bytes.  Halves eight rows at a time, each lane its own out of shared memory (pairs
+// exchanged between lanes, row by row: 33 rows of 2001 x 512 8.1 us, now 6.7).  Not inlined: the kernel's loop has no registers for it
 template <bool F32>
 __device__ __noinline__ void store_rows(const unsigned char* buf, void* Y, size_t at, long ldy, int rows, int cols, bool pairs) {
     const int lane = threadIdx.x & 31;
+    auto piece = [&](int rr, int p) { return buf + rr * 128 + ((p ^ (rr & 7)) << 4); };
+    if constexpr (F32) {
 #pragma unroll 4
-    for (int rr = 0; rr < rows; ++rr, at += ldy) {
-        // 4 bytes per lane: piece lane / 4 of the row, which lies at (lane / 4) ^ (rr & 7)
-        const uint32_t w = *reinterpret_cast<const uint32_t*>(buf + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
-        if (F32) {
+        for (int rr = 0; rr < rows; ++rr, at += ldy) {
+            const uint32_t w = *reinterpret_cast<const uint32_t*>(piece(rr, lane >> 2) + (lane & 3) * 4);
             if (lane < cols) static_cast<float*>(Y)[at + lane] = __uint_as_float(w);
-        } else if (pairs) {
-            __half* y = static_cast<__half*>(Y) + at + 2 * lane;
-            if (2 * lane + 1 < cols) *reinterpret_cast<uint32_t*>(y) = w;
-            else if (2 * lane < cols) *reinterpret_cast<uint16_t*>(y) = (uint16_t)w;
-        } else {
-            // 2-byte stores of neighbours: lane l takes elements l and 32 + l
-            const uint32_t lo = __shfl_sync(0xffffffffu, w, lane >> 1), hi = __shfl_sync(0xffffffffu, w, 16 + (lane >> 1));
-            uint16_t* y = static_cast<uint16_t*>(Y) + at;
-            if (lane < cols) y[lane] = (uint16_t)(lane & 1 ? lo >> 16 : lo);
-            if (32 + lane < cols) y[32 + lane] = (uint16_t)(lane & 1 ? hi >> 16 : hi);
+        }
+        return;
+    }
+    constexpr int AT_ONCE = 8;             // (the chunk has 32 rows: those behind the last one are read, not stored)
+    uint16_t* y = static_cast<uint16_t*>(Y) + at;
+    if (pairs) {
+        for (int r0 = 0; r0 < rows; r0 += AT_ONCE) {
+            uint32_t w[AT_ONCE];
+#pragma unroll
+            for (int i = 0; i < AT_ONCE; ++i) w[i] = *reinterpret_cast<const uint32_t*>(piece(r0 + i, lane >> 2) + (lane & 3) * 4);
+#pragma unroll
+            for (int i = 0; i < AT_ONCE; ++i, y += ldy) {
+                if (r0 + i >= rows) return;
+                if (2 * lane + 1 < cols) *reinterpret_cast<uint32_t*>(y + 2 * lane) = w[i];
+                else if (2 * lane < cols) y[2 * lane] = (uint16_t)w[i];
+            }
+        }
+        return;
+    }
+    for (int r0 = 0; r0 < rows; r0 += AT_ONCE) {
+        uint16_t lo[AT_ONCE], hi[AT_ONCE];                 // 2-byte stores of neighbours: lane l takes elements l and 32 + l
+#pragma unroll
+        for (int i = 0; i < AT_ONCE; ++i) {
+            lo[i] = *reinterpret_cast<const uint16_t*>(piece(r0 + i, lane >> 3) + (lane & 7) * 2);
+            hi[i] = *reinterpret_cast<const uint16_t*>(piece(r0 + i, 4 + (lane >> 3)) + (lane & 7) * 2);
+        }
+#pragma unroll
+        for (int i = 0; i < AT_ONCE; ++i, y += ldy) {
+            if (r0 + i >= rows) return;
+            if (lane < cols) y[lane] = lo[i];
+            if (32 + lane < cols) y[32 + lane] = hi[i];
         }
     }
 }

@@ -229,6 +229,21 @@ def test_columns_behind_the_result_stay(N, J, f32):
     assert bool((out[:, N:] == 7.0).all())
 
 
+# rows of Y that no tensor map takes, stored by the warps eight at a time: one to 32 rows in a warp, even and odd widths, a ragged last column
+@pytest.mark.parametrize("N", [65, 130, 2001, 2498])
+@pytest.mark.parametrize("J", [33, 39, 40, 41, 63, 64, 65, 131])
+@pytest.mark.parametrize("f32", [False, True])
+def test_rows_that_no_tensor_map_takes(N, J, f32):
+    ops = _ops()
+    K = 2056                                            # (a matrix that the few-row kernel leaves to the tensor cores from 33 rows)
+    g = torch.Generator(device="cuda").manual_seed(N + J)
+    W, X, b = ((torch.randn(*s, generator=g, device="cuda") * f).half() for s, f in (((N, K), K ** -0.5), ((J, K), 1.0), ((N,), 1.0)))
+    ref = (X.double() @ W.double().T + b.double()).cpu().numpy()
+    out = torch.full((J, N + 25 - N % 2 * 3), 7.0, dtype=torch.float32 if f32 else torch.float16, device="cuda")
+    assert_close(ops.gemm_wx(W, X, b, ops.ACT_NONE, out=out[:, :N]), ref, 1e-4 if f32 else GEMV_ATOL, 1e-4 if f32 else GEMV_RTOL, f"{N}x{K}x{J}")
+    assert bool((out[:, N:] == 7.0).all())
+
+
 @pytest.mark.parametrize("N,K,J", [(1, 1, 2), (63, 9, 3), (64, 63, 64), (65, 65, 65), (129, 127, 2), (1280, 761, 130), (333, 2047, 40), (70, 130, 300)])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_ragged_gemm(N, K, J, shift):
