@@ -58,13 +58,16 @@ struct SkinnyArgs {
 // in flight while the current one is multiplied.
 // UB: 32-wide K blocks per register buffer.  One is all that a warp has at K <= 512, and leaves room for CTAs of the launches behind
 // this one on the same SM (20 rows: 250 registers with buffers of four).
-template <int NT, int MTW, int UB>
-__global__ void __launch_bounds__(kSkinnyThreads, UB == 1 ? 2 : 1) gemm_skinny_kernel(const __grid_constant__ SkinnyArgs a) {
+// AHEAD: both buffers are under way before the first product; else the second one is asked for ahead of the first one's products.
+// PER_SM: CTAs that an SM has to hold (0: as the compiler likes).  The arguments come by value: as a grid constant they give the
+// form of <1, 2, 2, false, 0> other registers and 20 % more time.
+template <int NT, int MTW, int UB, bool AHEAD, int PER_SM>
+__global__ void __launch_bounds__(kSkinnyThreads, PER_SM) gemm_skinny_kernel(SkinnyArgs a) {
     constexpr int KS = kSkinnyWarps;
     constexpr int ROWS = MTW * kSkinnyRows;
     __shared__ float part[KS][ROWS][NT * 8 + 1];
     pdl_launch_dependents();
-    if (!a.fixed) pdl_wait();
+    if (!AHEAD || !a.fixed) pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int n0 = blockIdx.x * ROWS;
@@ -126,23 +129,46 @@ __global__ void __launch_bounds__(kSkinnyThreads, UB == 1 ? 2 : 1) gemm_skinny_k
                     mma16816(acc[m][j], w[u][m][0].z, w[u][m][1].z, w[u][m][0].w, w[u][m][1].w, x[u][j].z, x[u][j].w);
                 }
     };
-    // two register buffers used alternately (no copies between them: a move would wait for the load it moves); weights that
-    // nobody writes are on their way before the predecessor has ended
-    if (a.fixed) {
-        load_w(wc, b_lo);
-        load_w(wn, b_lo + UB);
-        pdl_wait();
-        load_x(xc, b_lo);
-        load_x(xn, b_lo + UB);
+    // two register buffers used alternately (no copies between them: a move would wait for the load it moves)
+    if constexpr (AHEAD) {
+        if (a.fixed) {             // weights that nobody writes are on their way before the predecessor has ended
+            load_w(wc, b_lo);
+            load_w(wn, b_lo + UB);
+            pdl_wait();
+            load_x(xc, b_lo);
+            load_x(xn, b_lo + UB);
+        } else {
+            load_w(wc, b_lo); load_x(xc, b_lo);
+            load_w(wn, b_lo + UB); load_x(xn, b_lo + UB);
+        }
+        for (int b0 = b_lo; b0 < b_hi; b0 += 2 * UB) {
+            multiply(wc, xc);
+            load_w(wc, b0 + 2 * UB); load_x(xc, b0 + 2 * UB);
+            multiply(wn, xn);
+            load_w(wn, b0 + 3 * UB); load_x(xn, b0 + 3 * UB);
+        }
     } else {
-        load_w(wc, b_lo); load_x(xc, b_lo);
-        load_w(wn, b_lo + UB); load_x(xn, b_lo + UB);
-    }
-    for (int b0 = b_lo; b0 < b_hi; b0 += 2 * UB) {
-        multiply(wc, xc);
-        load_w(wc, b0 + 2 * UB); load_x(xc, b0 + 2 * UB);
-        multiply(wn, xn);
-        load_w(wn, b0 + 3 * UB); load_x(xn, b0 + 3 * UB);
+        auto load = [&](uint4 (&w)[UB][MTW][2], uint4 (&x)[UB][NT], int b0) {
+#pragma unroll
+            for (int u = 0; u < UB; ++u) {
+                const int b = b0 + u;
+                const bool in = b < b_hi && b * 32 + 8 * t < K;
+#pragma unroll
+                for (int m = 0; m < MTW; ++m) {
+                    w[u][m][0] = in ? ld_stream_v4(wrow[m][0] + (size_t)b * 32) : zero;
+                    w[u][m][1] = in ? ld_stream_v4(wrow[m][1] + (size_t)b * 32) : zero;
+                }
+#pragma unroll
+                for (int j = 0; j < NT; ++j) x[u][j] = in ? ld_v4(xrow[j] + (size_t)b * 32) : zero;
+            }
+        };
+        load(wc, xc, b_lo);
+        for (int b0 = b_lo; b0 < b_hi; b0 += 2 * UB) {
+            load(wn, xn, b0 + UB);
+            multiply(wc, xc);
+            load(wc, xc, b0 + 2 * UB);
+            multiply(wn, xn);
+        }
     }
     // accumulator layout: (row g, cols 2t, 2t+1), (row g+8, same cols) of each n-tile
 #pragma unroll
@@ -563,20 +589,33 @@ int launch_gemm_wx_skinny(const __half* W, const __half* X, const __half* bias, 
     // K blocks per buffer (two buffers per warp).  16 weight rows: as few as hold the warp's share of K, at most four.  32: one at
     // K <= 512, and where a second CTA per SM has work (8192 x 2048, 1 / 20 / 32 rows: 5.1 / 7.4 / 9.0 us with two, 3.9 / 6.4 / 8.0
     // with one), else two (4096 x 1024, 20 rows: 2.8 us, 4.0 with one).
-    static void (*const narrow[3][4])(SkinnyArgs) = {
-        {gemm_skinny_kernel<1, 1, 1>, gemm_skinny_kernel<2, 1, 1>, gemm_skinny_kernel<3, 1, 1>, gemm_skinny_kernel<4, 1, 1>},
-        {gemm_skinny_kernel<1, 1, 2>, gemm_skinny_kernel<2, 1, 2>, gemm_skinny_kernel<3, 1, 2>, gemm_skinny_kernel<4, 1, 2>},
-        {gemm_skinny_kernel<1, 1, 4>, gemm_skinny_kernel<2, 1, 4>, gemm_skinny_kernel<3, 1, 4>, gemm_skinny_kernel<4, 1, 4>}};
-    static void (*const broad[2][4])(SkinnyArgs) = {
-        {gemm_skinny_kernel<1, 2, 1>, gemm_skinny_kernel<2, 2, 1>, gemm_skinny_kernel<3, 2, 1>, gemm_skinny_kernel<4, 2, 1>},
-        {gemm_skinny_kernel<1, 2, 2>, gemm_skinny_kernel<2, 2, 2>, gemm_skinny_kernel<3, 2, 2>, gemm_skinny_kernel<4, 2, 2>}};
-    const bool one_wave = grid.x * grid.y <= kNumSmB200;
-    // up to 8 rows against several waves of CTAs: two where weights are loaded ahead of the wait or the waves are many (32320 x 1024,
-    // 2 rows: 11.9 / 13.4 us with two / one ahead of it, 13.2 / 13.8 behind), else one (16384 x 1024: 8.2 / 7.75).  17..24 rows
-    // at K <= 1024: two ahead of the wait (1024 x 1024: 2.5 / 3.1), one behind (512 x 768: 3.3 / 3.1)
-    const bool ahead = fixed || grid.x > 4 * kNumSmB200;
-    void (*const kernel)(SkinnyArgs) = wide ? broad[K > 512 ? one_wave || (nt == 1 && ahead) : one_wave && nt == 3][nt - 1]
-                                              : narrow[K <= 512 || (nt == 3 && K <= 1024 && !fixed) ? 0 : K <= 1024 ? 1 : 2][nt - 1];
+#define PIMB200_ROW(MTW, UB, AHEAD, PER_SM) \
+    {gemm_skinny_kernel<1, MTW, UB, AHEAD, PER_SM>, gemm_skinny_kernel<2, MTW, UB, AHEAD, PER_SM>, \
+     gemm_skinny_kernel<3, MTW, UB, AHEAD, PER_SM>, gemm_skinny_kernel<4, MTW, UB, AHEAD, PER_SM>}
+    static void (*const narrow[3][4])(SkinnyArgs) = {PIMB200_ROW(1, 1, true, 2), PIMB200_ROW(1, 2, true, 1), PIMB200_ROW(1, 4, true, 1)};
+    static void (*const broad[2][4])(SkinnyArgs) = {PIMB200_ROW(2, 1, true, 2), PIMB200_ROW(2, 2, true, 1)};
+#undef PIMB200_ROW
+    const int ctas = grid.x * grid.y;
+    void (*kernel)(SkinnyArgs);
+    if (wide) {
+        const bool one_wave = ctas <= kNumSmB200;
+        // up to 8 rows whose weights are loaded ahead of the wait: two in any number of waves (32320 x 1024, 2 rows: 11.9, 13.4 with one)
+        kernel = broad[K > 512 ? one_wave || (nt == 1 && fixed) : one_wave && nt == 3][nt - 1];
+        // Behind the wait, up to 16 rows and more CTAs than two per SM hold: as many CTAs per SM as registers allow, the buffers one
+        // after the other (12000 x 768, 2 / 12 rows: 5.7 / 6.4 us, 6.4 / 8.2 with both under way; 16384 x 512, 2 rows: 5.1 / 5.5; 24000 x
+        // 1024: 9.9 / 10.5; 32320 x 1024, weights in L2: 8.5 / 9.7).  17..24 rows in more than one wave: the buffers one after the other
+        // (8192 x 1024: 5.9 / 6.5)
+        if (!fixed && nt <= 2 && ctas > 2 * kNumSmB200)
+            kernel = nt == 2 ? gemm_skinny_kernel<2, 2, 1, false, 0> : K <= 512 ? gemm_skinny_kernel<1, 2, 1, false, 0> : gemm_skinny_kernel<1, 2, 2, false, 0>;
+        else if (!fixed && nt == 3 && !one_wave) kernel = gemm_skinny_kernel<3, 2, 1, false, 2>;
+    } else {
+        int form = K <= 512 ? 0 : K <= 1024 ? 1 : 2;
+        // behind the wait: 17..24 rows with one (512 x 768: 3.1 us, 3.3 with two), and 9..24 rows of more than 32 CTAs at K > 768 with four
+        // (1024 x 1024, 16 / 24 rows: 2.9 / 3.3, 3.1 / 3.7 with fewer)
+        if (!fixed && nt == 3 && K <= 1024) form = 0;
+        if (!fixed && (nt == 2 || nt == 3) && K > 768 && grid.x > 32) form = 2;
+        kernel = narrow[form][nt - 1];
+    }
     const cudaError_t rc = launch_pdl(kernel, grid, dim3(kSkinnyThreads), 0, st, a);
     return cuda_status(rc);
 }

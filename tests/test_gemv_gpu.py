@@ -214,6 +214,19 @@ def test_gemm_row_tiles(N, K, J, f32):
     assert _lib.lib().pimb200_gemm_last_status() == 0
 
 
+# forms of the few-row kernel: 16 weight rows with one, two and four K blocks per buffer, 32 with one and two, both buffers under way or
+# one, few CTAs and many; and blocks of 32 rows
+@pytest.mark.parametrize("N,K", [(512, 512), (528, 776), (1000, 1024), (1040, 1032), (2048, 520), (4096, 1024), (4800, 1000), (8208, 520), (9500, 776)])
+@pytest.mark.parametrize("J", [1, 8, 9, 17, 24, 25, 32, 40])
+def test_few_row_kernel_forms(N, K, J):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(N + K + J)
+    W, X, b = ((torch.randn(*s, generator=g, device="cuda") * f).half() for s, f in (((N, K), K ** -0.5), ((J, K), 1.0), ((N,), 1.0)))
+    ref = torch.relu(X.double() @ W.double().T + b.double()).cpu().numpy()
+    assert_close(ops.gemm_wx(W, X, b, ops.ACT_RELU), ref, GEMV_ATOL, GEMV_RTOL, f"{N}x{K}x{J}")
+    assert_close(ops.gemm_wx(W, X, b, ops.ACT_RELU, out_f32=True), ref, 1e-4, 1e-4, f"f32 {N}x{K}x{J}")
+
+
 # rows of Y that start at 16-byte boundaries and end between them: what lies behind them in a wider buffer stays
 @pytest.mark.parametrize("N", [65, 130, 2001, 2002, 2004])
 @pytest.mark.parametrize("J", [33, 130, 520])
