@@ -201,7 +201,9 @@ __global__ void __launch_bounds__(kSkinnyThreads, PER_SM) gemm_skinny_kernel(Ski
 // As two products and a gate kernel a step of 9 sequences (2048 inputs, H = 1024) took 12.8 us, the first 1.1 of each
 // kernel in launch and ramp; one launch takes 8.9.  The weights are constants of the handle, so the first group of them is
 // loaded before the kernel's predecessor has finished.
-template <int NT>
+// BLOCKS: more than 32 sequences, in blocks of 32 (of their own instance: with the block's start in a register 9..16 sequences of
+// 320..768 units took 3..8 % longer)
+template <int NT, bool BLOCKS>
 __global__ void __launch_bounds__(kSkinnyThreads) lstm_cell_skinny_kernel(const __grid_constant__ RowsCell a) {
     constexpr int KS = kSkinnyWarps, ROWS = 2 * kSkinnyRows, UB = 2;
     __shared__ float part[KS][ROWS][NT * 8 + 1];
@@ -209,7 +211,7 @@ __global__ void __launch_bounds__(kSkinnyThreads) lstm_cell_skinny_kernel(const 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int n0 = blockIdx.x * ROWS;                              // 4H is a multiple of 32
-    const int j_base = blockIdx.y * kSkinnyMaxJ, J = min(a.J - j_base, kSkinnyMaxJ);   // this CTA's sequences
+    const int j_base = BLOCKS ? blockIdx.y * kSkinnyMaxJ : 0, J = BLOCKS ? min(a.J - j_base, kSkinnyMaxJ) : a.J;   // this CTA's sequences
     const int bx = a.I >> 5, blocks = bx + (a.h0 ? a.H >> 5 : 0);  // 32-wide K blocks of both products
     const int per = (blocks + KS - 1) / KS;
     const int b_lo = min(blocks, warp * per), b_hi = min(blocks, b_lo + per);
@@ -260,7 +262,7 @@ __global__ void __launch_bounds__(kSkinnyThreads) lstm_cell_skinny_kernel(const 
                 }
     };
     // the CTA's rows of both matrices, 128 to 256 KB, on their way into L2 while the predecessor finishes
-    if (blockIdx.y > 0) {
+    if (BLOCKS && blockIdx.y > 0) {
     } else if (threadIdx.x < 32) prefetch_l2(a.Wx + (size_t)(n0 + lane) * a.I, (uint32_t)a.I * 2);
     else if (threadIdx.x < 64 && a.h0) prefetch_l2(a.Wh + (size_t)(n0 + lane) * a.H, (uint32_t)a.H * 2);
     load_w(wc, b_lo);
@@ -624,11 +626,12 @@ int launch_lstm_cell_skinny(const RowsCell& c, cudaStream_t st) {
     if (c.J < 1 || c.J > 65535 * kSkinnyMaxJ || c.I % 32 != 0 || c.H % 32 != 0 || c.x_ld % 8 != 0 || !aligned16(c.x) || (c.h0 && !aligned16(c.h0)))
         return PIMB200_ERR_UNSUPPORTED;
     const dim3 grid(4 * c.H / (2 * kSkinnyRows), ceil_div(c.J, kSkinnyMaxJ)), block(kSkinnyThreads);
-    switch (grid.y > 1 ? 4 : ceil_div(c.J, 8)) {
-        case 1: return cuda_status(launch_pdl(lstm_cell_skinny_kernel<1>, grid, block, 0, st, c));
-        case 2: return cuda_status(launch_pdl(lstm_cell_skinny_kernel<2>, grid, block, 0, st, c));
-        case 3: return cuda_status(launch_pdl(lstm_cell_skinny_kernel<3>, grid, block, 0, st, c));
-        default: return cuda_status(launch_pdl(lstm_cell_skinny_kernel<4>, grid, block, 0, st, c));
+    if (grid.y > 1) return cuda_status(launch_pdl(lstm_cell_skinny_kernel<4, true>, grid, block, 0, st, c));
+    switch (ceil_div(c.J, 8)) {
+        case 1: return cuda_status(launch_pdl(lstm_cell_skinny_kernel<1, false>, grid, block, 0, st, c));
+        case 2: return cuda_status(launch_pdl(lstm_cell_skinny_kernel<2, false>, grid, block, 0, st, c));
+        case 3: return cuda_status(launch_pdl(lstm_cell_skinny_kernel<3, false>, grid, block, 0, st, c));
+        default: return cuda_status(launch_pdl(lstm_cell_skinny_kernel<4, false>, grid, block, 0, st, c));
     }
 }
 
