@@ -286,10 +286,19 @@ def test_recurrence_kernels_at_the_edges_of_their_ranges(B, L, H):
 
 @pytest.mark.parametrize("B,L", [(3, 2), (8, 2), (3, 1), (9, 1), (20, 1), (70, 1)])
 def test_initial_state_of_nans_with_every_bit_set(B, L):
+    _nan_state(B, L, 256)
+
+
+@pytest.mark.parametrize("B", [70, 128])
+def test_initial_state_of_nans_in_two_halves_of_a_large_layer(B):
+    _nan_state(B, 1, 1024)
+
+
+def _nan_state(B, L, H):
     # 0xffff is a NaN and the exchange's mark of a record that has not arrived
     ops = _ops()
     g = torch.Generator().manual_seed(B)
-    T, I, H = 12, 24, 256
+    T, I = 12, 24
     m = ops.Lstm([to_dev(p) for p in lstm_params(L, 1, I, H, g)], L, False, I, H, True)
     x, h0, c0 = (to_dev(torch.randn(*s, generator=g)) for s in ((T, B, I), (L, B, H), (L, B, H)))
     want = [t.clone() for t in m.forward(x, h0, c0)]
@@ -305,11 +314,21 @@ def test_initial_state_of_nans_with_every_bit_set(B, L):
 @pytest.mark.parametrize("L,B,T", [(1, 1, 10), (1, 1, 11), (1, 8, 12), (1, 16, 13), (2, 1, 8), (2, 3, 9), (2, 8, 10), (3, 2, 11),
                                    (1, 20, 8), (1, 40, 10), (2, 70, 11), (1, 128, 9)])
 def test_captured_recurrence_replayed_among_eager_calls(L, B, T):
+    _captured_among_eager_calls(L, B, T, 256)
+
+
+@pytest.mark.parametrize("L,B,T", [(2, 70, 11), (1, 128, 9)])
+def test_captured_recurrence_of_a_large_layer(L, B, T):
+    # 65..128 sequences of 1024 units: the pipelined kernel in two halves
+    _captured_among_eager_calls(L, B, T, 1024)
+
+
+def _captured_among_eager_calls(L, B, T, H):
     # a call that was captured and never run, and replays of graphs with one, two or three recurrences of a handle between
     # eager calls: always what a handle of its own gives, bit for bit
     ops = _ops()
     g = torch.Generator().manual_seed(L * 100 + B)
-    I, H = 24, 256
+    I = 24
     ps = [to_dev(p) for p in lstm_params(L, 1, I, H, g)]
     m = ops.Lstm(ps, L, False, I, H, True)
     xs = [to_dev(torch.randn(T, B, I, generator=g)) for _ in range(7)]
