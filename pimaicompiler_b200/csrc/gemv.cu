@@ -380,17 +380,18 @@ __global__ void __launch_bounds__(256) gemv_vm_cluster_kernel(const __half* x, c
 }
 
 // Column tile and slices of K: as many slices as keep every CTA resident at once (a second wave of a few CTAs costs as much as the
-// first: 20000 columns x 4096 36.7 us with eight slices of 256 columns, 27.6 with seven, 29.2 by the split through memory), with at
-// least four passes over the rows in each.  Narrow tiles hold 5.2 CTAs per SM, wide ones 4.  Wide tiles from where narrow ones would
-// have less than four slices (12000 columns x 4096: 17.3 us in narrow ones, 18.9 in wide ones; 14000: 25.6 and 20.4), and up to
-// K = 1024 from where they fill a quarter of the SMs (9480 x 512: 4.1 us, 5.1 in narrow ones).
+// first: 20000 columns x 4096 36.7 us with eight slices of 256 columns, 27.0 with seven, 29.3 by the split through memory), with at
+// least four passes over the rows in each.  Narrow tiles hold 5.25 CTAs per SM (7000 x 4096: 770 CTAs 11.7..12.0 us, 660 12.6, 880
+// 17.1), wide ones 4.  Wide tiles from where narrow ones would have less than four slices (12000 columns x 4096: 17.3 us in narrow
+// ones, 18.9 in wide ones; 14000: 25.6 and 20.4), and up to K = 1024 from where they fill a quarter of the SMs (9480 x 512: 4.1 us,
+// 5.1 in narrow ones).
 struct VmSplit {
     bool wide;
     int tiles, slices;
 };
 static VmSplit split_vm(int K, int N) {
     const int narrow = ceil_div(N, 64);
-    const int narrow_most = kNumSmB200 * 26 / 5;
+    const int narrow_most = kNumSmB200 * 21 / 4;
     const bool wide = narrow * 4 > narrow_most || (K <= 1024 && ceil_div(N, 256) >= kNumSmB200 / 4);
     VmSplit v{wide, wide ? ceil_div(N, 256) : narrow, 8};
     const int passes = K / (wide ? 8 : 32), most = wide ? kNumSmB200 * 4 : narrow_most;
