@@ -37,6 +37,22 @@ inline size_t lstm_batch_smem(int H, int nj, int subs) {
     return alone_on_sm((size_t)own * kBlockBytes + kRingBytes + 1024 /*align*/ + 512 /*barriers*/);
 }
 
+// Launch of B sequences where `most` groups are resident, each with up to 256: as many groups as there are, and two sub-batches where
+// a group has more than the 32 columns that cost as much as 16
+struct LstmBatchPlan {
+    int groups, subs, nj;
+};
+inline LstmBatchPlan lstm_batch_plan(int B, int most) {
+    auto up = [](int a, int b) { return (a + b - 1) / b; };
+    LstmBatchPlan p;
+    p.groups = most < up(B, 16) ? most : up(B, 16);
+    p.subs = up(B, p.groups) > 32 ? 2 : 1;
+    p.nj = up(up(B, p.groups * p.subs), 16);
+    if (p.nj == 7) p.nj = 8;               // (sixteen gate warps share an even number of octets)
+    p.groups = up(B, p.subs * p.nj * 16);
+    return p;
+}
+
 // Stage uses of a CTA pair, numbered from 0: each CTA asks for its half of use q's copies, and the bytes of both count at the
 // leader's barrier of stage q % STAGES, where the leader expects them when it asks for its own half.  A pair that gave up may
 // have asked for different numbers of uses.  What the leader then adds to the barrier of use q, so that its phase completes

@@ -610,13 +610,13 @@ int launch_gemm_rows(const __half* W, const __half* X, const __half* bias, void*
 int gemm_rows_max_parts(int N) { return 2 * ceil_div(N, 64); }
 
 int launch_gemm_rows_argmax(const __half* W, const __half* X, const __half* bias, float* best_v, int* best_i, int* parts, int N,
-                            int K, int J, int ldx, cudaStream_t st, int fixed) {
+                            int K, int J, int ldx, cudaStream_t st) {
     using namespace tc;
     if (!operands_ok(W, X, K, ldx)) return PIMB200_ERR_UNSUPPORTED;
     Args a = {};
     int dev = 0, rc;
     if ((rc = tc_prepare(&dev, &a.status, &a.gen)) != PIMB200_OK) return rc;
-    a.bias = bias; a.N = N; a.J = J; a.act = PIMB200_ACT_NONE; a.fixed = fixed;
+    a.bias = bias; a.N = N; a.J = J; a.act = PIMB200_ACT_NONE;
     a.jrows = tile_rows(J);
     a.kb1 = ceil_div(K, BK);
     const Plan p = pick(N, J, a.jrows, a.kb1, 32, tc_sm_count(dev));

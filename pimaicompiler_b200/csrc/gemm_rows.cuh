@@ -31,7 +31,7 @@ int launch_gemm_rows(const __half* W, const __half* X, const __half* bias, void*
 // The largest of fp16(X W^T + bias) of every row in pieces: best_v / best_i [*parts][J], *parts <= gemm_rows_max_parts(N).
 int gemm_rows_max_parts(int N);
 int launch_gemm_rows_argmax(const __half* W, const __half* X, const __half* bias, float* best_v, int* best_i, int* parts, int N,
-                            int K, int J, int ldx, cudaStream_t st, int fixed = 0);
+                            int K, int J, int ldx, cudaStream_t st);
 
 // One LSTM step of J sequences: gates = X Wx^T + H0 Wh^T + bias (H0 may be NULL), cell update, y = h (+ residual)
 struct RowsCell {

@@ -637,9 +637,9 @@ int launch_lstm_cell_skinny(const RowsCell& c, cudaStream_t st) {
 
 // The arg max form for up to 32 activation rows: best_v / best_i [*parts][J]
 int launch_skinny_argmax(const __half* W, const __half* X, const __half* bias, float* best_v, int* best_i, int* parts, int N, int K,
-                         int J, int ldx, cudaStream_t st, int fixed) {
+                         int J, int ldx, cudaStream_t st) {
     if (J < 1 || J > kSkinnyMaxJ || K % 64 != 0 || ldx % 8 != 0 || !aligned16(W) || !aligned16(X)) return PIMB200_ERR_UNSUPPORTED;
-    const SkinnyArgs a{W, X, bias, nullptr, N, K, J, ldx, 0, PIMB200_ACT_NONE, 0, best_v, best_i, fixed};
+    const SkinnyArgs a{W, X, bias, nullptr, N, K, J, ldx, 0, PIMB200_ACT_NONE, 0, best_v, best_i, 0};
     const int nt = ceil_div(J, 8);
     *parts = skinny_rows_grid(N, (size_t)nt * 8 * K * 2);
     switch (nt) {

@@ -8,7 +8,7 @@
 namespace pimb200 {
 
 int launch_skinny_argmax(const __half* W, const __half* X, const __half* bias, float* best_v, int* best_i, int* parts, int N, int K,
-                         int J, int ldx, cudaStream_t st, int fixed);
+                         int J, int ldx, cudaStream_t st);
 
 namespace {
 
@@ -103,7 +103,7 @@ extern "C" int pimb200_greedy_token_step(const void* W, const void* X, const voi
     float* best_v = static_cast<float*>(workspace);
     int parts = J <= 32 ? kMaxParts : gemm_rows_max_parts(N);
     int* best_i = reinterpret_cast<int*>(best_v + (size_t)parts * J);
-    const int rc = J <= 32 ? launch_skinny_argmax(w, x, b, best_v, best_i, &parts, N, K, J, ldx, st, 0)
+    const int rc = J <= 32 ? launch_skinny_argmax(w, x, b, best_v, best_i, &parts, N, K, J, ldx, st)
                            : launch_gemm_rows_argmax(w, x, b, best_v, best_i, &parts, N, K, J, ldx, st);
     if (rc != PIMB200_OK) return rc;
     auto run = [&](auto kernel, int slices) {

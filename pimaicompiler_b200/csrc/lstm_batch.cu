@@ -436,16 +436,16 @@ __global__ void __launch_bounds__(threads_of(NJ), 1) lstm_batch_kernel(const __g
 }
 
 using BatchFn = void (*)(BatchMaps, BatchArgs);
-template <int SUBS>
-BatchFn pick_nj(int nj) {
+// one sub-batch has up to 32 columns, each of two more than 16
+BatchFn pick(int nj, int subs) {
+    if (subs == 1) return nj == 1 ? lstm_batch_kernel<1, 1> : lstm_batch_kernel<2, 1>;
     switch (nj) {
-        case 1: return lstm_batch_kernel<1, SUBS>;
-        case 2: return lstm_batch_kernel<2, SUBS>;
-        case 3: return lstm_batch_kernel<3, SUBS>;
-        case 4: return lstm_batch_kernel<4, SUBS>;
-        case 5: return lstm_batch_kernel<5, SUBS>;
-        case 6: return lstm_batch_kernel<6, SUBS>;
-        default: return lstm_batch_kernel<8, SUBS>;
+        case 2: return lstm_batch_kernel<2, 2>;
+        case 3: return lstm_batch_kernel<3, 2>;
+        case 4: return lstm_batch_kernel<4, 2>;
+        case 5: return lstm_batch_kernel<5, 2>;
+        case 6: return lstm_batch_kernel<6, 2>;
+        default: return lstm_batch_kernel<8, 2>;
     }
 }
 
@@ -509,18 +509,14 @@ int launch_lstm_batch(BatchArgs& a, cudaStream_t st) {
     int dev = 0, rc, gen;
     int* status;
     if ((rc = tc_prepare(&dev, &status, &gen)) != PIMB200_OK) return rc;
-    int groups = groups_per_dir(a.H, a.dirs, dev);
-    if (groups == 0 || a.B > groups * 256 || a.y_bstride % 8 != 0 || a.y_tstride % 8 != 0 || a.T % a.y_fold != 0) return PIMB200_ERR_UNSUPPORTED;
+    const int most = groups_per_dir(a.H, a.dirs, dev);
+    if (most == 0 || a.B > most * 256 || a.y_bstride % 8 != 0 || a.y_tstride % 8 != 0 || a.T % a.y_fold != 0) return PIMB200_ERR_UNSUPPORTED;
     for (int d = 0; d < a.dirs; ++d) {
         const BatchDir& r = a.dir[d];
         if (!aligned16(r.y) || (r.hn && !aligned16(r.hn)) || (r.h0 && !aligned16(r.h0)) || !aligned16(r.Whh)) return PIMB200_ERR_UNSUPPORTED;
     }
-    // as many groups as there are, and two sub-batches where a group has more than the 32 columns that cost as much as 16
-    groups = std::min(groups, ceil_div(a.B, 16));
-    const int subs = ceil_div(a.B, groups) > 32 ? 2 : 1;
-    int nj = ceil_div(ceil_div(a.B, groups * subs), 16);
-    if (nj == 7) nj = 8;                   // (sixteen gate warps share an even number of octets)
-    groups = ceil_div(a.B, subs * nj * 16);
+    const LstmBatchPlan plan = lstm_batch_plan(a.B, most);
+    const int groups = plan.groups, subs = plan.subs, nj = plan.nj;
     BatchMaps m = {};
     for (int d = 0; d < a.dirs; ++d) {
         const BatchDir& r = a.dir[d];
@@ -528,7 +524,7 @@ int launch_lstm_batch(BatchArgs& a, cudaStream_t st) {
         m.h0[d] = m.h[d];
         if (r.h0 && !encode_3d(&m.h0[d], r.h0, a.H, a.B, 1, (uint64_t)a.H * 2, (uint64_t)a.B * a.H * 2, 8 * nj)) return PIMB200_ERR_UNSUPPORTED;
     }
-    const BatchFn fn = subs == 2 ? pick_nj<2>(nj) : pick_nj<1>(nj);
+    const BatchFn fn = pick(nj, subs);
     const int blocks = a.H / 64;
     if ((rc = raise_smem_limit(fn)) != PIMB200_OK) return rc;
     PIMB200_CUDA_TRY(cudaMemsetAsync(a.counters, 0, (size_t)groups * a.dirs * subs * blocks * kBatchFlagWords * 4, st));

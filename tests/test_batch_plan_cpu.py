@@ -14,6 +14,10 @@ extern "C" {
 size_t smem_per_sm() { return kSmemPerSm; }
 size_t smem_per_cta() { return kSmemPerCta; }
 size_t lstm_smem(int H, int nj, int subs) { return lstm_batch_smem(H, nj, subs); }
+void batch(int B, int most, int* out) {
+    const LstmBatchPlan p = lstm_batch_plan(B, most);
+    out[0] = p.groups, out[1] = p.subs, out[2] = p.nj;
+}
 int stages(int nj) { return stages_of(nj); }
 int per_stage(int nj) { return blocks_per_stage(nj); }
 void debt(unsigned q, unsigned leader, unsigned other, unsigned bytes, unsigned* out) {
@@ -68,6 +72,18 @@ def test_groups_of_the_greedy_loop_have_all_their_ctas_resident(plan):
         assert groups * ctas <= min(resident, 148) and capacity == groups * max_nj * 16
     assert of(320, 1000, 148)[4] == 0                                 # more joint rows per CTA than one K block
     assert of(320, 512, 148, smem=150 * 1024)[3] < 5 and of(320, 512, 148, smem=100 * 1024)[4] == 0
+
+
+def test_every_batch_has_an_instance_of_the_recurrence(plan):
+    instances = {(1, 1), (2, 1), (2, 2), (3, 2), (4, 2), (5, 2), (6, 2), (8, 2)}       # those that are compiled
+    out, seen = (ctypes.c_int * 3)(), set()
+    for most in (1, 2, 4, 7, 14, 37, 74):
+        for B in range(1, 256 * most + 1):
+            plan.batch(B, most, out)
+            groups, subs, nj = out
+            assert 1 <= groups <= most and groups * subs * nj * 16 >= B > (groups - 1) * subs * nj * 16
+            seen.add((nj, subs))
+    assert seen == instances
 
 
 class _Barrier:
