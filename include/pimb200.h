@@ -291,8 +291,9 @@ int pimb200_lstm_destroy(pimb200_lstm* h);
 
 /* variant selection for A/B profiling: 0 = automatic, 1 = streamed per-step kernels,
  * 2 = persistent weight-stationary kernels (one cooperative launch per layer and direction; W_hh slice in registers,
- * flag + bulk-copy exchange, 1..64 sequences, H a multiple of 16 up to 1024; larger H falls back to the variants with
- * W_hh in shared memory; fails with UNSUPPORTED when the shape does not fit), 3 = persistent with the tagged-word
+ * flag + bulk-copy exchange, 1..128 sequences, H a multiple of 16 up to 1024; any number of sequences of at least 8 steps
+ * where H is a multiple of 64; larger H falls back to the variants with W_hh in shared memory; fails with UNSUPPORTED when the
+ * shape does not fit), 3 = persistent with the tagged-word
  * exchange (W_hh in shared memory) for up to 8 sequences. */
 enum { PIMB200_LSTM_AUTO = 0, PIMB200_LSTM_STREAMED = 1, PIMB200_LSTM_PERSISTENT = 2,
        PIMB200_LSTM_PERSISTENT_TAGGED = 3 };
@@ -327,7 +328,7 @@ int pimb200_lstm_forward_packed(pimb200_lstm* h, const void* data, const int64_t
                                 const void* h0, const void* c0, void* y, void* hn, void* cn, void* stream);
 
 /* How many sequences of a packed batch this handle walks in lock step, in one launch per layer (0: none; larger batches run
- * timestep by timestep). */
+ * timestep by timestep, and so does one of more than 128 for whose padded rows the device has no memory). */
 int pimb200_lstm_packed_capacity(const pimb200_lstm* h);
 
 /* The last device-side status of a handle's asynchronous work: call after synchronising the
@@ -364,9 +365,9 @@ int pimb200_lstm_set_bulk_wide(pimb200_lstm* h, int on);
  * 0 = chosen by batch size, the default).  Same results.  No counterpart in the reference. */
 int pimb200_lstm_set_pipe_group_size(pimb200_lstm* h, int seqs);
 
-/* Packed input (pimb200_lstm_forward_packed) of up to 128 sequences and H % 16 == 0 runs as a padded lock-step batch on
+/* Packed input (pimb200_lstm_forward_packed) of up to pimb200_lstm_packed_capacity sequences runs as a padded lock-step batch on
  * the persistent recurrences (default, on = 1): the sequences are scattered into padded rows (the backward direction
- * reversed sequence by sequence), the gate terms behind a sequence's end freeze its cell state, outputs are gathered
+ * reversed sequence by sequence), the gate terms behind a sequence's end hold its cell state, outputs are gathered
  * back into packed rows.  on = 0 keeps the timestep-by-timestep streamed kernels (A/B and parity tests). */
 int pimb200_lstm_set_packed_lockstep(pimb200_lstm* h, int on);
 

@@ -2511,7 +2511,9 @@ constexpr long kBatchChunkRows = 131072;     // rows of gate terms per chunk (2 
 // sequences as for 256, and shorter for smaller matrices, of which more lies in tensor memory; the pipelined kernel's grows with
 // the groups of 16 that it walks.  100 steps with their projection, us, pipelined / batched: H = 256 at 64 sequences 345 / 328, 65:
 // 383 / 328; H = 512 at 64: 370 / 394, 65: 402 / 396, 128: 536 / 412; H = 768 at 96: 431 / 477, 112: 557 / 531; H = 1024 at 128:
-// 469 / 611.  Two directions share one launch of it (H = 1024, 33: 660 / 586; 24: 597 for both by the kernels above)
+// 469 / 611.  Two directions share one launch of it: 33 sequences, 50 and 8 steps, one direction after the other on the kernels above /
+// in one launch: H = 64 276, 66 / 151, 39; 256 293, 71 / 173, 44; 512 317, 84 / 203, 51; 768 346, 92 / 238, 55; 1024 350, 99 / 304, 67
+// (24 sequences of 1024 units, 100 steps, on the kernels above: 597, where 33 take 586 here)
 static int batch_min(int H, int dirs) { return dirs == 2 ? 33 : H <= 512 ? 65 : H <= 768 ? 112 : kPipeMaxB + 1; }
 constexpr long kBatchMaxPackedRows = 4 * kBatchChunkRows;
 struct PackedMeta {

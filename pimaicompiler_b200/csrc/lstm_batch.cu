@@ -20,6 +20,9 @@
 // lstm_persistent_pipe_kernel takes 3.9 for every 128 (31 at 1024); the cycles of a step at 256..1024 sequences: states 1.1 k,
 // products 3.3..6 k, commit 1.2 k, gates 2.6..5.4 k, counters 1.5..2.5 k.
 //
+// Sums of all K in one fp32 accumulator of tensor memory, where the kernels for fewer sequences add four quarters: the error of the
+// outputs against 64 bits is the same to three digits (1024 units, 150..1000 sequences: 2.10e-4..2.30e-4, the rounding of the states).
+//
 // Every wait of the loops is bounded; on giving up a CTA records the error, lets its copies land and frees its tensor memory.
 // What has no bound waits for no other CTA's progress: the allocation of tensor memory finds it free (a CTA has its SM's shared
 // memory for itself), and both CTAs of a pair reach the barriers at either end.
